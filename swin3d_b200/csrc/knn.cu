@@ -280,7 +280,8 @@ knn_kernel(int K, const float *__restrict__ src, const float *__restrict__ query
         for (int r = 0; r < NQ; ++r) same = same && jb[r] == jb_w && je[r] == je_w;
         same = __all_sync(0xffffffffu, same);
         int j = jb_w & ~3;
-        if (same) {
+        // (jb_w >= je_w: every query of the warp belongs to a scene that lies outside this tile)
+        if (same && jb_w < je_w) {
             if (j < jb_w) { step(j, std::true_type{}); j += KNN_STEP; }
             for (; j + KNN_STEP <= je_w; j += KNN_STEP) step(j, std::false_type{});
         }

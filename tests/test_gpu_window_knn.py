@@ -142,6 +142,19 @@ def test_knn_fewer_candidates_than_k_and_empty_scene():
     assert d2[1].tolist() == [2.0 ** 31] * 4 and idx[1].tolist() == [0] * 4
 
 
+def test_knn_block_over_several_scenes_with_ragged_source_offsets():
+    """One block holds the end of a scene's queries and whole warps of the next scenes', whose sources
+    start far outside the tile and not at a multiple of four."""
+    sizes = [(1692, 5367), (97, 1021), (3, 2), (700, 3333)]
+    qrys, srcs = zip(*[S.make_knn_scene(60 + i, q, s)[::-1] for i, (q, s) in enumerate(sizes)])
+    src, qry = np.concatenate(srcs), np.concatenate(qrys)
+    so, qo = np.cumsum([len(s) for s in srcs]), np.cumsum([len(q) for q in qrys])
+    for K in (3, 16):
+        idx, d2 = _knn_gpu(K, src, qry, so, qo)
+        ridx, rd2 = O.knn(K, src, qry, so, qo, fma_mode=2)
+        assert np.array_equal(idx, ridx) and np.array_equal(d2.view(np.uint32), rd2.view(np.uint32))
+
+
 def test_knn_function_returns_sqrt_distance():
     from swin3d_b200.sparse_dl.knn import KNN
     src, qry = S.make_knn_scene(9, 500, 400)
