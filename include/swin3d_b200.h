@@ -242,6 +242,19 @@ int s3d_knn(int K, const float *src, const float *query, const int32_t *src_offs
             const int32_t *query_offset, int B, int64_t Ns, int64_t Nq,
             int32_t *ret_idx, float *ret_dist, void *stream);
 
+/* The same search with scratch memory from the caller, which lets large problems build a spatial
+ * index first instead of scanning every source for every query.  The results are those of s3d_knn, bit
+ * for bit; root != 0 writes distances (correctly rounded square roots) instead of squared distances.
+ * s3d_knn_workspace_bytes: what `workspace` (16-byte aligned, device memory, contents irrelevant) has
+ * to hold; 0 when the call would not use it.  A null workspace is allowed and means s3d_knn's kernels.
+ */
+int s3d_debug_knn_path(int path);   /* tests: 0 by size, 1 / 2 thread / warp per query, 3 index; -> previous */
+int64_t s3d_knn_workspace_bytes(int K, int B, int64_t Ns, int64_t Nq);
+int s3d_knn_search(int K, const float *src, const float *query, const int32_t *src_offset,
+                   const int32_t *query_offset, int B, int64_t Ns, int64_t Nq, int root,
+                   int32_t *ret_idx, float *ret_dist, void *workspace, int64_t workspace_bytes,
+                   void *stream);
+
 /* ---------------------------------------------------------------------------------------------
  * Consumers of the KNN result (the callers either side of s3d_knn).
  *

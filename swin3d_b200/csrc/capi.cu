@@ -305,17 +305,61 @@ int s3d_window_build(const int32_t *coords, const float *feats, int64_t N, int F
                                counts_out, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
 }
 
-int s3d_knn(int K, const float *src, const float *query, const int32_t *src_offset,
-            const int32_t *query_offset, int B, int64_t Ns, int64_t Nq, int32_t *ret_idx,
-            float *ret_dist, void *stream)
+// Set through s3d_debug_knn_path(): 0 = by size, 1 = thread-per-query scan, 2 = warp-per-query scan,
+// 3 = spatial index where it exists (K <= 16).  The tests run every kernel at every size with it.
+static int g_knn_path = 0;
+
+int s3d_debug_knn_path(int path)
+{
+    const int was = g_knn_path;
+    g_knn_path = path;
+    return was;
+}
+
+static bool use_warp(int K, int B, int64_t Ns, int64_t Nq) { return g_knn_path ? g_knn_path == 2 : knn_warp_wanted(K, B, Ns, Nq); }
+static bool use_tree(int K, int B, int64_t Ns, int64_t Nq)
+{
+    return knn_tree_supported(K, B, Ns, Nq) && (g_knn_path ? g_knn_path == 3 : !knn_warp_wanted(K, B, Ns, Nq));
+}
+
+static int knn_impl(int K, const float *src, const float *query, const int32_t *src_offset,
+                    const int32_t *query_offset, int B, int64_t Ns, int64_t Nq, bool root, int32_t *ret_idx,
+                    float *ret_dist, void *workspace, int64_t workspace_bytes, void *stream)
 {
     if (K < 1 || K > S3D_KNN_MAX_K) return S3D_ERR_UNSUPPORTED;
     if (B < 1 || Ns < 0 || Nq < 0) return S3D_ERR_BAD_ARG;
     if (Nq == 0) return S3D_OK;
     if (!query || !src_offset || !query_offset || !ret_idx || !ret_dist || (Ns > 0 && !src))
         return S3D_ERR_BAD_ARG;
-    return knn_launch(K, src, query, src_offset, query_offset, B, Nq, ret_idx, ret_dist,
-                      static_cast<cudaStream_t>(stream));
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (use_warp(K, B, Ns, Nq))
+        return knn_launch_warp(K, src, query, src_offset, query_offset, B, Nq, root, ret_idx, ret_dist, st);
+    if (workspace && use_tree(K, B, Ns, Nq)) {
+        if (workspace_bytes < knn_tree_bytes(B, Ns, Nq)) return S3D_ERR_WORKSPACE;
+        return knn_launch_tree(K, src, query, src_offset, query_offset, B, Ns, Nq, root, ret_idx, ret_dist, workspace, st);
+    }
+    return knn_launch(K, src, query, src_offset, query_offset, B, Nq, root, ret_idx, ret_dist, st);
+}
+
+int s3d_knn(int K, const float *src, const float *query, const int32_t *src_offset,
+            const int32_t *query_offset, int B, int64_t Ns, int64_t Nq, int32_t *ret_idx,
+            float *ret_dist, void *stream)
+{
+    return knn_impl(K, src, query, src_offset, query_offset, B, Ns, Nq, false, ret_idx, ret_dist, nullptr, 0, stream);
+}
+
+int64_t s3d_knn_workspace_bytes(int K, int B, int64_t Ns, int64_t Nq)
+{
+    if (K < 1 || B < 1 || Ns < 0 || Nq < 1 || !use_tree(K, B, Ns, Nq)) return 0;
+    return knn_tree_bytes(B, Ns, Nq);
+}
+
+int s3d_knn_search(int K, const float *src, const float *query, const int32_t *src_offset,
+                   const int32_t *query_offset, int B, int64_t Ns, int64_t Nq, int root, int32_t *ret_idx,
+                   float *ret_dist, void *workspace, int64_t workspace_bytes, void *stream)
+{
+    return knn_impl(K, src, query, src_offset, query_offset, B, Ns, Nq, root != 0, ret_idx, ret_dist, workspace,
+                    workspace_bytes, stream);
 }
 
 }  // extern "C"

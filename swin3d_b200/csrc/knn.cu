@@ -23,36 +23,13 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "knn_common.cuh"
 #include "knn_kernels.cuh"
 
 namespace s3d {
 
 constexpr int KNN_TILE = 768;          // source points per shared-memory tile (a multiple of KNN_STEP)
 constexpr int KNN_STEP = 8;            // candidates per step of the scan
-
-__device__ __forceinline__ void knn_sift_down(float *heap, int *idx, int start, int end)
-{
-    int curr = start;
-    int child = curr * 2 + 1;
-    while (child < end) {
-        if (child + 1 < end && heap[child] < heap[child + 1]) child++;
-        if (heap[curr] > heap[child]) return;
-        const float tf = heap[curr]; heap[curr] = heap[child]; heap[child] = tf;
-        const int ti = idx[curr]; idx[curr] = idx[child]; idx[child] = ti;
-        curr = child;
-        child = curr * 2 + 1;
-    }
-}
-
-// fp32 squared distance.  The reference writes dx*dx + dy*dy + dz*dz and lets nvcc contract it;
-// its compiled kernel (nvcc 12.9, default -fmad=true, sm_100) evaluates
-// fma(dz,dz, fma(dx,dx, dy*dy)), established by comparing bit patterns of its output with the
-// three possible contractions.  The expression is spelled with intrinsics so that it cannot
-// drift with compiler versions; the GPU parity test re-checks it against the compiled reference.
-__device__ __forceinline__ float knn_dist2(float dx, float dy, float dz)
-{
-    return __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
-}
 
 // Two candidates per instruction: element 0 in the low half of the 64-bit register.
 __device__ __forceinline__ uint64_t pack2(float lo, float hi)
@@ -107,11 +84,14 @@ __device__ __forceinline__ float knn_threshold(float top, float sq, float pmax2)
 // The heaps are thread-private arrays (local memory beyond a few entries; heaps in shared memory as
 // [entry][thread] were measured at the same speed for K = 16: the cost there is the number of heap
 // updates, K (1 + ln(N / K)) per query, each entered by a whole warp).
-template <int KMAX, int NQ, int NT, int QCAP>
+// LIST: the queries are those of a list in device memory (tied queries of the search over the spatial
+// index), walked by a fixed grid; nothing happens unless it holds more than list_min.
+template <int KMAX, int NQ, int NT, int QCAP, bool LIST>
 __global__ void __launch_bounds__(NT)
 knn_kernel(int K, const float *__restrict__ src, const float *__restrict__ query,
            const int32_t *__restrict__ src_offset, const int32_t *__restrict__ query_offset,
-           int B, int64_t Nq, int32_t *__restrict__ ret_idx, float *__restrict__ ret_dist)
+           int B, int64_t Nq, const int32_t *__restrict__ list, const int *__restrict__ list_count, int list_min,
+           bool root, int32_t *__restrict__ ret_idx, float *__restrict__ ret_dist)
 {
     // planes x, y, z, |p|^2 of a tile; a step may read past the last point
     __shared__ __align__(16) float s_p[4][KNN_TILE + KNN_STEP];
@@ -119,7 +99,10 @@ knn_kernel(int K, const float *__restrict__ src, const float *__restrict__ query
     __shared__ int s_lo, s_hi;
     __shared__ unsigned s_pmax;                    // bits of the largest |p|^2 loaded so far
 
-    const int64_t g0 = (int64_t)blockIdx.x * (NT * NQ) + threadIdx.x;
+    const int64_t total = LIST ? (int64_t)__ldg(list_count) : Nq;
+    if (LIST && total <= list_min) return;
+    for (int64_t blk = blockIdx.x; blk * (NT * NQ) < total; blk += gridDim.x) {
+    const int64_t g0 = blk * (NT * NQ) + threadIdx.x;
 
     float heap[NQ][KMAX];
     int hidx[NQ][KMAX];
@@ -127,6 +110,7 @@ knn_kernel(int K, const float *__restrict__ src, const float *__restrict__ query
     uint64_t a2[NQ], b2[NQ], c2[NQ];
     int s0[NQ], s1[NQ], qn[NQ];
     bool active[NQ];
+    int64_t gq[NQ];
 #pragma unroll
     for (int r = 0; r < NQ; ++r) {
 #pragma unroll
@@ -134,8 +118,10 @@ knn_kernel(int K, const float *__restrict__ src, const float *__restrict__ query
             heap[r][i] = 2147483648.0f;  // (float)0x7fffffff
             hidx[r][i] = 0;
         }
-        const int64_t g = g0 + (int64_t)r * NT;
-        active[r] = g < Nq;
+        const int64_t at = g0 + (int64_t)r * NT;
+        active[r] = at < total;
+        const int64_t g = LIST && active[r] ? (int64_t)__ldg(list + at) : at;
+        gq[r] = g;
         qx[r] = qy[r] = qz[r] = 0.f;
         s0[r] = s1[r] = 0;
         qn[r] = 0;
@@ -143,10 +129,7 @@ knn_kernel(int K, const float *__restrict__ src, const float *__restrict__ query
             qx[r] = __ldg(query + g * 3);
             qy[r] = __ldg(query + g * 3 + 1);
             qz[r] = __ldg(query + g * 3 + 2);
-            int b = 0;
-            for (; b < B; ++b)
-                if (g < __ldg(query_offset + b)) break;
-            if (b >= B) b = B - 1;
+            const int b = knn_scene(g, query_offset, B);
             s0[r] = b > 0 ? __ldg(src_offset + b - 1) : 0;
             s1[r] = __ldg(src_offset + b);
         }
@@ -155,6 +138,7 @@ knn_kernel(int K, const float *__restrict__ src, const float *__restrict__ query
         c2[r] = pack2(-2.f * qz[r], -2.f * qz[r]);
         sq[r] = __fmaf_rn(qz[r], qz[r], __fmaf_rn(qy[r], qy[r], __fmul_rn(qx[r], qx[r])));
     }
+    if (LIST) __syncthreads();                     // the previous round of the block is over
     if (threadIdx.x == 0) { s_lo = 0x7fffffff; s_hi = 0; s_pmax = 0u; }
     __syncthreads();
 #pragma unroll
@@ -291,31 +275,40 @@ knn_kernel(int K, const float *__restrict__ src, const float *__restrict__ query
 #pragma unroll
     for (int r = 0; r < NQ; ++r) {
         if (!active[r]) continue;
-        const int64_t g = g0 + (int64_t)r * NT;
-        for (int i = K - 1; i > 0; --i) {
-            const float tf = heap[r][0]; heap[r][0] = heap[r][i]; heap[r][i] = tf;
-            const int ti = hidx[r][0]; hidx[r][0] = hidx[r][i]; hidx[r][i] = ti;
-            knn_sift_down(heap[r], hidx[r], 0, i);
-        }
+        knn_heap_sort(heap[r], hidx[r], K);
         for (int i = 0; i < K; ++i) {
-            ret_dist[g * K + i] = heap[r][i];
-            ret_idx[g * K + i] = hidx[r][i];
+            ret_dist[gq[r] * K + i] = root ? __fsqrt_rn(heap[r][i]) : heap[r][i];
+            ret_idx[gq[r] * K + i] = hidx[r][i];
         }
+    }
     }
 }
 
 template <int KMAX, int NQ, int NT, int QCAP>
 static int knn_launch_as(int K, const float *src, const float *query, const int32_t *src_offset,
-                         const int32_t *query_offset, int B, int64_t Nq, int32_t *ret_idx, float *ret_dist,
+                         const int32_t *query_offset, int B, int64_t Nq, bool root, int32_t *ret_idx, float *ret_dist,
                          cudaStream_t st)
 {
     const unsigned blocks = (unsigned)((Nq + NT * NQ - 1) / (NT * NQ));
-    knn_kernel<KMAX, NQ, NT, QCAP><<<blocks, NT, 0, st>>>(K, src, query, src_offset, query_offset, B, Nq, ret_idx, ret_dist);
+    knn_kernel<KMAX, NQ, NT, QCAP, false><<<blocks, NT, 0, st>>>(K, src, query, src_offset, query_offset, B, Nq, nullptr, nullptr, 0, root, ret_idx, ret_dist);
+    return cudaGetLastError() == cudaSuccess ? S3D_OK : S3D_ERR_LAUNCH;
+}
+
+int knn_launch_list(int K, const float *src, const float *query, const int32_t *src_offset,
+                    const int32_t *query_offset, int B, int64_t Nq, const int32_t *list, const int *list_count,
+                    int list_min, bool root, int32_t *ret_idx, float *ret_dist, cudaStream_t st)
+{
+    if (K > 16) return S3D_ERR_UNSUPPORTED;
+    const unsigned blocks = (unsigned)((Nq + 127) / 128 < 148 * 8 ? (Nq + 127) / 128 : 148 * 8);
+    if (K <= 4)
+        knn_kernel<4, 1, 128, KNN_STEP + 4, true><<<blocks, 128, 0, st>>>(K, src, query, src_offset, query_offset, B, Nq, list, list_count, list_min, root, ret_idx, ret_dist);
+    else
+        knn_kernel<16, 1, 128, KNN_STEP + 4, true><<<blocks, 128, 0, st>>>(K, src, query, src_offset, query_offset, B, Nq, list, list_count, list_min, root, ret_idx, ret_dist);
     return cudaGetLastError() == cudaSuccess ? S3D_OK : S3D_ERR_LAUNCH;
 }
 
 int knn_launch(int K, const float *src, const float *query, const int32_t *src_offset,
-               const int32_t *query_offset, int B, int64_t Nq, int32_t *ret_idx, float *ret_dist,
+               const int32_t *query_offset, int B, int64_t Nq, bool root, int32_t *ret_idx, float *ret_dist,
                cudaStream_t st)
 {
     if (Nq == 0) return S3D_OK;
@@ -325,14 +318,14 @@ int knn_launch(int K, const float *src, const float *query, const int32_t *src_o
     // queries: smaller blocks of one query per thread keep more warps resident (measured on 200 k to
     // 1.6 M queries: the smaller blocks win below about 300 k queries for K <= 4, 600 k for K <= 16)
     if (K <= 4) {
-        if (Nq < 300000) return knn_launch_as<4, 1, 128, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, ret_idx, ret_dist, st);
-        return knn_launch_as<4, 2, 128, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, ret_idx, ret_dist, st);
+        if (Nq < 300000) return knn_launch_as<4, 1, 128, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, root, ret_idx, ret_dist, st);
+        return knn_launch_as<4, 2, 128, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, root, ret_idx, ret_dist, st);
     }
     if (K <= 16) {
-        if (Nq < 600000) return knn_launch_as<16, 1, 128, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, ret_idx, ret_dist, st);
-        return knn_launch_as<16, 1, 256, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, ret_idx, ret_dist, st);
+        if (Nq < 600000) return knn_launch_as<16, 1, 128, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, root, ret_idx, ret_dist, st);
+        return knn_launch_as<16, 1, 256, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, root, ret_idx, ret_dist, st);
     }
-    return knn_launch_as<64, 1, 256, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, ret_idx, ret_dist, st);
+    return knn_launch_as<64, 1, 256, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, root, ret_idx, ret_dist, st);
 }
 
 }  // namespace s3d

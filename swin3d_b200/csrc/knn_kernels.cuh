@@ -1,10 +1,30 @@
-// Host entry point of the KNN kernel.
+// Host entry points of the KNN kernels.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 namespace s3d {
+
+// thread-per-query scan; root: write distances instead of squared distances
 int knn_launch(int K, const float *src, const float *query, const int32_t *src_offset,
-               const int32_t *query_offset, int B, int64_t Nq, int32_t *ret_idx, float *ret_dist,
+               const int32_t *query_offset, int B, int64_t Nq, bool root, int32_t *ret_idx, float *ret_dist,
                cudaStream_t st);
-}
+// the same for the queries of a list in device memory; nothing happens unless it holds more than list_min
+int knn_launch_list(int K, const float *src, const float *query, const int32_t *src_offset,
+                    const int32_t *query_offset, int B, int64_t Nq, const int32_t *list, const int *list_count,
+                    int list_min, bool root, int32_t *ret_idx, float *ret_dist, cudaStream_t st);
+
+// warp-per-query scan
+bool knn_warp_wanted(int K, int B, int64_t Ns, int64_t Nq);
+int knn_launch_warp(int K, const float *src, const float *query, const int32_t *src_offset,
+                    const int32_t *query_offset, int B, int64_t Nq, bool root, int32_t *ret_idx, float *ret_dist,
+                    cudaStream_t st);
+
+// search over a spatial index
+bool knn_tree_supported(int K, int B, int64_t Ns, int64_t Nq);
+int64_t knn_tree_bytes(int B, int64_t Ns, int64_t Nq);
+int knn_launch_tree(int K, const float *src, const float *query, const int32_t *src_offset,
+                    const int32_t *query_offset, int B, int64_t Ns, int64_t Nq, bool root, int32_t *ret_idx,
+                    float *ret_dist, void *work, cudaStream_t st);
+
+}  // namespace s3d

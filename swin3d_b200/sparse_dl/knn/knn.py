@@ -9,8 +9,7 @@ from torch.autograd.function import Function
 from ... import _lib
 
 
-def knn_raw(K: int, src_xyz, query_xyz, src_offset, query_offset):
-    """-> (idx int32 [Nq,K], squared distance float32 [Nq,K])."""
+def _search(K: int, src_xyz, query_xyz, src_offset, query_offset, root: bool, out=None):
     for name, t in (("src_xyz", src_xyz), ("query_xyz", query_xyz)):
         if not t.is_cuda:
             raise RuntimeError(f"{name} must be a CUDA tensor")
@@ -19,23 +18,33 @@ def knn_raw(K: int, src_xyz, query_xyz, src_offset, query_offset):
     assert src_xyz.is_contiguous() and query_xyz.is_contiguous()
     if src_offset.shape != query_offset.shape:
         raise ValueError("src_offset and query_offset must have one entry per scene")
+    K = int(K)
     so = src_offset.to(torch.int32).contiguous()
     qo = query_offset.to(torch.int32).contiguous()
-    Nq, Ns = query_xyz.shape[0], src_xyz.shape[0]
-    idx = torch.empty((Nq, K), dtype=torch.int32, device=query_xyz.device)
-    d2 = torch.empty((Nq, K), dtype=torch.float32, device=query_xyz.device)
-    with torch.cuda.device(query_xyz.device):
+    dev = query_xyz.device
+    B, Nq, Ns = so.shape[0], query_xyz.shape[0], src_xyz.shape[0]
+    if out is None:
+        out = (torch.empty((Nq, K), dtype=torch.int32, device=dev), torch.empty((Nq, K), dtype=torch.float32, device=dev))
+    idx, dist = out
+    nbytes = _lib.lib.s3d_knn_workspace_bytes(K, B, Ns, Nq)
+    work = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
+    with torch.cuda.device(dev):
         st = torch.cuda.current_stream().cuda_stream
-        rc = _lib.lib.s3d_knn(int(K), src_xyz.data_ptr(), query_xyz.data_ptr(), so.data_ptr(),
-                              qo.data_ptr(), so.shape[0], Ns, Nq, idx.data_ptr(), d2.data_ptr(), st)
+        rc = _lib.lib.s3d_knn_search(K, src_xyz.data_ptr(), query_xyz.data_ptr(), so.data_ptr(), qo.data_ptr(), B, Ns, Nq,
+                                     int(root), idx.data_ptr(), dist.data_ptr(), None if work is None else work.data_ptr(),
+                                     nbytes, st)
     _lib.check(rc, "s3d_knn")
-    return idx, d2
+    return idx, dist
+
+
+def knn_raw(K: int, src_xyz, query_xyz, src_offset, query_offset):
+    """-> (idx int32 [Nq,K], squared distance float32 [Nq,K])."""
+    return _search(K, src_xyz, query_xyz, src_offset, query_offset, False)
 
 
 class KNN(Function):
     @staticmethod
     def forward(ctx, K, src_xyz, query_xyz, src_offset, query_offset):
-        idx, d2 = knn_raw(K, src_xyz, query_xyz, src_offset, query_offset)
-        dist = torch.sqrt(d2)
+        idx, dist = _search(K, src_xyz, query_xyz, src_offset, query_offset, True)
         ctx.mark_non_differentiable(idx, dist)
         return idx, dist

@@ -10,7 +10,7 @@ and index 0 (the reference leaves the index uninitialised).
 """
 import torch
 
-from .. import _lib
+from .knn.knn import _search
 
 
 def knn_cuda(K, src_xyz, query_xyz, src_offset, query_offset, ret_idx, ret_dist) -> None:
@@ -26,10 +26,4 @@ def knn_cuda(K, src_xyz, query_xyz, src_offset, query_offset, ret_idx, ret_dist)
         raise ValueError("ret_dist must be a contiguous float32 [Nq, K] tensor")
     if src_offset.shape != query_offset.shape:
         raise ValueError("src_offset and query_offset must have one entry per scene")
-    so = src_offset.to(torch.int32).contiguous()
-    qo = query_offset.to(torch.int32).contiguous()
-    with torch.cuda.device(query_xyz.device):
-        st = torch.cuda.current_stream().cuda_stream
-        rc = _lib.lib.s3d_knn(int(K), src_xyz.data_ptr(), query_xyz.data_ptr(), so.data_ptr(), qo.data_ptr(),
-                              so.shape[0], Ns, Nq, ret_idx.data_ptr(), ret_dist.data_ptr(), st)
-    _lib.check(rc, "s3d_knn")
+    _search(K, src_xyz, query_xyz, src_offset, query_offset, False, (ret_idx, ret_dist))

@@ -155,6 +155,75 @@ def test_knn_block_over_several_scenes_with_ragged_source_offsets():
         assert np.array_equal(idx, ridx) and np.array_equal(d2.view(np.uint32), rd2.view(np.uint32))
 
 
+@pytest.mark.parametrize("path", [1, 2, 3], ids=["scan", "warp", "index"])
+@pytest.mark.parametrize("case", ["ragged", "one_scene", "lattice", "offset_1e5", "scale_1e-22", "scale_3e19", "nonfinite",
+                                  "duplicates", "few", "far_outlier"])
+def test_knn_kernels_agree_with_the_heap_at_every_size(path, case):
+    """Each of the three kernels (by size, a call takes one of them) on inputs where it can go wrong:
+    leaves and warps that straddle scenes, scenes smaller than K or empty, partial leaves, more than
+    one node, distance ties everywhere, magnitudes at the ends of the fp32 range."""
+    from swin3d_b200 import _lib
+    rng = np.random.default_rng(7)
+    if case == "ragged":
+        parts = [S.make_knn_scene(70 + i, q, s) for i, (q, s) in enumerate([(45, 33), (1, 1), (700, 2053), (31, 1024), (3, 17)])]
+        src, qry = np.concatenate([p[0] for p in parts]), np.concatenate([p[1] for p in parts])
+        so, qo = np.cumsum([len(p[0]) for p in parts]), np.cumsum([len(p[1]) for p in parts])
+        so, qo = np.insert(so, 2, so[1]), np.insert(qo, 2, qo[1] + 0)      # a scene without sources or queries
+    elif case == "one_scene":
+        src, qry = S.make_knn_scene(80, 1001, 40_001)
+        so, qo = [len(src)], [len(qry)]
+    elif case == "lattice":
+        g = np.stack(np.meshgrid(*[np.arange(14)] * 3, indexing="ij"), -1).reshape(-1, 3).astype(np.float32)
+        src, qry = g[rng.permutation(len(g))], g[::5] + np.float32(0.5)
+        so, qo = [1000, len(src)], [200, len(qry)]
+    elif case == "few":
+        src, qry = rng.random((5, 3), dtype=np.float32), rng.random((70, 3), dtype=np.float32)
+        so, qo = [2, 2, 5], [30, 50, 70]
+    else:
+        src, qry, so, qo = _two_scenes(50)
+        src, qry = src.copy(), qry.copy()
+        if case.startswith("offset"):
+            src, qry = src + np.float32(1e5), qry + np.float32(1e5)
+        elif case.startswith("scale"):
+            sc = np.float32(case.split("_")[1])
+            src, qry = src * sc, qry * sc
+        elif case == "nonfinite":
+            bad = rng.choice(len(src), 60, replace=False)
+            src[bad[:20], rng.integers(0, 3, 20)] = np.nan
+            src[bad[20:40], rng.integers(0, 3, 20)] = np.inf
+            src[bad[40:], rng.integers(0, 3, 20)] = -np.inf
+            qry[5, 1], qry[6, 0], qry[7, 2] = np.nan, np.inf, -np.inf
+        elif case == "duplicates":
+            src[:400], src[400:600] = qry[:400], qry[:200]
+        elif case == "far_outlier":
+            src[3], qry[9] = 1e9, -1e9
+    was = _lib.lib.s3d_debug_knn_path(path)
+    try:
+        for K in (1, 3, 5, 16):
+            idx, d2 = _knn_gpu(K, src, qry, so, qo)
+            with np.errstate(all="ignore"):
+                ridx, rd2 = O.knn(K, src, qry, so, qo, fma_mode=2)
+            assert np.array_equal(d2.view(np.uint32), rd2.view(np.uint32)), K
+            assert np.array_equal(idx, ridx), K
+    finally:
+        _lib.lib.s3d_debug_knn_path(was)
+
+
+def test_knn_index_hands_many_ties_to_the_scan():
+    """More tied queries than the warp-per-query pass takes (16384): a lattice, where every query ties."""
+    from swin3d_b200 import _lib
+    g = np.stack(np.meshgrid(*[np.arange(30)] * 3, indexing="ij"), -1).reshape(-1, 3).astype(np.float32)
+    src, qry = g[::13], g + np.float32(0.5)
+    was = _lib.lib.s3d_debug_knn_path(3)
+    try:
+        for K in (3, 16):
+            idx, d2 = _knn_gpu(K, src, qry, [len(src)], [len(qry)])
+            ridx, rd2 = O.knn(K, src, qry, [len(src)], [len(qry)], fma_mode=2)
+            assert np.array_equal(idx, ridx) and np.array_equal(d2, rd2)
+    finally:
+        _lib.lib.s3d_debug_knn_path(was)
+
+
 def test_knn_function_returns_sqrt_distance():
     from swin3d_b200.sparse_dl.knn import KNN
     src, qry = S.make_knn_scene(9, 500, 400)
