@@ -37,7 +37,8 @@ struct TreeBufs {
     uint32_t *hist;          // [2][B * cells]: sources, queries; after the scan the start of every cell
     uint32_t *tile;          // sums of SCAN_TILE cells
     uint32_t *rank;          // [Ns + Nq] position of a point inside its cell
-    float4 *pts;             // [Ns + Nq] x, y, z, row number: sources in cell order, then queries
+    float *src;              // [leaves][4][32] x, y, z, row number of the sources in cell order, a leaf at a time
+    float4 *qry;             // [Nq] x, y, z, row number of the queries in cell order
     float4 *leaf;            // [leaves][2] lowest and highest corner
     float4 *node;            // [nodes][2]
     int32_t *ties;           // [Nq] queries to scan again
@@ -73,7 +74,8 @@ TreeBufs tree_bufs(char *base, int B, int64_t Ns, int64_t Nq)
     t.zero_bytes = off;
     t.tile = (uint32_t *)take((int64_t)t.n_tiles * 4);
     t.rank = (uint32_t *)take((Ns + Nq) * 4);
-    t.pts = (float4 *)take((Ns + Nq) * 16);
+    t.src = (float *)take((Ns / LEAF + B + 1) * LEAF * 16);
+    t.qry = (float4 *)take(Nq * 16);
     t.leaf = (float4 *)take((Ns / LEAF + B + 1) * 32);
     t.node = (float4 *)take((Ns / (LEAF * 32) + B + 1) * 32);
     t.ties = (int32_t *)take(Nq * 4);
@@ -148,6 +150,11 @@ __device__ __forceinline__ uint32_t cell_of(float x, float y, float z, const uin
     return spread3(axis((x - lx) * inv)) | (spread3(axis((y - ly) * inv)) << 1) | (spread3(axis((z - lz) * inv)) << 2);
 }
 
+// Leaves and nodes of scene b, whose sources start at s0, start at these places of their arrays, which
+// leaves room for the partial last one of every scene.
+__device__ __forceinline__ int64_t first_leaf(int64_t s0, int b) { return s0 / LEAF + b; }
+__device__ __forceinline__ int64_t first_node(int64_t s0, int b) { return s0 / (LEAF * 32) + b; }
+
 // One point per thread, sources then queries.  COUNT: rank inside the cell; otherwise: into cell order.
 template <bool COUNT>
 __global__ void __launch_bounds__(KT_THREADS)
@@ -170,8 +177,18 @@ tree_sort_kernel(const float *__restrict__ src, const float *__restrict__ query,
     const float x = __ldg(p), y = __ldg(p + 1), z = __ldg(p + 2);
     const int64_t cells = (int64_t)B << (3 * t.bits);
     uint32_t *h = t.hist + (is_q ? cells : 0) + ((int64_t)b << (3 * t.bits)) + cell_of(x, y, z, t.bbox, b, t.bits);
-    if (COUNT) t.rank[i] = atomicAdd(h, 1u);
-    else t.pts[*h + t.rank[i]] = make_float4(x, y, z, __int_as_float((int)g));
+    if (COUNT) {
+        t.rank[i] = atomicAdd(h, 1u);
+        return;
+    }
+    const uint32_t at = *h + t.rank[i];
+    if (is_q) {
+        t.qry[at - t.hist[cells]] = make_float4(x, y, z, __int_as_float((int)g));   // the first query cell follows the last source
+    } else {
+        const uint32_t s0 = t.hist[(int64_t)b << (3 * t.bits)];
+        float *o = t.src + (first_leaf(s0, b) + (at - s0) / LEAF) * (4 * LEAF) + (at - s0) % LEAF;
+        o[0] = x; o[LEAF] = y; o[2 * LEAF] = z; o[3 * LEAF] = __int_as_float((int)g);
+    }
 }
 
 // Exclusive scan of the histograms in two launches: tile sums, then every block adds up the sums of the
@@ -235,9 +252,8 @@ tree_scan_kernel(uint32_t *__restrict__ hist, const uint32_t *__restrict__ tile)
     }
 }
 
-// Boxes: a warp makes a leaf, a block (32 warps) a node.  grid = nodes of all scenes, in scene order;
-// leaves and nodes of scene b, whose sources start at s0, start at s0 / 32 + b and s0 / 1024 + b of
-// their arrays, which leaves room for the partial last one of every scene.
+// Boxes: a warp makes a leaf, a block (32 warps) a node.  grid = nodes of all scenes, in scene order.
+// The places of a partial leaf that hold no source get NaN coordinates, which no comparison lets in.
 __global__ void __launch_bounds__(1024)
 tree_boxes_kernel(int B, TreeBufs t)
 {
@@ -256,10 +272,15 @@ tree_boxes_kernel(int B, TreeBufs t)
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int leaf = j * 32 + wid, at = leaf * LEAF + lane;
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    float *p = t.src + (first_leaf(s0, b) + leaf) * (4 * LEAF) + lane;
     if (at < n) {
-        const float4 p = t.pts[s0 + at];
-        lo[0] = fminf(lo[0], p.x); lo[1] = fminf(lo[1], p.y); lo[2] = fminf(lo[2], p.z);    // a NaN never counts
-        hi[0] = fmaxf(hi[0], p.x); hi[1] = fmaxf(hi[1], p.y); hi[2] = fmaxf(hi[2], p.z);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {                        // a NaN never counts
+            lo[d] = fminf(lo[d], p[d * LEAF]);
+            hi[d] = fmaxf(hi[d], p[d * LEAF]);
+        }
+    } else if (leaf * LEAF < n) {
+        p[0] = p[LEAF] = p[2 * LEAF] = NAN;
     }
     auto reduce = [&]() {
 #pragma unroll
@@ -273,7 +294,7 @@ tree_boxes_kernel(int B, TreeBufs t)
     reduce();
     if (lane == 0) {
         if (leaf * LEAF < n) {
-            float4 *o = t.leaf + 2 * ((int64_t)(s0 / LEAF) + b + leaf);
+            float4 *o = t.leaf + 2 * (first_leaf(s0, b) + leaf);
             o[0] = make_float4(lo[0], lo[1], lo[2], 0.f);
             o[1] = make_float4(hi[0], hi[1], hi[2], 0.f);
         }
@@ -286,7 +307,7 @@ tree_boxes_kernel(int B, TreeBufs t)
         for (int d = 0; d < 3; ++d) { lo[d] = s_lo[d][lane]; hi[d] = s_hi[d][lane]; }
         reduce();
         if (lane == 0) {
-            float4 *o = t.node + 2 * ((int64_t)(s0 / (LEAF * 32)) + b + j);
+            float4 *o = t.node + 2 * (first_node(s0, b) + j);
             o[0] = make_float4(lo[0], lo[1], lo[2], 0.f);
             o[1] = make_float4(hi[0], hi[1], hi[2], 0.f);
         }
@@ -302,6 +323,27 @@ __device__ __forceinline__ float box_gap(float lo, float hi, float ql, float qh)
 __device__ __forceinline__ float box_dist(const float4 &lo, const float4 &hi, const float (&ql)[3], const float (&qh)[3])
 {
     return knn_dist2(box_gap(lo.x, hi.x, ql[0], qh[0]), box_gap(lo.y, hi.y, ql[1], qh[1]), box_gap(lo.z, hi.z, ql[2], qh[2]));
+}
+
+// Two candidates per instruction (element 0 in the low half).  The packed operations round each half as
+// the scalar ones do, so the distances are those of knn_dist2 bit for bit.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void dist2x2(float &d0, float &d1, uint64_t px, uint64_t py, uint64_t pz, uint64_t nx, uint64_t ny, uint64_t nz)
+{
+    asm("{\n\t.reg .b64 x, y, z;\n\t"
+        "add.rn.f32x2 x, %2, %5;\n\t"
+        "add.rn.f32x2 y, %3, %6;\n\t"
+        "add.rn.f32x2 z, %4, %7;\n\t"
+        "mul.rn.f32x2 y, y, y;\n\t"
+        "fma.rn.f32x2 y, x, x, y;\n\t"
+        "fma.rn.f32x2 y, z, z, y;\n\t"
+        "mov.b64 {%0, %1}, y;\n\t}"
+        : "=f"(d0), "=f"(d1) : "l"(px), "l"(py), "l"(pz), "l"(nx), "l"(ny), "l"(nz));
 }
 
 // The KL smallest distances of a query, ascending, in registers; the first KL - K entries are -1 when
@@ -333,6 +375,32 @@ struct TopK {
         }
         if (x < d[0]) { d[0] = x; i[0] = id; }
     }
+    // the eight candidates (x, id), unsorted, INFINITY where there is none: sort them, keep the KL smallest of
+    // both lists (a bitonic sequence), sort that
+    __device__ __forceinline__ void merge8(float (&x)[8], int (&id)[8])
+    {
+        static_assert(KL == 8 || KL == 16, "a power of two");
+        auto order = [](float &a, float &b, int &ia, int &ib) {
+            const bool swap = b < a;
+            const float lo = fminf(a, b), hi = fmaxf(a, b);
+            const int il = swap ? ib : ia, ih = swap ? ia : ib;
+            a = lo; b = hi; ia = il; ib = ih;
+        };
+        constexpr int net[19][2] = {{0, 1}, {2, 3}, {4, 5}, {6, 7}, {0, 2}, {1, 3}, {4, 6}, {5, 7}, {1, 2}, {5, 6},
+                                    {0, 4}, {1, 5}, {2, 6}, {3, 7}, {2, 4}, {3, 5}, {1, 2}, {3, 4}, {5, 6}};
+#pragma unroll
+        for (int k = 0; k < 19; ++k) order(x[net[k][0]], x[net[k][1]], id[net[k][0]], id[net[k][1]]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            order(d[KL - 1 - j], x[j], i[KL - 1 - j], id[j]);
+            ex = fminf(ex, x[j]);
+        }
+#pragma unroll
+        for (int h = KL / 2; h > 0; h /= 2)
+#pragma unroll
+            for (int j = 0; j < KL; ++j)
+                if (!(j & h)) order(d[j], d[j + h], i[j], i[j + h]);
+    }
     __device__ __forceinline__ bool tied() const
     {
         bool tie = ex == d[KL - 1] && ex < KNN_FAR;
@@ -342,21 +410,29 @@ struct TopK {
     }
 };
 
+// Longer lists do not take their candidates one by one (an insertion costs five instructions per entry,
+// for one lane of the warp as for all): a lane parks what beats its K-th distance in shared memory,
+// and when a lane has eight or more parked, all lanes merge eight each.
+constexpr int QUEUE = 16;
+
 template <int KL, bool ROOT>
 __global__ void __launch_bounds__(SEARCH_THREADS)
 tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, TreeBufs t,
                    int32_t *__restrict__ ret_idx, float *__restrict__ ret_dist)
 {
+    constexpr bool PARK = KL >= 8;
+    __shared__ float s_qd[PARK ? QUEUE : 1][PARK ? SEARCH_THREADS : 1];
+    __shared__ int s_qi[PARK ? QUEUE : 1][PARK ? SEARCH_THREADS : 1];
     const int64_t at = (int64_t)blockIdx.x * SEARCH_THREADS + threadIdx.x;
     const int lane = threadIdx.x & 31;
     if ((at & ~(int64_t)31) >= Nq) return;                   // the whole warp
-    const uint32_t n_src = __ldg(t.hist + ((int64_t)B << (3 * t.bits)));     // the first query cell follows the last source
     float4 q = make_float4(NAN, NAN, NAN, __int_as_float(-1));
-    if (at < Nq) q = t.pts[n_src + at];
+    if (at < Nq) q = t.qry[at];
     const int g = __float_as_int(q.w);
     const int scene = g >= 0 ? knn_scene(g, qo, B) : -1;
     TopK<KL> best;
     best.init(K);
+    int parked = 0;
     // a query that is not finite has no distance below the heap's initial entry
     unsigned todo = __ballot_sync(0xffffffffu, scene >= 0 && finite3(q.x, q.y, q.z));
     while (todo) {
@@ -369,6 +445,7 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
         if (n <= 0) continue;
         // queries of other scenes take part as NaN: no comparison holds for them
         const float qx = mine ? q.x : NAN, qy = mine ? q.y : NAN, qz = mine ? q.z : NAN;
+        const uint64_t nx = pack2(-qx, -qx), ny = pack2(-qy, -qy), nz = pack2(-qz, -qz);
         float ql[3], qh[3];
         {
             const float c[3] = {q.x, q.y, q.z};
@@ -379,27 +456,72 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
                 qh[d] = from_order_key(__reduce_max_sync(0xffffffffu, mine ? k : 0u));
             }
         }
-        const float4 *pts = t.pts + s0;
-        const float4 *leaves = t.leaf + 2 * ((int64_t)(s0 / LEAF) + b), *nodes = t.node + 2 * ((int64_t)(s0 / (LEAF * 32)) + b);
+        const float *points = t.src + first_leaf(s0, b) * (4 * LEAF);
+        const float4 *leaves = t.leaf + 2 * first_leaf(s0, b), *nodes = t.node + 2 * first_node(s0, b);
         const int n_leaf = (n + LEAF - 1) / LEAF, n_node = (n_leaf + 31) / 32;
 
-        auto offer = [&](const float4 &p) {
-            const float d = knn_dist2(p.x - qx, p.y - qy, p.z - qz);
-            const bool in = d < best.top();
-            if (__any_sync(0xffffffffu, in)) {
-                if (in) best.insert(d, __float_as_int(p.w));
-                else best.ex = fminf(best.ex, d);
-            } else {
-                best.ex = fminf(best.ex, d);
+        auto drain = [&]() {
+            if constexpr (PARK) {
+                while (__any_sync(0xffffffffu, parked > 0)) {
+                    float x[8];
+                    int id[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const bool in = parked > j;
+                        const int from = in ? parked - 1 - j : 0;
+                        x[j] = in ? s_qd[from][threadIdx.x] : INFINITY;
+                        id[j] = s_qi[from][threadIdx.x];
+                    }
+                    parked = max(parked - 8, 0);
+                    best.merge8(x, id);
+                }
             }
         };
         auto visit = [&](int leaf) {
-            const float4 *p = pts + leaf * LEAF;
-            if ((leaf + 1) * LEAF <= n) {
-#pragma unroll 4
-                for (int j = 0; j < LEAF; ++j) offer(__ldg(p + j));
-            } else {
-                for (int j = 0; j < n - leaf * LEAF; ++j) offer(__ldg(p + j));
+            const float *p = points + leaf * (4 * LEAF);
+#pragma unroll 2
+            for (int j = 0; j < LEAF; j += 8) {
+                float d[8];
+#pragma unroll
+                for (int u = 0; u < 8; u += 4) {
+                    const ulonglong2 x = __ldg(reinterpret_cast<const ulonglong2 *>(p + j + u));
+                    const ulonglong2 y = __ldg(reinterpret_cast<const ulonglong2 *>(p + LEAF + j + u));
+                    const ulonglong2 z = __ldg(reinterpret_cast<const ulonglong2 *>(p + 2 * LEAF + j + u));
+                    dist2x2(d[u], d[u + 1], x.x, y.x, z.x, nx, ny, nz);
+                    dist2x2(d[u + 2], d[u + 3], x.y, y.y, z.y, nx, ny, nz);
+                }
+                const float m = fminf(fminf(fminf(d[0], d[1]), fminf(d[2], d[3])), fminf(fminf(d[4], d[5]), fminf(d[6], d[7])));
+                if (!__any_sync(0xffffffffu, m < best.top())) {
+                    best.ex = fminf(best.ex, m);
+                    continue;
+                }
+                int id[8];
+#pragma unroll
+                for (int u = 0; u < 8; u += 4) {
+                    const int4 v = __ldg(reinterpret_cast<const int4 *>(p + 3 * LEAF + j + u));
+                    id[u] = v.x; id[u + 1] = v.y; id[u + 2] = v.z; id[u + 3] = v.w;
+                }
+                if constexpr (PARK) {
+                    const float top = best.top();
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        if (d[u] < top) {
+                            s_qd[parked][threadIdx.x] = d[u];
+                            s_qi[parked][threadIdx.x] = id[u];
+                            ++parked;
+                        } else {
+                            best.ex = fminf(best.ex, d[u]);
+                        }
+                    }
+                    if (__any_sync(0xffffffffu, parked > QUEUE - 8)) drain();
+                } else {
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const bool in = d[u] < best.top();
+                        if (!in) best.ex = fminf(best.ex, d[u]);
+                        if (__any_sync(0xffffffffu, in) && in) best.insert(d[u], id[u]);
+                    }
+                }
             }
         };
         // begin with the leaf at the place of the warp's middle query, so that later boxes meet a bound
@@ -410,11 +532,11 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
             const uint32_t start = __ldg(t.hist + ((int64_t)b << (3 * t.bits)) + cell_of(mx, my, mz, t.bbox, b, t.bits));
             first = min((int)start - s0, n - 1) / LEAF;
             visit(first);
+            drain();
         }
-        auto top_max = [&]() { return __uint_as_float(__reduce_max_sync(0xffffffffu, mine ? __float_as_uint(best.top()) : 0u)); };
         // the nearest of the boxes held by the lanes that can still matter; -1 if there is none
         auto nearest = [&](float lb, bool &open) {
-            const float most = top_max();                    // by all lanes, open or not
+            const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, mine ? __float_as_uint(best.top()) : 0u));
             const bool can = open && lb <= most;
             const uint32_t key = can ? __float_as_uint(lb) : 0xffffffffu;
             const uint32_t m = __reduce_min_sync(0xffffffffu, key);
@@ -450,6 +572,7 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
                 }
             }
         }
+        drain();
     }
     if (g < 0) return;
     if (best.tied()) {
@@ -475,123 +598,299 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
     }
 }
 
-// ---- a warp per query, straight over the scene's sources ------------------------------------------------
-// For K <= 32 the warp keeps the sorted list one entry per lane; a distance tie (as above) or a larger
-// K makes it scan again with the literal heap (lane 0, in shared memory).  Serves the small problems,
-// where building the index costs more than it saves, and the tied queries of the search above
-// (LIST: the queries come from a list and are known to tie).
-constexpr int WARP_THREADS = 128;
-constexpr int WARP_BATCH = 4;
-
-template <bool LIST, bool ROOT>
-__global__ void __launch_bounds__(WARP_THREADS)
-knn_warp_kernel(int K, const float *__restrict__ src, const float *__restrict__ query, const int32_t *__restrict__ so,
-                const int32_t *__restrict__ qo, int B, int64_t Nq, const int32_t *__restrict__ list,
-                const int *__restrict__ list_count, int list_max, int32_t *__restrict__ ret_idx, float *__restrict__ ret_dist)
-{
-    __shared__ float s_heap[WARP_THREADS / 32][S3D_KNN_MAX_K];
-    __shared__ int s_hidx[WARP_THREADS / 32][S3D_KNN_MAX_K];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int64_t total = Nq;
-    if (LIST) {
-        total = __ldg(list_count);
-        if (total > list_max) return;                        // too many: the thread-per-query scan takes them
+// ---- the literal heap, one entry per lane (K <= 32) ---------------------------------------------------------
+// Entry i of the reference's heap lives in lane i.  The path a new root sinks along -- always to the larger
+// child, the left one when they are equal -- depends on the heap alone, so every lane knows from one ballot
+// (bit j: "entry j's right child is strictly larger") whether it is on it.  The new value sinks past every
+// entry of the path that is not smaller than it; those move up one step.
+struct LaneHeap {
+    float h;
+    int id;
+    unsigned anc, way;       // entries above this one, and on which of them the path turns right to get here
+    bool kid, kid2;
+    __device__ __forceinline__ void init(int K, int lane)
+    {
+        h = KNN_FAR;
+        id = 0;
+        anc = way = 0;
+        for (int i = lane; i > 0; i = (i - 1) / 2) {
+            anc |= 1u << ((i - 1) / 2);
+            if (!(i & 1)) way |= 1u << ((i - 1) / 2);
+        }
+        kid = 2 * lane + 1 < K;
+        kid2 = 2 * lane + 2 < K;
+        if (lane >= K) anc = 1u, way = 0xffffffffu;          // never on the path
     }
-    for (int64_t w = (int64_t)blockIdx.x * (WARP_THREADS / 32) + wid; w < total; w += (int64_t)gridDim.x * (WARP_THREADS / 32)) {
-        const int64_t g = LIST ? list[w] : w;
+    __device__ __forceinline__ float root() const { return __shfl_sync(0xffffffffu, h, 0); }
+    // d < root()
+    __device__ __forceinline__ void replace(float d, int row, int lane)
+    {
+        const float v1 = __shfl_sync(0xffffffffu, h, (2 * lane + 1) & 31), v2 = __shfl_sync(0xffffffffu, h, (2 * lane + 2) & 31);
+        const int i1 = __shfl_sync(0xffffffffu, id, (2 * lane + 1) & 31), i2 = __shfl_sync(0xffffffffu, id, (2 * lane + 2) & 31);
+        const bool right = kid2 && v1 < v2;
+        const float v = right ? v2 : v1;
+        const unsigned turns = __ballot_sync(0xffffffffu, right);
+        const bool left_empty = lane == 0 || ((turns & anc) == way && !(d > h));   // this entry moved up
+        if (left_empty) {
+            const bool up = kid && !(d > v);
+            h = up ? v : d;
+            id = up ? (right ? i2 : i1) : row;
+        }
+    }
+};
+
+// Result of a literal heap: the reference's heap sort, by lane 0 in shared memory.
+template <bool ROOT>
+__device__ __forceinline__ void finish_heap(float *heap, int *hidx, int K, int64_t g, int lane, int32_t *__restrict__ ret_idx,
+                                            float *__restrict__ ret_dist)
+{
+    __syncwarp();
+    if (lane == 0) knn_heap_sort(heap, hidx, K);
+    __syncwarp();
+    for (int j = lane; j < K; j += 32) {
+        ret_idx[g * K + j] = hidx[j];
+        ret_dist[g * K + j] = ROOT ? __fsqrt_rn(heap[j]) : heap[j];
+    }
+    __syncwarp();
+}
+
+// ---- tied queries of the search: a block per query ----------------------------------------------------------
+// The heap is a serial chain over the candidates that enter it, several thousand when the sources are in
+// spatial order.  Warp 0 runs it; the other warps scan the sources ahead of it, 8 per lane and round, and
+// hand over, in index order, those below the heap root of two rounds ago -- all that can still enter.
+// A list of more than list_max queries is left to the thread-per-query scan.
+constexpr int TIE_THREADS = 512, TIE_WARPS = TIE_THREADS / 32 - 1, TIE_PER = 8;
+
+template <bool ROOT>
+__global__ void __launch_bounds__(TIE_THREADS)
+knn_tie_kernel(int K, const float *__restrict__ src, const float *__restrict__ query, const int32_t *__restrict__ so,
+               const int32_t *__restrict__ qo, int B, const int32_t *__restrict__ list, const int *__restrict__ list_count,
+               int list_max, int32_t *__restrict__ ret_idx, float *__restrict__ ret_dist)
+{
+    __shared__ float s_d[2][TIE_WARPS][32 * TIE_PER];
+    __shared__ uint16_t s_o[2][TIE_WARPS][32 * TIE_PER];     // offset from the first source of the warp's share
+    __shared__ int s_n[2][TIE_WARPS];
+    __shared__ float s_root[2];
+    __shared__ float s_heap[32];
+    __shared__ int s_hidx[32];
+    const int total = __ldg(list_count);
+    if (total > list_max) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    constexpr int ROUND = TIE_WARPS * 32 * TIE_PER;
+    for (int w = blockIdx.x; w < total; w += gridDim.x) {
+        const int64_t g = list[w];
         const int b = knn_scene(g, qo, B);
         const int s0 = b > 0 ? __ldg(so + b - 1) : 0, s1 = __ldg(so + b);
-        const float qx = __ldg(query + g * 3), qy = __ldg(query + g * 3 + 1), qz = __ldg(query + g * 3 + 2);
-        // one pass over the sources in index order: 32 per step, every candidate that beats top() is handed to
-        // take(distance, row) in order
-        auto scan = [&](auto top, auto take, auto reject) {
-            for (int base = s0; base < s1; base += 32 * WARP_BATCH) {
-                float d[WARP_BATCH];
-#pragma unroll
-                for (int u = 0; u < WARP_BATCH; ++u) {
-                    const int j = base + 32 * u + lane;
-                    d[u] = INFINITY;
-                    if (j < s1) {
-                        const float *p = src + (int64_t)j * 3;
-                        d[u] = knn_dist2(__ldg(p) - qx, __ldg(p + 1) - qy, __ldg(p + 2) - qz);
+        const int rounds = s1 > s0 ? (s1 - s0 + ROUND - 1) / ROUND : 0;
+        __syncthreads();                                     // the previous query is over
+        if (threadIdx.x < 2) s_root[threadIdx.x] = KNN_FAR;
+        __syncthreads();
+        if (wid == 0) {
+            LaneHeap heap;
+            heap.init(K, lane);
+            for (int r = 0; r <= rounds; ++r) {
+                if (r > 0) {
+                    const int buf = (r - 1) & 1;
+                    for (int v = 0; v < TIE_WARPS; ++v) {
+                        const int cnt = s_n[buf][v];
+                        const int base = s0 + (r - 1) * ROUND + v * (32 * TIE_PER);
+                        for (int j = 0; j < cnt; j += 32) {
+                            float d = j + lane < cnt ? s_d[buf][v][j + lane] : INFINITY;
+                            const int row = base + (j + lane < cnt ? s_o[buf][v][j + lane] : 0);
+                            unsigned m;
+                            while ((m = __ballot_sync(0xffffffffu, d < heap.root())) != 0) {
+                                const int who = __ffs(m) - 1;
+                                heap.replace(__shfl_sync(0xffffffffu, d, who), __shfl_sync(0xffffffffu, row, who), lane);
+                                if (lane <= who) d = INFINITY;             // earlier ones had their turn
+                            }
+                        }
                     }
+                    if (lane == 0) s_root[buf] = heap.h;
                 }
+                __syncthreads();
+            }
+            s_heap[lane] = heap.h;
+            s_hidx[lane] = heap.id;
+            finish_heap<ROOT>(s_heap, s_hidx, K, g, lane, ret_idx, ret_dist);
+        } else {
+            const float qx = __ldg(query + g * 3), qy = __ldg(query + g * 3 + 1), qz = __ldg(query + g * 3 + 2);
+            const int v = wid - 1;
+            for (int r = 0; r <= rounds; ++r) {
+                if (r < rounds) {
+                    const int buf = r & 1;
+                    const float root = s_root[buf];          // after round r - 2
+                    const int base = s0 + r * ROUND + v * (32 * TIE_PER);
+                    float d[TIE_PER];
 #pragma unroll
-                for (int u = 0; u < WARP_BATCH; ++u) {
-                    float tp = top();
-                    unsigned m = __ballot_sync(0xffffffffu, d[u] < tp);
-                    while (m) {
-                        const int who = __ffs(m) - 1;
-                        const float dd = __shfl_sync(0xffffffffu, d[u], who);
-                        take(dd, base + 32 * u + who);
-                        if (lane == who) d[u] = INFINITY;
-                        tp = top();
-                        m = __ballot_sync(0xffffffffu, d[u] < tp);
+                    for (int u = 0; u < TIE_PER; ++u) {
+                        const int j = base + 32 * u + lane;
+                        d[u] = INFINITY;
+                        if (j < s1) {
+                            const float *p = src + (int64_t)j * 3;
+                            d[u] = knn_dist2(__ldg(p) - qx, __ldg(p + 1) - qy, __ldg(p + 2) - qz);
+                        }
                     }
-                    reject(d[u]);
-                }
-            }
-        };
-        bool exact = LIST || K > 32;
-        if (!exact) {
-            float a = lane < K ? KNN_FAR : INFINITY, ex = INFINITY;
-            int ai = 0;
-            scan([&]() { return __shfl_sync(0xffffffffu, a, K - 1); },
-                 [&](float dd, int row) {
-                     const float last = __shfl_sync(0xffffffffu, a, K - 1);
-                     ex = fminf(ex, last);
-                     const int at = __popc(__ballot_sync(0xffffffffu, a <= dd));
-                     const float up_a = __shfl_up_sync(0xffffffffu, a, 1);
-                     const int up_i = __shfl_up_sync(0xffffffffu, ai, 1);
-                     if (lane < K) {
-                         if (lane > at) { a = up_a; ai = up_i; }
-                         else if (lane == at) { a = dd; ai = row; }
-                     }
-                 },
-                 [&](float d) { ex = fminf(ex, d); });
+                    int cnt = 0;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) ex = fminf(ex, __shfl_xor_sync(0xffffffffu, ex, o));
-            const float before = __shfl_up_sync(0xffffffffu, a, 1), last = __shfl_sync(0xffffffffu, a, K - 1);
-            const bool tie = (lane > 0 && lane < K && a == before && a < KNN_FAR) || (last < KNN_FAR && ex == last);
-            exact = __any_sync(0xffffffffu, tie);
-            if (!exact && lane < K) {
-                ret_idx[g * K + lane] = ai;
-                ret_dist[g * K + lane] = ROOT ? __fsqrt_rn(a) : a;
+                    for (int u = 0; u < TIE_PER; ++u) {
+                        const bool in = d[u] < root;
+                        const unsigned m = __ballot_sync(0xffffffffu, in);
+                        if (in) {
+                            const int at = cnt + __popc(m & ((1u << lane) - 1u));
+                            s_d[buf][v][at] = d[u];
+                            s_o[buf][v][at] = (uint16_t)(32 * u + lane);
+                        }
+                        cnt += __popc(m);
+                    }
+                    if (lane == 0) s_n[buf][v] = cnt;
+                }
+                __syncthreads();
             }
-        }
-        if (exact) {
-            float *heap = s_heap[wid];
-            int *hidx = s_hidx[wid];
-            __syncwarp();
-            for (int j = lane; j < K; j += 32) { heap[j] = KNN_FAR; hidx[j] = 0; }
-            __syncwarp();
-            scan([&]() { return *(volatile float *)heap; },
-                 [&](float dd, int row) {
-                     if (lane == 0) {
-                         heap[0] = dd;
-                         hidx[0] = row;
-                         knn_sift_down(heap, hidx, 0, K);
-                     }
-                     __syncwarp();
-                 },
-                 [&](float) {});
-            if (lane == 0) knn_heap_sort(heap, hidx, K);
-            __syncwarp();
-            for (int j = lane; j < K; j += 32) {
-                ret_idx[g * K + j] = hidx[j];
-                ret_dist[g * K + j] = ROOT ? __fsqrt_rn(heap[j]) : heap[j];
-            }
-            __syncwarp();
         }
     }
 }
 
-template <bool LIST>
-void launch_warp(int K, const float *src, const float *query, const int32_t *so, const int32_t *qo, int B, int64_t Nq,
-                 const int32_t *list, const int *count, int list_max, bool root, int32_t *idx, float *dist, unsigned blocks, cudaStream_t st)
+// ---- a warp per query, straight over the scene's sources --------------------------------------------------
+// For small problems, where building the index costs more than it saves.  First pass: the smallest distance
+// each lane meets on its 32nd of the sources; the K-th smallest of these 32 is a bound of the K-th
+// distance, since they belong to different sources.  Second pass: the candidates within the bound, a few
+// more than K, go to shared memory, and every one finds its rank by counting.  A distance tie among
+// them that reaches into the result, more than 64 of them, or K > 32: scan with the literal heap.
+constexpr int WARP_THREADS = 128, WARP_BATCH = 8, WARP_KEEP = 64;
+
+template <bool ROOT>
+__global__ void __launch_bounds__(WARP_THREADS)
+knn_warp_kernel(int K, const float *__restrict__ src, const float *__restrict__ query, const int32_t *__restrict__ so,
+                const int32_t *__restrict__ qo, int B, int64_t Nq, int32_t *__restrict__ ret_idx, float *__restrict__ ret_dist)
 {
-    if (root) knn_warp_kernel<LIST, true><<<blocks, WARP_THREADS, 0, st>>>(K, src, query, so, qo, B, Nq, list, count, list_max, idx, dist);
-    else knn_warp_kernel<LIST, false><<<blocks, WARP_THREADS, 0, st>>>(K, src, query, so, qo, B, Nq, list, count, list_max, idx, dist);
+    static_assert(WARP_KEEP >= S3D_KNN_MAX_K, "the candidates and the heap share the array");
+    __shared__ float s_d[WARP_THREADS / 32][WARP_KEEP];
+    __shared__ int s_i[WARP_THREADS / 32][WARP_KEEP];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float *keep = s_d[wid];
+    int *kidx = s_i[wid];
+    const int64_t g = (int64_t)blockIdx.x * (WARP_THREADS / 32) + wid;
+    if (g >= Nq) return;
+    const int b = knn_scene(g, qo, B);
+    const int s0 = b > 0 ? __ldg(so + b - 1) : 0, s1 = __ldg(so + b);
+    const float qx = __ldg(query + g * 3), qy = __ldg(query + g * 3 + 1), qz = __ldg(query + g * 3 + 2);
+    // distances of WARP_BATCH x 32 sources, source = base + 32 u + lane
+    auto batch = [&](int base, float (&d)[WARP_BATCH]) {
+#pragma unroll
+        for (int u = 0; u < WARP_BATCH; ++u) {
+            const int j = base + 32 * u + lane;
+            d[u] = INFINITY;
+            if (j < s1) {
+                const float *p = src + (int64_t)j * 3;
+                d[u] = knn_dist2(__ldg(p) - qx, __ldg(p + 1) - qy, __ldg(p + 2) - qz);
+            }
+        }
+    };
+    bool exact = K > 32;
+    if (!exact) {
+        float mn = INFINITY;
+        for (int base = s0; base < s1; base += 32 * WARP_BATCH) {
+            float d[WARP_BATCH];
+            batch(base, d);
+#pragma unroll
+            for (int u = 0; u < WARP_BATCH; ++u) mn = fminf(mn, d[u]);       // a NaN never counts
+        }
+        // bitonic sort over the lanes
+#pragma unroll
+        for (int k = 2; k <= 32; k *= 2)
+#pragma unroll
+            for (int h = k / 2; h > 0; h /= 2) {
+                const float o = __shfl_xor_sync(0xffffffffu, mn, h);
+                mn = ((lane & h) != 0) == ((lane & k) == 0) ? fmaxf(mn, o) : fminf(mn, o);
+            }
+        const float bound = __shfl_sync(0xffffffffu, mn, K - 1);
+        int cnt = 0;
+        for (int base = s0; base < s1; base += 32 * WARP_BATCH) {
+            float d[WARP_BATCH];
+            batch(base, d);
+#pragma unroll
+            for (int u = 0; u < WARP_BATCH; ++u) {
+                const bool in = d[u] <= bound && d[u] < KNN_FAR;
+                const unsigned m = __ballot_sync(0xffffffffu, in);
+                if (m) {
+                    const int at = cnt + __popc(m & ((1u << lane) - 1u));
+                    if (in && at < WARP_KEEP) {
+                        keep[at] = d[u];
+                        kidx[at] = base + 32 * u + lane;
+                    }
+                    cnt += __popc(m);
+                }
+            }
+        }
+        __syncwarp();
+        exact = cnt > WARP_KEEP;
+        if (!exact) {
+            const float d0 = lane < cnt ? keep[lane] : INFINITY, d1 = lane + 32 < cnt ? keep[lane + 32] : INFINITY;
+            int r0 = 0, r1 = 0, e0 = 0, e1 = 0;
+            for (int j = 0; j < cnt; ++j) {
+                const float d = keep[j];
+                r0 += d < d0; r1 += d < d1;
+                e0 += d == d0; e1 += d == d1;
+            }
+            exact = __any_sync(0xffffffffu, (lane < cnt && r0 < K && e0 > 1) || (lane + 32 < cnt && r1 < K && e1 > 1));
+            if (!exact) {
+                if (lane < cnt && r0 < K) {
+                    ret_idx[g * K + r0] = kidx[lane];
+                    ret_dist[g * K + r0] = ROOT ? __fsqrt_rn(d0) : d0;
+                }
+                if (lane + 32 < cnt && r1 < K) {
+                    ret_idx[g * K + r1] = kidx[lane + 32];
+                    ret_dist[g * K + r1] = ROOT ? __fsqrt_rn(d1) : d1;
+                }
+                if (lane < K && lane >= cnt) {                                // fewer candidates than K
+                    ret_idx[g * K + lane] = 0;
+                    ret_dist[g * K + lane] = ROOT ? __fsqrt_rn(KNN_FAR) : KNN_FAR;
+                }
+            }
+        }
+        __syncwarp();
+    }
+    if (!exact) return;
+    if (K <= 32) {
+        LaneHeap heap;
+        heap.init(K, lane);
+        for (int base = s0; base < s1; base += 32 * WARP_BATCH) {
+            float d[WARP_BATCH];
+            batch(base, d);
+#pragma unroll
+            for (int u = 0; u < WARP_BATCH; ++u) {
+                unsigned m;
+                while ((m = __ballot_sync(0xffffffffu, d[u] < heap.root())) != 0) {
+                    const int who = __ffs(m) - 1;
+                    heap.replace(__shfl_sync(0xffffffffu, d[u], who), base + 32 * u + who, lane);
+                    if (lane <= who) d[u] = INFINITY;
+                }
+            }
+        }
+        if (lane < K) { keep[lane] = heap.h; kidx[lane] = heap.id; }
+    } else {
+        for (int j = lane; j < K; j += 32) { keep[j] = KNN_FAR; kidx[j] = 0; }
+        __syncwarp();
+        for (int base = s0; base < s1; base += 32 * WARP_BATCH) {
+            float d[WARP_BATCH];
+            batch(base, d);
+#pragma unroll
+            for (int u = 0; u < WARP_BATCH; ++u) {
+                unsigned m;
+                while ((m = __ballot_sync(0xffffffffu, d[u] < *(volatile float *)keep)) != 0) {
+                    const int who = __ffs(m) - 1;
+                    if (lane == who) {
+                        keep[0] = d[u];
+                        kidx[0] = base + 32 * u + who;
+                        knn_sift_down(keep, kidx, 0, K);
+                    }
+                    if (lane <= who) d[u] = INFINITY;
+                    __syncwarp();
+                }
+            }
+        }
+    }
+    finish_heap<ROOT>(keep, kidx, K, g, lane, ret_idx, ret_dist);
 }
 
 }  // namespace
@@ -612,7 +911,8 @@ int knn_launch_warp(int K, const float *src, const float *query, const int32_t *
                     bool root, int32_t *idx, float *dist, cudaStream_t st)
 {
     const unsigned blocks = (unsigned)((Nq + WARP_THREADS / 32 - 1) / (WARP_THREADS / 32));
-    launch_warp<false>(K, src, query, so, qo, B, Nq, nullptr, nullptr, 0, root, idx, dist, blocks, st);
+    if (root) knn_warp_kernel<true><<<blocks, WARP_THREADS, 0, st>>>(K, src, query, so, qo, B, Nq, idx, dist);
+    else knn_warp_kernel<false><<<blocks, WARP_THREADS, 0, st>>>(K, src, query, so, qo, B, Nq, idx, dist);
     return cudaGetLastError() == cudaSuccess ? S3D_OK : S3D_ERR_LAUNCH;
 }
 
@@ -639,10 +939,12 @@ int knn_launch_tree(int K, const float *src, const float *query, const int32_t *
     else { S3D_KNN_SEARCH(16); }
 #undef S3D_KNN_SEARCH
     if (cudaGetLastError() != cudaSuccess) return S3D_ERR_LAUNCH;
-    // tied queries: a warp each while they are few, otherwise the thread-per-query scan; both kernels read
+    // tied queries: a block each while they are few, otherwise the thread-per-query scan; both kernels read
     // the count and one of them returns at once
-    constexpr int FEW = 16384;
-    launch_warp<true>(K, src, query, so, qo, B, Nq, t.ties, t.tie_count, FEW, root, idx, dist, 148 * 8, st);
+    constexpr int FEW = 2048;
+    const unsigned tie_blocks = (unsigned)(Nq < 148 * 4 ? Nq : 148 * 4);
+    if (root) knn_tie_kernel<true><<<tie_blocks, TIE_THREADS, 0, st>>>(K, src, query, so, qo, B, t.ties, t.tie_count, FEW, idx, dist);
+    else knn_tie_kernel<false><<<tie_blocks, TIE_THREADS, 0, st>>>(K, src, query, so, qo, B, t.ties, t.tie_count, FEW, idx, dist);
     if (cudaGetLastError() != cudaSuccess) return S3D_ERR_LAUNCH;
     return Nq > FEW ? knn_launch_list(K, src, query, so, qo, B, Nq, t.ties, t.tie_count, FEW, root, idx, dist, st) : S3D_OK;
 }
