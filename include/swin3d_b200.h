@@ -286,6 +286,24 @@ int s3d_knn_maxpool_fwd(const int32_t *idx, const void *g, void *out, int32_t *a
 int s3d_knn_maxpool_bwd(const int32_t *arg, const void *dout, float *dg,
                         int64_t Nq, int64_t Ns, int C, int dtype, void *stream);
 
+/* The same operations with the gradient gathered per source row instead of scattered.
+ *  s3d_knn_maxpool_slots_fwd keeps slot uint8[Nq,C], the position (0..K-1) of the maximum in the query's
+ *  list, instead of the source row.  The two _bwd calls turn idx around in `workspace`
+ *  (s3d_knn_gather_workspace_bytes, 16-byte aligned device memory; 0: too large for this form) and
+ *  write dsrc / dg [Ns,C] in `dtype`, every row once, summed in fp32.  The sum runs over the queries that
+ *  refer to a row one after the other, so lists of many thousands are better scattered.
+ */
+int64_t s3d_knn_gather_workspace_bytes(int64_t Ns, int64_t Nq, int K);
+int s3d_knn_interpolate_gather_bwd(const int32_t *idx, const float *dist, const void *dout, void *dsrc,
+                                   int64_t Nq, int64_t Ns, int K, int C, int dtype, void *workspace,
+                                   int64_t workspace_bytes, void *stream);
+int s3d_knn_maxpool_slots_fwd(const int32_t *idx, const void *g, void *out, uint8_t *slot,
+                              int64_t Nq, int K, int C, int dtype, void *stream);
+int s3d_knn_maxpool_slots_bwd(const int32_t *idx, const uint8_t *slot, const void *dout, void *dg,
+                              int64_t Nq, int64_t Ns, int K, int C, int dtype, void *workspace,
+                              int64_t workspace_bytes, void *stream);
+
+
 #ifdef __cplusplus
 }
 #endif

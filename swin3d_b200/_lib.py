@@ -59,6 +59,10 @@ SIGNATURES = {
     "s3d_knn_interpolate_bwd": (_i32, [_c_void_p] * 4 + [_i64, _i64, _i32, _i32, _i32, _c_void_p]),
     "s3d_knn_maxpool_fwd": (_i32, [_c_void_p] * 4 + [_i64, _i32, _i32, _i32, _c_void_p]),
     "s3d_knn_maxpool_bwd": (_i32, [_c_void_p] * 3 + [_i64, _i64, _i32, _i32, _c_void_p]),
+    "s3d_knn_gather_workspace_bytes": (_i64, [_i64, _i64, _i32]),
+    "s3d_knn_interpolate_gather_bwd": (_i32, [_c_void_p] * 4 + [_i64, _i64, _i32, _i32, _i32, _c_void_p, _i64, _c_void_p]),
+    "s3d_knn_maxpool_slots_fwd": (_i32, [_c_void_p] * 4 + [_i64, _i32, _i32, _i32, _c_void_p]),
+    "s3d_knn_maxpool_slots_bwd": (_i32, [_c_void_p] * 4 + [_i64, _i64, _i32, _i32, _i32, _c_void_p, _i64, _c_void_p]),
 }
 
 

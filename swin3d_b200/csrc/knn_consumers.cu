@@ -10,19 +10,28 @@
 //    out[q][c] = max_i g[idx[q,i]][c] with g = linear(norm(src_feat)) evaluated once per SOURCE row.
 //    The arg-max source row is kept for the backward scatter (first maximum wins, as MaxPool1d).
 //
-// Both are HBM-bound row gathers: a warp owns a query, lanes run over channels with 16-byte
-// accesses; the scatter-adds of the backward are fp32 reductions in L2 (red.global.add).
+// Both forwards are row gathers bound by L2 and HBM: a block takes a tile of queries, works out their
+// rows and weights once into shared memory, and its threads then run over (query, 16-byte piece), so
+// that every lane carries data whatever C is.  (A warp per query with the lanes over the channels
+// left 22 of 32 lanes idle at C = 80: 466 against 127 us for 1.6 M queries, fp16, K = 3.)
+//
+// Two backwards.  The scatter form adds into an fp32 array with reductions in L2 (red.global.add).  The
+// gather form (workspace given) first turns idx around -- a counting sort of the Nq * K (query,
+// neighbour) entries by source -- and then a thread per (source, 16-byte piece) sums its entries in
+// registers: no fp32 array to clear, add into and convert, one store per result.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "common.cuh"
+#include "scan.cuh"
 
 namespace s3d {
 namespace {
 
 constexpr int KC_MAX_K = 64;
 constexpr int KC_THREADS = 256;
+constexpr int KC_TILE = 64;              // queries per block of the forwards
 
 template <typename T> struct Vec;
 template <> struct Vec<float> {
@@ -79,39 +88,41 @@ knn_interp_fwd_kernel(const int32_t *__restrict__ idx, const float *__restrict__
 {
     constexpr int VN = Vec<T>::N;
     using Raw = typename Vec<T>::Raw;
+    extern __shared__ int2 s_iw[];                           // [KC_TILE][K] row, weight
     const int K = KT ? KT : Krt;
-    const int lane = threadIdx.x & 31;
-    const int64_t warp0 = (int64_t)blockIdx.x * (KC_THREADS / 32) + (threadIdx.x >> 5);
-    const int64_t nwarp = (int64_t)gridDim.x * (KC_THREADS / 32);
     const int CV = C / VN;   // C is a whole number of vectors (checked by the entry point)
-    for (int64_t q = warp0; q < Nq; q += nwarp) {
-        float w[KT ? KT : KC_MAX_K];
-        int32_t id[KT ? KT : KC_MAX_K];
-        {
-            float norm = 0.f;
+    const int64_t q0 = (int64_t)blockIdx.x * KC_TILE;
+    const int nq = (int)min((int64_t)KC_TILE, Nq - q0);
+    if (threadIdx.x < nq) {
+        const int64_t q = q0 + threadIdx.x;
+        float norm = 0.f;
+        int2 *e = s_iw + threadIdx.x * K;
 #pragma unroll 4
-            for (int i = 0; i < K; ++i) {
-                id[i] = __ldg(idx + q * K + i);
-                w[i] = __fdiv_rn(1.0f, __fadd_rn(__ldg(dist + q * K + i), 1e-8f));
-                norm = __fadd_rn(norm, w[i]);
-            }
-#pragma unroll 4
-            for (int i = 0; i < K; ++i) w[i] = __fdiv_rn(w[i], norm);
+        for (int i = 0; i < K; ++i) {
+            const float w = __fdiv_rn(1.0f, __fadd_rn(__ldg(dist + q * K + i), 1e-8f));
+            norm = __fadd_rn(norm, w);
+            e[i] = make_int2(__ldg(idx + q * K + i), __float_as_int(w));
         }
-        for (int cv = lane; cv < CV; cv += 32) {
-            float acc[VN];
-#pragma unroll
-            for (int j = 0; j < VN; ++j) acc[j] = 0.f;
 #pragma unroll 4
-            for (int i = 0; i < K; ++i) {
-                const Raw r = __ldg(reinterpret_cast<const Raw *>(src + (int64_t)id[i] * C) + cv);
-                float f[VN];
-                Vec<T>::unpack(r, f);
+        for (int i = 0; i < K; ++i) e[i].y = __float_as_int(__fdiv_rn(__int_as_float(e[i].y), norm));
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < nq * CV; t += KC_THREADS) {
+        const int ql = t / CV, cv = t - ql * CV;
+        const int2 *e = s_iw + ql * K;
+        float acc[VN];
 #pragma unroll
-                for (int j = 0; j < VN; ++j) acc[j] = round_acc<T>(__fadd_rn(acc[j], __fmul_rn(f[j], w[i])));
-            }
-            reinterpret_cast<Raw *>(out + q * C)[cv] = Vec<T>::pack(acc);
+        for (int j = 0; j < VN; ++j) acc[j] = 0.f;
+#pragma unroll 4
+        for (int i = 0; i < K; ++i) {
+            const int2 iw = e[i];
+            const float w = __int_as_float(iw.y);
+            float f[VN];
+            Vec<T>::unpack(__ldg(reinterpret_cast<const Raw *>(src + (int64_t)iw.x * C) + cv), f);
+#pragma unroll
+            for (int j = 0; j < VN; ++j) acc[j] = round_acc<T>(__fadd_rn(acc[j], __fmul_rn(f[j], w)));
         }
+        reinterpret_cast<Raw *>(out + (q0 + ql) * C)[cv] = Vec<T>::pack(acc);
     }
 }
 
@@ -143,38 +154,152 @@ knn_interp_bwd_kernel(const int32_t *__restrict__ idx, const float *__restrict__
     }
 }
 
-template <typename T>
+// A: what is kept of the arg-max, the source row (int32_t) or the position in the query's list (uint8_t).
+template <typename T, typename A, int KT /*0: runtime K*/>
 __global__ void __launch_bounds__(KC_THREADS)
 knn_maxpool_fwd_kernel(const int32_t *__restrict__ idx, const T *__restrict__ g, T *__restrict__ out,
-                       int32_t *__restrict__ arg, int64_t Nq, int K, int C)
+                       A *__restrict__ arg, int64_t Nq, int Krt, int C)
 {
     constexpr int VN = Vec<T>::N;
     using Raw = typename Vec<T>::Raw;
-    const int lane = threadIdx.x & 31;
-    const int64_t warp0 = (int64_t)blockIdx.x * (KC_THREADS / 32) + (threadIdx.x >> 5);
-    const int64_t nwarp = (int64_t)gridDim.x * (KC_THREADS / 32);
+    extern __shared__ int32_t s_id[];                        // [KC_TILE][K] (K <= KC_MAX_K; longer lists stay in global memory)
+    const int K = KT ? KT : Krt;
     const int CV = C / VN;
-    for (int64_t q = warp0; q < Nq; q += nwarp) {
-        for (int cv = lane; cv < CV; cv += 32) {
-            float best[VN] = {};
-            int32_t who[VN] = {};
-            for (int i = 0; i < K; ++i) {
-                const int32_t s = __ldg(idx + q * K + i);
-                float f[VN];
-                Vec<T>::unpack(__ldg(reinterpret_cast<const Raw *>(g + (int64_t)s * C) + cv), f);
+    const int64_t q0 = (int64_t)blockIdx.x * KC_TILE;
+    const int nq = (int)min((int64_t)KC_TILE, Nq - q0);
+    const bool staged = KT || K <= KC_MAX_K;
+    if (staged)
+        for (int i = threadIdx.x; i < nq * K; i += KC_THREADS) s_id[i] = __ldg(idx + q0 * K + i);
+    __syncthreads();
+    for (int t = threadIdx.x; t < nq * CV; t += KC_THREADS) {
+        const int ql = t / CV, cv = t - ql * CV;
+        const int32_t *e = staged ? s_id + ql * K : idx + (q0 + ql) * K;
+        float best[VN] = {};
+        A who[VN] = {};
+#pragma unroll 8
+        for (int i = 0; i < K; ++i) {
+            const int32_t s = e[i];
+            float f[VN];
+            Vec<T>::unpack(__ldg(reinterpret_cast<const Raw *>(g + (int64_t)s * C) + cv), f);
 #pragma unroll
-                for (int j = 0; j < VN; ++j)
-                    if (i == 0 || f[j] > best[j] || f[j] != f[j]) {   // first maximum wins; NaN propagates
-                        best[j] = f[j];
-                        who[j] = s;
-                    }
-            }
-            reinterpret_cast<Raw *>(out + q * C)[cv] = Vec<T>::pack(best);
+            for (int j = 0; j < VN; ++j)
+                if (i == 0 || f[j] > best[j] || f[j] != f[j]) {   // first maximum wins; NaN propagates
+                    best[j] = f[j];
+                    who[j] = sizeof(A) == 1 ? (A)i : (A)s;
+                }
+        }
+        reinterpret_cast<Raw *>(out + (q0 + ql) * C)[cv] = Vec<T>::pack(best);
+        A *a = arg + (q0 + ql) * C + cv * VN;
 #pragma unroll
-            for (int j = 0; j < VN; j += 4)
-                *reinterpret_cast<int4 *>(arg + q * C + cv * VN + j) = make_int4(who[j], who[j + 1], who[j + 2], who[j + 3]);
+        for (int j = 0; j < VN; j += 4) {
+            if (sizeof(A) == 1) *reinterpret_cast<uchar4 *>(a + j) = make_uchar4(who[j], who[j + 1], who[j + 2], who[j + 3]);
+            else *reinterpret_cast<int4 *>(a + j) = make_int4(who[j], who[j + 1], who[j + 2], who[j + 3]);
         }
     }
+}
+
+// ---- gather backward -----------------------------------------------------------------------------------
+// Workspace: one counter per source (then the start of its entries), tile sums of their scan, the rank
+// of every (query, neighbour) among the entries of its source, the entries.
+struct Inverse {
+    uint32_t *start, *tile, *rank;
+    int2 *entry;
+    int64_t start_bytes, total;
+    int n_tiles;
+};
+
+Inverse inverse_layout(char *base, int64_t Ns, int64_t Nq, int K)
+{
+    Inverse v{};
+    v.n_tiles = (int)((Ns + 1 + SCAN_TILE - 1) / SCAN_TILE);
+    int64_t off = 0;
+    auto take = [&](int64_t bytes) { const int64_t o = off; off = (off + bytes + 255) / 256 * 256; return base + o; };
+    v.start_bytes = (int64_t)v.n_tiles * SCAN_TILE * 4;
+    v.start = (uint32_t *)take(v.start_bytes);
+    v.tile = (uint32_t *)take((int64_t)v.n_tiles * 4);
+    v.rank = (uint32_t *)take(Nq * K * 4);
+    v.entry = (int2 *)take(Nq * K * 8);
+    v.total = off;
+    return v;
+}
+
+__global__ void __launch_bounds__(KC_THREADS)
+inverse_count_kernel(const int32_t *__restrict__ idx, int64_t n, Inverse v)
+{
+    const int64_t e = (int64_t)blockIdx.x * KC_THREADS + threadIdx.x;
+    if (e < n) v.rank[e] = atomicAdd(v.start + __ldg(idx + e), 1u);
+}
+
+// entries (query, weight)
+__global__ void __launch_bounds__(KC_THREADS)
+inverse_fill_weights_kernel(const int32_t *__restrict__ idx, const float *__restrict__ dist, int64_t Nq, int K, Inverse v)
+{
+    const int64_t q = (int64_t)blockIdx.x * KC_THREADS + threadIdx.x;
+    if (q >= Nq) return;
+    float norm = 0.f;
+#pragma unroll 4
+    for (int i = 0; i < K; ++i) norm = __fadd_rn(norm, __fdiv_rn(1.0f, __fadd_rn(__ldg(dist + q * K + i), 1e-8f)));
+#pragma unroll 4
+    for (int i = 0; i < K; ++i) {
+        const float w = __fdiv_rn(__fdiv_rn(1.0f, __fadd_rn(__ldg(dist + q * K + i), 1e-8f)), norm);
+        const int64_t e = q * K + i;
+        v.entry[v.start[__ldg(idx + e)] + v.rank[e]] = make_int2((int)q, __float_as_int(w));
+    }
+}
+
+// entries (query, position in its list)
+__global__ void __launch_bounds__(KC_THREADS)
+inverse_fill_slots_kernel(const int32_t *__restrict__ idx, int64_t n, int K, Inverse v)
+{
+    const int64_t e = (int64_t)blockIdx.x * KC_THREADS + threadIdx.x;
+    if (e >= n) return;
+    const int q = (int)((uint32_t)e / (uint32_t)K);
+    v.entry[v.start[__ldg(idx + e)] + v.rank[e]] = make_int2(q, (int)(e - (int64_t)q * K));
+}
+
+// dsrc[s] = sum over the entries of s of w * dout[q]          (SLOT: of dout[q] where slot[q] is the entry's)
+template <typename T, bool SLOT>
+__global__ void __launch_bounds__(KC_THREADS)
+inverse_gather_kernel(const T *__restrict__ dout, const uint8_t *__restrict__ slot, T *__restrict__ dsrc, int64_t Ns, int C, Inverse v)
+{
+    constexpr int VN = Vec<T>::N;
+    using Raw = typename Vec<T>::Raw;
+    const int CV = C / VN;
+    const int64_t t = (int64_t)blockIdx.x * KC_THREADS + threadIdx.x;
+    const int64_t s = t / CV;
+    if (s >= Ns) return;
+    const int cv = (int)(t - s * CV);
+    const uint32_t e0 = __ldg(v.start + s), e1 = __ldg(v.start + s + 1);
+    float acc[VN];
+#pragma unroll
+    for (int j = 0; j < VN; ++j) acc[j] = 0.f;
+#pragma unroll 4
+    for (uint32_t e = e0; e < e1; ++e) {
+        const int2 it = __ldg(v.entry + e);
+        if (SLOT) {
+            const uint8_t *sp = slot + (int64_t)it.x * C + cv * VN;
+            uint32_t sl[VN / 4], any = 0;
+            const uint32_t want = 0x01010101u * (uint32_t)it.y;
+#pragma unroll
+            for (int j = 0; j < VN / 4; ++j) {
+                sl[j] = __vcmpeq4(__ldg(reinterpret_cast<const uint32_t *>(sp) + j), want);
+                any |= sl[j];
+            }
+            if (any) {
+                float g[VN];
+                Vec<T>::unpack(__ldg(reinterpret_cast<const Raw *>(dout + (int64_t)it.x * C) + cv), g);
+#pragma unroll
+                for (int j = 0; j < VN; ++j) acc[j] += (sl[j / 4] >> (8 * (j & 3))) & 1u ? g[j] : 0.f;
+            }
+        } else {
+            float g[VN];
+            Vec<T>::unpack(__ldg(reinterpret_cast<const Raw *>(dout + (int64_t)it.x * C) + cv), g);
+            const float w = __int_as_float(it.y);
+#pragma unroll
+            for (int j = 0; j < VN; ++j) acc[j] = fmaf(g[j], w, acc[j]);
+        }
+    }
+    reinterpret_cast<Raw *>(dsrc + s * C)[cv] = Vec<T>::pack(acc);
 }
 
 template <typename T>
@@ -191,12 +316,35 @@ knn_maxpool_bwd_kernel(const int32_t *__restrict__ arg, const T *__restrict__ do
 
 int grid_for(int64_t warps_needed)
 {
+    static int sms_of[64] = {0};
     int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
+        if (!sms_of[dev] && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) sms_of[dev] = sms;
+        if (sms_of[dev]) sms = sms_of[dev];
+    }
     const int64_t blocks = (warps_needed + KC_THREADS / 32 - 1) / (KC_THREADS / 32);
     const int64_t cap = (int64_t)sms * 8;     // 8 resident blocks of 256 threads per SM
     return (int)(blocks < 1 ? 1 : (blocks < cap ? blocks : cap));
+}
+
+unsigned blocks_of(int64_t n, int per) { return (unsigned)((n + per - 1) / per); }
+
+template <typename T>
+void launch_interp_fwd(const int32_t *idx, const float *dist, const void *src, void *out, int64_t Nq, int K, int C, cudaStream_t st)
+{
+    const unsigned grid = blocks_of(Nq, KC_TILE);
+    const size_t smem = (size_t)KC_TILE * K * sizeof(int2);
+    if (K == 3) knn_interp_fwd_kernel<T, 3><<<grid, KC_THREADS, smem, st>>>(idx, dist, (const T *)src, (T *)out, Nq, K, C);
+    else knn_interp_fwd_kernel<T, 0><<<grid, KC_THREADS, smem, st>>>(idx, dist, (const T *)src, (T *)out, Nq, K, C);
+}
+
+template <typename T, typename A>
+void launch_maxpool_fwd(const int32_t *idx, const void *g, void *out, A *arg, int64_t Nq, int K, int C, cudaStream_t st)
+{
+    const unsigned grid = blocks_of(Nq, KC_TILE);
+    const size_t smem = K <= KC_MAX_K ? (size_t)KC_TILE * K * sizeof(int32_t) : 0;
+    if (K == 16) knn_maxpool_fwd_kernel<T, A, 16><<<grid, KC_THREADS, smem, st>>>(idx, (const T *)g, (T *)out, arg, Nq, K, C);
+    else knn_maxpool_fwd_kernel<T, A, 0><<<grid, KC_THREADS, smem, st>>>(idx, (const T *)g, (T *)out, arg, Nq, K, C);
 }
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -217,18 +365,8 @@ extern "C" int s3d_knn_interpolate_fwd(const int32_t *idx, const float *dist, co
     const int vn = dtype == S3D_F32 ? 4 : 8;
     if (C % vn != 0 || !aligned16(src_feat) || !aligned16(out)) return S3D_ERR_UNSUPPORTED;
     cudaStream_t st = (cudaStream_t)stream;
-    const int grid = grid_for(Nq);
-    if (dtype == S3D_F32) {
-        if (K == 3)
-            knn_interp_fwd_kernel<float, 3><<<grid, KC_THREADS, 0, st>>>(idx, dist, (const float *)src_feat, (float *)out, Nq, K, C);
-        else
-            knn_interp_fwd_kernel<float, 0><<<grid, KC_THREADS, 0, st>>>(idx, dist, (const float *)src_feat, (float *)out, Nq, K, C);
-    } else {
-        if (K == 3)
-            knn_interp_fwd_kernel<__half, 3><<<grid, KC_THREADS, 0, st>>>(idx, dist, (const __half *)src_feat, (__half *)out, Nq, K, C);
-        else
-            knn_interp_fwd_kernel<__half, 0><<<grid, KC_THREADS, 0, st>>>(idx, dist, (const __half *)src_feat, (__half *)out, Nq, K, C);
-    }
+    if (dtype == S3D_F32) launch_interp_fwd<float>(idx, dist, src_feat, out, Nq, K, C, st);
+    else launch_interp_fwd<__half>(idx, dist, src_feat, out, Nq, K, C, st);
     return last_status();
 }
 
@@ -261,11 +399,8 @@ extern "C" int s3d_knn_maxpool_fwd(const int32_t *idx, const void *g, void *out,
     const int vn = dtype == S3D_F32 ? 4 : 8;
     if (C % vn != 0 || !aligned16(g) || !aligned16(out) || !aligned16(arg)) return S3D_ERR_UNSUPPORTED;
     cudaStream_t st = (cudaStream_t)stream;
-    const int grid = grid_for(Nq);
-    if (dtype == S3D_F32)
-        knn_maxpool_fwd_kernel<float><<<grid, KC_THREADS, 0, st>>>(idx, (const float *)g, (float *)out, arg, Nq, K, C);
-    else
-        knn_maxpool_fwd_kernel<__half><<<grid, KC_THREADS, 0, st>>>(idx, (const __half *)g, (__half *)out, arg, Nq, K, C);
+    if (dtype == S3D_F32) launch_maxpool_fwd<float>(idx, g, out, arg, Nq, K, C, st);
+    else launch_maxpool_fwd<__half>(idx, g, out, arg, Nq, K, C, st);
     return last_status();
 }
 
@@ -290,4 +425,69 @@ extern "C" int s3d_knn_maxpool_bwd(const int32_t *arg, const void *dout, float *
     else
         knn_maxpool_bwd_kernel<__half><<<grid, KC_THREADS, 0, st>>>(arg, (const __half *)dout, dg, total, C);
     return last_status();
+}
+
+extern "C" int s3d_knn_maxpool_slots_fwd(const int32_t *idx, const void *g, void *out, uint8_t *slot,
+                                         int64_t Nq, int K, int C, int dtype, void *stream)
+{
+    if (Nq < 0 || K < 1 || K > KC_MAX_K || C < 1 || (dtype != S3D_F32 && dtype != S3D_F16)) return S3D_ERR_BAD_ARG;
+    if (Nq == 0) return S3D_OK;
+    if (!idx || !g || !out || !slot) return S3D_ERR_BAD_ARG;
+    const int vn = dtype == S3D_F32 ? 4 : 8;
+    if (C % vn != 0 || !aligned16(g) || !aligned16(out) || !aligned16(slot)) return S3D_ERR_UNSUPPORTED;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (dtype == S3D_F32) launch_maxpool_fwd<float>(idx, g, out, slot, Nq, K, C, st);
+    else launch_maxpool_fwd<__half>(idx, g, out, slot, Nq, K, C, st);
+    return last_status();
+}
+
+extern "C" int64_t s3d_knn_gather_workspace_bytes(int64_t Ns, int64_t Nq, int K)
+{
+    if (Ns < 1 || Nq < 1 || K < 1 || Nq * K >= (int64_t)1 << 31) return 0;
+    return inverse_layout(nullptr, Ns, Nq, K).total;
+}
+
+static int gather_impl(const int32_t *idx, const float *dist, const uint8_t *slot, const void *dout, void *dsrc,
+                       int64_t Nq, int64_t Ns, int K, int C, int dtype, void *workspace, int64_t workspace_bytes, void *stream)
+{
+    if (Nq < 0 || Ns < 0 || K < 1 || K > KC_MAX_K || C < 1 || (dtype != S3D_F32 && dtype != S3D_F16)) return S3D_ERR_BAD_ARG;
+    if (Ns == 0) return S3D_OK;
+    if (!dsrc) return S3D_ERR_BAD_ARG;
+    const int vn = dtype == S3D_F32 ? 4 : 8;
+    if (C % vn != 0 || !aligned16(dout) || !aligned16(dsrc)) return S3D_ERR_UNSUPPORTED;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (Nq == 0) return cudaMemsetAsync(dsrc, 0, (size_t)Ns * C * (dtype == S3D_F32 ? 4 : 2), st) == cudaSuccess ? S3D_OK : S3D_ERR_LAUNCH;
+    if (!idx || (!dist && !slot) || !dout || !workspace) return S3D_ERR_BAD_ARG;
+    if (Nq * K >= (int64_t)1 << 31) return S3D_ERR_UNSUPPORTED;
+    const Inverse v = inverse_layout((char *)workspace, Ns, Nq, K);
+    if (workspace_bytes < v.total) return S3D_ERR_WORKSPACE;
+    if (cudaMemsetAsync(v.start, 0, (size_t)v.start_bytes, st) != cudaSuccess) return S3D_ERR_LAUNCH;
+    const int64_t n = Nq * K;
+    inverse_count_kernel<<<blocks_of(n, KC_THREADS), KC_THREADS, 0, st>>>(idx, n, v);
+    scan_in_place(v.start, v.tile, v.n_tiles, st);
+    if (slot) inverse_fill_slots_kernel<<<blocks_of(n, KC_THREADS), KC_THREADS, 0, st>>>(idx, n, K, v);
+    else inverse_fill_weights_kernel<<<blocks_of(Nq, KC_THREADS), KC_THREADS, 0, st>>>(idx, dist, Nq, K, v);
+    const unsigned grid = blocks_of(Ns * (C / vn), KC_THREADS);
+    if (dtype == S3D_F32) {
+        if (slot) inverse_gather_kernel<float, true><<<grid, KC_THREADS, 0, st>>>((const float *)dout, slot, (float *)dsrc, Ns, C, v);
+        else inverse_gather_kernel<float, false><<<grid, KC_THREADS, 0, st>>>((const float *)dout, slot, (float *)dsrc, Ns, C, v);
+    } else {
+        if (slot) inverse_gather_kernel<__half, true><<<grid, KC_THREADS, 0, st>>>((const __half *)dout, slot, (__half *)dsrc, Ns, C, v);
+        else inverse_gather_kernel<__half, false><<<grid, KC_THREADS, 0, st>>>((const __half *)dout, slot, (__half *)dsrc, Ns, C, v);
+    }
+    return last_status();
+}
+
+extern "C" int s3d_knn_interpolate_gather_bwd(const int32_t *idx, const float *dist, const void *dout, void *dsrc,
+                                              int64_t Nq, int64_t Ns, int K, int C, int dtype, void *workspace,
+                                              int64_t workspace_bytes, void *stream)
+{
+    return gather_impl(idx, dist, nullptr, dout, dsrc, Nq, Ns, K, C, dtype, workspace, workspace_bytes, stream);
+}
+
+extern "C" int s3d_knn_maxpool_slots_bwd(const int32_t *idx, const uint8_t *slot, const void *dout, void *dg,
+                                         int64_t Nq, int64_t Ns, int K, int C, int dtype, void *workspace,
+                                         int64_t workspace_bytes, void *stream)
+{
+    return gather_impl(idx, nullptr, slot, dout, dg, Nq, Ns, K, C, dtype, workspace, workspace_bytes, stream);
 }

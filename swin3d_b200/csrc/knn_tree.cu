@@ -21,13 +21,13 @@
 // K = 3; 4 x 30 k x 120 k, K = 16): see knn_launch_tree.
 #include "knn_common.cuh"
 #include "knn_kernels.cuh"
+#include "scan.cuh"
 
 namespace s3d {
 namespace {
 
 constexpr int LEAF = 32;
 constexpr int KT_THREADS = 256;
-constexpr int SCAN_T = 256, SCAN_PER = 16, SCAN_TILE = SCAN_T * SCAN_PER;
 constexpr int SEARCH_THREADS = 128;
 
 struct TreeBufs {
@@ -188,67 +188,6 @@ tree_sort_kernel(const float *__restrict__ src, const float *__restrict__ query,
         const uint32_t s0 = t.hist[(int64_t)b << (3 * t.bits)];
         float *o = t.src + (first_leaf(s0, b) + (at - s0) / LEAF) * (4 * LEAF) + (at - s0) % LEAF;
         o[0] = x; o[LEAF] = y; o[2 * LEAF] = z; o[3 * LEAF] = __int_as_float((int)g);
-    }
-}
-
-// Exclusive scan of the histograms in two launches: tile sums, then every block adds up the sums of the
-// tiles before its own (at most a few thousand words from L2) and scans its tile in place.
-__global__ void __launch_bounds__(SCAN_T)
-tree_tile_sums_kernel(const uint32_t *__restrict__ hist, uint32_t *__restrict__ tile)
-{
-    const uint4 *p = reinterpret_cast<const uint4 *>(hist + (int64_t)blockIdx.x * SCAN_TILE);
-    uint32_t s = 0;
-#pragma unroll
-    for (int j = 0; j < SCAN_PER / 4; ++j) {
-        const uint4 v = p[j * SCAN_T + threadIdx.x];
-        s += v.x + v.y + v.z + v.w;
-    }
-    __shared__ uint32_t s_w[SCAN_T / 32];
-    s = __reduce_add_sync(0xffffffffu, s);
-    if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const uint32_t v = __reduce_add_sync(0xffffffffu, threadIdx.x < SCAN_T / 32 ? s_w[threadIdx.x] : 0u);
-        if (threadIdx.x == 0) tile[blockIdx.x] = v;
-    }
-}
-
-__global__ void __launch_bounds__(SCAN_T)
-tree_scan_kernel(uint32_t *__restrict__ hist, const uint32_t *__restrict__ tile)
-{
-    __shared__ uint32_t s_w[SCAN_T / 32], s_base[SCAN_T / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t before = 0;
-    for (int i = threadIdx.x; i < (int)blockIdx.x; i += SCAN_T) before += __ldg(tile + i);
-    before = __reduce_add_sync(0xffffffffu, before);
-    uint4 *p = reinterpret_cast<uint4 *>(hist + (int64_t)blockIdx.x * SCAN_TILE) + threadIdx.x * (SCAN_PER / 4);
-    uint4 v[SCAN_PER / 4];
-    uint32_t sum = 0;
-#pragma unroll
-    for (int j = 0; j < SCAN_PER / 4; ++j) {
-        v[j] = p[j];
-        sum += v[j].x + v[j].y + v[j].z + v[j].w;
-    }
-    uint32_t incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) s_w[wid] = incl;
-    if (lane == 0) s_base[wid] = before;
-    __syncthreads();
-    uint32_t run = incl - sum;
-#pragma unroll
-    for (int w = 0; w < SCAN_T / 32; ++w) run += s_base[w] + (w < wid ? s_w[w] : 0u);
-#pragma unroll
-    for (int j = 0; j < SCAN_PER / 4; ++j) {
-        uint4 o;
-        o.x = run; run += v[j].x;
-        o.y = run; run += v[j].y;
-        o.z = run; run += v[j].z;
-        o.w = run; run += v[j].w;
-        p[j] = o;
     }
 }
 
@@ -926,8 +865,7 @@ int knn_launch_tree(int K, const float *src, const float *query, const int32_t *
     tree_bbox_kernel<<<dim3(gx, (unsigned)B), KT_THREADS, 0, st>>>(src, query, so, qo, B, Nq, t.bbox);
     const unsigned nb = (unsigned)((Ns + Nq + KT_THREADS - 1) / KT_THREADS);
     tree_sort_kernel<true><<<nb, KT_THREADS, 0, st>>>(src, query, so, qo, B, Ns, Nq, t);
-    tree_tile_sums_kernel<<<(unsigned)t.n_tiles, SCAN_T, 0, st>>>(t.hist, t.tile);
-    tree_scan_kernel<<<(unsigned)t.n_tiles, SCAN_T, 0, st>>>(t.hist, t.tile);
+    scan_in_place(t.hist, t.tile, t.n_tiles, st);
     tree_sort_kernel<false><<<nb, KT_THREADS, 0, st>>>(src, query, so, qo, B, Ns, Nq, t);
     tree_boxes_kernel<<<(unsigned)(Ns / (LEAF * 32) + B), 1024, 0, st>>>(B, t);
     const unsigned blocks = (unsigned)((Nq + SEARCH_THREADS - 1) / SEARCH_THREADS);

@@ -37,6 +37,19 @@ def get_offset(batch: torch.Tensor) -> torch.Tensor:
     return torch.cumsum(torch.bincount(batch.long()), 0).to(torch.int32)
 
 
+# The gather form of the backwards walks the queries of a source row one after the other: with more than
+# this many on average (few sources, many queries) the scatter form keeps more of the GPU busy.
+GATHER_MOST_PER_SOURCE = 256
+
+
+def _gather_workspace(n_src: int, Nq: int, K: int, dev):
+    """(workspace, bytes) of the gather backward, or (None, 0) where the scatter backward is the better one."""
+    if Nq * K > GATHER_MOST_PER_SOURCE * n_src:
+        return None, 0
+    nbytes = _lib.lib.s3d_knn_gather_workspace_bytes(n_src, Nq, K)
+    return (torch.empty(nbytes, dtype=torch.uint8, device=dev), nbytes) if nbytes else (None, 0)
+
+
 class KNNInterpolate(Function):
     """out[q] = sum_i src_feat[idx[q,i]] * w_i with normalised inverse-distance weights."""
 
@@ -64,6 +77,16 @@ class KNNInterpolate(Function):
         grad_out = grad_out.contiguous()
         Nq, K = idx.shape
         C = grad_out.shape[1]
+        work, nbytes = _gather_workspace(ctx.n_src, Nq, K, grad_out.device)
+        if work is not None and grad_out.data_ptr() % 16 == 0:
+            dsrc = torch.empty((ctx.n_src, C), dtype=grad_out.dtype, device=grad_out.device)
+            with torch.cuda.device(grad_out.device):
+                st = torch.cuda.current_stream().cuda_stream
+                rc = _lib.lib.s3d_knn_interpolate_gather_bwd(idx.data_ptr(), dist.data_ptr(), grad_out.data_ptr(),
+                                                             dsrc.data_ptr(), Nq, ctx.n_src, K, C, _dtype_code(grad_out),
+                                                             work.data_ptr(), nbytes, st)
+            _lib.check(rc, "s3d_knn_interpolate_gather_bwd")
+            return dsrc, None, None
         dsrc = torch.empty((ctx.n_src, C), dtype=torch.float32, device=grad_out.device)
         with torch.cuda.device(grad_out.device):
             st = torch.cuda.current_stream().cuda_stream
@@ -117,13 +140,55 @@ class KNNMaxPool(Function):
         return dg.to(grad_out.dtype), None
 
 
+class _KNNMaxPoolSlots(Function):
+    """KNNMaxPool without the arg-max rows among its outputs: one byte per value is kept for the backward,
+    which gathers the gradient of every source row."""
+
+    @staticmethod
+    def forward(ctx, g, idx):
+        _check_feat("g", g)
+        g = g.contiguous()
+        Nq, K = idx.shape
+        C = g.shape[1]
+        out = torch.empty((Nq, C), dtype=g.dtype, device=g.device)
+        slot = torch.empty((Nq, C), dtype=torch.uint8, device=g.device)
+        with torch.cuda.device(g.device):
+            st = torch.cuda.current_stream().cuda_stream
+            rc = _lib.lib.s3d_knn_maxpool_slots_fwd(idx.data_ptr(), g.data_ptr(), out.data_ptr(), slot.data_ptr(),
+                                                    Nq, K, C, _dtype_code(g), st)
+        _lib.check(rc, "s3d_knn_maxpool_slots_fwd")
+        ctx.save_for_backward(idx, slot)
+        ctx.n_src = g.shape[0]
+        return out
+
+    @staticmethod
+    def backward(ctx, grad_out):
+        idx, slot = ctx.saved_tensors
+        Nq, K = idx.shape
+        C = grad_out.shape[1]
+        grad_out = grad_out.contiguous()
+        if grad_out.data_ptr() % 16:
+            grad_out = grad_out.clone()
+        dg = torch.empty((ctx.n_src, C), dtype=grad_out.dtype, device=grad_out.device)
+        nbytes = _lib.lib.s3d_knn_gather_workspace_bytes(ctx.n_src, Nq, K)
+        work = torch.empty(nbytes, dtype=torch.uint8, device=grad_out.device)
+        with torch.cuda.device(grad_out.device):
+            st = torch.cuda.current_stream().cuda_stream
+            rc = _lib.lib.s3d_knn_maxpool_slots_bwd(idx.data_ptr(), slot.data_ptr(), grad_out.data_ptr(), dg.data_ptr(),
+                                                    Nq, ctx.n_src, K, C, _dtype_code(grad_out), work.data_ptr(), nbytes, st)
+        _lib.check(rc, "s3d_knn_maxpool_slots_bwd")
+        return dg, None
+
+
 def knn_max_pool(K, src_xyz, query_xyz, g, src_offset, query_offset):
     """``MaxPool1d(K)(g[idx].transpose(1, 2))`` of GridKNNDownsample.forward (:302-309) for
     ``g = linear(norm(src_feat))`` evaluated per source row (LayerNorm and the bias-free Linear
     act row by row, so they commute with the reference's gather)."""
     idx, _ = KNN.apply(K, src_xyz, query_xyz, src_offset, query_offset)
-    out, _ = KNNMaxPool.apply(g, idx)
-    return out
+    Nq, n_src = idx.shape[0], g.shape[0]
+    if 0 < Nq * K <= GATHER_MOST_PER_SOURCE * n_src and Nq * K < 2 ** 31:
+        return _KNNMaxPoolSlots.apply(g, idx)
+    return KNNMaxPool.apply(g, idx)[0]
 
 
 def query_knn_feature(K, src_xyz, query_xyz, src_feat, src_offset, query_offset, return_idx=False):

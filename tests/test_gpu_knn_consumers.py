@@ -131,3 +131,44 @@ def test_downsample_tail_matches_reference_vectors():
     out.backward(_dev(G["down.dout"]))
     np.testing.assert_allclose(out.detach().cpu().numpy(), G["down.out"], rtol=1e-4, atol=1e-5)
     np.testing.assert_allclose(feat.grad.cpu().numpy(), G["down.dfeat"], rtol=1e-3, atol=1e-4)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("K,C,n_src,Nq", [(3, 8, 1, 1), (3, 80, 4095, 1000), (3, 48, 4097, 12_293), (16, 40, 300, 65),
+                                          (5, 320, 70, 129), (64, 16, 257, 64)])
+def test_gather_backwards_match_the_scatter(dtype, K, C, n_src, Nq):
+    """Gradient gathered per source row against the scatter form and fp64: sources without an entry,
+    ends of the scan's tiles, one query, lists longer than a warp, every K of the templates."""
+    from swin3d_b200.sparse_dl.knn import KNNInterpolate, KNNMaxPool, consumers
+    g = torch.Generator(device="cuda").manual_seed(K * Nq)
+    idx = torch.randint(0, n_src, (Nq, K), generator=g, device="cuda", dtype=torch.int32)
+    dist = torch.rand((Nq, K), generator=g, device="cuda")
+    feat = torch.randn((n_src, C), generator=g, device="cuda").to(dtype).requires_grad_()
+    dout = torch.randn((Nq, C), generator=g, device="cuda").to(dtype)
+    w = 1.0 / (dist + 1e-8)
+    w = (w / w.sum(1, keepdim=True)).double()
+    want = torch.zeros((n_src, C), dtype=torch.float64, device="cuda")
+    size = torch.zeros((n_src, C), dtype=torch.float64, device="cuda")
+    for i in range(K):
+        want.index_add_(0, idx[:, i].long(), w[:, i, None] * dout.double())
+        size.index_add_(0, idx[:, i].long(), w[:, i, None] * dout.double().abs())
+    # fp32 sums of n terms: n eps of the sum of magnitudes at most (n <= a few hundred), then one rounding to dtype
+    eps = 2.0 ** -24 if dtype == torch.float32 else 2.0 ** -11
+    n_max = int(torch.bincount(idx.flatten().long(), minlength=n_src).max()) + 8
+    bound = size * n_max * 2.0 ** -24 + want.abs() * eps + 2.0 ** -24
+    was = consumers.GATHER_MOST_PER_SOURCE
+    try:
+        for most in (0, 1 << 30):
+            consumers.GATHER_MOST_PER_SOURCE = most
+            (got,) = torch.autograd.grad(KNNInterpolate.apply(feat, idx, dist), [feat], dout)
+            assert ((got.double() - want).abs() <= bound).all()
+    finally:
+        consumers.GATHER_MOST_PER_SOURCE = was
+    out, arg = KNNMaxPool.apply(feat, idx)
+    (ref,) = torch.autograd.grad(out, [feat], dout)
+    out2 = consumers._KNNMaxPoolSlots.apply(feat, idx)
+    (got,) = torch.autograd.grad(out2, [feat], dout)
+    assert torch.equal(out, out2)
+    size = torch.zeros((n_src, C), dtype=torch.float64, device="cuda").scatter_add_(0, arg.long(), dout.double().abs())
+    if K <= n_src:                                    # a row listed twice by a query: the first position counts, as here
+        assert ((got.double() - ref.double()).abs() <= size * n_max * 2.0 ** -23 + 2 * ref.double().abs() * eps + 2.0 ** -24).all()
