@@ -230,6 +230,21 @@ int s3d_window_build_static(const int32_t *coords, const float *feats, int64_t N
                             int32_t *n2n, float *n_coords, int32_t *w_sizes, int32_t *w2n,
                             int64_t *counts_out, void *stream);
 
+/* The same grouping, synchronous, for voxels that are distinct and fill their bounding box of windows
+ * reasonably well (no sort: a dense grid of windows with a bit per cell).
+ *  xyz, rest: the first three and the other F - 3 signals of a voxel, rows xyz_stride / rest_stride floats
+ *  apart.  w2m int64[N]: exclusive sum of the squared window sizes.  counts_host[4] (host memory):
+ *  windows, attention pairs, largest window, flags: 1 = a coordinate outside the supported range,
+ *  2 = the box holds too many windows, 4 = repeated voxels; with a flag set the outputs are incomplete
+ *  and (2, 4) s3d_window_build does the job.
+ *  workspace: s3d_window_groups_workspace_bytes, 16-byte aligned device memory.
+ */
+int64_t s3d_window_groups_workspace_bytes(int64_t N, int ws);
+int s3d_window_groups(const int32_t *coords, const float *xyz, int xyz_stride, const float *rest, int rest_stride,
+                      int64_t N, int F, int stride, int ws, int shift, int32_t *n2n, float *n_coords,
+                      int32_t *w_sizes, int32_t *w2n, int64_t *w2m, int64_t *counts_host,
+                      void *workspace, int64_t workspace_bytes, void *stream);
+
 /* ---------------------------------------------------------------------------------------------
  * Brute-force KNN.  Replaces knn_cuda.knn_cuda (Swin3D/src/knn/knn_cuda_kernel.h:5-12,
  * Swin3D/src/knn/knn_api.cpp:4-6).

@@ -322,6 +322,54 @@ static bool use_tree(int K, int B, int64_t Ns, int64_t Nq)
     return knn_tree_supported(K, B, Ns, Nq) && (g_knn_path ? g_knn_path == 3 : !knn_warp_wanted(K, B, Ns, Nq));
 }
 
+// 32 bytes of pinned memory per calling thread, given back when the thread ends: the counts of the
+// synchronous window grouping arrive there.
+namespace {
+struct PinnedCounts {
+    int64_t *p = nullptr;
+    int64_t *get()
+    {
+        if (!p && cudaHostAlloc(reinterpret_cast<void **>(&p), 4 * sizeof(int64_t), cudaHostAllocPortable) != cudaSuccess) p = nullptr;
+        return p;
+    }
+    ~PinnedCounts() { if (p) cudaFreeHost(p); }
+};
+}  // namespace
+
+int64_t s3d_window_groups_workspace_bytes(int64_t N, int ws)
+{
+    if (N < 0 || N >= (int64_t)1 << 31 || ws < 1 || ws > 8) return 0;
+    return window_dense_workspace_bytes(N, ws);
+}
+
+int s3d_window_groups(const int32_t *coords, const float *xyz, int xyz_stride, const float *rest, int rest_stride,
+                      int64_t N, int F, int stride, int ws, int shift, int32_t *n2n, float *n_coords, int32_t *w_sizes,
+                      int32_t *w2n, int64_t *w2m, int64_t *counts_host, void *workspace, int64_t workspace_bytes,
+                      void *stream)
+{
+    if (N < 0 || stride < 1 || shift < 0 || F < 3 || F > 3 + 2 * 3) return S3D_ERR_BAD_ARG;
+    if (ws < 1 || ws > 8) return S3D_ERR_UNSUPPORTED;
+    if (N >= (int64_t)1 << 31) return S3D_ERR_UNSUPPORTED;
+    if (!counts_host || !workspace) return S3D_ERR_BAD_ARG;
+    if (N > 0 && (!coords || !xyz || (F > 3 && !rest) || !n2n || !n_coords || !w_sizes || !w2n || !w2m)) return S3D_ERR_BAD_ARG;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    static thread_local PinnedCounts pinned;
+    int64_t *host = pinned.get();
+    if (!host) return S3D_ERR_LAUNCH;
+    int64_t *counts = nullptr;
+    const int rc = window_dense_launch(coords, xyz, xyz_stride, rest, rest_stride, N, F, stride, ws, shift, n2n, n_coords,
+                                       w_sizes, w2n, w2m, &counts, workspace, workspace_bytes, st);
+    if (rc != S3D_OK) return rc;
+    cudaError_t e = cudaMemcpyAsync(host, counts, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) {
+        note_cuda_error(e);
+        return S3D_ERR_LAUNCH;
+    }
+    memcpy(counts_host, host, 4 * sizeof(int64_t));
+    return S3D_OK;
+}
+
 static int knn_impl(int K, const float *src, const float *query, const int32_t *src_offset,
                     const int32_t *query_offset, int B, int64_t Ns, int64_t Nq, bool root, int32_t *ret_idx,
                     float *ret_dist, void *workspace, int64_t workspace_bytes, void *stream)

@@ -18,6 +18,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "window_common.cuh"
 #include "window_kernels.cuh"
 
 namespace s3d {
@@ -29,31 +30,9 @@ constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
-constexpr int CELL_BITS = 9, W_BITS = 15, B_BITS = 10;
-constexpr int W_BIAS = 1 << (W_BITS - 1);
 constexpr int NPASS = 8;
 
-__device__ __forceinline__ int floor_div(int a, int b) { int q = a / b; return (a % b != 0 && ((a < 0) != (b < 0))) ? q - 1 : q; }
-
 // ---- keys ------------------------------------------------------------------------------------
-struct VoxelWindow {
-    int b, wx, wy, wz, cell;
-};
-
-__device__ __forceinline__ VoxelWindow voxel_window(const int32_t *__restrict__ coords, int64_t i, int stride, int ws, int shift)
-{
-    const int4 c = __ldg(reinterpret_cast<const int4 *>(coords) + i);  // b, x, y, z
-    const int wstride = ws * stride;
-    const int sx = c.y + shift * stride, sy = c.z + shift * stride, sz = c.w + shift * stride;
-    VoxelWindow v;
-    v.b = c.x;
-    v.wx = floor_div(sx, wstride); v.wy = floor_div(sy, wstride); v.wz = floor_div(sz, wstride);
-    const int cx = (sx - v.wx * wstride) / stride, cy = (sy - v.wy * wstride) / stride,
-              cz = (sz - v.wz * wstride) / stride;
-    v.cell = (cx * ws + cy) * ws + cz;
-    return v;
-}
-
 // range[0..3] = min of (batch, wx, wy, wz), range[4..7] = max; also flags coordinates outside the
 // supported range (batch < 2^10, |window index| < 2^14, cell id < 2^9)
 __global__ void wb_range_kernel(const int32_t *__restrict__ coords, int64_t N, int stride, int ws, int shift,
@@ -62,16 +41,14 @@ __global__ void wb_range_kernel(const int32_t *__restrict__ coords, int64_t N, i
     int lo[4] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX}, hi[4] = {INT_MIN, INT_MIN, INT_MIN, INT_MIN};
     bool bad = false;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        const VoxelWindow v = voxel_window(coords, i, stride, ws, shift);
+        const VoxelWindow v = voxel_window(coords, i, WindowGrid{stride, ws, shift});
         const int f[4] = {v.b, v.wx, v.wy, v.wz};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             lo[k] = min(lo[k], f[k]);
             hi[k] = max(hi[k], f[k]);
         }
-        const int bx = v.wx + W_BIAS, by = v.wy + W_BIAS, bz = v.wz + W_BIAS;
-        bad = bad || v.b < 0 || v.b >= (1 << B_BITS) || bx < 0 || bx >= (1 << W_BITS) || by < 0 ||
-              by >= (1 << W_BITS) || bz < 0 || bz >= (1 << W_BITS) || v.cell >= (1 << CELL_BITS);
+        bad = bad || !voxel_in_range(v);
     }
     // warp, then block, then one set of atomics per block
     __shared__ int s_lo[4], s_hi[4];
@@ -117,7 +94,7 @@ __global__ void wb_keys_kernel(const int32_t *__restrict__ coords, int64_t N, in
     }
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
-    const VoxelWindow v = voxel_window(coords, i, stride, ws, shift);
+    const VoxelWindow v = voxel_window(coords, i, WindowGrid{stride, ws, shift});
     uint64_t key = (uint64_t)(uint32_t)(v.b - range[0]) & ((1ull << B_BITS) - 1);
     key = (key << wbx) | ((uint64_t)(uint32_t)(v.wx - range[1]) & ((1ull << W_BITS) - 1));
     key = (key << wby) | ((uint64_t)(uint32_t)(v.wy - range[2]) & ((1ull << W_BITS) - 1));

@@ -23,7 +23,29 @@ def _check_window(coords, feats, ws, shift, stride=1):
     assert np.array_equal(wi.w2n.cpu().numpy(), ref[3])
     assert wi.num_pairs == int((ref[2].astype(np.int64) ** 2).sum())
     assert wi.max_window == int(ref[2].max())
+    w2 = ref[2].astype(np.int64) ** 2
+    assert np.array_equal(wi.w2m.cpu().numpy(), np.cumsum(w2) - w2)
     return wi
+
+
+@pytest.mark.parametrize("ws", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("kind", ["full", "sparse", "repeated", "line"])
+def test_window_build_every_window_size(ws, kind):
+    """Masks of 1 to 16 words, completely filled windows, and the inputs the dense grid hands to the sort:
+    windows scattered over a box far larger than their number, voxels that occur twice."""
+    rng = np.random.default_rng(ws)
+    if kind == "full":
+        pts = np.stack(np.meshgrid(*[np.arange(-9, 12)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    elif kind == "sparse":
+        pts = np.concatenate([rng.integers(0, 8000, size=(300, 3)), [[0, 0, 0], [8000, 8000, 8000]]])
+        pts = np.unique(pts, axis=0)
+    elif kind == "repeated":
+        pts = rng.integers(0, 9, size=(2500, 3))
+    else:                                              # a scan of 1024 windows: the edge of a scan tile
+        pts = np.stack([np.arange(1025 * ws), np.zeros(1025 * ws, int), np.zeros(1025 * ws, int)], 1)
+    pts = rng.permutation(pts)
+    coords = np.concatenate([rng.integers(0, 3, size=(len(pts), 1)) if kind == "sparse" else np.zeros((len(pts), 1), int), pts], 1)
+    _check_window(coords.astype(np.int32), rng.random((len(pts), 6), dtype=np.float32), ws, ws // 2)
 
 
 @pytest.mark.parametrize("ws,shift", [(5, 0), (5, 2), (7, 0), (7, 3)])
