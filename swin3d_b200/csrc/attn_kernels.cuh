@@ -56,4 +56,8 @@ int attn_tc_backward(const AttnArgs &a, cudaStream_t st);   // dtq/dtk/dtv zeroe
 bool attn_tc_bwd_small_supported(const AttnArgs &a);          // attn_tc_bwd_small.cu: windows <= 32 voxels
 int attn_tc_backward_small(const AttnArgs &a, cudaStream_t st);
 
+// fp32 backward, factorised (attn_f32_bwd.cu): head_dim 8 and 16, tables of at most 63 rows per dimension
+bool attn_f32_bwd_supported(const AttnArgs &a);
+int attn_f32_backward(const AttnArgs &a, cudaStream_t st);
+
 }  // namespace s3d

@@ -20,6 +20,10 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include <mutex>
+#include <vector>
+
+#include "attn_kernels.cuh"
 #include "common.cuh"
 
 namespace s3d {
@@ -282,6 +286,90 @@ __device__ __forceinline__ uint32_t perm_tile_mask_warp(const uint16_t *lut_d, i
     return __reduce_or_sync(0xffffffffu, m);
 }
 
+// 16-row tiles a tile pair can touch: index range of every dimension from the extrema of the coordinates
+// of its nq queries and nk keys (lane = voxel).  Warp-wide; every lane returns the mask.
+template <int D>
+__device__ __forceinline__ uint32_t item_tile_mask(const float (&cq)[D], const float (&ck)[D], int nq, int nk, const uint16_t *lut,
+                                                   const PermMeta &pm, const PairConsts &pc, int lane)
+{
+    uint32_t used = 0;
+    bool odd = false;           // a NaN or infinite coordinate: no range argument, use every tile
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+        odd = odd || (lane < nq && !(fabsf(cq[d]) < INFINITY)) || (lane < nk && !(fabsf(ck[d]) < INFINITY));
+        const int kq = float_order_key(cq[d]), kk = float_order_key(ck[d]);
+        const float qmn = float_from_order_key(__reduce_min_sync(0xffffffffu, lane < nq ? kq : 0x7fffffff));
+        const float qmx = float_from_order_key(__reduce_max_sync(0xffffffffu, lane < nq ? kq : (int)0x80000000));
+        const float kmn = float_from_order_key(__reduce_min_sync(0xffffffffu, lane < nk ? kk : 0x7fffffff));
+        const float kmx = float_from_order_key(__reduce_max_sync(0xffffffffu, lane < nk ? kk : (int)0x80000000));
+        const int lo = (int)crse_index_pc(qmn, kmx, pc.half[d], pc.clamp[d]);
+        const int hi = (int)crse_index_pc(qmx, kmn, pc.half[d], pc.clamp[d]);
+        used |= perm_tile_mask_warp(lut + d * pm.lut_stride, pm.n[d], lo, hi, lane);
+    }
+    return __any_sync(0xffffffffu, odd) ? 0xffffffffu : used;
+}
+
+// The windows of block blockIdx.x of gridDim.x: a contiguous range of equal cost, the cost of a window
+// being its number of 32 x 32 tile pairs.  Every block scans all window sizes (a few hundred KB from
+// L2), so the assignment is balanced to within one window, needs no global counter and is the same on
+// every run.  All NTA threads of the block call this; scratch: (NTA + 4) * 8 bytes of shared memory.
+template <int NTA>
+__device__ __forceinline__ void balanced_range(const int32_t *__restrict__ w_sizes, int64_t W, void *scratch, int64_t &w_begin,
+                                               int64_t &w_end)
+{
+    int64_t *s_seg = static_cast<int64_t *>(scratch);                  // [NTA + 1] segment sums, then their exclusive scan
+    int64_t *s_range = s_seg + NTA + 2;                                // [2] first window, one past the last
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int64_t per = (W + NTA - 1) / NTA;
+    const int64_t w0 = (int64_t)tid * per, w1 = w0 + per < W ? w0 + per : W;
+    auto cost = [&](int64_t w) {
+        const int64_t nt = (__ldg(w_sizes + w) + QT - 1) / QT;
+        return nt * nt;
+    };
+    int64_t sum = 0;
+    for (int64_t w = w0; w < w1; ++w) sum += cost(w);
+    s_seg[tid] = sum;
+    __syncthreads();
+    if (tid < 32) {                       // exclusive scan of the NTA segment sums by one warp
+        int64_t carry = 0;
+        for (int b0 = 0; b0 < NTA; b0 += 32) {
+            const int64_t v = s_seg[b0 + lane];
+            int64_t x = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            s_seg[b0 + lane] = carry + x - v;
+            carry += __shfl_sync(0xffffffffu, x, 31);
+        }
+        if (lane == 0) s_seg[NTA] = carry;
+    }
+    __syncthreads();
+    const int64_t total = s_seg[NTA];
+    // window index at which the cumulative cost reaches the target: first w with prefix(w) >= target
+    const int64_t lo_t = total * blockIdx.x / gridDim.x, hi_t = total * (blockIdx.x + 1) / gridDim.x;
+    const int64_t mine = s_seg[tid], next = tid + 1 < NTA ? s_seg[tid + 1] : total + 1;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int64_t target = k == 0 ? lo_t : hi_t;
+        if (target >= total) {
+            if (tid == 0) s_range[k] = W;
+        } else if (mine <= target && target < next && w0 < w1) {
+            int64_t acc = mine, w = w0;
+            for (; w < w1; ++w) {
+                if (acc >= target) break;
+                acc += cost(w);
+            }
+            s_range[k] = w;
+        }
+    }
+    __syncthreads();
+    w_begin = s_range[0];
+    w_end = s_range[1];
+    __syncthreads();
+}
+
 // Head modes of the tiled kernels.  A thread block always works on two "slots" packed as half2:
 //   HDM_PAIR8   head_dim 8 : slots = heads 2hp, 2hp+1, 8 channels each, one plane
 //   HDM_SINGLE16 head_dim 16: slots = the two 8-channel halves of head hp (partial scores are summed)
@@ -481,6 +569,28 @@ __host__ __device__ inline SmemLayout make_layout(int R, int n_rowq_arrays, int 
     L.off_misc = off; off += 1024 + WL_BYTES;
     L.total = off;
     return L;
+}
+
+// Lets a kernel use 227 KB of shared memory and returns the SM count of the current device; both are asked
+// of the runtime once per kernel and device.
+inline int kernel_setup(const void *kern, int &sms)
+{
+    struct Done { const void *kern; int dev, sms; };
+    static std::mutex m;
+    static std::vector<Done> done;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return S3D_ERR_LAUNCH;
+    std::lock_guard<std::mutex> lock(m);
+    for (const Done &d : done)
+        if (d.kern == kern && d.dev == dev) {
+            sms = d.sms;
+            return S3D_OK;
+        }
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    note_cuda_error(e);
+    if (e != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return S3D_ERR_LAUNCH;
+    done.push_back({kern, dev, sms});
+    return S3D_OK;
 }
 
 }  // namespace tc

@@ -167,63 +167,9 @@ attn_bwd_small_kernel(const SmallParams P, const PermMeta pm, const PairConsts p
         mbar_init_fence();
     }
     fill_perm_lut(s_lut, pm, tid, blockDim.x);
-    // ---- this block's windows: a contiguous range of equal cost --------------------------------------------------
-    // cost of a window = its number of tile pairs; every block scans all window sizes (a few hundred KB
-    // from L2) and takes the range whose cumulative cost falls into its share, so the assignment is
-    // balanced to within one window, needs no global counter and is the same on every run.
-    {
-        constexpr int NTA = (NW + 1) * 32;
-        int64_t *s_seg = reinterpret_cast<int64_t *>(smem + L.off_pq);     // [NTA + 1] segment sums, then their exclusive scan
-        int64_t *s_range = s_seg + NTA + 2;                                // [2] first window, one past the last
-        const int64_t per = (P.W + NTA - 1) / NTA;
-        const int64_t w0 = (int64_t)tid * per, w1 = w0 + per < P.W ? w0 + per : P.W;
-        int64_t sum = 0;
-        for (int64_t w = w0; w < w1; ++w) {
-            const int nt = (__ldg(P.w_sizes + w) + QT - 1) / QT;
-            sum += (int64_t)nt * nt;
-        }
-        s_seg[tid] = sum;
-        __syncthreads();
-        if (wid == 0) {                       // exclusive scan of the NTA segment sums by one warp
-            int64_t carry = 0;
-            for (int b0 = 0; b0 < NTA; b0 += 32) {
-                const int64_t v = s_seg[b0 + lane];
-                int64_t x = v;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
-                    if (lane >= o) x += y;
-                }
-                s_seg[b0 + lane] = carry + x - v;
-                carry += __shfl_sync(0xffffffffu, x, 31);
-            }
-            if (lane == 0) s_seg[NTA] = carry;
-        }
-        __syncthreads();
-        const int64_t total = s_seg[NTA];
-        // window index at which the cumulative cost reaches the target: first w with prefix(w) >= target
-        const int64_t lo_t = total * blockIdx.x / gridDim.x, hi_t = total * (blockIdx.x + 1) / gridDim.x;
-        const int64_t mine = s_seg[tid], next = tid + 1 < NTA ? s_seg[tid + 1] : total + 1;
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int64_t target = k == 0 ? lo_t : hi_t;
-            if (target >= total) {
-                if (tid == 0) s_range[k] = P.W;
-            } else if (mine <= target && target < next && w0 < w1) {
-                int64_t acc = mine, w = w0;
-                for (; w < w1; ++w) {
-                    if (acc >= target) break;
-                    const int nt = (__ldg(P.w_sizes + w) + QT - 1) / QT;
-                    acc += (int64_t)nt * nt;
-                }
-                s_range[k] = w;
-            }
-        }
-        __syncthreads();
-    }
-    const int64_t w_begin = reinterpret_cast<const int64_t *>(smem + L.off_pq)[(NW + 1) * 32 + 2];
-    const int64_t w_end = reinterpret_cast<const int64_t *>(smem + L.off_pq)[(NW + 1) * 32 + 3];
-    __syncthreads();
+    // this block's windows: a contiguous range of equal cost
+    int64_t w_begin, w_end;
+    balanced_range<(NW + 1) * 32>(P.w_sizes, P.W, smem + L.off_pq, w_begin, w_end);
 
     if (wid == NW) {
         // ================================ producer warp ================================================
@@ -298,24 +244,7 @@ attn_bwd_small_kernel(const SmallParams P, const PermMeta pm, const PairConsts p
                 gdo[0] = __ldg(gd); gdo[1] = __ldg(gd + 1);
                 go[0] = __ldg(gg); go[1] = __ldg(gg + 1);
             }
-            // tiles this item can touch: index range of every dimension from the coordinate extrema
-            uint32_t used = 0;
-            {
-                bool odd = false;           // a NaN or infinite coordinate: no range argument, use every tile
-#pragma unroll
-                for (int d = 0; d < D; ++d) {
-                    odd = odd || (lane < nq && !(fabsf(cq[d]) < INFINITY)) || (lane < nk && !(fabsf(ck[d]) < INFINITY));
-                    const int kq = float_order_key(cq[d]), kk = float_order_key(ck[d]);
-                    const float qmn = float_from_order_key(__reduce_min_sync(0xffffffffu, lane < nq ? kq : 0x7fffffff));
-                    const float qmx = float_from_order_key(__reduce_max_sync(0xffffffffu, lane < nq ? kq : (int)0x80000000));
-                    const float kmn = float_from_order_key(__reduce_min_sync(0xffffffffu, lane < nk ? kk : 0x7fffffff));
-                    const float kmx = float_from_order_key(__reduce_max_sync(0xffffffffu, lane < nk ? kk : (int)0x80000000));
-                    const int lo = (int)crse_index_pc(qmn, kmx, pc.half[d], pc.clamp[d]);
-                    const int hi = (int)crse_index_pc(qmx, kmn, pc.half[d], pc.clamp[d]);
-                    used |= perm_tile_mask_warp(s_lut + d * pm.lut_stride, pm.n[d], lo, hi, lane);
-                }
-                if (__any_sync(0xffffffffu, odd)) used = 0xffffffffu;
-            }
+            const uint32_t used = item_tile_mask<D>(cq, ck, nq, nk, s_lut, pm, pc, lane);
             // delta[slot] = sum_c dO . O over the eight channels of the slot
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -742,19 +671,11 @@ static int launch_small_m(const SmallParams &p, const BwdMirrors &mm, const Crse
     constexpr int NW = bwd_small_warps(D);
     const SmallSmem L = make_small_layout(pm.R, NW, pm.D * pm.lut_stride);
     auto kern = attn_bwd_small_kernel<D, NPU, NHU, HD16, MIRROR>;
-    static int sms_of[64] = {0};     // 0: this instantiation has not been set up on the device yet
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return S3D_ERR_LAUNCH;
-    if (sms_of[dev] == 0) {
-        int sms = 0;
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        note_cuda_error(e);
-        if (e != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
-            return S3D_ERR_LAUNCH;
-        sms_of[dev] = sms;
-    }
+    int sms = 0;
+    const int rc = kernel_setup(reinterpret_cast<const void *>(kern), sms);
+    if (rc != S3D_OK) return rc;
     const int hp = HD16 ? p.H : p.H / 2;
-    int gx = sms_of[dev] / hp;
+    int gx = sms / hp;
     if (gx > p.W) gx = (int)p.W;
     if (gx < 1) gx = 1;
     dim3 grid((unsigned)gx, (unsigned)hp);

@@ -230,6 +230,7 @@ static int attn_bwd_impl(const void *q, const void *k, const void *v, const void
         return S3D_ERR_BAD_ARG;
     if (!force_scalar() && attn_tc_bwd_supported(a)) return attn_tc_backward(a, st);
     if (n_mirrors) return S3D_ERR_UNSUPPORTED;
+    if (!force_scalar() && attn_f32_bwd_supported(a)) return attn_f32_backward(a, st);
     return attn_scalar_backward(a, st);
 }
 
