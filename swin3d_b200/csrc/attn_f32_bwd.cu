@@ -37,16 +37,34 @@ using tc::IDX_BITS;
 
 constexpr int STAGES = 2;
 constexpr int ES = 33;                                       // row stride of the pair planes
-constexpr int NDT = 3;                                       // 32-row table-gradient units per warp
 __host__ __device__ constexpr int warps_for(int D) { return D == 9 ? 15 : (D == 6 ? 11 : 7); }
+
+// How the warps share the last two kinds of products.  A step of the table gradients reads a voxel row per
+// lane, and every 32-row unit a warp holds reuses it: head_dim 8 gives the gradients to 3 * DTW warps
+// with up to NDT units each (8 registers a unit) and the hist.T products to the others at the same
+// time.  (All warps doing both in turn, one or two units each: 19 k shared-memory wavefronts per item,
+// the pipe 80 % busy, 3.39 instead of 2.72 ms for 115 k voxels, 6 heads.)  At head_dim 16 a unit is 16
+// registers: every warp takes its share of both, up to three units.
+template <int D, int HD>
+struct Split {
+    static constexpr int NW = warps_for(D);
+    static constexpr bool APART = HD == 8;
+    static constexpr int DTW = APART ? (D == 9 ? 3 : (D == 6 ? 2 : 1)) : NW / 3;   // gradient warps per table
+    static constexpr int NDT = APART ? (D == 9 ? 4 : (D == 6 ? 5 : 6)) : 3;        // 32-row units per warp
+    static constexpr int HT0 = APART ? 3 * DTW : 0;                                // first warp of the hist.T products
+    static constexpr int SG = (NW - HT0) / 2;                                      // warps per side of them
+};
+constexpr int row_stride(int hd) { return hd + 4; }          // lanes = voxels read 16-byte pieces without conflicts
 
 struct Smem {
     int R16, Rp;
     int off_pq, off_db, off_pk, off_pl, off_rows, off_c, off_pg, off_st, off_lut, off_map, off_misc, total;
 };
 
-__host__ __device__ inline Smem make_smem(int R, int nw, int hd, int lut_entries)
+template <int D, int HD>
+__host__ __device__ inline Smem make_smem(int R, int lut_entries)
 {
+    constexpr int nw = warps_for(D), hd = HD, rs = row_stride(HD);
     Smem L;
     L.R16 = (R + 15) / 16 * 16;
     L.Rp = L.R16 + 1;                                        // odd: lanes = keys write P_k without conflicts
@@ -56,9 +74,9 @@ __host__ __device__ inline Smem make_smem(int R, int nw, int hd, int lut_entries
     L.off_db = off; off += arr;                              // dB, later histV
     L.off_pk = off; off += (32 * L.Rp * 4 + 15) / 16 * 16;   // P_k, later histK
     // the pair planes; over them, once the histograms exist, the partial dQ and dK of the warps
-    const int planes = 4 * 32 * ES * 4, part = 2 * (nw / 2) * 32 * hd * 4;
+    const int planes = 4 * 32 * ES * 4, part = 2 * Split<D, HD>::SG * 32 * hd * 4;
     L.off_pl = off; off += planes > part ? planes : part;
-    L.off_rows = off; off += STAGES * 4 * 32 * hd * 4;       // Q, dO (query tile), K, V (key tile), per stage
+    L.off_rows = off; off += STAGES * 4 * 32 * rs * 4;       // Q, dO (query tile), K, V (key tile), per stage
     L.off_c = off; off += STAGES * 2 * 32 * 12 * 4;          // coordinates of both tiles, per stage
     L.off_pg = off; off += 3 * 32 * hd * 4;                  // dQ, dV, dK of the pair products
     L.off_st = off; off += nw * 16 * hd * 4;                 // a 16-row table tile per warp
@@ -186,11 +204,12 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
     constexpr int GEMM_WARP = D + NKW;           // dQ and dK pair products
     constexpr int DV_WARP = (D & 1) ? D + NKW - 1 : D + NKW + 1;
     static_assert(DV_WARP < NW && GEMM_WARP < NW, "not enough warps");
-    constexpr int SG = NW / 2;                   // warps per side of the hist.T products
+    using SP = Split<D, HD>;
+    constexpr int SG = SP::SG, NDT = SP::NDT, DTW = SP::DTW, RS = row_stride(HD);
     constexpr int KPW = (QT + NW - 1) / NW;      // keys per warp in the score phase
     constexpr int HP = HD / 2;
     extern __shared__ __align__(16) unsigned char smem[];
-    const Smem L = make_smem(pm.R, NW, HD, pm.D * pm.lut_stride);
+    const Smem L = make_smem<D, HD>(pm.R, pm.D * pm.lut_stride);
     float *s_pq = reinterpret_cast<float *>(smem + L.off_pq);
     float *s_db = reinterpret_cast<float *>(smem + L.off_db);
     float *s_pk = reinterpret_cast<float *>(smem + L.off_pk);
@@ -198,7 +217,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
     float *s_P = reinterpret_cast<float *>(smem + L.off_pl), *s_DS = s_P + 32 * ES;
     uint32_t *s_W0 = reinterpret_cast<uint32_t *>(s_DS + 32 * ES), *s_W1 = s_W0 + 32 * ES;
     float *s_part = s_P;                                                // [2][SG][32][HD]
-    float *s_rows = reinterpret_cast<float *>(smem + L.off_rows);       // [stage][Q,dO,K,V][32][HD]
+    float *s_rows = reinterpret_cast<float *>(smem + L.off_rows);       // [stage][Q,dO,K,V][32][RS]
     float *s_cs = reinterpret_cast<float *>(smem + L.off_c);            // [stage][query tile, key tile][32][12]
     float *s_pg = reinterpret_cast<float *>(smem + L.off_pg);           // [3][32][HD]
     uint16_t *s_lut = reinterpret_cast<uint16_t *>(smem + L.off_lut);
@@ -307,7 +326,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
                 g_f32_async_error = 1;
                 nq = nk = 0;                                  // tell the consumers to stop
             }
-            float *rq = s_rows + s * (4 * 32 * HD);
+            float *rq = s_rows + s * (4 * 32 * RS);
             float *cs = s_cs + s * 768;
 #pragma unroll
             for (int d = 0; d < D; ++d) {
@@ -323,7 +342,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
                 if (lane >= (a < 2 ? nq : nk)) {
 #pragma unroll
                     for (int i = 0; i < HD / 4; ++i)
-                        reinterpret_cast<float4 *>(rq + (a * 32 + lane) * HD)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        reinterpret_cast<float4 *>(rq + (a * 32 + lane) * RS)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
             if (lane == 0) {
                 s_n[s * 8] = nq;
@@ -338,13 +357,13 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
             __syncwarp();
             if (lane < nq) {
                 const int64_t off = (int64_t)rowq * HC + co;
-                bulk_copy_g2s(rq + lane * HD, P.q + off, HD * 4, s_full + s);
-                bulk_copy_g2s(rq + (32 + lane) * HD, P.dout + off, HD * 4, s_full + s);
+                bulk_copy_g2s(rq + lane * RS, P.q + off, HD * 4, s_full + s);
+                bulk_copy_g2s(rq + (32 + lane) * RS, P.dout + off, HD * 4, s_full + s);
             }
             if (lane < nk) {
                 const int64_t off = (int64_t)rowk * HC + co;
-                bulk_copy_g2s(rq + (64 + lane) * HD, P.k + off, HD * 4, s_full + s);
-                bulk_copy_g2s(rq + (96 + lane) * HD, P.v + off, HD * 4, s_full + s);
+                bulk_copy_g2s(rq + (64 + lane) * RS, P.k + off, HD * 4, s_full + s);
+                bulk_copy_g2s(rq + (96 + lane) * RS, P.v + off, HD * 4, s_full + s);
             }
             if (nq == 0) break;
             advance();
@@ -358,7 +377,8 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
     // 32-row units (gradients) are dealt round-robin inside a group
     const int tg = wid / TG, wsub = wid - tg * TG;
     const float *Tproj = tg == 0 ? P.tq : (tg == 1 ? P.tv : P.tk);
-    const int side = wid / SG, ws2 = wid - side * SG;         // hist.T: 0 = histQ.Tq, 1 = histK.Tk
+    const int dtg = wid / DTW, dsub = wid - dtg * DTW;        // table gradients: the same order of tables
+    const int side = wid < SP::HT0 ? 2 : (wid - SP::HT0) / SG, ws2 = (wid - SP::HT0) - side * SG;   // hist.T: 0 = histQ.Tq, 1 = histK.Tk
     float *st = reinterpret_cast<float *>(smem + L.off_st) + wid * (16 * HD);
     uint64_t dt_acc[NDT][HP];
 #pragma unroll
@@ -377,13 +397,13 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
         const bool add_q = s_n[s * 8 + 2] != 0, add_k = s_n[s * 8 + 3] != 0;
         const uint32_t used = (uint32_t)s_n[s * 8 + 4];
         if (nq == 0 || *s_fail) break;
-        const float *s_q = s_rows + s * (4 * 32 * HD), *s_do = s_q + 32 * HD, *s_k = s_do + 32 * HD, *s_v = s_k + 32 * HD;
+        const float *s_q = s_rows + s * (4 * 32 * RS), *s_do = s_q + 32 * RS, *s_k = s_do + 32 * RS, *s_v = s_k + 32 * RS;
         const float *s_c = s_cs + s * 768, *s_ck = s_c + 384;
         const int *s_rowq = s_rowi + s * 64, *s_rowk = s_rowq + 32;
         // ---- projections ------------------------------------------------------------------------------------
         if (tg < 3) {
             uint64_t x[HP];
-            load_row<HD>(x, (tg == 0 ? s_q : (tg == 1 ? s_do : s_k)) + lane * HD);
+            load_row<HD>(x, (tg == 0 ? s_q : (tg == 1 ? s_do : s_k)) + lane * RS);
             TableTile<HD> tile;
             int mt = next_used(wsub, TG, n_mt, used);
             if (mt < n_mt) tile.fetch(Tproj, HC, co, s_map, mt, lane);
@@ -409,8 +429,8 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
         // ---- scores: keys wid, wid + NW, ... ; lane = query ---------------------------------------------------
         {
             uint64_t q2[HP], g2[HP];
-            load_row<HD>(q2, s_q + lane * HD);
-            load_row<HD>(g2, s_do + lane * HD);
+            load_row<HD>(q2, s_q + lane * RS);
+            load_row<HD>(g2, s_do + lane * RS);
             float cx[D];
             tc::load_coords12<D>(s_c + lane * 12, cx);
             const float lse = s_lses[s * 32 + lane], del = s_dels[s * 32 + lane];
@@ -425,7 +445,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
                         float ck[D];
                         tc::load_coords12<D>(s_ck + kk * 12, ck);
                         const float *pk_row = s_pk + kk * Rp;
-                        float b0 = dot_row<HD>(q2, s_k + kk * HD), b1 = 0.f, b2 = dot_row<HD>(g2, s_v + kk * HD);
+                        float b0 = dot_row<HD>(q2, s_k + kk * RS), b1 = 0.f, b2 = dot_row<HD>(g2, s_v + kk * RS);
 #pragma unroll
                         for (int d = 0; d < D; ++d) {
                             const uint32_t idx = tc::crse_index_pc(cx[d], ck[d], pc.half[d], pc.clamp[d]);
@@ -517,39 +537,39 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
 #pragma unroll
             for (int i = 0; i < HP; ++i) acc[i] = 0ull;
 #pragma unroll 4
-            for (int kk = 0; kk < nk; ++kk) axpy_row<HD>(acc, s_DS[kk * ES + lane], s_k + kk * HD);      // dQ[q] = sum_k ds K[k]
+            for (int kk = 0; kk < nk; ++kk) axpy_row<HD>(acc, s_DS[kk * ES + lane], s_k + kk * RS);      // dQ[q] = sum_k ds K[k]
             store_row<HD>(s_pg + lane * HD, acc);
 #pragma unroll
             for (int i = 0; i < HP; ++i) acc[i] = 0ull;
 #pragma unroll 4
-            for (int qq = 0; qq < nq; ++qq) axpy_row<HD>(acc, s_DS[lane * ES + qq], s_q + qq * HD);      // dK[k] = sum_q ds Q[q]
+            for (int qq = 0; qq < nq; ++qq) axpy_row<HD>(acc, s_DS[lane * ES + qq], s_q + qq * RS);      // dK[k] = sum_q ds Q[q]
             store_row<HD>(s_pg + (64 + lane) * HD, acc);
         } else if (wid == DV_WARP) {
             uint64_t acc[HP];
 #pragma unroll
             for (int i = 0; i < HP; ++i) acc[i] = 0ull;
 #pragma unroll 4
-            for (int qq = 0; qq < nq; ++qq) axpy_row<HD>(acc, s_P[lane * ES + qq], s_do + qq * HD);      // dV[k] = sum_q p dO[q]
+            for (int qq = 0; qq < nq; ++qq) axpy_row<HD>(acc, s_P[lane * ES + qq], s_do + qq * RS);      // dV[k] = sum_q p dO[q]
             store_row<HD>(s_pg + (32 + lane) * HD, acc);
         }
         consumer_sync<NT>();
         // ---- table gradients: lane = row of a 32-row unit ---------------------------------------------------------
-        if (tg < 3) {
-            const float *hist = tg == 0 ? s_hq : (tg == 1 ? s_hv : s_hk);
-            const float *X = tg == 0 ? s_q : (tg == 1 ? s_do : s_k);
+        if (dtg < 3) {
+            const float *hist = dtg == 0 ? s_hq : (dtg == 1 ? s_hv : s_hk);
+            const float *X = dtg == 0 ? s_q : (dtg == 1 ? s_do : s_k);
             bool on[NDT];
             const float *hrow[NDT];
 #pragma unroll
             for (int u = 0; u < NDT; ++u) {
-                const int tile = 2 * (wsub + TG * u) + (lane >> 4);
+                const int tile = 2 * (dsub + DTW * u) + (lane >> 4);
                 on[u] = tile < n_mt && ((used >> tile) & 1u);
-                hrow[u] = hist + (on[u] ? (wsub + TG * u) * 32 + lane : 0) * QT;
+                hrow[u] = hist + (on[u] ? (dsub + DTW * u) * 32 + lane : 0) * QT;
             }
-            constexpr int STEP = HD == 8 ? 4 : 2;
+            constexpr int STEP = 2;
             for (int i = 0; i < QT; i += STEP) {
                 uint64_t x[STEP][HP];
 #pragma unroll
-                for (int j = 0; j < STEP; ++j) load_row<HD>(x[j], X + ((i + j + lane) & 31) * HD);
+                for (int j = 0; j < STEP; ++j) load_row<HD>(x[j], X + ((i + j + lane) & 31) * RS);
 #pragma unroll
                 for (int u = 0; u < NDT; ++u)
                     if (__any_sync(0xffffffffu, on[u])) {
@@ -625,11 +645,11 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
     }
 
     // ---- the table gradients of this block ---------------------------------------------------------------------------
-    if (tg < 3) {
-        float *dst = tg == 0 ? P.dtq : (tg == 1 ? P.dtv : P.dtk);
+    if (dtg < 3) {
+        float *dst = dtg == 0 ? P.dtq : (dtg == 1 ? P.dtv : P.dtk);
 #pragma unroll
         for (int u = 0; u < NDT; ++u) {
-            const int r = (wsub + TG * u) * 32 + lane;
+            const int r = (dsub + DTW * u) * 32 + lane;
             const int row = r < L.R16 ? s_map[r] : 0xffff;      // aliases go to the row they stand for
             if (row != 0xffff) {
                 float f[HD];
@@ -646,7 +666,7 @@ template <int D, int HD>
 static int launch(const Params &p, const CrseMeta &meta, const PermMeta &pm, cudaStream_t st)
 {
     constexpr int NW = warps_for(D);
-    const Smem L = make_smem(pm.R, NW, HD, pm.D * pm.lut_stride);
+    const Smem L = make_smem<D, HD>(pm.R, pm.D * pm.lut_stride);
     auto kern = attn_bwd_f32_kernel<D, HD>;
     int sms = 0;
     const int rc = tc::kernel_setup(reinterpret_cast<const void *>(kern), sms);
@@ -660,6 +680,14 @@ static int launch(const Params &p, const CrseMeta &meta, const PermMeta &pm, cud
     return le == cudaSuccess ? S3D_OK : S3D_ERR_LAUNCH;
 }
 
+template <int D, int HD>
+static bool fits(const PermMeta &pm)
+{
+    const int n_mt = (pm.R + 15) / 16;                       // the tile mask is one word
+    return n_mt <= 32 && (n_mt + 1) / 2 <= Split<D, HD>::NDT * Split<D, HD>::DTW &&
+           make_smem<D, HD>(pm.R, pm.D * pm.lut_stride).total <= 227 * 1024;
+}
+
 }  // namespace f32
 
 bool attn_f32_bwd_supported(const AttnArgs &a)
@@ -668,9 +696,12 @@ bool attn_f32_bwd_supported(const AttnArgs &a)
     for (int d = 0; d < a.meta.D; ++d)
         if (a.meta.L[d] >= (1 << tc::IDX_BITS)) return false;
     const tc::PermMeta pm = tc::make_perm_meta(a.meta);
-    const int nw = f32::warps_for(a.meta.D), n_mt = (pm.R + 15) / 16;
-    if (n_mt > 32 || (n_mt + 1) / 2 > f32::NDT * (nw / 3)) return false;      // the tile mask is one word; units per warp
-    return f32::make_smem(pm.R, nw, a.hd, pm.D * pm.lut_stride).total <= 227 * 1024;
+    switch (a.meta.D) {
+        case 3: return a.hd == 8 ? f32::fits<3, 8>(pm) : f32::fits<3, 16>(pm);
+        case 6: return a.hd == 8 ? f32::fits<6, 8>(pm) : f32::fits<6, 16>(pm);
+        case 9: return a.hd == 8 ? f32::fits<9, 8>(pm) : f32::fits<9, 16>(pm);
+        default: return false;
+    }
 }
 
 // dtq, dtk, dtv must be zero on entry (accumulated into).
