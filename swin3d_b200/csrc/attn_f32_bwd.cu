@@ -489,18 +489,23 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
             const uint16_t *lut = s_lut + d * pm.lut_stride;
             float *cell = s_hq + lane;
             const int hv = L.R16 * QT;                     // histV follows histQ
+            // software pipeline: the rows of this step are known; its cells, the rows of the next step and
+            // the pair entries after that are fetched together
+            auto row_of = [&](uint32_t x) { return (int)lut[(x >> sh) & ((1u << IDX_BITS) - 1u)] * QT; };
+            int r0 = row_of(wcol[0]), r1 = row_of(wcol[ES]);
+            uint32_t x0 = wcol[2 * ES], x1 = wcol[3 * ES];
             float p0 = pcol[0], d0 = dcol[0], p1 = pcol[ES], d1 = dcol[ES];
-            uint32_t x0 = wcol[0], x1 = wcol[ES];
             for (int kk = 0; kk < nk; kk += 2) {           // entries beyond the window are zero
-                const uint32_t i0 = lut[(x0 >> sh) & ((1u << IDX_BITS) - 1u)], i1 = lut[(x1 >> sh) & ((1u << IDX_BITS) - 1u)];
-                float *a0 = cell + i0 * QT, *a1 = cell + i1 * QT;
-                const bool second = kk + 1 < nk;
+                float *a0 = cell + r0, *a1 = cell + r1;
+                const bool second = kk + 1 < nk, same = r1 == r0;
                 const float q0 = a0[0], v0 = a0[hv], q1 = a1[0], v1 = a1[hv];
+                r0 = row_of(x0); r1 = row_of(x1);
                 const float cp0 = p0, cd0 = d0, cp1 = p1, cd1 = d1;
                 const int k2 = min(kk + 2, QT - 1) * ES, k3 = min(kk + 3, QT - 1) * ES;
-                p0 = pcol[k2]; d0 = dcol[k2]; x0 = wcol[k2];
-                p1 = pcol[k3]; d1 = dcol[k3]; x1 = wcol[k3];
-                const bool same = a1 == a0;
+                p0 = pcol[k2]; d0 = dcol[k2];
+                p1 = pcol[k3]; d1 = dcol[k3];
+                x0 = wcol[min(kk + 4, QT - 1) * ES];
+                x1 = wcol[min(kk + 5, QT - 1) * ES];
                 const float sq0 = q0 + cd0, sv0 = v0 + cp0;
                 const float sq1 = (same ? sq0 : q1) + cd1, sv1 = (same ? sv0 : v1) + cp1;
                 a0[0] = sq0; a0[hv] = sv0;
@@ -515,18 +520,21 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
                 const uint32_t *wrow = (lo ? s_W0 : s_W1) + lane * ES;
                 const uint16_t *lut = s_lut + d * pm.lut_stride;
                 float *cell = s_hk + lane;
+                auto row_of = [&](uint32_t x) { return (int)lut[(x >> sh) & ((1u << IDX_BITS) - 1u)] * QT; };
+                int r0 = row_of(wrow[0]), r1 = row_of(wrow[1]);
+                uint32_t x0 = wrow[2], x1 = wrow[3];
                 float d0 = drow[0], d1 = drow[1];
-                uint32_t x0 = wrow[0], x1 = wrow[1];
                 for (int qq = 0; qq < nq; qq += 2) {
-                    const uint32_t i0 = lut[(x0 >> sh) & ((1u << IDX_BITS) - 1u)], i1 = lut[(x1 >> sh) & ((1u << IDX_BITS) - 1u)];
-                    float *a0 = cell + i0 * QT, *a1 = cell + i1 * QT;
-                    const bool second = qq + 1 < nq;
+                    float *a0 = cell + r0, *a1 = cell + r1;
+                    const bool second = qq + 1 < nq, same = r1 == r0;
                     const float c0 = a0[0], c1 = a1[0];
+                    r0 = row_of(x0); r1 = row_of(x1);
                     const float cd0 = d0, cd1 = d1;
-                    const int q2 = min(qq + 2, QT - 1), q3 = min(qq + 3, QT - 1);
-                    d0 = drow[q2]; x0 = wrow[q2];
-                    d1 = drow[q3]; x1 = wrow[q3];
-                    const float s0 = c0 + cd0, s1 = (a1 == a0 ? s0 : c1) + cd1;
+                    d0 = drow[min(qq + 2, QT - 1)];
+                    d1 = drow[min(qq + 3, QT - 1)];
+                    x0 = wrow[min(qq + 4, QT - 1)];
+                    x1 = wrow[min(qq + 5, QT - 1)];
+                    const float s0 = c0 + cd0, s1 = (same ? s0 : c1) + cd1;
                     a0[0] = s0;
                     if (second) a1[0] = s1;
                 }
