@@ -187,13 +187,6 @@ struct TableTile {
     }
 };
 
-// Next used tile of a warp's share (first, first + step, ...); n_mt if there is none.
-__device__ __forceinline__ int next_used(int mt, int step, int n_mt, uint32_t used)
-{
-    while (mt < n_mt && !((used >> mt) & 1u)) mt += step;
-    return mt < n_mt ? mt : n_mt;
-}
-
 template <int D, int HD>
 __global__ void __launch_bounds__((warps_for(D) + 1) * 32, 1)
 attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
@@ -405,14 +398,15 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
             uint64_t x[HP];
             load_row<HD>(x, (tg == 0 ? s_q : (tg == 1 ? s_do : s_k)) + lane * RS);
             TableTile<HD> tile;
-            int mt = next_used(wsub, TG, n_mt, used);
-            if (mt < n_mt) tile.fetch(Tproj, HC, co, s_map, mt, lane);
-            while (mt < n_mt) {
+            tc::UsedTiles tiles(used, n_mt, wsub, TG);
+            int mt = tiles.next();
+            if (mt >= 0) tile.fetch(Tproj, HC, co, s_map, mt, lane);
+            while (mt >= 0) {
                 __syncwarp();
                 tile.put(st, lane);
                 __syncwarp();
-                const int nx = next_used(mt + TG, TG, n_mt, used);
-                if (nx < n_mt) tile.fetch(Tproj, HC, co, s_map, nx, lane);
+                const int nx = tiles.next();
+                if (nx >= 0) tile.fetch(Tproj, HC, co, s_map, nx, lane);
                 if (tg < 2) {
                     float *dst = (tg == 0 ? s_pq : s_db) + mt * 16 * QT + lane;
 #pragma unroll 4
@@ -598,14 +592,15 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
 #pragma unroll
             for (int i = 0; i < HP; ++i) acc[i] = 0ull;
             TableTile<HD> tile;
-            int mt = next_used(ws2, SG, n_mt, used);
-            if (mt < n_mt) tile.fetch(T, HC, co, s_map, mt, lane);
-            while (mt < n_mt) {
+            tc::UsedTiles tiles(used, n_mt, ws2, SG);
+            int mt = tiles.next();
+            if (mt >= 0) tile.fetch(T, HC, co, s_map, mt, lane);
+            while (mt >= 0) {
                 __syncwarp();
                 tile.put(st, lane);
                 __syncwarp();
-                const int nx = next_used(mt + SG, SG, n_mt, used);
-                if (nx < n_mt) tile.fetch(T, HC, co, s_map, nx, lane);
+                const int nx = tiles.next();
+                if (nx >= 0) tile.fetch(T, HC, co, s_map, nx, lane);
                 const float *h = hist + mt * 16 * QT + lane;
 #pragma unroll 4
                 for (int r = 0; r < 16; ++r) axpy_row<HD>(acc, h[r * QT], st + r * HD);

@@ -309,6 +309,25 @@ __device__ __forceinline__ uint32_t item_tile_mask(const float (&cq)[D], const f
     return __any_sync(0xffffffffu, odd) ? 0xffffffffu : used;
 }
 
+// The used tiles dealt to `parts` warps in turn: part p takes the p-th, (p + parts)-th, ... used tile, so the
+// shares differ by one tile at most whichever tiles an item uses.
+struct UsedTiles {
+    uint32_t m;
+    int parts;
+    __device__ __forceinline__ UsedTiles(uint32_t used, int n_mt, int part, int parts_) : m(n_mt < 32 ? used & ((1u << n_mt) - 1u) : used), parts(parts_)
+    {
+        for (int i = 0; i < part; ++i) m &= m - 1u;
+    }
+    // the next tile of this part, -1 when there is none
+    __device__ __forceinline__ int next()
+    {
+        if (!m) return -1;
+        const int t = __ffs(m) - 1;
+        for (int i = 0; i < parts; ++i) m &= m - 1u;
+        return t;
+    }
+};
+
 // The windows of block blockIdx.x of gridDim.x: a contiguous range of equal cost, the cost of a window
 // being its number of 32 x 32 tile pairs.  Every block scans all window sizes (a few hundred KB from
 // L2), so the assignment is balanced to within one window, needs no global counter and is the same on

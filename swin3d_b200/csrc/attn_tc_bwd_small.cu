@@ -385,10 +385,10 @@ attn_bwd_small_kernel(const SmallParams P, const PermMeta pm, const PairConsts p
         if (tg < 3 && S3D_KEEP(0)) {
             uint32_t bf[8][2];
             load_feat_bfrag(bf, tg == 0 ? s_q : (tg == 1 ? s_do : s_k), tg == 2 ? nk : nq, g, t);
-#pragma unroll
-            for (int i = 0; i < NPU; ++i) {
-                const int mt = wsub + TG * i;
-                if (mt < n_mt && ((used >> mt) & 1u)) {
+            UsedTiles tiles(used, n_mt, wsub, TG);
+#pragma unroll 1
+            for (int mt = tiles.next(); mt >= 0; mt = tiles.next()) {
+                {
                     const uint4 f = s_ta[(tg * n_mt + mt) * 32 + lane];
                     const uint32_t taf[2][2] = {{f.x, f.y}, {f.z, f.w}};
                     if (tg == 0) project_unit_b<true>(taf, bf, s_pq, mt, Rp, nq, g, t);
