@@ -477,70 +477,12 @@ attn_bwd_small_kernel(const SmallParams P, const PermMeta pm, const PairConsts p
         S3D_PHASE_MARK(3)
         // ---- histograms and pair GEMMs ------------------------------------------------------------------------
         if (wid < D) {
-            // histQ += ds, histV += p ; lanes = queries, two keys per step
-            if (S3D_KEEP(3)) {
-                const int d = wid;
-                const bool lo = d < 5;
-                const int sh = IDX_BITS * (lo ? d : d - 5);
-                const uint32_t *pcol = s_P + lane, *dcol = s_DS + lane, *wcol = (lo ? s_W0 : s_W1) + lane;
-                const uint16_t *lut = s_lut + d * pm.lut_stride;
-                uint32_t *cell = s_hq + mypos;
-                const int hv = L.R16 * QT;                 // histV follows histQ
-                uint32_t p0 = pcol[0], d0 = dcol[0], x0 = wcol[0];
-                uint32_t p1 = pcol[ES], d1 = dcol[ES], x1 = wcol[ES];
-                int kk = 0;
-                for (; kk + 1 < nk; kk += 2) {
-                    const uint32_t i0 = lut[(x0 >> sh) & ((1u << IDX_BITS) - 1u)], i1 = lut[(x1 >> sh) & ((1u << IDX_BITS) - 1u)];
-                    uint32_t *a0 = cell + i0 * QT, *a1 = cell + i1 * QT;
-                    const uint32_t q0 = a0[0], v0 = a0[hv], q1 = a1[0], v1 = a1[hv];
-                    const uint32_t cp0 = p0, cd0 = d0, cp1 = p1, cd1 = d1;
-                    const int k2 = min(kk + 2, QT - 1) * ES, k3 = min(kk + 3, QT - 1) * ES;
-                    p0 = pcol[k2]; d0 = dcol[k2]; x0 = wcol[k2];
-                    p1 = pcol[k3]; d1 = dcol[k3]; x1 = wcol[k3];
-                    const bool same = a1 == a0;
-                    const __half2 sq0 = __hadd2(u32_as_h2(q0), u32_as_h2(cd0));
-                    const __half2 sv0 = __hadd2(u32_as_h2(v0), u32_as_h2(cp0));
-                    const __half2 sq1 = __hadd2(same ? sq0 : u32_as_h2(q1), u32_as_h2(cd1));
-                    const __half2 sv1 = __hadd2(same ? sv0 : u32_as_h2(v1), u32_as_h2(cp1));
-                    a0[0] = h2_as_u32(sq0); a0[hv] = h2_as_u32(sv0);
-                    a1[0] = h2_as_u32(sq1); a1[hv] = h2_as_u32(sv1);
-                }
-                if (kk < nk) {
-                    const uint32_t i0 = lut[(x0 >> sh) & ((1u << IDX_BITS) - 1u)];
-                    uint32_t *a0 = cell + i0 * QT;
-                    a0[0] = h2_as_u32(__hadd2(u32_as_h2(a0[0]), u32_as_h2(d0)));
-                    a0[hv] = h2_as_u32(__hadd2(u32_as_h2(a0[hv]), u32_as_h2(p0)));
-                }
-            }
+            // histQ += ds, histV += p ; lanes = queries
+            if (S3D_KEEP(3)) hist_query_side(s_hq + mypos, L.R16 * QT, s_P, s_DS, s_W0, s_W1, s_lut, pm.lut_stride, wid, nk, lane);
         } else if (wid < D + NKW) {
-            // histK += ds ; lanes = keys, the planes are read column-wise, two queries per step
-            for (int d = 2 * (wid - D); d < 2 * (wid - D) + 2 && d < D && S3D_KEEP(7); ++d) {
-                const bool lo = d < 5;
-                const int sh = IDX_BITS * (lo ? d : d - 5);
-                const uint32_t *drow = s_DS + lane * ES, *wrow = (lo ? s_W0 : s_W1) + lane * ES;
-                const uint16_t *lut = s_lut + d * pm.lut_stride;
-                uint32_t *cell = s_hk + mypos;
-                uint32_t d0 = drow[0], x0 = wrow[0], d1 = drow[1], x1 = wrow[1];
-                int qq = 0;
-                for (; qq + 1 < nq; qq += 2) {
-                    const uint32_t i0 = lut[(x0 >> sh) & ((1u << IDX_BITS) - 1u)], i1 = lut[(x1 >> sh) & ((1u << IDX_BITS) - 1u)];
-                    uint32_t *a0 = cell + i0 * QT, *a1 = cell + i1 * QT;
-                    const uint32_t c0 = a0[0], c1 = a1[0];
-                    const uint32_t cd0 = d0, cd1 = d1;
-                    const int q2 = min(qq + 2, QT - 1), q3 = min(qq + 3, QT - 1);
-                    d0 = drow[q2]; x0 = wrow[q2];
-                    d1 = drow[q3]; x1 = wrow[q3];
-                    const __half2 s0 = __hadd2(u32_as_h2(c0), u32_as_h2(cd0));
-                    const __half2 s1 = __hadd2(a1 == a0 ? s0 : u32_as_h2(c1), u32_as_h2(cd1));
-                    a0[0] = h2_as_u32(s0);
-                    a1[0] = h2_as_u32(s1);
-                }
-                if (qq < nq) {
-                    const uint32_t i0 = lut[(x0 >> sh) & ((1u << IDX_BITS) - 1u)];
-                    uint32_t *a0 = cell + i0 * QT;
-                    a0[0] = h2_as_u32(__hadd2(u32_as_h2(a0[0]), u32_as_h2(d0)));
-                }
-            }
+            // histK += ds ; lanes = keys
+            for (int d = 2 * (wid - D); d < 2 * (wid - D) + 2 && d < D && S3D_KEEP(7); ++d)
+                hist_key_side(s_hk + mypos, s_DS, s_W0, s_W1, s_lut, pm.lut_stride, d, nq, lane);
         }
         if (wid == GEMM_WARP || wid == DV_WARP) {
             float pg[2][2][4];

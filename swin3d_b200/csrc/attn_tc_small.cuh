@@ -8,6 +8,34 @@ namespace tc {
 
 constexpr int ES = 33;   // entry-row stride of the [32][ES] pair array (16-byte entries)
 
+// Stores of a projection unit's accumulators (d0: rows g, d1: rows g + 8 of row tile mt; register j = voxels 4j + t).
+// Lane-major [row][qpos(voxel)]: 16-byte stores go out a quarter warp (rows g, g+1; t = 0..3) at a time; odd rows
+// write their upper half first so that the eight lanes of a quarter cover all 32 banks.
+__device__ __forceinline__ void store_lane_major(uint32_t *dst, const uint32_t (&d0)[8], const uint32_t (&d1)[8], int mt, int g, int t)
+{
+    uint32_t *r0 = dst + (mt * 16 + g) * QT + 4 * t;
+    const bool od = g & 1;
+    const int o0 = od ? 16 : 0, o1 = 16 - o0;
+    const uint4 a0 = make_uint4(d0[0], d0[2], d0[4], d0[6]), a1 = make_uint4(d0[1], d0[3], d0[5], d0[7]);
+    const uint4 b0 = make_uint4(d1[0], d1[2], d1[4], d1[6]), b1 = make_uint4(d1[1], d1[3], d1[5], d1[7]);
+    *reinterpret_cast<uint4 *>(r0 + o0) = od ? a1 : a0;
+    *reinterpret_cast<uint4 *>(r0 + o1) = od ? a0 : a1;
+    *reinterpret_cast<uint4 *>(r0 + 8 * QT + o0) = od ? b1 : b0;
+    *reinterpret_cast<uint4 *>(r0 + 8 * QT + o1) = od ? b0 : b1;
+}
+
+// Tile-major [voxel][Rp], the first nvalid voxels rounded up to a multiple of four.
+__device__ __forceinline__ void store_key_major(uint32_t *dst, const uint32_t (&d0)[8], const uint32_t (&d1)[8], int mt, int Rp, int nvalid, int g, int t)
+{
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        if (4 * j < nvalid) {
+            uint32_t *p = dst + (4 * j + t) * Rp + mt * 16 + g;
+            p[0] = d0[j];
+            p[8] = d1[j];
+        }
+}
+
 // One (table, 16-row tile) projection unit:  P^T[rows][(voxel, head)] = T . F^T  for the 32 voxels of
 // the window, written lane-major ([row][qpos(voxel)]) or tile-major ([voxel][Rp]).
 template <bool LANE_MAJOR>
@@ -25,27 +53,8 @@ __device__ __forceinline__ void project_unit(const uint32_t (&ta)[2][2], const _
             d1[j] = 0u;
         }
     }
-    if (LANE_MAJOR) {
-        // 16-byte stores go out a quarter warp (rows g, g+1 ; t = 0..3) at a time: odd rows write their
-        // upper half first so that the eight lanes of a quarter cover all 32 banks.
-        uint32_t *r0 = dst + (mt * 16 + g) * QT + 4 * t;
-        const bool od = g & 1;
-        const int o0 = od ? 16 : 0, o1 = 16 - o0;
-        const uint4 a0 = make_uint4(d0[0], d0[2], d0[4], d0[6]), a1 = make_uint4(d0[1], d0[3], d0[5], d0[7]);
-        const uint4 b0 = make_uint4(d1[0], d1[2], d1[4], d1[6]), b1 = make_uint4(d1[1], d1[3], d1[5], d1[7]);
-        *reinterpret_cast<uint4 *>(r0 + o0) = od ? a1 : a0;
-        *reinterpret_cast<uint4 *>(r0 + o1) = od ? a0 : a1;
-        *reinterpret_cast<uint4 *>(r0 + 8 * QT + o0) = od ? b1 : b0;
-        *reinterpret_cast<uint4 *>(r0 + 8 * QT + o1) = od ? b0 : b1;
-    } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (4 * j < nvalid) {
-                uint32_t *p = dst + (4 * j + t) * Rp + mt * 16 + g;
-                p[0] = d0[j];
-                p[8] = d1[j];
-            }
-    }
+    if (LANE_MAJOR) store_lane_major(dst, d0, d1, mt, g, t);
+    else store_key_major(dst, d0, d1, mt, Rp, nvalid, g, t);
 }
 
 // Block-diagonal B fragments of a staged feature array ([32 voxels][16 halves] = two slots of 8
@@ -78,25 +87,8 @@ __device__ __forceinline__ void project_unit_b(const uint32_t (&ta)[2][2], const
             d1[j] = 0u;
         }
     }
-    if (LANE_MAJOR) {
-        uint32_t *r0 = dst + (mt * 16 + g) * QT + 4 * t;
-        const bool od = g & 1;
-        const int o0 = od ? 16 : 0, o1 = 16 - o0;
-        const uint4 a0 = make_uint4(d0[0], d0[2], d0[4], d0[6]), a1 = make_uint4(d0[1], d0[3], d0[5], d0[7]);
-        const uint4 b0 = make_uint4(d1[0], d1[2], d1[4], d1[6]), b1 = make_uint4(d1[1], d1[3], d1[5], d1[7]);
-        *reinterpret_cast<uint4 *>(r0 + o0) = od ? a1 : a0;
-        *reinterpret_cast<uint4 *>(r0 + o1) = od ? a0 : a1;
-        *reinterpret_cast<uint4 *>(r0 + 8 * QT + o0) = od ? b1 : b0;
-        *reinterpret_cast<uint4 *>(r0 + 8 * QT + o1) = od ? b0 : b1;
-    } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (4 * j < nvalid) {
-                uint32_t *p = dst + (4 * j + t) * Rp + mt * 16 + g;
-                p[0] = d0[j];
-                p[8] = d1[j];
-            }
-    }
+    if (LANE_MAJOR) store_lane_major(dst, d0, d1, mt, g, t);
+    else store_key_major(dst, d0, d1, mt, Rp, nvalid, g, t);
 }
 
 // acc[head][m-tile] += A . B with A[m][kk] = field FIELD (0 = p, 1 = ds) of the pair entries and
@@ -270,16 +262,14 @@ __device__ __forceinline__ void dt_unit_b(float (&acc)[2][4], const uint32_t *hi
     }
 }
 
-// part[head][m-tile] += hist(16 rows of k-step ks) . T(16 rows)  for the 32 voxels (m) of the window.
-// The fragment an mma lane (g,t) needs (four rows, one 16-byte column chunk g) would make the four
-// t-lanes of a quarter warp hit the same banks; each lane therefore loads the conflict-free pattern
-// (lane L: rows L/8 + 4i, chunk L%8, i.e. four rows x 128 bytes per instruction) and the registers
-// are moved to their mma lane with shuffles.
-__device__ __forceinline__ void ht_unit(float (&part)[2][2][4], const uint32_t *hist, const uint32_t (&tb)[2][2], int ks, int g, int t)
+// The four histogram rows t + 4i of k-step ks, queries {g, g+8, g+16, g+24}, that an mma lane needs in the hist.T
+// products.  Loaded directly (one 16-byte column chunk g of four rows) they would make the four t-lanes of a
+// quarter warp hit the same banks; each lane therefore loads the conflict-free pattern (lane L: rows L/8 + 4i,
+// chunk L%8, i.e. four rows x 128 bytes per instruction) and shuffles move the registers to their mma lane.
+__device__ __forceinline__ void load_hist_rows(uint4 (&y)[4], const uint32_t *hist, int ks, int lane, int g, int t)
 {
-    const int lane = 4 * g + t, src = 8 * t + g;
+    const int src = 8 * t + g;
     const uint32_t *hp = hist + (ks * 16 + (lane >> 3)) * QT + 4 * (lane & 7);
-    uint4 y[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) y[i] = *reinterpret_cast<const uint4 *>(hp + 4 * i * QT);
 #pragma unroll
@@ -289,11 +279,98 @@ __device__ __forceinline__ void ht_unit(float (&part)[2][2][4], const uint32_t *
         y[i].z = __shfl_sync(0xffffffffu, y[i].z, src);
         y[i].w = __shfl_sync(0xffffffffu, y[i].w, src);
     }
+}
+
+// part[head][m-tile] += hist(16 rows of k-step ks) . T(16 rows)  for the 32 voxels (m) of the window.
+__device__ __forceinline__ void ht_unit(float (&part)[2][2][4], const uint32_t *hist, const uint32_t (&tb)[2][2], int ks, int g, int t)
+{
+    uint4 y[4];
+    load_hist_rows(y, hist, ks, 4 * g + t, g, t);
     // y[i] = row t + 4i, queries {g, g+8, g+16, g+24}
     mma_k16(part[0][0], pack_lo(y[0].x, y[1].x), pack_lo(y[0].y, y[1].y), pack_lo(y[2].x, y[3].x), pack_lo(y[2].y, y[3].y), tb[0][0], tb[0][1]);
     mma_k16(part[1][0], pack_hi(y[0].x, y[1].x), pack_hi(y[0].y, y[1].y), pack_hi(y[2].x, y[3].x), pack_hi(y[2].y, y[3].y), tb[1][0], tb[1][1]);
     mma_k16(part[0][1], pack_lo(y[0].z, y[1].z), pack_lo(y[0].w, y[1].w), pack_lo(y[2].z, y[3].z), pack_lo(y[2].w, y[3].w), tb[0][0], tb[0][1]);
     mma_k16(part[1][1], pack_hi(y[0].z, y[1].z), pack_hi(y[0].w, y[1].w), pack_hi(y[2].z, y[3].z), pack_hi(y[2].w, y[3].w), tb[1][0], tb[1][1]);
+}
+
+// Histograms of the single-sweep backward kernels.  The pair planes p, ds (half2), idx 0-4, idx 5-8 are
+// [key][query] with row stride ES; `cell` points at this lane's column.
+// Query side of dimension d (lanes = queries): histQ[row] += ds, histV[row] += p, histV lying hv words after
+// histQ.  Two keys per step, the next step's entries fetched before this step's stores.
+__device__ __forceinline__ void hist_query_side(uint32_t *cell, int hv, const uint32_t *s_P, const uint32_t *s_DS, const uint32_t *s_W0,
+                                                const uint32_t *s_W1, const uint16_t *s_lut, int lut_stride, int d, int nk, int lane)
+{
+    const bool lo = d < 5;
+    const int sh = IDX_BITS * (lo ? d : d - 5);
+    const uint32_t *pcol = s_P + lane, *dcol = s_DS + lane, *wcol = (lo ? s_W0 : s_W1) + lane;
+    const uint16_t *lut = s_lut + d * lut_stride;
+    uint32_t p0 = pcol[0], d0 = dcol[0], x0 = wcol[0];
+    uint32_t p1 = pcol[ES], d1 = dcol[ES], x1 = wcol[ES];
+    int kk = 0;
+    for (; kk + 1 < nk; kk += 2) {
+        const uint32_t i0 = lut[(x0 >> sh) & ((1u << IDX_BITS) - 1u)], i1 = lut[(x1 >> sh) & ((1u << IDX_BITS) - 1u)];
+        uint32_t *a0 = cell + i0 * QT, *a1 = cell + i1 * QT;
+        const uint32_t q0 = a0[0], v0 = a0[hv], q1 = a1[0], v1 = a1[hv];
+        const uint32_t cp0 = p0, cd0 = d0, cp1 = p1, cd1 = d1;
+        const int k2 = min(kk + 2, QT - 1) * ES, k3 = min(kk + 3, QT - 1) * ES;
+        p0 = pcol[k2]; d0 = dcol[k2]; x0 = wcol[k2];
+        p1 = pcol[k3]; d1 = dcol[k3]; x1 = wcol[k3];
+        const bool same = a1 == a0;
+        const __half2 sq0 = __hadd2(u32_as_h2(q0), u32_as_h2(cd0));
+        const __half2 sv0 = __hadd2(u32_as_h2(v0), u32_as_h2(cp0));
+        const __half2 sq1 = __hadd2(same ? sq0 : u32_as_h2(q1), u32_as_h2(cd1));
+        const __half2 sv1 = __hadd2(same ? sv0 : u32_as_h2(v1), u32_as_h2(cp1));
+        a0[0] = h2_as_u32(sq0); a0[hv] = h2_as_u32(sv0);
+        a1[0] = h2_as_u32(sq1); a1[hv] = h2_as_u32(sv1);
+    }
+    if (kk < nk) {
+        const uint32_t i0 = lut[(x0 >> sh) & ((1u << IDX_BITS) - 1u)];
+        uint32_t *a0 = cell + i0 * QT;
+        a0[0] = h2_as_u32(__hadd2(u32_as_h2(a0[0]), u32_as_h2(d0)));
+        a0[hv] = h2_as_u32(__hadd2(u32_as_h2(a0[hv]), u32_as_h2(p0)));
+    }
+}
+
+// Key side of dimension d (lanes = keys, the planes are read along their rows): histK[row] += ds.
+__device__ __forceinline__ void hist_key_side(uint32_t *cell, const uint32_t *s_DS, const uint32_t *s_W0, const uint32_t *s_W1,
+                                              const uint16_t *s_lut, int lut_stride, int d, int nq, int lane)
+{
+    const bool lo = d < 5;
+    const int sh = IDX_BITS * (lo ? d : d - 5);
+    const uint32_t *drow = s_DS + lane * ES, *wrow = (lo ? s_W0 : s_W1) + lane * ES;
+    const uint16_t *lut = s_lut + d * lut_stride;
+    uint32_t d0 = drow[0], x0 = wrow[0], d1 = drow[1], x1 = wrow[1];
+    int qq = 0;
+    for (; qq + 1 < nq; qq += 2) {
+        const uint32_t i0 = lut[(x0 >> sh) & ((1u << IDX_BITS) - 1u)], i1 = lut[(x1 >> sh) & ((1u << IDX_BITS) - 1u)];
+        uint32_t *a0 = cell + i0 * QT, *a1 = cell + i1 * QT;
+        const uint32_t c0 = a0[0], c1 = a1[0];
+        const uint32_t cd0 = d0, cd1 = d1;
+        const int q2 = min(qq + 2, QT - 1), q3 = min(qq + 3, QT - 1);
+        d0 = drow[q2]; x0 = wrow[q2];
+        d1 = drow[q3]; x1 = wrow[q3];
+        const __half2 s0 = __hadd2(u32_as_h2(c0), u32_as_h2(cd0));
+        const __half2 s1 = __hadd2(a1 == a0 ? s0 : u32_as_h2(c1), u32_as_h2(cd1));
+        a0[0] = h2_as_u32(s0);
+        a1[0] = h2_as_u32(s1);
+    }
+    if (qq < nq) {
+        const uint32_t i0 = lut[(x0 >> sh) & ((1u << IDX_BITS) - 1u)];
+        uint32_t *a0 = cell + i0 * QT;
+        a0[0] = h2_as_u32(__hadd2(u32_as_h2(a0[0]), u32_as_h2(d0)));
+    }
+}
+
+// Four fp16 channels of a result row: written, or added to what the same thread wrote before.
+__device__ __forceinline__ void add_store_h4(__half *p, float4 a, bool add)
+{
+    uint2 *d = reinterpret_cast<uint2 *>(p);
+    if (add) {
+        const uint2 old = *d;
+        const float2 lo = __half22float2(u32_as_h2(old.x)), hi = __half22float2(u32_as_h2(old.y));
+        a.x += lo.x; a.y += lo.y; a.z += hi.x; a.w += hi.y;
+    }
+    *d = make_uint2(h2_as_u32(__floats2half2_rn(a.x, a.y)), h2_as_u32(__floats2half2_rn(a.z, a.w)));
 }
 
 __device__ __forceinline__ void store_part(float *red, const float (&part)[2][2][4], int g, int t)

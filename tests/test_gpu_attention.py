@@ -310,6 +310,51 @@ def test_fp16_index_equal_to_L_alias_rows_and_determinism():
         assert rel_err(a[2][i], b[2][i]) < 1e-4
 
 
+def _scene_of_window_sizes(ws, sizes, seed=3):
+    """One window per entry of `sizes`, filled with that many voxels; normals all along +z but two windows
+    with mixed ones, so that items use few and many table row tiles."""
+    rng = np.random.default_rng(seed)
+    pts, nrm = [], []
+    cells = np.stack(np.meshgrid(*[np.arange(ws)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    for i, n in enumerate(sizes):
+        pts.append(cells[np.sort(rng.choice(len(cells), n, replace=False))] + [i * ws, 0, 0])
+        v = np.tile([[0, 0, 1]], (n, 1)).astype(np.float32)
+        if i % 3 == 1:
+            v[::2] = [1, 0, 0]
+            v[1::4] = [-0.9, 0, 0.1]                          # differences below 2: no index reaches its limit
+        nrm.append(v)
+    pts = np.concatenate(pts)
+    n = len(pts)
+    return S.Scene(np.concatenate([np.zeros((n, 1)), pts], 1).astype(np.int32), rng.random((n, 3), dtype=np.float32) * 0.999,
+                   rng.random((n, 3), dtype=np.float32), np.concatenate(nrm))
+
+
+@pytest.mark.parametrize("dtype,H,hd,ws,crse", [("float16", 2, 16, 7, "XYZ_RGB_NORM"), ("float16", 4, 16, 5, "XYZ_RGB"),
+                                                ("float16", 2, 16, 7, "XYZ"), ("float32", 3, 8, 5, "XYZ_RGB_NORM"),
+                                                ("float32", 1, 16, 7, "XYZ_RGB_NORM"), ("float32", 2, 16, 7, "XYZ_RGB"),
+                                                ("float32", 2, 8, 7, "XYZ"), ("float32", 1, 16, 5, "XYZ")])
+def test_backward_kernels_at_the_edges_of_their_tiles(dtype, H, hd, ws, crse):
+    """Windows of 1 voxel up to several tiles, each side of every multiple of the 32-voxel tile; the gradients
+    of a window of several tiles are sums over its tile pairs."""
+    from tests.gpu_helpers import cuda_fwd_bwd
+    sizes = [1, 2, 3, 15, 16, 17, 31, 32, 33, 63, 64, 65, 96, 97, ws ** 3]
+    p = make_problem(seed=91, ws=ws, H=H, hd=hd, crse=crse, scene=_scene_of_window_sizes(ws, sizes),
+                     round_fp16=dtype == "float16")
+    assert sorted(p.w_sizes.tolist()) == sorted(sizes)
+    tol = FP16_TOL if dtype == "float16" else FP32_TOL
+    o_ref, _, g_ref = oracle_fwd_bwd(p, np.float64)
+    out, _, grads = cuda_fwd_bwd(p, getattr(torch, dtype))
+    assert rel_err(out, o_ref) < tol
+    for name, a, b in zip("dq dk dv dtq dtk dtv".split(), grads, g_ref):
+        assert rel_err(a, b) < tol, name
+    # Row by row in fp32 only.  A row that every pair of a window hits (signals equal throughout: index L/2) has the
+    # gradient sum_q q_q sum_k ds_qk = 0 exactly, of terms that each carry a rounding error of up to
+    # eps * n * max|ds q|: with fp16 histograms (eps = 2^-11) that is of the size of the other rows' values.
+    if dtype == "float32":
+        for name, a, b in zip("dtq dtk dtv".split(), grads[3:], g_ref[3:]):
+            assert table_row_errors(a, b, H * hd, tol, 2e-2) == [], name
+
+
 @pytest.mark.parametrize("crse,H,ws,shift", [("XYZ_RGB_NORM", 5, 5, 2), ("XYZ_RGB", 3, 5, 0), ("XYZ", 2, 7, 3),
                                              ("XYZ_RGB_NORM", 4, 7, 0), ("XYZ_RGB_NORM", 10, 7, 3), ("XYZ_RGB", 6, 5, 2)])
 def test_fp16_head_dim_16_tensor_core_path(crse, H, ws, shift):
