@@ -73,6 +73,34 @@ __device__ __forceinline__ void bulk_copy_g2s(void *dst_smem, const void *src_gm
                  : "memory");
 }
 
+// 16 bytes global -> shared by the load/store unit, without a register in between; zeros where !valid (src is not read).
+// A row piece of 32 or 64 bytes is too small for the bulk copy engine: one bulk copy per row and array, 64 to 128 of
+// them per item, took the producer warp longer than the consumers' work on the smaller items.
+__device__ __forceinline__ void cp_async16(void *dst_smem, const void *src_gmem, bool valid)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst_smem)), "l"(src_gmem), "r"(valid ? 16 : 0) : "memory");
+}
+
+// One arrival on the barrier (counted in its initial count) once this thread's earlier cp_async16 have landed.
+__device__ __forceinline__ void mbar_arrive_cp_async(uint64_t *bar)
+{
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+// A warp fetches 32 rows of PIECES 16-byte pieces: row r (lane r holds its row number) from src + row * row_elems, to
+// dst + r * dst_elems; rows from n on become zeros.
+template <int PIECES, typename T>
+__device__ __forceinline__ void stage_rows(T *dst, int dst_elems, const T *src, int64_t row_elems, int row, int n, int lane)
+{
+    constexpr int PER = 16 / sizeof(T);
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+        const int c = lane + 32 * i, r = c / PIECES, e = c % PIECES * PER;
+        const int64_t from = __shfl_sync(0xffffffffu, row, r);
+        cp_async16(dst + r * dst_elems + e, src + from * row_elems + e, r < n);
+    }
+}
+
 // Barrier among the first `count` threads of the block (a multiple of 32), id 1; the producer warp,
 // which runs ahead, does not take part.
 template <int COUNT>

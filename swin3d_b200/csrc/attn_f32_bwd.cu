@@ -227,7 +227,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
 
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
-            mbar_init(s_full + s, 1);
+            mbar_init(s_full + s, 64);         // every producer lane: its stores, its copies
             mbar_init(s_empty + s, NW);
         }
         *s_fail = 0;
@@ -330,13 +330,6 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
             s_rowi[s * 64 + 32 + lane] = rowk;
             s_lses[s * 32 + lane] = ls;
             s_dels[s * 32 + lane] = de;
-#pragma unroll
-            for (int a = 0; a < 4; ++a)                       // rows beyond the tiles are zero
-                if (lane >= (a < 2 ? nq : nk)) {
-#pragma unroll
-                    for (int i = 0; i < HD / 4; ++i)
-                        reinterpret_cast<float4 *>(rq + (a * 32 + lane) * RS)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                }
             if (lane == 0) {
                 s_n[s * 8] = nq;
                 s_n[s * 8 + 1] = nk;
@@ -344,20 +337,12 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
                 s_n[s * 8 + 3] = ti > 0;
                 s_n[s * 8 + 4] = (int)used;
             }
-            async_proxy_fence();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_expect_tx(s_full + s, (unsigned)((nq + nk) * 2 * HD * 4));
-            __syncwarp();
-            if (lane < nq) {
-                const int64_t off = (int64_t)rowq * HC + co;
-                bulk_copy_g2s(rq + lane * RS, P.q + off, HD * 4, s_full + s);
-                bulk_copy_g2s(rq + (32 + lane) * RS, P.dout + off, HD * 4, s_full + s);
-            }
-            if (lane < nk) {
-                const int64_t off = (int64_t)rowk * HC + co;
-                bulk_copy_g2s(rq + (64 + lane) * RS, P.k + off, HD * 4, s_full + s);
-                bulk_copy_g2s(rq + (96 + lane) * RS, P.v + off, HD * 4, s_full + s);
-            }
+            mbar_arrive(s_full + s);
+            stage_rows<HD / 4>(rq, RS, P.q + co, HC, rowq, nq, lane);
+            stage_rows<HD / 4>(rq + 32 * RS, RS, P.dout + co, HC, rowq, nq, lane);
+            stage_rows<HD / 4>(rq + 64 * RS, RS, P.k + co, HC, rowk, nk, lane);
+            stage_rows<HD / 4>(rq + 96 * RS, RS, P.v + co, HC, rowk, nk, lane);
+            mbar_arrive_cp_async(s_full + s);
             if (nq == 0) break;
             advance();
         }

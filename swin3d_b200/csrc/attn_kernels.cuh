@@ -56,6 +56,8 @@ int attn_tc_backward(const AttnArgs &a, cudaStream_t st);   // dtq/dtk/dtv zeroe
 bool attn_tc_bwd_small_supported(const AttnArgs &a);          // attn_tc_bwd_small.cu: windows <= 32 voxels
 int attn_tc_backward_small(const AttnArgs &a, cudaStream_t st);
 
+bool attn_tc_fwd_pair16_supported(const AttnArgs &a);         // attn_tc_fwd_pair16.cu: head_dim 16, even head count
+int attn_tc_forward_pair16(const AttnArgs &a, cudaStream_t st);
 bool attn_tc_bwd_pair16_supported(const AttnArgs &a);         // attn_tc_bwd_pair16.cu: head_dim 16, even head count
 int attn_tc_backward_pair16(const AttnArgs &a, cudaStream_t st);
 

@@ -328,25 +328,26 @@ struct UsedTiles {
     }
 };
 
-// The windows of block blockIdx.x of gridDim.x: a contiguous range of equal cost, the cost of a window
-// being its number of 32 x 32 tile pairs.  Every block scans all window sizes (a few hundred KB from
-// L2), so the assignment is balanced to within one window, needs no global counter and is the same on
-// every run.  All NTA threads of the block call this; scratch: (NTA + 4) * 8 bytes of shared memory.
-template <int NTA>
-__device__ __forceinline__ void balanced_range(const int32_t *__restrict__ w_sizes, int64_t W, void *scratch, int64_t &w_begin,
-                                               int64_t &w_end)
+// The share of block blockIdx.x of gridDim.x: a contiguous range of equal cost, the cost of a window being its number of
+// 32 x 32 tile pairs.  Every block scans all window sizes (a few hundred KB from L2), so the assignment needs no global
+// counter and is the same on every run.  The range is [(w_begin, i_begin), (w_end, i_end)) in (window, query tile) units,
+// a query tile costing as many tile pairs as its window has tiles; with whole windows (BY_WINDOW) i_begin = i_end = 0.
+// All NTA threads of the block call this; scratch: (NTA + 6) * 8 bytes of shared memory.
+template <int NTA, bool BY_WINDOW>
+__device__ __forceinline__ void balanced_units(const int32_t *__restrict__ w_sizes, int64_t W, void *scratch, int64_t &w_begin,
+                                               int64_t &w_end, int &i_begin, int &i_end)
 {
     int64_t *s_seg = static_cast<int64_t *>(scratch);                  // [NTA + 1] segment sums, then their exclusive scan
-    int64_t *s_range = s_seg + NTA + 2;                                // [2] first window, one past the last
+    int64_t *s_range = s_seg + NTA + 2;                                // [4] window and tile of the first unit, of one past the last
     const int tid = threadIdx.x, lane = tid & 31;
     const int64_t per = (W + NTA - 1) / NTA;
     const int64_t w0 = (int64_t)tid * per, w1 = w0 + per < W ? w0 + per : W;
-    auto cost = [&](int64_t w) {
-        const int64_t nt = (__ldg(w_sizes + w) + QT - 1) / QT;
-        return nt * nt;
-    };
+    auto tiles = [&](int64_t w) { return (int64_t)((__ldg(w_sizes + w) + QT - 1) / QT); };
     int64_t sum = 0;
-    for (int64_t w = w0; w < w1; ++w) sum += cost(w);
+    for (int64_t w = w0; w < w1; ++w) {
+        const int64_t nt = tiles(w);
+        sum += nt * nt;
+    }
     s_seg[tid] = sum;
     __syncthreads();
     if (tid < 32) {                       // exclusive scan of the NTA segment sums by one warp
@@ -366,27 +367,42 @@ __device__ __forceinline__ void balanced_range(const int32_t *__restrict__ w_siz
     }
     __syncthreads();
     const int64_t total = s_seg[NTA];
-    // window index at which the cumulative cost reaches the target: first w with prefix(w) >= target
+    // the first unit (window) at which the cumulative cost reaches the target
     const int64_t lo_t = total * blockIdx.x / gridDim.x, hi_t = total * (blockIdx.x + 1) / gridDim.x;
     const int64_t mine = s_seg[tid], next = tid + 1 < NTA ? s_seg[tid + 1] : total + 1;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         const int64_t target = k == 0 ? lo_t : hi_t;
         if (target >= total) {
-            if (tid == 0) s_range[k] = W;
+            if (tid == 0) { s_range[2 * k] = W; s_range[2 * k + 1] = 0; }
         } else if (mine <= target && target < next && w0 < w1) {
-            int64_t acc = mine, w = w0;
-            for (; w < w1; ++w) {
-                if (acc >= target) break;
-                acc += cost(w);
+            int64_t acc = mine, w = w0, i = 0;
+            for (; w < w1 && acc < target; ++w) {
+                const int64_t nt = tiles(w);
+                if (!BY_WINDOW && acc + nt * nt > target) {
+                    i = (target - acc + nt - 1) / nt;
+                    if (i < nt) break;
+                    i = 0;
+                }
+                acc += nt * nt;
             }
-            s_range[k] = w;
+            s_range[2 * k] = w;
+            s_range[2 * k + 1] = i;
         }
     }
     __syncthreads();
     w_begin = s_range[0];
-    w_end = s_range[1];
+    i_begin = (int)s_range[1];
+    w_end = s_range[2];
+    i_end = (int)s_range[3];
     __syncthreads();
+}
+
+template <int NTA>
+__device__ __forceinline__ void balanced_range(const int32_t *__restrict__ w_sizes, int64_t W, void *scratch, int64_t &w_begin, int64_t &w_end)
+{
+    int i_begin, i_end;
+    balanced_units<NTA, true>(w_sizes, W, scratch, w_begin, w_end, i_begin, i_end);
 }
 
 // Head modes of the tiled kernels.  A thread block always works on two "slots" packed as half2:

@@ -2,11 +2,7 @@
 // size: the single-sweep tile-pair scheme of attn_tc_bwd_small.cu with two heads of 16 channels per block.
 //
 // The look-ups, histograms and pair planes are those of a head_dim-8 pair (half2 = two heads); only the
-// products see the 16 channels.  A product that contracts over channels runs as two k-steps: an mma lane t
-// holds channels 4t, 4t+1 in the first and 4t+2, 4t+3 in the second (any split serves as long as both
-// operands use it), so that its part of a row is one 8-byte load.  A product whose columns are channels
-// runs once for the even and once for the odd channels: lane g loads channels 2g, 2g+1 of the two rows
-// of a k pair with 4-byte loads and swaps halves, and an accumulator lane ends with channels 4t..4t+3.
+// products see the 16 channels (attn_tc_pair16.cuh).
 //
 // What does not fit beside 24 row tiles of projections (148 KB) stays outside shared memory: the table
 // operands are fetched per tile from L1/L2, one tile ahead, and the table gradients of a block (24 tiles x
@@ -19,6 +15,7 @@
 // Swin3D-L, 144 k voxels, 10 heads: 11.84 -> 5.78 ms.
 #include "attn_kernels.cuh"
 #include "attn_tc.cuh"
+#include "attn_tc_pair16.cuh"
 #include "attn_tc_small.cuh"
 #include "async_stage.cuh"
 
@@ -26,8 +23,6 @@ namespace s3d {
 namespace tc {
 
 constexpr int P16_STAGES = 2;
-constexpr int P16_RS = 40;                       // halves per staged voxel row: 32 + 8, so that 8 rows start in different banks
-__host__ __device__ constexpr int p16_warps(int D) { return D == 9 ? 15 : (D == 6 ? 11 : 7); }
 
 template <int D>
 struct P16Split {
@@ -84,107 +79,6 @@ struct P16Params {
 // Set when a bounded wait of this kernel ran out (it never should).
 __device__ int g_bwd_p16_async_error;
 
-__device__ __forceinline__ void mma_f32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
-{
-    mma_k16(d, a[0], a[1], a[2], a[3], b0, b1);
-}
-
-// Table rows of a 16-row tile as A operands of the projections: [slot][row g, g + 8], .x / .y = first / second k-step.
-struct P16TileA {
-    uint2 f[2][2];
-    __device__ __forceinline__ void fetch(const __half *T, int HC, int co, const uint16_t *map, int mt, int g, int t)
-    {
-        const int r0 = map[mt * 16 + g], r1 = map[mt * 16 + g + 8];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            f[h][0] = r0 != 0xffff ? __ldg(reinterpret_cast<const uint2 *>(T + (int64_t)r0 * HC + co + h * 16 + 4 * t)) : make_uint2(0, 0);
-            f[h][1] = r1 != 0xffff ? __ldg(reinterpret_cast<const uint2 *>(T + (int64_t)r1 * HC + co + h * 16 + 4 * t)) : make_uint2(0, 0);
-        }
-    }
-};
-
-// The same rows as B operands of the hist.T products (k = row in ht_krow order, n = channel): raw[slot][half][first, second
-// row of the pair] = channels 2g, 2g + 1.
-struct P16TileB {
-    uint32_t raw[2][2][2];
-    __device__ __forceinline__ void fetch(const __half *T, int HC, int co, const uint16_t *map, int ks, int g, int t)
-    {
-#pragma unroll
-        for (int half = 0; half < 2; ++half)
-#pragma unroll
-            for (int second = 0; second < 2; ++second) {
-                const int r = map[ks * 16 + ht_krow(t, half, second)];
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    raw[h][half][second] = r != 0xffff ? __ldg(reinterpret_cast<const uint32_t *>(T + (int64_t)r * HC + co + h * 16 + 2 * g)) : 0u;
-            }
-    }
-};
-
-// acc[slot][even / odd channels][m-tile] += A . rows with A from a [32][ES] plane of half2 pair entries: TRANSPOSED = false:
-// m = query, k = key (entry [k][m]); true: m = key, k = query (entry [m][k]).
-template <bool TRANSPOSED>
-__device__ __forceinline__ void p16_pair_gemm(float (&acc)[2][2][2][4], const uint32_t *e32, const __half *rows, int nk, int g, int t)
-{
-#pragma unroll
-    for (int ks = 0; ks < 2; ++ks) {
-        if (16 * ks < nk) {
-            uint32_t b[2][2][2];                               // [slot][parity][half]
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int kh = 0; kh < 2; ++kh) {
-                    const int ka = 16 * ks + 2 * t + 8 * kh;
-                    const uint32_t u = *reinterpret_cast<const uint32_t *>(rows + ka * P16_RS + h * 16 + 2 * g);
-                    const uint32_t w = *reinterpret_cast<const uint32_t *>(rows + (ka + 1) * P16_RS + h * 16 + 2 * g);
-                    b[h][0][kh] = pack_lo(u, w);
-                    b[h][1][kh] = pack_hi(u, w);
-                }
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                uint32_t fa[2][4];
-#pragma unroll
-                for (int kh = 0; kh < 2; ++kh)
-#pragma unroll
-                    for (int rr = 0; rr < 2; ++rr) {
-                        const int m = 16 * i + g + 8 * rr, ka = 16 * ks + 2 * t + 8 * kh;
-                        const uint32_t u = TRANSPOSED ? e32[m * ES + ka] : e32[ka * ES + m];
-                        const uint32_t w = TRANSPOSED ? e32[m * ES + ka + 1] : e32[(ka + 1) * ES + m];
-                        fa[0][2 * kh + rr] = pack_lo(u, w);
-                        fa[1][2 * kh + rr] = pack_hi(u, w);
-                    }
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int p = 0; p < 2; ++p) mma_f32(acc[h][p][i], fa[h], b[h][p][0], b[h][p][1]);
-            }
-        }
-    }
-}
-
-// Accumulators [slot][parity][m-tile] to a [32][32] array: lane (g, t) holds channels 4t..4t+3 of rows g, g + 8.
-__device__ __forceinline__ void p16_store(float *dst, const float (&acc)[2][2][2][4], int g, int t)
-{
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int rr = 0; rr < 2; ++rr)
-                *reinterpret_cast<float4 *>(dst + (16 * i + g + 8 * rr) * 32 + h * 16 + 4 * t) =
-                    make_float4(acc[h][0][i][2 * rr], acc[h][1][i][2 * rr], acc[h][0][i][2 * rr + 1], acc[h][1][i][2 * rr + 1]);
-}
-
-__device__ __forceinline__ void p16_zero(float (&acc)[2][2][2][4])
-{
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int p = 0; p < 2; ++p)
-#pragma unroll
-            for (int i = 0; i < 2; ++i) acc[h][p][i][0] = acc[h][p][i][1] = acc[h][p][i][2] = acc[h][p][i][3] = 0.f;
-}
-
 template <int D>
 __global__ void __launch_bounds__((p16_warps(D) + 1) * 32, 1)
 attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc)
@@ -226,7 +120,7 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
 
     if (tid == 0) {
         for (int s = 0; s < P16_STAGES; ++s) {
-            mbar_init(s_full + s, 1);
+            mbar_init(s_full + s, 64);         // every producer lane: its stores, its copies
             mbar_init(s_empty + s, NW);
         }
         *s_fail = 0;
@@ -343,13 +237,6 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
             s_lses[s * 64 + lane * 2 + 1] = ls1;
             s_dels[s * 64 + lane * 2] = de0;
             s_dels[s * 64 + lane * 2 + 1] = de1;
-#pragma unroll
-            for (int a = 0; a < 4; ++a)                   // rows beyond the tiles are zero
-                if (lane >= (a < 2 ? nq : nk)) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        *reinterpret_cast<uint4 *>(rq + a * ROWS + lane * RS + i * 8) = make_uint4(0, 0, 0, 0);
-                }
             if (lane == 0) {
                 s_n[s * 8] = nq;
                 s_n[s * 8 + 1] = nk;
@@ -357,20 +244,12 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
                 s_n[s * 8 + 3] = ti > 0;
                 s_n[s * 8 + 4] = (int)used;
             }
-            async_proxy_fence();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_expect_tx(s_full + s, (unsigned)((nq + nk) * 128));
-            __syncwarp();
-            if (lane < nq) {
-                const int64_t off = (int64_t)rowq * HC + co;
-                bulk_copy_g2s(rq + lane * RS, P.q + off, 64, s_full + s);
-                bulk_copy_g2s(rq + ROWS + lane * RS, P.dout + off, 64, s_full + s);
-            }
-            if (lane < nk) {
-                const int64_t off = (int64_t)rowk * HC + co;
-                bulk_copy_g2s(rq + 2 * ROWS + lane * RS, P.k + off, 64, s_full + s);
-                bulk_copy_g2s(rq + 3 * ROWS + lane * RS, P.v + off, 64, s_full + s);
-            }
+            mbar_arrive(s_full + s);
+            stage_rows<4>(rq, RS, P.q + co, HC, rowq, nq, lane);
+            stage_rows<4>(rq + ROWS, RS, P.dout + co, HC, rowq, nq, lane);
+            stage_rows<4>(rq + 2 * ROWS, RS, P.k + co, HC, rowk, nk, lane);
+            stage_rows<4>(rq + 3 * ROWS, RS, P.v + co, HC, rowk, nk, lane);
+            mbar_arrive_cp_async(s_full + s);
             if (nq == 0) break;
             advance();                                    // the next item's position-indexed loads fly during the wait above
         }
@@ -419,27 +298,15 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
             P16TileA tile;
             if (mt >= 0) tile.fetch(Tproj, HC, co, s_map, mt, g, t);
             const int nv = tg == 2 ? nk : nq;
-            uint2 bf[8];                                     // voxel 4j + g/2, slot g&1, channels 4t..4t+3
-            {
-                const __half *feat = (tg == 0 ? s_q : (tg == 1 ? s_do : s_k)) + (g >> 1) * RS + (g & 1) * 16 + 4 * t;
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    bf[j] = 4 * j < nv ? *reinterpret_cast<const uint2 *>(feat + 4 * j * RS) : make_uint2(0, 0);
-            }
+            uint2 bf[8];
+            p16_feat_frag(bf, tg == 0 ? s_q : (tg == 1 ? s_do : s_k), nv, g, t);
 #pragma unroll 1
             while (mt >= 0) {
                 const P16TileA cur = tile;
                 const int nx = tiles.next();
                 if (nx >= 0) tile.fetch(Tproj, HC, co, s_map, nx, g, t);
                 uint32_t d0[8], d1[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    d0[j] = d1[j] = 0u;
-                    if (4 * j < nv) {
-                        mma_k16_h(d0[j], d1[j], cur.f[0][0].x, cur.f[0][1].x, cur.f[1][0].x, cur.f[1][1].x, od ? 0u : bf[j].x, od ? bf[j].x : 0u);
-                        mma_k16_ha(d0[j], d1[j], cur.f[0][0].y, cur.f[0][1].y, cur.f[1][0].y, cur.f[1][1].y, od ? 0u : bf[j].y, od ? bf[j].y : 0u);
-                    }
-                }
+                p16_project(d0, d1, cur, bf, nv, od);
                 if (tg < 2) store_lane_major(tg == 0 ? s_pq : s_db, d0, d1, mt, g, t);
                 else store_key_major(s_pk, d0, d1, mt, Rp, nv, g, t);
                 mt = nx;
@@ -448,13 +315,8 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
         for (int u = wid; u < 32; u += NW) {
             const int a = u >> 4, mt = (u >> 3) & 1, j = u & 7;     // key rows 16mt.., query columns 4j..
             if (16 * mt < nk && 4 * j < nq) {
-                const __half *y = (a == 0 ? s_k : s_v) + (16 * mt + g) * RS + 4 * t;
-                const uint2 x = *reinterpret_cast<const uint2 *>((a == 0 ? s_q : s_do) + (4 * j + (g >> 1)) * RS + (g & 1) * 16 + 4 * t);
-                const uint2 a0 = *reinterpret_cast<const uint2 *>(y), a1 = *reinterpret_cast<const uint2 *>(y + 8 * RS);
-                const uint2 a2 = *reinterpret_cast<const uint2 *>(y + 16), a3 = *reinterpret_cast<const uint2 *>(y + 8 * RS + 16);
                 float c[4];
-                mma_k16_z(c, a0.x, a1.x, a2.x, a3.x, od ? 0u : x.x, od ? x.x : 0u);
-                mma_k16(c, a0.y, a1.y, a2.y, a3.y, od ? 0u : x.y, od ? x.y : 0u);
+                p16_dot_block(c, a == 0 ? s_k : s_v, 16 * mt, a == 0 ? s_q : s_do, 4 * j, g, t);
                 float *e0 = reinterpret_cast<float *>(s_s0 + (16 * mt + g) * ES + 4 * j + t) + 2 * a;
                 float *e1 = reinterpret_cast<float *>(s_s0 + (16 * mt + g + 8) * ES + 4 * j + t) + 2 * a;
                 *reinterpret_cast<float2 *>(e0) = make_float2(c[0], c[1]);
@@ -600,21 +462,7 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
                 const P16TileB cur = tile;
                 const int nx = tiles.next();
                 if (nx >= 0) tile.fetch(T, HC, co, s_map, nx, g, t);
-                uint4 y[4];
-                load_hist_rows(y, hist, ks, lane, g, t);       // y[i] = row t + 4i, queries {g, g+8, g+16, g+24}
-                const uint32_t a[2][2][4] = {{{pack_lo(y[0].x, y[1].x), pack_lo(y[0].y, y[1].y), pack_lo(y[2].x, y[3].x), pack_lo(y[2].y, y[3].y)},
-                                              {pack_lo(y[0].z, y[1].z), pack_lo(y[0].w, y[1].w), pack_lo(y[2].z, y[3].z), pack_lo(y[2].w, y[3].w)}},
-                                             {{pack_hi(y[0].x, y[1].x), pack_hi(y[0].y, y[1].y), pack_hi(y[2].x, y[3].x), pack_hi(y[2].y, y[3].y)},
-                                              {pack_hi(y[0].z, y[1].z), pack_hi(y[0].w, y[1].w), pack_hi(y[2].z, y[3].z), pack_hi(y[2].w, y[3].w)}}};
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int p = 0; p < 2; ++p) {
-                        const uint32_t b0 = p == 0 ? pack_lo(cur.raw[h][0][0], cur.raw[h][0][1]) : pack_hi(cur.raw[h][0][0], cur.raw[h][0][1]);
-                        const uint32_t b1 = p == 0 ? pack_lo(cur.raw[h][1][0], cur.raw[h][1][1]) : pack_hi(cur.raw[h][1][0], cur.raw[h][1][1]);
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) mma_f32(acc[h][p][i], a[h][i], b0, b1);
-                    }
+                p16_hist_t(acc, hist, cur, ks, lane, g, t);
                 ks = nx;
             }
             p16_store(s_part + (side * SG + ws2) * 1024, acc, g, t);

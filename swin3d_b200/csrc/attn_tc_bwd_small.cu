@@ -160,7 +160,7 @@ attn_bwd_small_kernel(const SmallParams P, const PermMeta pm, const PairConsts p
 
     if (tid == 0) {
         for (int s = 0; s < BS_STAGES; ++s) {
-            mbar_init(s_full + s, 1);
+            mbar_init(s_full + s, 64);         // every producer lane: its stores, its copies
             mbar_init(s_empty + s, NW);
         }
         *s_fail = 0;
@@ -275,12 +275,6 @@ attn_bwd_small_kernel(const SmallParams P, const PermMeta pm, const PairConsts p
             s_lses[s * 64 + lane * 2 + 1] = ls1;
             s_dels[s * 64 + lane * 2] = de0;
             s_dels[s * 64 + lane * 2 + 1] = de1;
-#pragma unroll
-            for (int a = 0; a < 4; ++a)                   // rows beyond the tiles are zero
-                if (lane >= (a < 2 ? nq : nk)) {
-                    *reinterpret_cast<uint4 *>(rq + a * 512 + lane * 16) = make_uint4(0, 0, 0, 0);
-                    *reinterpret_cast<uint4 *>(rq + a * 512 + lane * 16 + 8) = make_uint4(0, 0, 0, 0);
-                }
             if (lane == 0) {
                 s_n[s * 8] = nq;
                 s_n[s * 8 + 1] = nk;
@@ -288,20 +282,12 @@ attn_bwd_small_kernel(const SmallParams P, const PermMeta pm, const PairConsts p
                 s_n[s * 8 + 3] = ti > 0;
                 s_n[s * 8 + 4] = (int)used;
             }
-            async_proxy_fence();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_expect_tx(s_full + s, (unsigned)((nq + nk) * 64));
-            __syncwarp();
-            if (lane < nq) {
-                const int64_t off = (int64_t)rowq * HC + co;
-                bulk_copy_g2s(rq + lane * 16, P.q + off, 32, s_full + s);
-                bulk_copy_g2s(rq + 512 + lane * 16, P.dout + off, 32, s_full + s);
-            }
-            if (lane < nk) {
-                const int64_t off = (int64_t)rowk * HC + co;
-                bulk_copy_g2s(rq + 1024 + lane * 16, P.k + off, 32, s_full + s);
-                bulk_copy_g2s(rq + 1536 + lane * 16, P.v + off, 32, s_full + s);
-            }
+            mbar_arrive(s_full + s);
+            stage_rows<2>(rq, 16, P.q + co, HC, rowq, nq, lane);
+            stage_rows<2>(rq + 512, 16, P.dout + co, HC, rowq, nq, lane);
+            stage_rows<2>(rq + 1024, 16, P.k + co, HC, rowk, nk, lane);
+            stage_rows<2>(rq + 1536, 16, P.v + co, HC, rowk, nk, lane);
+            mbar_arrive_cp_async(s_full + s);
             if (nq == 0) break;
             advance();                                    // the next item's position-indexed loads fly during the wait above
         }

@@ -567,6 +567,7 @@ int attn_tc_forward(const AttnArgs &a0, cudaStream_t st)
     a.meta = tc::internal_meta(a0.meta);   // kernels work in the internal row numbering
     const int hdm = attn_tc_head_mode(a0);
     int skip_upto = 0;
+    if (hdm == tc::HDM_PAIR16 && attn_tc_fwd_pair16_supported(a0)) return attn_tc_forward_pair16(a0, st);
     // the single-tile kernel serves head pairs of 8 channels and single heads of 16
     if (hdm != tc::HDM_PAIR16 && attn_tc_fwd_small_supported(a0)) {
         // window_class: the caller's word that every window has at most QT voxels (1) or more (2); each

@@ -120,7 +120,7 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
 
     if (tid == 0) {
         for (int s = 0; s < FS_STAGES; ++s) {
-            mbar_init(s_full + s, 1);
+            mbar_init(s_full + s, 64);         // every producer lane: its stores, its copies
             mbar_init(s_empty + s, NW);
         }
         *s_fail = 0;
@@ -169,24 +169,12 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
 #pragma unroll
             for (int d = 0; d < D; ++d) cs[lane * 12 + d] = c[d];
             s_rowi[s * 32 + lane] = row;
-            if (lane >= n) {                              // rows beyond the window are zero
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    *reinterpret_cast<uint4 *>(rq + a * 512 + lane * 16) = make_uint4(0, 0, 0, 0);
-                    *reinterpret_cast<uint4 *>(rq + a * 512 + lane * 16 + 8) = make_uint4(0, 0, 0, 0);
-                }
-            }
             if (lane == 0) s_n[s] = n;
-            async_proxy_fence();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_expect_tx(s_full + s, (unsigned)(n * 96));
-            __syncwarp();
-            if (lane < n) {
-                const int64_t off = (int64_t)row * HC + co;
-                bulk_copy_g2s(rq + lane * 16, P.q + off, 32, s_full + s);
-                bulk_copy_g2s(rq + 512 + lane * 16, P.k + off, 32, s_full + s);
-                bulk_copy_g2s(rq + 1024 + lane * 16, P.v + off, 32, s_full + s);
-            }
+            mbar_arrive(s_full + s);
+            stage_rows<2>(rq, 16, P.q + co, HC, row, n, lane);
+            stage_rows<2>(rq + 512, 16, P.k + co, HC, row, n, lane);
+            stage_rows<2>(rq + 1024, 16, P.v + co, HC, row, n, lane);
+            mbar_arrive_cp_async(s_full + s);
             if (n == 0) break;
         }
         return;
