@@ -3,9 +3,9 @@
 //
 // Both point sets are put into Morton order of a per-scene grid by a counting sort (histogram, scan,
 // scatter).  32 consecutive sources are a leaf and 32 leaves a node, each with its bounding box.
-// A warp searches for 32 consecutive queries, which lie close together: the lanes test the boxes
-// of 32 nodes or leaves at a time against the box of the warp's queries, nearest first, and a leaf that
-// survives is offered to all 32 queries with one broadcast load per source.
+// A warp searches for 32 consecutive queries (K > 3: 16 or 8, several lanes each), which lie close together:
+// the lanes test the boxes of 32 nodes or leaves at a time against the box of the warp's queries, nearest
+// first, and a leaf that survives is offered to all its queries with broadcast loads.
 //
 // Why the results are the same.  (1) The K smallest distances of a query do not depend on the order
 // of the scan, and neither do their indices as long as no two candidates at or below the K-th distance
@@ -17,8 +17,9 @@
 // the history of its heap.  The search notices that (it keeps the smallest excluded distance) and puts
 // the query on a list; those queries are scanned again in index order with the literal heap.
 //
-// Bound: instruction issue of the leaf evaluation.  Measured (8 scenes x 200 k queries x 50 k sources,
-// K = 3; 4 x 30 k x 120 k, K = 16): see knn_launch_tree.
+// Bound: instruction issue of the leaf evaluation for K = 3, the merges of the lists and their latency for
+// K = 16.  Measured, whole search: 8 scenes x (200 k queries, 50 k sources), K = 3: 0.53 ms, the scan of knn.cu
+// 16.9; 4 x (30 k, 120 k), K = 16: 0.72 ms (the scan: 62).
 #include "knn_common.cuh"
 #include "knn_kernels.cuh"
 #include "scan.cuh"
@@ -319,12 +320,6 @@ struct TopK {
     __device__ __forceinline__ void merge8(float (&x)[8], int (&id)[8])
     {
         static_assert(KL == 8 || KL == 16, "a power of two");
-        auto order = [](float &a, float &b, int &ia, int &ib) {
-            const bool swap = b < a;
-            const float lo = fminf(a, b), hi = fmaxf(a, b);
-            const int il = swap ? ib : ia, ih = swap ? ia : ib;
-            a = lo; b = hi; ia = il; ib = ih;
-        };
         constexpr int net[19][2] = {{0, 1}, {2, 3}, {4, 5}, {6, 7}, {0, 2}, {1, 3}, {4, 6}, {5, 7}, {1, 2}, {5, 6},
                                     {0, 4}, {1, 5}, {2, 6}, {3, 7}, {2, 4}, {3, 5}, {1, 2}, {3, 4}, {5, 6}};
 #pragma unroll
@@ -334,6 +329,35 @@ struct TopK {
             order(d[KL - 1 - j], x[j], i[KL - 1 - j], id[j]);
             ex = fminf(ex, x[j]);
         }
+        sort_bitonic();
+    }
+    // the KL smallest of this lane's list and that of lane ^ h, in both lanes
+    __device__ __forceinline__ void merge_lane(int h)
+    {
+        float od[KL];
+        int oi[KL];
+#pragma unroll
+        for (int j = 0; j < KL; ++j) {
+            od[j] = __shfl_xor_sync(0xffffffffu, d[KL - 1 - j], h);
+            oi[j] = __shfl_xor_sync(0xffffffffu, i[KL - 1 - j], h);
+        }
+        ex = fminf(ex, __shfl_xor_sync(0xffffffffu, ex, h));
+#pragma unroll
+        for (int j = 0; j < KL; ++j) {
+            order(d[j], od[j], i[j], oi[j]);
+            ex = fminf(ex, od[j]);
+        }
+        sort_bitonic();
+    }
+    static __device__ __forceinline__ void order(float &a, float &b, int &ia, int &ib)
+    {
+        const bool swap = b < a;
+        const float lo = fminf(a, b), hi = fmaxf(a, b);
+        const int il = swap ? ib : ia, ih = swap ? ia : ib;
+        a = lo; b = hi; ia = il; ib = ih;
+    }
+    __device__ __forceinline__ void sort_bitonic()
+    {
 #pragma unroll
         for (int h = KL / 2; h > 0; h /= 2)
 #pragma unroll
@@ -354,7 +378,16 @@ struct TopK {
 // and when a lane has eight or more parked, all lanes merge eight each.
 constexpr int QUEUE = 16;
 
-template <int KL, bool ROOT>
+// Long lists are also shared: the SHARE lanes of a query each take their part of every leaf's sources and keep
+// their own list.  A lane's K-th distance is a bound of the query's, and so is the largest of the lanes'
+// ceil(K / SHARE)-th.  The lists are merged at the end.  A warp then has fewer queries, so a smaller box and
+// fewer leaves to look at, and there are more warps.  K = 16, whole search with SHARE = 1 / 2 / 4: 4 x (30 k
+// queries in 120 k sources) 940 / 719 / 855 us, 3 x (16 k in 60 k) 604 / 567 / 466, 8 x (6 k in 20 k) 291 / 225 /
+// 200, 40 k in 135 k 674 / 456 / 448, 3 k in 12 k 159 / 182 / 133: four lanes while two would leave the GPU
+// with fewer than 4096 warps.
+inline int search_share(int64_t Nq) { return Nq < 65536 ? 4 : 2; }
+
+template <int KL, int SHARE, bool ROOT>
 __global__ void __launch_bounds__(SEARCH_THREADS)
 tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, TreeBufs t,
                    int32_t *__restrict__ ret_idx, float *__restrict__ ret_dist)
@@ -362,16 +395,35 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
     constexpr bool PARK = KL >= 8;
     __shared__ float s_qd[PARK ? QUEUE : 1][PARK ? SEARCH_THREADS : 1];
     __shared__ int s_qi[PARK ? QUEUE : 1][PARK ? SEARCH_THREADS : 1];
-    const int64_t at = (int64_t)blockIdx.x * SEARCH_THREADS + threadIdx.x;
-    const int lane = threadIdx.x & 31;
-    if ((at & ~(int64_t)31) >= Nq) return;                   // the whole warp
+    constexpr int PER = LEAF / SHARE;
+    static_assert(PER % 8 == 0 && (SHARE == 1 || PARK), "a lane takes its sources eight at a time");
+    const int64_t at = ((int64_t)blockIdx.x * SEARCH_THREADS + threadIdx.x) / SHARE;
+    const int lane = threadIdx.x & 31, sub = threadIdx.x % SHARE;
+    if (at - lane / SHARE >= Nq) return;                     // the whole warp
     float4 q = make_float4(NAN, NAN, NAN, __int_as_float(-1));
     if (at < Nq) q = t.qry[at];
     const int g = __float_as_int(q.w);
     const int scene = g >= 0 ? knn_scene(g, qo, B) : -1;
     TopK<KL> best;
-    best.init(K);
+    best.init(sub == 0 ? K : KL);                            // the entries that are -1 come once
     int parked = 0;
+    float bound = KNN_FAR;                                   // of the query's K-th distance
+    auto tighten = [&]() {
+        bound = best.top();
+        if constexpr (SHARE > 1) {
+            float part = 0.f;
+            const int at_part = KL - K + (K + SHARE - 1) / SHARE - 1;
+#pragma unroll
+            for (int j = 0; j < KL; ++j)
+                if (j == at_part) part = best.d[j];
+#pragma unroll
+            for (int h = 1; h < SHARE; h *= 2) {
+                bound = fminf(bound, __shfl_xor_sync(0xffffffffu, bound, h));
+                part = fmaxf(part, __shfl_xor_sync(0xffffffffu, part, h));
+            }
+            bound = fminf(bound, part);
+        }
+    };
     // a query that is not finite has no distance below the heap's initial entry
     unsigned todo = __ballot_sync(0xffffffffu, scene >= 0 && finite3(q.x, q.y, q.z));
     while (todo) {
@@ -414,12 +466,13 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
                     parked = max(parked - 8, 0);
                     best.merge8(x, id);
                 }
+                tighten();
             }
         };
         auto visit = [&](int leaf) {
-            const float *p = points + leaf * (4 * LEAF);
+            const float *p = points + leaf * (4 * LEAF) + sub * PER;
 #pragma unroll 2
-            for (int j = 0; j < LEAF; j += 8) {
+            for (int j = 0; j < PER; j += 8) {
                 float d[8];
 #pragma unroll
                 for (int u = 0; u < 8; u += 4) {
@@ -430,7 +483,7 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
                     dist2x2(d[u + 2], d[u + 3], x.y, y.y, z.y, nx, ny, nz);
                 }
                 const float m = fminf(fminf(fminf(d[0], d[1]), fminf(d[2], d[3])), fminf(fminf(d[4], d[5]), fminf(d[6], d[7])));
-                if (!__any_sync(0xffffffffu, m < best.top())) {
+                if (!__any_sync(0xffffffffu, m < bound)) {
                     best.ex = fminf(best.ex, m);
                     continue;
                 }
@@ -441,10 +494,9 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
                     id[u] = v.x; id[u + 1] = v.y; id[u + 2] = v.z; id[u + 3] = v.w;
                 }
                 if constexpr (PARK) {
-                    const float top = best.top();
 #pragma unroll
                     for (int u = 0; u < 8; ++u) {
-                        if (d[u] < top) {
+                        if (d[u] < bound) {
                             s_qd[parked][threadIdx.x] = d[u];
                             s_qi[parked][threadIdx.x] = id[u];
                             ++parked;
@@ -456,9 +508,12 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
                 } else {
 #pragma unroll
                     for (int u = 0; u < 8; ++u) {
-                        const bool in = d[u] < best.top();
+                        const bool in = d[u] < bound;
                         if (!in) best.ex = fminf(best.ex, d[u]);
-                        if (__any_sync(0xffffffffu, in) && in) best.insert(d[u], id[u]);
+                        if (__any_sync(0xffffffffu, in) && in) {
+                            best.insert(d[u], id[u]);
+                            bound = best.top();
+                        }
                     }
                 }
             }
@@ -475,7 +530,7 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
         }
         // the nearest of the boxes held by the lanes that can still matter; -1 if there is none
         auto nearest = [&](float lb, bool &open) {
-            const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, mine ? __float_as_uint(best.top()) : 0u));
+            const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, mine ? __float_as_uint(bound) : 0u));
             const bool can = open && lb <= most;
             const uint32_t key = can ? __float_as_uint(lb) : 0xffffffffu;
             const uint32_t m = __reduce_min_sync(0xffffffffu, key);
@@ -507,32 +562,36 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
                     const float4 a = make_float4(__shfl_sync(0xffffffffu, lo.x, lf), __shfl_sync(0xffffffffu, lo.y, lf), __shfl_sync(0xffffffffu, lo.z, lf), 0.f);
                     const float4 c = make_float4(__shfl_sync(0xffffffffu, hi.x, lf), __shfl_sync(0xffffffffu, hi.y, lf), __shfl_sync(0xffffffffu, hi.z, lf), 0.f);
                     const float o[3] = {q.x, q.y, q.z};
-                    if (__any_sync(0xffffffffu, mine && box_dist(a, c, o, o) <= best.top())) visit((nb + nd) * 32 + lf);
+                    if (__any_sync(0xffffffffu, mine && box_dist(a, c, o, o) <= bound)) visit((nb + nd) * 32 + lf);
                 }
             }
         }
         drain();
     }
+    if constexpr (SHARE > 1)
+#pragma unroll
+        for (int h = 1; h < SHARE; h *= 2) best.merge_lane(h);
     if (g < 0) return;
     if (best.tied()) {
-        t.ties[atomicAdd(t.tie_count, 1)] = g;
+        if (sub == 0) t.ties[atomicAdd(t.tie_count, 1)] = g;
         return;
     }
+    const bool put_idx = sub == 0, put_dist = sub == SHARE - 1;
     const int64_t o = (int64_t)g * K;
     if (KL == 16 && K == 16 && !((reinterpret_cast<uintptr_t>(ret_idx) | reinterpret_cast<uintptr_t>(ret_dist)) & 15)) {
 #pragma unroll
         for (int j = 0; j < KL; j += 4) {
-            reinterpret_cast<int4 *>(ret_idx + o)[j / 4] = make_int4(best.i[j % KL], best.i[(j + 1) % KL], best.i[(j + 2) % KL], best.i[(j + 3) % KL]);
+            if (put_idx) reinterpret_cast<int4 *>(ret_idx + o)[j / 4] = make_int4(best.i[j % KL], best.i[(j + 1) % KL], best.i[(j + 2) % KL], best.i[(j + 3) % KL]);
             float4 d = make_float4(best.d[j % KL], best.d[(j + 1) % KL], best.d[(j + 2) % KL], best.d[(j + 3) % KL]);
             if (ROOT) d = make_float4(__fsqrt_rn(d.x), __fsqrt_rn(d.y), __fsqrt_rn(d.z), __fsqrt_rn(d.w));
-            reinterpret_cast<float4 *>(ret_dist + o)[j / 4] = d;
+            if (put_dist) reinterpret_cast<float4 *>(ret_dist + o)[j / 4] = d;
         }
     } else {
 #pragma unroll
         for (int j = 0; j < KL; ++j)
             if (j >= KL - K) {
-                ret_idx[o + j - (KL - K)] = best.i[j];
-                ret_dist[o + j - (KL - K)] = ROOT ? __fsqrt_rn(best.d[j]) : best.d[j];
+                if (put_idx) ret_idx[o + j - (KL - K)] = best.i[j];
+                if (put_dist) ret_dist[o + j - (KL - K)] = ROOT ? __fsqrt_rn(best.d[j]) : best.d[j];
             }
     }
 }
@@ -868,13 +927,16 @@ int knn_launch_tree(int K, const float *src, const float *query, const int32_t *
     scan_in_place(t.hist, t.tile, t.n_tiles, st);
     tree_sort_kernel<false><<<nb, KT_THREADS, 0, st>>>(src, query, so, qo, B, Ns, Nq, t);
     tree_boxes_kernel<<<(unsigned)(Ns / (LEAF * 32) + B), 1024, 0, st>>>(B, t);
-    const unsigned blocks = (unsigned)((Nq + SEARCH_THREADS - 1) / SEARCH_THREADS);
-#define S3D_KNN_SEARCH(KL)                                                                                          \
-    if (root) tree_search_kernel<KL, true><<<blocks, SEARCH_THREADS, 0, st>>>(K, qo, B, Nq, t, idx, dist);       \
-    else tree_search_kernel<KL, false><<<blocks, SEARCH_THREADS, 0, st>>>(K, qo, B, Nq, t, idx, dist)
-    if (K <= 3) { S3D_KNN_SEARCH(3); }
-    else if (K <= 8) { S3D_KNN_SEARCH(8); }
-    else { S3D_KNN_SEARCH(16); }
+    const int share = K <= 3 ? 1 : search_share(Nq);
+    const unsigned blocks = (unsigned)((Nq * share + SEARCH_THREADS - 1) / SEARCH_THREADS);
+#define S3D_KNN_SEARCH(KL, SHARE)                                                                                   \
+    if (root) tree_search_kernel<KL, SHARE, true><<<blocks, SEARCH_THREADS, 0, st>>>(K, qo, B, Nq, t, idx, dist);   \
+    else tree_search_kernel<KL, SHARE, false><<<blocks, SEARCH_THREADS, 0, st>>>(K, qo, B, Nq, t, idx, dist)
+    if (K <= 3) { S3D_KNN_SEARCH(3, 1); }
+    else if (K <= 8 && share == 2) { S3D_KNN_SEARCH(8, 2); }
+    else if (K <= 8) { S3D_KNN_SEARCH(8, 4); }
+    else if (share == 2) { S3D_KNN_SEARCH(16, 2); }
+    else { S3D_KNN_SEARCH(16, 4); }
 #undef S3D_KNN_SEARCH
     if (cudaGetLastError() != cudaSuccess) return S3D_ERR_LAUNCH;
     // tied queries: a block each while they are few, otherwise the thread-per-query scan; both kernels read

@@ -246,6 +246,27 @@ def test_knn_index_hands_many_ties_to_the_scan():
         _lib.lib.s3d_debug_knn_path(was)
 
 
+@pytest.mark.parametrize("n_query", [65_533, 65_536])
+@pytest.mark.parametrize("K", [4, 5, 8, 9, 16])
+def test_knn_index_lanes_of_a_query_agree_with_the_heap(K, n_query):
+    """The index search gives a query of K > 3 four lanes below 65536 queries and two from there on, each with
+    its own list: lists of fewer entries than the kernel's, scenes with fewer sources than K, and a part of
+    the queries that tie."""
+    from swin3d_b200 import _lib
+    src, qry = S.make_knn_scene(90, n_query, 1_500)
+    src = src.copy()
+    src[1400:1450] = src[:50]                                # equal distances for the queries near them
+    so, qo = [1_451, 1_458, 1_500], [n_query // 2, n_query // 2 + 7, n_query]
+    was = _lib.lib.s3d_debug_knn_path(3)
+    try:
+        idx, d2 = _knn_gpu(K, src, qry, so, qo)
+    finally:
+        _lib.lib.s3d_debug_knn_path(was)
+    ridx, rd2 = O.knn(K, src, qry, so, qo, fma_mode=2)
+    assert np.array_equal(d2.view(np.uint32), rd2.view(np.uint32))
+    assert np.array_equal(idx, ridx)
+
+
 def test_knn_function_returns_sqrt_distance():
     from swin3d_b200.sparse_dl.knn import KNN
     src, qry = S.make_knn_scene(9, 500, 400)
