@@ -65,14 +65,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity)
     return false;
 }
 
-// bytes: a multiple of 16; dst and src 16-byte aligned.
-__device__ __forceinline__ void bulk_copy_g2s(void *dst_smem, const void *src_gmem, unsigned bytes, uint64_t *bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_addr(dst_smem)), "l"(src_gmem), "r"(bytes), "r"(smem_addr(bar))
-                 : "memory");
-}
-
 // 16 bytes global -> shared by the load/store unit, without a register in between; zeros where !valid (src is not read).
 // A row piece of 32 or 64 bytes is too small for the bulk copy engine: one bulk copy per row and array, 64 to 128 of
 // them per item, took the producer warp longer than the consumers' work on the smaller items.

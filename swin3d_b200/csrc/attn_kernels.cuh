@@ -45,15 +45,15 @@ int crse_indices_dump_variant(const float *n_coords, const CrseMeta &meta, int f
 int crse_index_values(const float *cq, const float *ck, int64_t n, int L, int last, int variant, int32_t *out,
                       cudaStream_t st);
 
-// Tensor-core path (attn_tc_fwd.cu): fp16 storage, head_dim 8, even head count.
+// Tensor-core path (attn_tc_fwd.cu): fp16 storage, head_dim 8 with an even head count, or 16.
 bool attn_tc_supported(const AttnArgs &a);
 int attn_tc_forward(const AttnArgs &a, cudaStream_t st);
 int attn_tc_head_mode(const AttnArgs &a);                      // HDM_* of attn_tc.cuh for this call
-bool attn_tc_fwd_small_supported(const AttnArgs &a);          // attn_tc_fwd_small.cu: windows <= 32 voxels
+bool attn_tc_fwd_small_supported(const AttnArgs &a);          // attn_tc_fwd_small.cu: head_dim 8, or 16 with an odd head count
 int attn_tc_forward_small(const AttnArgs &a, cudaStream_t st);
 bool attn_tc_bwd_supported(const AttnArgs &a);
 int attn_tc_backward(const AttnArgs &a, cudaStream_t st);   // dtq/dtk/dtv zeroed by the caller
-bool attn_tc_bwd_small_supported(const AttnArgs &a);          // attn_tc_bwd_small.cu: windows <= 32 voxels
+bool attn_tc_bwd_small_supported(const AttnArgs &a);          // attn_tc_bwd_small.cu
 int attn_tc_backward_small(const AttnArgs &a, cudaStream_t st);
 
 bool attn_tc_fwd_pair16_supported(const AttnArgs &a);         // attn_tc_fwd_pair16.cu: head_dim 16, even head count

@@ -37,9 +37,6 @@ __device__ __forceinline__ void store_h2_mirrored(__half *base, const Mirrors &m
 }
 
 constexpr int QT = 32;        // queries per tile (= lanes)
-constexpr int KT = 16;        // keys per tile
-constexpr int NWARP = 8;
-constexpr int NTHREADS = NWARP * 32;
 constexpr int IDX_BITS = 6;   // cRSE indices are packed 5 per 32-bit word, 6 bits each
 
 __device__ __forceinline__ int qpos(int q) { return ((q & 7) << 2) | (q >> 3); }
@@ -332,17 +329,21 @@ struct UsedTiles {
 // 32 x 32 tile pairs.  Every block scans all window sizes (a few hundred KB from L2), so the assignment needs no global
 // counter and is the same on every run.  The range is [(w_begin, i_begin), (w_end, i_end)) in (window, query tile) units,
 // a query tile costing as many tile pairs as its window has tiles; with whole windows (BY_WINDOW) i_begin = i_end = 0.
+// Windows of fewer than n_min or more than n_max voxels cost nothing.
 // All NTA threads of the block call this; scratch: (NTA + 6) * 8 bytes of shared memory.
 template <int NTA, bool BY_WINDOW>
 __device__ __forceinline__ void balanced_units(const int32_t *__restrict__ w_sizes, int64_t W, void *scratch, int64_t &w_begin,
-                                               int64_t &w_end, int &i_begin, int &i_end)
+                                               int64_t &w_end, int &i_begin, int &i_end, int n_min = 1, int n_max = 0x7fffffff)
 {
     int64_t *s_seg = static_cast<int64_t *>(scratch);                  // [NTA + 1] segment sums, then their exclusive scan
     int64_t *s_range = s_seg + NTA + 2;                                // [4] window and tile of the first unit, of one past the last
     const int tid = threadIdx.x, lane = tid & 31;
     const int64_t per = (W + NTA - 1) / NTA;
     const int64_t w0 = (int64_t)tid * per, w1 = w0 + per < W ? w0 + per : W;
-    auto tiles = [&](int64_t w) { return (int64_t)((__ldg(w_sizes + w) + QT - 1) / QT); };
+    auto tiles = [&](int64_t w) {
+        const int n = __ldg(w_sizes + w);
+        return (int64_t)(n >= n_min && n <= n_max ? (n + QT - 1) / QT : 0);
+    };
     int64_t sum = 0;
     for (int64_t w = w0; w < w1; ++w) {
         const int64_t nt = tiles(w);
@@ -576,34 +577,6 @@ __device__ __forceinline__ bool next_work_item(const uint16_t *list, const int *
         dt = (int)(((int64_t)b - (c0 + dw)) % nb);
         if (dt < 0) dt += nb;
     }
-}
-
-// Shared-memory carve-up (byte offsets) for a table of R rows.
-struct SmemLayout {
-    int R16;      // rows rounded up to a multiple of 16
-    int Rp;       // row stride (words) of the per-key array, == 8 (mod 32)
-    int off_pq, off_hist, off_pk, off_s, off_idx, off_kv, off_kc, off_misc, total;
-};
-
-__host__ __device__ inline SmemLayout make_layout(int R, int n_rowq_arrays, int n_planes = 1, int n_warps = NWARP)
-{
-    const int kt = 2 * n_warps;                                  // keys per tile: two per warp
-    SmemLayout L;
-    L.R16 = (R + 15) / 16 * 16;
-    L.Rp = (L.R16 + 31) / 32 * 32 + 8;
-    int off = 0;
-    L.off_pq = off;   off += n_rowq_arrays * L.R16 * QT * 4;   // P_q (and dB in the backward)
-    L.off_hist = off; off += n_rowq_arrays * L.R16 * QT * 4;   // histograms
-    // the per-key array doubles as the cross-warp reduction buffer of the epilogue (2.25 KB per warp)
-    const int red = n_warps * (QT * 16 + QT * 2) * 4;
-    L.off_pk = off;   off += (kt * L.Rp * 4 > red) ? kt * L.Rp * 4 : red;
-    L.off_s = off;    off += kt * QT * 8;                      // float2 scores / half2 probabilities
-    L.off_idx = off;  off += kt * 2 * QT * 4;                  // packed cRSE indices
-    L.off_kv = off;   off += n_planes * 2 * kt * 16 * 2;       // key and value rows of the tile, per plane
-    L.off_kc = off;   off += kt * 12 * 4;                      // key coordinates, padded to 12
-    L.off_misc = off; off += 1024 + WL_BYTES;
-    L.total = off;
-    return L;
 }
 
 // Lets a kernel use 227 KB of shared memory and returns the SM count of the current device; both are asked

@@ -1,12 +1,15 @@
-// Forward of the cRSE window attention for windows of at most 32 voxels, tensor-core path (fp16).
+// Forward of the cRSE window attention, tensor-core path (fp16), windows of any size: two heads of 8 channels
+// per block, or one of 16 (an odd head count).  Even head counts of 16 channels: attn_tc_fwd_pair16.cu.
 //
-// The whole window is one 32 x 32 tile, so the softmax needs no running maximum across key tiles
-// and nothing is ever rescaled.  A block of D+1 warps (at least 8) serves one head pair (head_dim 8)
-// or one head (head_dim 16) and walks the windows x, x + gridDim.x, ...; per window:
-//   stage      Q, K, V rows of the head pair, the signal coordinates
+// A window of n voxels is cut into nt = ceil(n / 32) tiles of equal size.  A block of D+1 warps (at least 8) takes
+// query tiles (window, i) and runs over the key tiles j of their window: every tile pair is an independent
+// 32 x 32 problem with its own row maximum; a thread of the store phase keeps two output channels of one
+// query and merges the tile pairs' (maximum, sum, output) as they come.  Most windows of the first
+// stage have at most 32 voxels and are a single item, where nothing is merged.  Per item:
+//   stage      Q rows (query tile), K, V rows (key tile) of the head pair, the signal coordinates of both
 //   GEMM       P_q = Tq.Q^T (lane-major), P_k = Tk.K^T (key-major), S0 = K.Q^T     [tensor cores]
 //              the first half of the warps owns the Tq tiles, the second half the Tk tiles, so a
-//              warp builds the block-diagonal B fragments of its feature array once per window
+//              warp builds the block-diagonal B fragments of its feature array once per item
 //   scores     lane = query, the keys dealt to the warps: D indices, 2*D look-ups, score; the
 //              scores and the packed indices of a thread's (at most four) pairs stay in registers;
 //              exact row maxima through shared-memory atomics
@@ -15,10 +18,16 @@
 //   histogram  warp d owns signal dimension d (rows of different dimensions are disjoint):
 //              hist[row][q] += p, two keys per step, the next step's entries fetched before the
 //              stores of this one; warp D: O = P.V                                    [tensor cores]
-//   epilogue   O += hist.Tv (k-steps dealt to the warps) [tensor cores], reduce, normalise, store
-// The histogram reuses the shared memory of P_q, which is dead once the scores exist; 108 KB of
-// shared memory per block, two blocks per SM.
-// grid = (x, H/2) (head_dim 8) or (x, H) (head_dim 16).  Larger windows: attn_tc_fwd.cu.
+//   epilogue   O += hist.Tv (k-steps dealt to the warps) [tensor cores], reduce, merge, store
+// The histogram reuses the shared memory of P_q, which is dead once the scores exist, and P_q is projected
+// again for every key tile; about 110 KB of shared memory per block, two blocks per SM.
+// The blocks take contiguous ranges of (window, query tile) units of equal cost (tile pairs).
+// grid = (x, H/2) (head_dim 8) or (x, H) (head_dim 16).
+//
+// Bound: shared-memory wavefronts (65 % of the pipe's peak) and instruction issue (58 %), see profiles/.
+// Measured against the version for windows of at most 32 voxels (blocks took every gridDim.x-th window) plus a kernel of
+// one block per SM with an online softmax for the larger ones: 964 k voxels, 10 heads 8.38 -> 7.69 ms; 115 k
+// voxels, 6 heads 680 -> 559 us.
 #include "attn_kernels.cuh"
 #include "attn_tc.cuh"
 #include "attn_tc_small.cuh"
@@ -44,7 +53,7 @@ __device__ unsigned int g_ablate;      // bit i set: piece i of the kernel is sk
 #define S3D_PHASE_FLUSH(base)
 #endif
 
-constexpr int FS_STAGES = 2;      // windows staged ahead of the one being computed
+constexpr int FS_STAGES = 2;      // items staged ahead of the one being computed
 
 struct FwdSmallSmem {
     int R16, Rp;
@@ -62,7 +71,7 @@ __host__ __device__ inline FwdSmallSmem make_fwd_small_layout(int R, int nw)
     L.off_pk = off; off += pk > red ? pk : red;                              // P_k, later the reduction buffer
     L.off_e = off; off += 2 * 32 * ES * 8;                                   // pair entries, two planes
     L.off_rows = off; off += FS_STAGES * 3 * 32 * 16 * 2;                    // Q, K, V rows, per stage
-    L.off_c = off; off += FS_STAGES * 32 * 12 * 4;                           // signal coordinates, per stage
+    L.off_c = off; off += FS_STAGES * 2 * 32 * 12 * 4;                       // signal coordinates of both tiles, per stage
     L.off_misc = off; off += 1024;
     L.total = off;
     return L;
@@ -76,6 +85,7 @@ struct FwdSmallParams {
     const float *n_coords;
     int64_t W;
     int H;
+    int n_min, n_max;      // the window sizes of this call
     Mirrors m_out;
 };
 
@@ -83,11 +93,10 @@ struct FwdSmallParams {
 // s3d_debug_async_error().
 __device__ int g_fwd_small_async_error;
 
-// Block = NW consumer warps + one producer warp.  The producer walks the block's windows
-// (x, x + gridDim.x, ... of at most 32 voxels) ahead of the consumers: it finds the next window,
-// reads its row numbers and coordinates and has the copy engine bring the 32-byte Q, K, V pieces
-// of its voxels into the next stage of shared memory (cp.async.bulk, completion on the stage's
-// "full" mbarrier); the consumers hand a stage back through its "empty" mbarrier.
+// Block = NW consumer warps + one producer warp.  The producer walks the block's tile pairs ahead of the
+// consumers: it reads row numbers and coordinates and copies the 32-byte Q, K, V pieces of the voxels
+// into the next stage of shared memory (cp.async, completion on the stage's "full" mbarrier); the
+// consumers hand a stage back through its "empty" mbarrier.
 template <int D, int NW, int NPU /*projection units per warp*/, int NHU /*hist.T units per warp*/, bool HD16>
 __global__ void __launch_bounds__((NW + 1) * 32, 2)
 attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta meta, const PairConsts pc)
@@ -104,11 +113,11 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
     uint2 *s_elo = reinterpret_cast<uint2 *>(smem + L.off_e);        // [32][ES] (p, idx 0-4); S0 before
     uint2 *s_ehi = s_elo + 32 * ES;                                  // [32][ES] (idx 5-8, p)
     __half *s_rows = reinterpret_cast<__half *>(smem + L.off_rows);  // [stage][Q,K,V][32][16]
-    float *s_cs = reinterpret_cast<float *>(smem + L.off_c);         // [stage][32][12]
+    float *s_cs = reinterpret_cast<float *>(smem + L.off_c);         // [stage][query tile, key tile][32][12]
     float *s_max = reinterpret_cast<float *>(smem + L.off_misc);     // [32][2]
-    int *s_rowi = reinterpret_cast<int *>(s_max + 64);               // [stage][32]
-    int *s_n = s_rowi + FS_STAGES * 32;                              // [stage] voxels of the window, 0: no more windows
-    int *s_fail = s_n + FS_STAGES;
+    int *s_rowi = reinterpret_cast<int *>(s_max + 64);               // [stage][32] rows of the query tile
+    int *s_n = s_rowi + FS_STAGES * 32;                              // [stage][4]: nq, nk, first key tile, last key tile; nq = 0: no more items
+    int *s_fail = s_n + FS_STAGES * 4;
     uint64_t *s_full = reinterpret_cast<uint64_t *>(smem + L.off_misc + 768);   // [stage]
     uint64_t *s_empty = s_full + FS_STAGES;                                      // [stage]
     float *s_red = reinterpret_cast<float *>(smem + L.off_pk);       // [NW][32][16], P_k is dead by then
@@ -126,56 +135,98 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
         *s_fail = 0;
         mbar_init_fence();
     }
-    __syncthreads();
+    int64_t w_begin, w_end;
+    int i_begin, i_end;                          // first query tile of window w_begin, one past the last of window w_end
+    balanced_units<(NW + 1) * 32, false>(P.w_sizes, P.W, smem + L.off_pq, w_begin, w_end, i_begin, i_end, P.n_min, P.n_max);
 
     if (wid == NW) {
         // ================================ producer warp ================================================
-        int64_t w = (int64_t)blockIdx.x - gridDim.x;
+        int64_t w = w_begin - 1;
+        int n = 0, base = 0, nt = 0, ts = 0, ti = 0, tj = 0, ti_end = 0;
+        int n_nx = 0, base_nx = 0;
+        if (w_begin < P.W) {
+            n_nx = __ldg(P.w_sizes + w_begin);
+            base_nx = __ldg(P.w2n + w_begin);
+        }
+        bool have = false;
+        int nq = 0, nk = 0, rowq = 0, rowk = 0;
+        float cq[D], ck[D];
+        auto advance = [&]() {
+            if (have && tj + 1 < nt) {
+                ++tj;
+            } else if (have && ti + 1 < ti_end) {
+                ++ti;
+                tj = 0;
+            } else {
+                do {                              // the range may end inside window w_end, and begin inside w_begin
+                    ++w;
+                    have = w < w_end || (w == w_end && i_end > 0);
+                    if (have) {
+                        n = n_nx;
+                        base = base_nx;
+                        if (w + 1 < P.W) {
+                            n_nx = __ldg(P.w_sizes + w + 1);
+                            base_nx = __ldg(P.w2n + w + 1);
+                        }
+                        nt = n >= P.n_min && n <= P.n_max ? (n + QT - 1) / QT : 0;
+                        ts = nt > 0 ? (n + nt - 1) / nt : 0;
+                        ti = w == w_begin ? i_begin : 0;
+                        ti_end = w == w_end ? i_end : nt;
+                        tj = 0;
+                    }
+                } while (have && ti >= ti_end);
+            }
+            nq = have ? min(ts, n - ti * ts) : 0;
+            nk = have ? min(ts, n - tj * ts) : 0;
+            rowq = rowk = 0;
+#pragma unroll
+            for (int d = 0; d < D; ++d) cq[d] = ck[d] = 0.f;
+            if (lane < nq) {
+                const int pos = base + ti * ts + lane;
+                rowq = __ldg(P.n2n + pos);
+#pragma unroll
+                for (int d = 0; d < D; ++d) cq[d] = __ldg(P.n_coords + (int64_t)pos * D + d);
+            }
+            if (ti == tj) {                       // the only case of a window of one tile
+                rowk = rowq;
+#pragma unroll
+                for (int d = 0; d < D; ++d) ck[d] = cq[d];
+            } else if (lane < nk) {
+                const int pos = base + tj * ts + lane;
+                rowk = __ldg(P.n2n + pos);
+#pragma unroll
+                for (int d = 0; d < D; ++d) ck[d] = __ldg(P.n_coords + (int64_t)pos * D + d);
+            }
+        };
+        advance();
         for (int it = 0;; ++it) {
-            // next window of at most QT voxels among this block's windows, 32 candidates at a time
-            int n = 0;
-            for (;;) {
-                const int64_t cand = w + (int64_t)(lane + 1) * gridDim.x;
-                const int nn = cand < P.W ? __ldg(P.w_sizes + cand) : 0;
-                const unsigned ok = __ballot_sync(0xffffffffu, nn >= 1 && nn <= QT);
-                if (ok) {
-                    const int j = __ffs(ok) - 1;
-                    w += (int64_t)(j + 1) * gridDim.x;
-                    n = __shfl_sync(0xffffffffu, nn, j);
-                    break;
-                }
-                w += (int64_t)32 * gridDim.x;
-                if (w + gridDim.x >= P.W) break;         // n stays 0: no more windows
-            }
-            int row = 0;
-            float c[D];
-#pragma unroll
-            for (int d = 0; d < D; ++d) c[d] = 0.f;
-            if (n > 0) {
-                const int base = __ldg(P.w2n + w);
-                if (lane < n) {
-                    row = __ldg(P.n2n + base + lane);
-#pragma unroll
-                    for (int d = 0; d < D; ++d) c[d] = __ldg(P.n_coords + (int64_t)(base + lane) * D + d);
-                }
-            }
             const int s = it % FS_STAGES;
             if (it >= FS_STAGES && !mbar_wait(s_empty + s, ((it / FS_STAGES) - 1) & 1)) {
                 g_fwd_small_async_error = 1;
-                n = 0;                                    // tell the consumers to stop
+                have = false;                             // tell the consumers to stop
             }
+            if (!have) nq = nk = 0;
             __half *rq = s_rows + s * 1536;
-            float *cs = s_cs + s * 384;
+            float *cs = s_cs + s * 768;
 #pragma unroll
-            for (int d = 0; d < D; ++d) cs[lane * 12 + d] = c[d];
-            s_rowi[s * 32 + lane] = row;
-            if (lane == 0) s_n[s] = n;
+            for (int d = 0; d < D; ++d) {
+                cs[lane * 12 + d] = cq[d];
+                cs[384 + lane * 12 + d] = ck[d];
+            }
+            s_rowi[s * 32 + lane] = rowq;
+            if (lane == 0) {
+                s_n[s * 4] = nq;
+                s_n[s * 4 + 1] = nk;
+                s_n[s * 4 + 2] = tj == 0;
+                s_n[s * 4 + 3] = tj + 1 == nt;
+            }
             mbar_arrive(s_full + s);
-            stage_rows<2>(rq, 16, P.q + co, HC, row, n, lane);
-            stage_rows<2>(rq + 512, 16, P.k + co, HC, row, n, lane);
-            stage_rows<2>(rq + 1024, 16, P.v + co, HC, row, n, lane);
+            stage_rows<2>(rq, 16, P.q + co, HC, rowq, nq, lane);
+            stage_rows<2>(rq + 512, 16, P.k + co, HC, rowk, nk, lane);
+            stage_rows<2>(rq + 1024, 16, P.v + co, HC, rowk, nk, lane);
             mbar_arrive_cp_async(s_full + s);
-            if (n == 0) break;
+            if (!have) break;
+            advance();
         }
         return;
     }
@@ -219,6 +270,9 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
                 tb[i][h][half] = h2_as_u32(__halves2half2(lo, hi));
             }
     }
+    // the store phase: this thread's query and two channels, merged over the key tiles
+    float2 o_run = make_float2(0.f, 0.f);
+    float m_run = 0.f, l_run = 0.f;
     S3D_PHASE_DECL
 #ifdef S3D_PHASE_CLOCK
     const unsigned ablate = g_ablate;
@@ -229,32 +283,31 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
             *s_fail = 1;
             g_fwd_small_async_error = 2;
         }
-        consumer_sync<NT>();          // the previous window's epilogue is over; the flag is settled
+        consumer_sync<NT>();          // the previous item's epilogue is over; the flag is settled
         S3D_PHASE_MARK(0)
-        const int n = s_n[s];
-        if (n == 0 || *s_fail) break;
+        const int nq = s_n[s * 4], nk = s_n[s * 4 + 1];
+        if (nq == 0 || *s_fail) break;
         const __half *s_q = s_rows + s * 1536, *s_k = s_q + 512, *s_v = s_q + 1024;
-        const float *s_c = s_cs + s * 384;
-        const int *s_row = s_rowi + s * 32;
+        const float *s_c = s_cs + s * 768, *s_ck = s_c + 384;
         float cx[D];
         load_coords12<D>(s_c + lane * 12, cx);
         if (tid < 64) s_max[tid] = -INFINITY;
         // ---- projections P_q (lane-major), P_k (key-major); S0 = K.Q^T ------------------------------
         if (p_side && S3D_KEEP(0)) {
             uint32_t bf[8][2];
-            load_feat_bfrag(bf, q_side ? s_q : s_k, n, g, t);
+            load_feat_bfrag(bf, q_side ? s_q : s_k, q_side ? nq : nk, g, t);
 #pragma unroll
             for (int i = 0; i < NPU; ++i) {
                 const int mt = wsub + HALF * i;
                 if (mt < n_mt) {
-                    if (q_side) project_unit_b<true>(ta[i], bf, s_pq, mt, Rp, n, g, t);
-                    else project_unit_b<false>(ta[i], bf, s_pk, mt, Rp, n, g, t);
+                    if (q_side) project_unit_b<true>(ta[i], bf, s_pq, mt, Rp, nq, g, t);
+                    else project_unit_b<false>(ta[i], bf, s_pk, mt, Rp, nk, g, t);
                 }
             }
         }
         for (int u = wid; u < 16 && S3D_KEEP(1); u += NW) {
             const int mt = u >> 3, j = u & 7;       // key rows 16mt.., query columns 4j..
-            if (16 * mt < n && 4 * j < n) {
+            if (16 * mt < nk && 4 * j < nq) {
                 const __half *ysrc = s_k + mt * 256;
                 const uint32_t wv = *reinterpret_cast<const uint32_t *>(s_q + (4 * j + (g >> 1)) * 16 + (g & 1) * 8 + 2 * t);
                 const uint32_t a0 = *reinterpret_cast<const uint32_t *>(ysrc + g * 16 + 2 * t);
@@ -279,9 +332,9 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
             const int kk = wid + NW * j;
             sreg[j][0] = sreg[j][1] = 0.f;
             wreg[j][0] = wreg[j][1] = 0u;
-            if (kk < n && S3D_KEEP(2)) {
+            if (kk < nk && S3D_KEEP(2)) {
                 float ck[D];
-                load_coords12<D>(s_c + kk * 12, ck);
+                load_coords12<D>(s_ck + kk * 12, ck);
                 const uint32_t *pk_row = s_pk + kk * Rp;
                 __half2 bq = __float2half2_rn(0.f), bk = bq;
                 uint32_t w0 = 0, w1 = 0;
@@ -306,7 +359,7 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
                 mloc1 = fmaxf(mloc1, sy);
             }
         }
-        if (wid < n) {
+        if (wid < nk) {
             atomic_max_float(s_max + lane * 2, mloc0);
             atomic_max_float(s_max + lane * 2 + 1, mloc1);
         }
@@ -319,8 +372,8 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
         for (int j = 0; j < KPW; ++j) {
             const int kk = wid + NW * j;
             if (kk < QT && S3D_KEEP(3)) {
-                uint32_t ph = 0u;                         // zero for keys beyond the window: P.V reads whole 16-key steps
-                if (kk < n && lane < n) {
+                uint32_t ph = 0u;                         // zero for keys beyond the tile: P.V reads whole 16-key steps
+                if (kk < nk && lane < nq) {
                     const float p0 = ex2_approx(fmaf(sreg[j][0], LOG2E, -m0));
                     const float p1 = ex2_approx(fmaf(sreg[j][1], LOG2E, -m1));
                     l0 += p0;
@@ -348,9 +401,9 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
             // the half of a pair entry this dimension needs: (p, idx 0-4) or (idx 5-8, p)
             const uint2 *ecol = (lo ? s_elo : s_ehi) + lane;
             uint32_t *cell = s_hist + meta.rowbase[d] * QT + mypos;
-            uint2 e0 = ecol[0], e1 = ecol[ES];              // keys beyond the window hold zero entries
+            uint2 e0 = ecol[0], e1 = ecol[ES];              // keys beyond the tile hold zero entries
             int kk = 0;
-            for (; kk + 1 < n; kk += 2) {
+            for (; kk + 1 < nk; kk += 2) {
                 const uint32_t p0 = lo ? e0.x : e0.y, i0 = ((lo ? e0.y : e0.x) >> sh) & ((1u << IDX_BITS) - 1u);
                 const uint32_t p1 = lo ? e1.x : e1.y, i1 = ((lo ? e1.y : e1.x) >> sh) & ((1u << IDX_BITS) - 1u);
                 uint32_t *a0 = cell + i0 * QT, *a1 = cell + i1 * QT;
@@ -362,13 +415,13 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
                 *a0 = h2_as_u32(s0);
                 *a1 = h2_as_u32(s1);
             }
-            if (kk < n) {
+            if (kk < nk) {
                 const uint32_t p0 = lo ? e0.x : e0.y, i0 = ((lo ? e0.y : e0.x) >> sh) & ((1u << IDX_BITS) - 1u);
                 uint32_t *a0 = cell + i0 * QT;
                 *a0 = h2_as_u32(__hadd2(u32_as_h2(*a0), u32_as_h2(p0)));
             }
         } else if (wid == D && S3D_KEEP(6)) {
-            pair_gemm2<0, false>(part, s_elo, s_v, n, g, t);  // O[q] = sum_k p V[k]
+            pair_gemm2<0, false>(part, s_elo, s_v, nk, g, t);  // O[q] = sum_k p V[k]
         }
         consumer_sync<NT>();
         S3D_PHASE_MARK(5)
@@ -385,7 +438,7 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
         S3D_PHASE_MARK(6)
         if (tid < 256 && S3D_KEEP(8)) {
             const int qq = tid >> 3, ch = (tid & 7) * 2, h = ch >> 3;
-            if (qq < n) {
+            if (qq < nq) {
                 float a = 0.f, b = 0.f, ls = 0.f;
 #pragma unroll
                 for (int ww = 0; ww < NW; ++ww) {
@@ -394,20 +447,35 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
                     b += pr.y;
                     ls += s_lsum[(ww * QT + qq) * 2 + h];
                 }
-                const float inv = 1.f / ls;
-                const int64_t row = s_row[qq];
-                store_h2_mirrored(P.out, P.m_out, row * HC + co + ch, __floats2half2_rn(a * inv, b * inv));
-                if (HD16) {
-                    if (ch == 0) P.lse[row * H + hp] = s_max[qq * 2] + __logf(ls);
-                } else if ((ch & 7) == 0) {
-                    P.lse[row * H + 2 * hp + h] = s_max[qq * 2 + h] + __logf(ls);
+                float m = s_max[qq * 2 + h];
+                if (!s_n[s * 4 + 2]) {                     // not the first key tile
+                    const float mt = m;
+                    m = fmaxf(m_run, mt);
+                    const float f0 = ex2_approx((m_run - m) * LOG2E), f1 = ex2_approx((mt - m) * LOG2E);
+                    a = o_run.x * f0 + a * f1;
+                    b = o_run.y * f0 + b * f1;
+                    ls = l_run * f0 + ls * f1;
+                }
+                if (s_n[s * 4 + 3]) {                      // the last one
+                    const float inv = 1.f / ls;
+                    const int64_t row = s_rowi[s * 32 + qq];
+                    store_h2_mirrored(P.out, P.m_out, row * HC + co + ch, __floats2half2_rn(a * inv, b * inv));
+                    if (HD16) {
+                        if (ch == 0) P.lse[row * H + hp] = m + __logf(ls);
+                    } else if ((ch & 7) == 0) {
+                        P.lse[row * H + 2 * hp + h] = m + __logf(ls);
+                    }
+                } else {
+                    o_run = make_float2(a, b);
+                    m_run = m;
+                    l_run = ls;
                 }
             }
         }
         // this warp is done with the stage (rows, coordinates, row numbers)
         __syncwarp();
         if (lane == 0) mbar_arrive(s_empty + s);
-    }  // windows
+    }  // items
     S3D_PHASE_FLUSH(0)
 }
 
@@ -433,7 +501,6 @@ static int launch_fwd_small(const FwdSmallParams &p, const CrseMeta &meta, cudaS
     // reserved per block) decides whether two fit
     const int per_sm = 2 * (L.total + 1024) <= 228 * 1024 ? 2 : 1;
     int gx = sms_of[dev] * per_sm / hp;
-    if (gx > p.W) gx = (int)p.W;
     if (gx < 1) gx = 1;
     dim3 grid((unsigned)gx, (unsigned)hp);
     kern<<<grid, (NW + 1) * 32, L.total, st>>>(p, meta, make_pair_consts(meta));
@@ -474,7 +541,7 @@ bool attn_tc_fwd_small_supported(const AttnArgs &a)
     return tc::make_fwd_small_layout(Rint, nw).total <= 227 * 1024;
 }
 
-// Windows of at most 32 voxels only; the others are left untouched.
+// a.window_class: windows of the other class are left untouched.
 int attn_tc_forward_small(const AttnArgs &a0, cudaStream_t st)
 {
     if (a0.W == 0) return S3D_OK;
@@ -486,6 +553,8 @@ int attn_tc_forward_small(const AttnArgs &a0, cudaStream_t st)
     p.out = (__half *)a.out; p.lse = a.lse; p.m_out = a.m_out;
     p.w_sizes = a.w_sizes; p.w2n = a.w2n; p.n2n = a.n2n; p.n_coords = a.n_coords;
     p.W = a.W; p.H = a.H;
+    p.n_min = a.window_class == 2 ? tc::QT + 1 : 1;
+    p.n_max = a.window_class == 1 ? tc::QT : 0x7fffffff;
     const int n_mt = (a.meta.R + 15) / 16;
     const int nw = tc::fwd_small_warps(a.meta.D);
     const int npu = (n_mt + nw / 2 - 1) / (nw / 2);   // <= 6
