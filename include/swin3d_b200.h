@@ -99,10 +99,8 @@ int s3d_attn_bwd(const void *q, const void *k, const void *v,
  * are in place).  S3D_ERR_UNSUPPORTED for shapes served by kernels without mirrored stores (the
  * generic path and head_dim 16 with an even head count and large tables).
  * window_class (forward): 0 = windows of any size; 1 = the caller guarantees that every window of
- * this call has at most 32 voxels, 2 = that every window has more.  The forward runs one kernel for
- * each class and each walks the whole window list for its own windows; a caller that has the sizes
- * on the host (the multi-GPU split plans its ranges from them) passes the two classes in two calls
- * and saves both walks.  A window that breaks the guarantee is NOT processed.
+ * this call has at most 32 voxels, 2 = that every window has more.  A window that breaks the
+ * guarantee is NOT processed (head_dim 8, and 16 with an odd head count, on the fp16 path).
  * The reference has no multi-GPU attention; this replaces nothing in it.                        */
 #define S3D_MAX_MIRRORS 7
 int s3d_attn_fwd_mirrored(const void *q, const void *k, const void *v,
@@ -166,6 +164,11 @@ int s3d_debug_crse_indices_variant(const float *n_coords, const int32_t *table_s
  * (Swin3D/src/attn/attn_utils.cuh:444-450).                                                   */
 int s3d_debug_crse_index_values(const float *cq, const float *ck, int64_t n, int L, int last_dim,
                                 int variant, int32_t *idx_out, void *stream);
+
+/* The three fp32 tables of a layer (n elements each) rounded to fp16 in one launch: dst[t*n + i] =
+ * half(src_t[i]), the cast that the fp16 modes make before every call
+ * (Swin3D/sparse_dl/attn/attn_coff.py:172-178).  dst: 3 n halves.                                */
+int s3d_cast_tables(const float *tq, const float *tk, const float *tv, int64_t n, void *dst, void *stream);
 
 /* Row gather for the multi-GPU window split: dst[a][i][:] = src_a[idx[i]][:] for A <= 4 per-voxel
  * arrays that share one index list (rows of row_bytes, a multiple of 16; array a of the result

@@ -212,9 +212,13 @@ static int attn_bwd_impl(const void *q, const void *k, const void *v, const void
     if (!dtq || !dtk || !dtv) return S3D_ERR_BAD_ARG;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t tbytes = (size_t)a.meta.R * H * hd * sizeof(float);
-    if (cudaMemsetAsync(dtq, 0, tbytes, st) != cudaSuccess || cudaMemsetAsync(dtk, 0, tbytes, st) != cudaSuccess ||
-        cudaMemsetAsync(dtv, 0, tbytes, st) != cudaSuccess)
+    const size_t tcount = (size_t)a.meta.R * H * hd;
+    if (dtk == dtq + tcount && dtv == dtk + tcount) {          // one array of three: one launch
+        if (cudaMemsetAsync(dtq, 0, 3 * tbytes, st) != cudaSuccess) return S3D_ERR_LAUNCH;
+    } else if (cudaMemsetAsync(dtq, 0, tbytes, st) != cudaSuccess || cudaMemsetAsync(dtk, 0, tbytes, st) != cudaSuccess ||
+               cudaMemsetAsync(dtv, 0, tbytes, st) != cudaSuccess) {
         return S3D_ERR_LAUNCH;
+    }
     if (N == 0 || W == 0) return S3D_OK;
     if (!q || !k || !v || !tq || !tk || !tv || !w_sizes || !w2n || !n2n || !n_coords || !out || !lse ||
         !dout || !dq || !dk || !dv)

@@ -15,7 +15,7 @@ import torch
 from torch import Tensor
 from torch.autograd.function import Function
 
-from ... import _lib
+from ... import _lib, _stream
 
 
 class PosEmb(enum.Enum):
@@ -146,17 +146,16 @@ def attn_forward_raw(q, k, v, tq, tk, tv, sizes: List[int], w_sizes, w2n, n2n, n
     if out.shape != q.shape or out.dtype != q.dtype or not out.is_contiguous() or lse.shape != (N, H):
         raise ValueError("out / lse buffers must be contiguous and match the query")
     arr = (ctypes.c_int32 * D)(*sizes)
-    with torch.cuda.device(q.device):
-        st = torch.cuda.current_stream().cuda_stream
-        args = (q.data_ptr(), k.data_ptr(), v.data_ptr(), tq.data_ptr(), tk.data_ptr(), tv.data_ptr(),
-                ctypes.cast(arr, ctypes.c_void_p), D, w_sizes.data_ptr(), w2n.data_ptr(),
-                n2n.data_ptr(), n_coords.data_ptr(), N, W, H, hd, _DTYPE_CODE[q.dtype],
-                out.data_ptr(), lse.data_ptr())
-        if mirrors or window_class:
-            keep, mp = _pointer_array(mirrors) if mirrors else (None, None)
-            rc = _lib.lib.s3d_attn_fwd_mirrored(*args, len(mirrors) if mirrors else 0, mp, int(window_class), st)
-        else:
-            rc = _lib.lib.s3d_attn_fwd(*args, st)
+    args = (q.data_ptr(), k.data_ptr(), v.data_ptr(), tq.data_ptr(), tk.data_ptr(), tv.data_ptr(),
+            ctypes.cast(arr, ctypes.c_void_p), D, w_sizes.data_ptr(), w2n.data_ptr(),
+            n2n.data_ptr(), n_coords.data_ptr(), N, W, H, hd, _DTYPE_CODE[q.dtype],
+            out.data_ptr(), lse.data_ptr())
+    if mirrors or window_class:
+        keep, mp = _pointer_array(mirrors) if mirrors else (None, None)
+        rc = _stream.call(q.device, _lib.lib.s3d_attn_fwd_mirrored, *args, len(mirrors) if mirrors else 0, mp,
+                          int(window_class))
+    else:
+        rc = _stream.call(q.device, _lib.lib.s3d_attn_fwd, *args)
     _lib.check(rc, "s3d_attn_fwd")
     return out, lse
 
@@ -181,22 +180,35 @@ def attn_backward_raw(q, k, v, tq, tk, tv, sizes: List[int], w_sizes, w2n, n2n, 
     tn = sum(sizes)
     dt = torch.empty((3, tn), dtype=torch.float32, device=q.device)
     arr = (ctypes.c_int32 * D)(*sizes)
-    with torch.cuda.device(q.device):
-        st = torch.cuda.current_stream().cuda_stream
-        args = (q.data_ptr(), k.data_ptr(), v.data_ptr(), tq.data_ptr(), tk.data_ptr(), tv.data_ptr(),
-                ctypes.cast(arr, ctypes.c_void_p), D, w_sizes.data_ptr(), w2n.data_ptr(),
-                n2n.data_ptr(), n_coords.data_ptr(), N, W, H, hd, _DTYPE_CODE[q.dtype],
-                out.data_ptr(), lse.data_ptr(), dout.data_ptr(), dq.data_ptr(), dk.data_ptr(),
-                dv.data_ptr(), dt[0].data_ptr(), dt[1].data_ptr(), dt[2].data_ptr())
-        if mirrors and len(mirrors[0]):
-            if not (len(mirrors) == 3 and len(mirrors[0]) == len(mirrors[1]) == len(mirrors[2])):
-                raise ValueError("mirrors: three equally long address lists (dq, dk, dv)")
-            keep = [_pointer_array(m) for m in mirrors]
-            rc = _lib.lib.s3d_attn_bwd_mirrored(*args, len(mirrors[0]), keep[0][1], keep[1][1], keep[2][1], st)
-        else:
-            rc = _lib.lib.s3d_attn_bwd(*args, st)
+    dtq, dtk, dtv = dt.unbind(0)
+    args = (q.data_ptr(), k.data_ptr(), v.data_ptr(), tq.data_ptr(), tk.data_ptr(), tv.data_ptr(),
+            ctypes.cast(arr, ctypes.c_void_p), D, w_sizes.data_ptr(), w2n.data_ptr(),
+            n2n.data_ptr(), n_coords.data_ptr(), N, W, H, hd, _DTYPE_CODE[q.dtype],
+            out.data_ptr(), lse.data_ptr(), dout.data_ptr(), dq.data_ptr(), dk.data_ptr(),
+            dv.data_ptr(), dtq.data_ptr(), dtk.data_ptr(), dtv.data_ptr())
+    if mirrors and len(mirrors[0]):
+        if not (len(mirrors) == 3 and len(mirrors[0]) == len(mirrors[1]) == len(mirrors[2])):
+            raise ValueError("mirrors: three equally long address lists (dq, dk, dv)")
+        keep = [_pointer_array(m) for m in mirrors]
+        rc = _stream.call(q.device, _lib.lib.s3d_attn_bwd_mirrored, *args, len(mirrors[0]), keep[0][1], keep[1][1],
+                          keep[2][1])
+    else:
+        rc = _stream.call(q.device, _lib.lib.s3d_attn_bwd, *args)
     _lib.check(rc, "s3d_attn_bwd")
-    return dq, dk, dv, dt[0], dt[1], dt[2]
+    return dq, dk, dv, dtq, dtk, dtv
+
+
+def _tables_in(tables, dtype):
+    """The three tables as contiguous arrays of `dtype`: fp32 parameters to fp16 in one launch."""
+    tq = tables[0]
+    n = tq.numel()
+    if (dtype == torch.float16 and n and tq.is_cuda and
+            all(t.dtype == torch.float32 and t.device == tq.device and t.numel() == n and t.is_contiguous() for t in tables)):
+        buf = torch.empty((3, n), dtype=torch.float16, device=tq.device)
+        rc = _stream.call(tq.device, _lib.lib.s3d_cast_tables, *[t.data_ptr() for t in tables], n, buf.data_ptr())
+        _lib.check(rc, "s3d_cast_tables")
+        return buf.unbind(0)
+    return [t.to(dtype).contiguous() for t in tables]
 
 
 class SelfAttnAIOFunction(Function):
@@ -225,7 +237,7 @@ class SelfAttnAIOFunction(Function):
             raise ValueError(f"compute dtype {c_dtype} is not supported (float32 or float16)")
 
         qkv = [t.to(c_dtype) for t in (raw_query_feats, raw_key_feats, raw_value_feats)]
-        tabs = [t.to(c_dtype).contiguous() for t in (query_table, key_table, value_table)]
+        tabs = _tables_in((query_table, key_table, value_table), c_dtype)
         sizes = _table_sizes_host(table_offsets, query_table.numel(), raw_query_feats.shape[1],
                                   raw_query_feats.shape[2])
         _, w_sizes, _, w2n, n2n, n_coords = indices
@@ -254,7 +266,7 @@ class SelfAttnAIOFunction(Function):
         if c_dtype not in _DTYPE_CODE:
             raise ValueError(f"compute dtype {c_dtype} is not supported (float32 or float16)")
         qkv = [t.to(c_dtype) for t in (q, k, v)]
-        tabs = [t.to(c_dtype).contiguous() for t in (tq, tk, tv)]
+        tabs = _tables_in((tq, tk, tv), c_dtype)
         dq, dk, dv, dtq, dtk, dtv = attn_backward_raw(
             *qkv, *tabs, ctx.sizes, w_sizes, w2n, n2n, n_coords,
             out.to(c_dtype), lse, grad.to(c_dtype).contiguous())

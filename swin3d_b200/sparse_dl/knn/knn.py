@@ -6,7 +6,7 @@ with ``dist`` the Euclidean distance (sqrt of the kernel's squared distance, knn
 import torch
 from torch.autograd.function import Function
 
-from ... import _lib
+from ... import _lib, _stream
 
 
 def _search(K: int, src_xyz, query_xyz, src_offset, query_offset, root: bool, out=None):
@@ -28,11 +28,8 @@ def _search(K: int, src_xyz, query_xyz, src_offset, query_offset, root: bool, ou
     idx, dist = out
     nbytes = _lib.lib.s3d_knn_workspace_bytes(K, B, Ns, Nq)
     work = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
-    with torch.cuda.device(dev):
-        st = torch.cuda.current_stream().cuda_stream
-        rc = _lib.lib.s3d_knn_search(K, src_xyz.data_ptr(), query_xyz.data_ptr(), so.data_ptr(), qo.data_ptr(), B, Ns, Nq,
-                                     int(root), idx.data_ptr(), dist.data_ptr(), None if work is None else work.data_ptr(),
-                                     nbytes, st)
+    rc = _stream.call(dev, _lib.lib.s3d_knn_search, K, src_xyz.data_ptr(), query_xyz.data_ptr(), so.data_ptr(), qo.data_ptr(),
+                      B, Ns, Nq, int(root), idx.data_ptr(), dist.data_ptr(), None if work is None else work.data_ptr(), nbytes)
     _lib.check(rc, "s3d_knn")
     return idx, dist
 
