@@ -355,6 +355,45 @@ def test_backward_kernels_at_the_edges_of_their_tiles(dtype, H, hd, ws, crse):
             assert table_row_errors(a, b, H * hd, tol, 2e-2) == [], name
 
 
+@pytest.mark.parametrize("H,hd,ws,crse", [(2, 8, 5, "XYZ_RGB_NORM"), (4, 8, 7, "XYZ_RGB"), (2, 8, 7, "XYZ"), (10, 8, 7, "XYZ_RGB_NORM"),
+                                          (1, 16, 5, "XYZ_RGB_NORM"), (3, 16, 7, "XYZ_RGB"), (1, 16, 7, "XYZ")])
+def test_fp16_forward_at_the_edges_of_its_tiles(H, hd, ws, crse):
+    """Windows of 1 voxel up to several tiles in one call: a window of several tiles merges its key tiles, and its
+    query tiles fall to different blocks; the call limited to one size class writes the same bits to its rows
+    and none to the others."""
+    from tests.gpu_helpers import dev
+    from swin3d_b200.sparse_dl.attn.attn_coff import attn_forward_raw
+    sizes = [1, 2, 3, 15, 16, 17, 31, 32, 33, 63, 64, 65, 96, 97, ws ** 3]
+    p = make_problem(seed=92, ws=ws, H=H, hd=hd, crse=crse, scene=_scene_of_window_sizes(ws, sizes), round_fp16=True)
+    o_ref, _, _ = oracle_fwd_bwd(p, np.float64)
+    h = lambda a: dev(a).half()
+    args = (h(p.q), h(p.k), h(p.v), h(p.tq), h(p.tk), h(p.tv), p.sizes, dev(p.w_sizes), dev(p.w2n), dev(p.n2n), dev(p.n_crse))
+    out, lse = attn_forward_raw(*args)
+    assert rel_err(out.float().cpu().numpy(), o_ref) < FP16_TOL
+    assert bool(torch.isfinite(lse).all())
+    small = torch.zeros(len(p.q), dtype=torch.bool, device="cuda")
+    for a, n in zip(p.w2n, p.w_sizes):
+        if n <= 32:
+            small[args[9][int(a):int(a) + int(n)].long()] = True
+    for cls, rows in ((1, small), (2, ~small)):
+        part = attn_forward_raw(*args, out=torch.full_like(out, float("nan")), window_class=cls)[0]
+        assert torch.equal(part[rows], out[rows]) and bool(torch.isnan(part[~rows].float()).all())
+
+
+@pytest.mark.parametrize("n,offset", [(16, 0), (4096, 0), (30_720, 0), (7, 0), (1001, 0), (1000, 1)])
+def test_table_cast_equals_the_torch_cast(n, offset):
+    """One launch for the three tables; odd lengths and views that begin inside a vector take single elements."""
+    from swin3d_b200 import _lib
+    src = [torch.randn(n + offset, device="cuda", generator=torch.Generator("cuda").manual_seed(i))[offset:] * 10.0 ** (4 * i - 4)
+           for i in range(3)]
+    src[0][0], src[1][-1], src[2][n // 2] = float("nan"), float("inf"), -7e4
+    dst = torch.full((3, n), 7.0, dtype=torch.float16, device="cuda")
+    rc = _lib.lib.s3d_cast_tables(*[t.data_ptr() for t in src], n, dst.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    for a, b in zip(src, dst):
+        assert torch.equal(a.half().view(torch.int16), b.view(torch.int16))
+
+
 @pytest.mark.parametrize("crse,H,ws,shift", [("XYZ_RGB_NORM", 5, 5, 2), ("XYZ_RGB", 3, 5, 0), ("XYZ", 2, 7, 3),
                                              ("XYZ_RGB_NORM", 4, 7, 0), ("XYZ_RGB_NORM", 10, 7, 3), ("XYZ_RGB", 6, 5, 2)])
 def test_fp16_head_dim_16_tensor_core_path(crse, H, ws, shift):
