@@ -157,8 +157,9 @@ __device__ __forceinline__ void pair_tables(const LaneDims<LG, D> &ld, const flo
 // ---------------------------------------------------------------------------------------------
 // Forward: a group of LG = HD / VEC lanes (a lane holds VEC consecutive channels) owns one
 // (query, head) row and walks the keys of the query's window; every row of q, k, v and of the
-// tables is read as one coalesced piece.
-template <typename T, int HD, int D, int VEC>
+// tables is read as one coalesced piece.  KS such groups may share a row, each taking every KS-th key with its
+// own maximum and sum, merged at the end.
+template <typename T, int HD, int D, int VEC, int KS>
 __global__ void __launch_bounds__(256)
 attn_fwd_scalar_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__restrict__ v,
                        const T *__restrict__ tq, const T *__restrict__ tk, const T *__restrict__ tv,
@@ -167,10 +168,11 @@ attn_fwd_scalar_kernel(const T *__restrict__ q, const T *__restrict__ k, const T
                        const float *__restrict__ n_coords, int64_t N, int64_t W, int H,
                        T *__restrict__ out, float *__restrict__ lse)
 {
-    constexpr int LG = HD / VEC, G = 32 / LG;
+    constexpr int LG = HD / VEC, G = 32 / (LG * KS);
+    static_assert(LG * KS <= 32, "a row's groups are in one warp");
     constexpr int NDL = LaneDims<LG, D>::NDL;
-    const int lane = threadIdx.x & 31, c = lane % LG, gi = lane / LG;
-    const unsigned gmask = group_mask<LG>(gi);
+    const int lane = threadIdx.x & 31, c = lane % LG, sub = lane / LG, gi = sub / KS, ks = sub % KS;
+    const unsigned gmask = group_mask<LG>(sub);
     const int HC = H * HD;
     const int64_t group0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * G + gi;
     const int64_t ngroups = (int64_t)gridDim.x * (blockDim.x >> 5) * G;
@@ -195,22 +197,23 @@ attn_fwd_scalar_kernel(const T *__restrict__ q, const T *__restrict__ k, const T
         ld.load(n_coords + (int64_t)p * D, ld.own);
         float mx = -INFINITY, l = 0.f;
         // the next key's row number and coordinates are fetched one iteration ahead
-        int64_t krow_n = __ldg(n2n + base);
+        const int k0 = base + min(ks, n - 1);
+        int64_t krow_n = __ldg(n2n + k0);
         float oth_n[NDL];
-        ld.load(n_coords + (int64_t)base * D, oth_n);
-        for (int kj = 0; kj < n; ++kj) {
+        ld.load(n_coords + (int64_t)k0 * D, oth_n);
+        for (int kj = ks; kj < n; kj += KS) {
             const int64_t krow = krow_n;
             float oth[NDL];
 #pragma unroll
             for (int j = 0; j < NDL; ++j) oth[j] = oth_n[j];
-            const int nx = base + min(kj + 1, n - 1);
+            const int nx = base + min(kj + KS, n - 1);
             krow_n = __ldg(n2n + nx);
             ld.load(n_coords + (int64_t)nx * D, oth_n);
             float kc[VEC], vc[VEC], bq[VEC], bk[VEC], bv[VEC];
             ldv<T, VEC>(k + krow * HC + hc, kc);
             ldv<T, VEC>(v + krow * HC + hc, vc);
             int mine[NDL];
-            pair_tables<T, LG, D, VEC, true>(ld, oth, gi, gmask, tq, tk, tv, HC, hc, mine, bq, bk, bv);
+            pair_tables<T, LG, D, VEC, true>(ld, oth, sub, gmask, tq, tk, tv, HC, hc, mine, bq, bk, bv);
             float sp = 0.f;
 #pragma unroll
             for (int i = 0; i < VEC; ++i) sp += qc[i] * (kc[i] + bq[i]) + kc[i] * bk[i];
@@ -223,7 +226,21 @@ attn_fwd_scalar_kernel(const T *__restrict__ q, const T *__restrict__ k, const T
             for (int i = 0; i < VEC; ++i) acc[i] = acc[i] * scale + pr * (vc[i] + bv[i]);
             mx = mnew;
         }
-        if (live) {
+        if constexpr (KS > 1) {
+            __syncwarp();
+#pragma unroll
+            for (int o = LG; o < LG * KS; o *= 2) {
+                const float m2 = __shfl_xor_sync(0xffffffffu, mx, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
+                const float mnew = fmaxf(mx, m2);
+                // a group without keys: maximum -inf, sum 0
+                const float f1 = mx == mnew ? 1.f : __expf(mx - mnew), f2 = m2 == mnew ? 1.f : __expf(m2 - mnew);
+                l = l * f1 + l2 * f2;
+#pragma unroll
+                for (int i = 0; i < VEC; ++i) acc[i] = acc[i] * f1 + __shfl_xor_sync(0xffffffffu, acc[i], o) * f2;
+                mx = mnew;
+            }
+        }
+        if (live && ks == 0) {
             const float inv = 1.f / l;
 #pragma unroll
             for (int i = 0; i < VEC; ++i) acc[i] *= inv;
@@ -472,14 +489,14 @@ template <> struct ScalarVec<8> { static constexpr int FWD = 4, BWD = 1; };
 template <> struct ScalarVec<16> { static constexpr int FWD = 2, BWD = 1; };
 template <> struct ScalarVec<32> { static constexpr int FWD = 4, BWD = 4; };
 
-template <typename T, int HD, int D, int VEC>
+template <typename T, int HD, int D, int VEC, int KS>
 static int launch_fwd_v(const AttnArgs &a, cudaStream_t st)
 {
-    const int groups_per_block = 8 * (32 / (HD / VEC));
+    const int groups_per_block = 8 * (32 / (HD / VEC * KS));
     int64_t blocks = (a.N * a.H + groups_per_block - 1) / groups_per_block;
     const int64_t cap = 148 * 64;
     if (blocks > cap) blocks = cap;
-    attn_fwd_scalar_kernel<T, HD, D, VEC><<<(unsigned)blocks, 256, 0, st>>>(
+    attn_fwd_scalar_kernel<T, HD, D, VEC, KS><<<(unsigned)blocks, 256, 0, st>>>(
         (const T *)a.q, (const T *)a.k, (const T *)a.v, (const T *)a.tq, (const T *)a.tk,
         (const T *)a.tv, a.meta, a.w_sizes, a.w2n, a.n2n, a.n_coords, a.N, a.W, a.H, (T *)a.out, a.lse);
     return cudaGetLastError() == cudaSuccess ? S3D_OK : S3D_ERR_LAUNCH;
@@ -489,7 +506,13 @@ template <typename T, int HD, int D>
 static int launch_fwd(const AttnArgs &a, cudaStream_t st)
 {
     if (a.W == 0 || a.N == 0) return S3D_OK;
-    return launch_fwd_v<T, HD, D, ScalarVec<HD>::FWD>(a, st);
+    // Few items: the walk over the keys of the largest windows is what takes the time, and the lanes to share it are
+    // there.  fp32, KS = 1 against the one taken, by items: head_dim 8 (KS = 2) 21 k 98 / 60 us, 113 k 234 / 196,
+    // 701 k 810 / 867; head_dim 16 (KS = 4) 8 k 207 / 137 us, 20 k 230 / 189, 26 k 288 / 298, 78 k 754 / 924.
+    constexpr int VEC = ScalarVec<HD>::FWD, KS = HD == 8 ? 2 : (HD == 16 ? 4 : 1);
+    constexpr int64_t FEW = HD == 8 ? 148 * 1024 : 148 * 160;
+    if (KS > 1 && a.N * a.H < FEW) return launch_fwd_v<T, HD, D, VEC, KS>(a, st);
+    return launch_fwd_v<T, HD, D, VEC, 1>(a, st);
 }
 
 template <typename T, int HD, int D, int VEC>

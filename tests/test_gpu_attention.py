@@ -581,6 +581,19 @@ def test_tiled_kernels_work_list_overflow_falls_back_to_a_direct_walk():
         assert rel_err(a, b) < 1.5e-2
 
 
+@pytest.mark.parametrize("hd,H", [(8, 236), (8, 237), (16, 36), (16, 37)])
+def test_generic_forward_either_side_of_the_shared_rows(hd, H):
+    """Few (voxel, head) items: several groups of lanes share a row's keys (windows of fewer keys than groups among
+    them); from 151552 (head_dim 8) and 23680 items (16) on, one group walks them all."""
+    from tests.gpu_helpers import cuda_fwd_bwd
+    p = make_problem(seed=35, n_voxels=642, grid=18, H=H, hd=hd, crse="XYZ_RGB")
+    few = 151_552 if hd == 8 else 23_680
+    assert (p.N * H < few) == (H in (236, 36))
+    o_ref, lse_ref, _ = oracle_fwd_bwd(p, np.float64)
+    out, lse, _ = cuda_fwd_bwd(p, torch.float32)
+    assert rel_err(out, o_ref) < FP32_TOL and np.abs(lse - lse_ref).max() < 1e-4
+
+
 @pytest.mark.parametrize("H,hd,dtype", [(3, 8, "float32"), (1, 16, "float32"), (1, 32, "float32"), (3, 32, "float16")])
 def test_generic_kernels_with_item_counts_that_do_not_fill_the_last_warp(H, hd, dtype):
     """The generic kernels deal (voxel, head) items to groups of lanes; with an odd number of items
