@@ -428,25 +428,49 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
     unsigned todo = __ballot_sync(0xffffffffu, scene >= 0 && finite3(q.x, q.y, q.z));
     while (todo) {
         const int b = __shfl_sync(0xffffffffu, scene, __ffs(todo) - 1);
-        const bool mine = ((todo >> lane) & 1u) && scene == b;
-        const unsigned act = __ballot_sync(0xffffffffu, mine);
-        todo &= ~act;
+        unsigned act = __ballot_sync(0xffffffffu, ((todo >> lane) & 1u) && scene == b);
         const int s0 = (int)__ldg(t.hist + ((int64_t)b << (3 * t.bits)));
         const int n = (int)__ldg(t.hist + ((int64_t)(b + 1) << (3 * t.bits))) - s0;
-        if (n <= 0) continue;
-        // queries of other scenes take part as NaN: no comparison holds for them
-        const float qx = mine ? q.x : NAN, qy = mine ? q.y : NAN, qz = mine ? q.z : NAN;
-        const uint64_t nx = pack2(-qx, -qx), ny = pack2(-qy, -qy), nz = pack2(-qz, -qz);
+        if (n <= 0) {
+            todo &= ~act;
+            continue;
+        }
+        // Box of the queries.  Where the cell order jumps, the box of both sides holds far more leaves than the two
+        // boxes, and a leaf costs a test against every query: the queries beyond the widest gap are left for
+        // another pass if the extents of the two boxes together are less than half that of the one.
         float ql[3], qh[3];
-        {
+        auto box_of = [&](unsigned lanes, float (&lo)[3], float (&hi)[3]) {
             const float c[3] = {q.x, q.y, q.z};
+            const bool in = (lanes >> lane) & 1u;
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 const uint32_t k = order_key(c[d]);
-                ql[d] = from_order_key(__reduce_min_sync(0xffffffffu, mine ? k : 0xffffffffu));
-                qh[d] = from_order_key(__reduce_max_sync(0xffffffffu, mine ? k : 0u));
+                lo[d] = from_order_key(__reduce_min_sync(0xffffffffu, in ? k : 0xffffffffu));
+                hi[d] = from_order_key(__reduce_max_sync(0xffffffffu, in ? k : 0u));
             }
+            return (hi[0] - lo[0]) + (hi[1] - lo[1]) + (hi[2] - lo[2]);
+        };
+        for (;;) {
+            const float ext = box_of(act, ql, qh);
+            const unsigned above = act & ~((2u << lane) - 1u);
+            const int nx = above ? __ffs(above) - 1 : lane;
+            const float gx = fabsf(__shfl_sync(0xffffffffu, q.x, nx) - q.x), gy = fabsf(__shfl_sync(0xffffffffu, q.y, nx) - q.y),
+                        gz = fabsf(__shfl_sync(0xffffffffu, q.z, nx) - q.z);
+            const uint32_t gap = ((act >> lane) & 1u) ? __float_as_uint(fmaxf(fmaxf(gx, gy), gz)) : 0u;
+            const uint32_t most = __reduce_max_sync(0xffffffffu, gap);
+            // ext <= ext of the parts + three gaps, so a smaller gap cannot do
+            if (most == 0u || __uint_as_float(most) * 6.f < ext) break;
+            const int who = __ffs(__ballot_sync(0xffffffffu, gap == most)) - 1;
+            const unsigned lower = act & ((2u << who) - 1u);
+            float l0[3], h0[3], l1[3], h1[3];
+            if (!(box_of(lower, l0, h0) + box_of(act & ~lower, l1, h1) < 0.5f * ext)) break;
+            act = lower;
         }
+        todo &= ~act;
+        const bool mine = (act >> lane) & 1u;
+        // the other queries take part as NaN: no comparison holds for them
+        const float qx = mine ? q.x : NAN, qy = mine ? q.y : NAN, qz = mine ? q.z : NAN;
+        const uint64_t nx = pack2(-qx, -qx), ny = pack2(-qy, -qy), nz = pack2(-qz, -qz);
         const float *points = t.src + first_leaf(s0, b) * (4 * LEAF);
         const float4 *leaves = t.leaf + 2 * first_leaf(s0, b), *nodes = t.node + 2 * first_node(s0, b);
         const int n_leaf = (n + LEAF - 1) / LEAF, n_node = (n_leaf + 31) / 32;
