@@ -197,7 +197,7 @@ attn_fwd_scalar_kernel(const T *__restrict__ q, const T *__restrict__ k, const T
         ld.load(n_coords + (int64_t)p * D, ld.own);
         float mx = -INFINITY, l = 0.f;
         // the next key's row number and coordinates are fetched one iteration ahead
-        const int k0 = base + min(ks, n - 1);
+        const int k0 = KS > 1 ? base + min(ks, n - 1) : base;
         int64_t krow_n = __ldg(n2n + k0);
         float oth_n[NDL];
         ld.load(n_coords + (int64_t)k0 * D, oth_n);
