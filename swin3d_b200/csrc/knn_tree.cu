@@ -3,7 +3,7 @@
 //
 // Both point sets are put into Morton order of a per-scene grid by a counting sort (histogram, scan,
 // scatter).  32 consecutive sources are a leaf and 32 leaves a node, each with its bounding box.
-// A warp searches for 32 consecutive queries (K > 3: 16 or 8, several lanes each), which lie close together:
+// A warp searches for 32 consecutive queries (K > 3: 16, two lanes each), which lie close together:
 // the lanes test the boxes of 32 nodes or leaves at a time against the box of the warp's queries, nearest
 // first, and a leaf that survives is offered to all its queries with broadcast loads.
 //
@@ -18,8 +18,8 @@
 // the query on a list; those queries are scanned again in index order with the literal heap.
 //
 // Bound: instruction issue of the leaf evaluation for K = 3, the merges of the lists and their latency for
-// K = 16.  Measured, whole search: 8 scenes x (200 k queries, 50 k sources), K = 3: 0.53 ms, the scan of knn.cu
-// 16.9; 4 x (30 k, 120 k), K = 16: 0.72 ms (the scan: 62).
+// K = 16.  Measured, whole search: 8 scenes x (200 k queries, 50 k sources), K = 3: 0.42 ms, the scan of knn.cu
+// 16.9; 4 x (30 k, 120 k), K = 16: 0.37 ms (the scan: 62).
 #include "knn_common.cuh"
 #include "knn_kernels.cuh"
 #include "scan.cuh"
@@ -381,11 +381,10 @@ constexpr int QUEUE = 16;
 // Long lists are also shared: the SHARE lanes of a query each take their part of every leaf's sources and keep
 // their own list.  A lane's K-th distance is a bound of the query's, and so is the largest of the lanes'
 // ceil(K / SHARE)-th.  The lists are merged at the end.  A warp then has fewer queries, so a smaller box and
-// fewer leaves to look at, and there are more warps.  K = 16, whole search with SHARE = 1 / 2 / 4: 4 x (30 k
-// queries in 120 k sources) 940 / 719 / 855 us, 3 x (16 k in 60 k) 604 / 567 / 466, 8 x (6 k in 20 k) 291 / 225 /
-// 200, 40 k in 135 k 674 / 456 / 448, 3 k in 12 k 159 / 182 / 133: four lanes while two would leave the GPU
-// with fewer than 4096 warps.
-inline int search_share(int64_t Nq) { return Nq < 65536 ? 4 : 2; }
+// fewer leaves to look at, and there are more warps.  K = 16, whole search with one lane / two (before queries were
+// split at jumps): 4 x (30 k queries in 120 k sources) 940 / 719 us, 40 k in 135 k 674 / 456.  With the split, two /
+// four lanes: 374 / 430 and 200 / 200 us, 3 x (16 k in 60 k) 164 / 211, 8 x (6 k in 20 k) 186 / 179, 3 k in 12 k 99 / 104.
+constexpr int SHARED = 2;
 
 template <int KL, int SHARE, bool ROOT>
 __global__ void __launch_bounds__(SEARCH_THREADS)
@@ -437,7 +436,8 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
         }
         // Box of the queries.  Where the cell order jumps, the box of both sides holds far more leaves than the two
         // boxes, and a leaf costs a test against every query: the queries beyond the widest gap are left for
-        // another pass if the extents of the two boxes together are less than half that of the one.
+        // another pass if the extents of the two boxes together are less than 0.4 of that of the one (0.2 / 0.3 / 0.4 /
+        // 0.5 / 0.7 / 0.85, K = 16, 4 x (30 k in 120 k): 447 / 385 / 373 / 374 / 397 / 469 us, 721 without).
         float ql[3], qh[3];
         auto box_of = [&](unsigned lanes, float (&lo)[3], float (&hi)[3]) {
             const float c[3] = {q.x, q.y, q.z};
@@ -459,11 +459,11 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
             const uint32_t gap = ((act >> lane) & 1u) ? __float_as_uint(fmaxf(fmaxf(gx, gy), gz)) : 0u;
             const uint32_t most = __reduce_max_sync(0xffffffffu, gap);
             // ext <= ext of the parts + three gaps, so a smaller gap cannot do
-            if (most == 0u || __uint_as_float(most) * 6.f < ext) break;
+            if (most == 0u || __uint_as_float(most) * 5.f < ext) break;
             const int who = __ffs(__ballot_sync(0xffffffffu, gap == most)) - 1;
             const unsigned lower = act & ((2u << who) - 1u);
             float l0[3], h0[3], l1[3], h1[3];
-            if (!(box_of(lower, l0, h0) + box_of(act & ~lower, l1, h1) < 0.5f * ext)) break;
+            if (!(box_of(lower, l0, h0) + box_of(act & ~lower, l1, h1) < 0.4f * ext)) break;
             act = lower;
         }
         todo &= ~act;
@@ -951,16 +951,14 @@ int knn_launch_tree(int K, const float *src, const float *query, const int32_t *
     scan_in_place(t.hist, t.tile, t.n_tiles, st);
     tree_sort_kernel<false><<<nb, KT_THREADS, 0, st>>>(src, query, so, qo, B, Ns, Nq, t);
     tree_boxes_kernel<<<(unsigned)(Ns / (LEAF * 32) + B), 1024, 0, st>>>(B, t);
-    const int share = K <= 3 ? 1 : search_share(Nq);
+    const int share = K <= 3 ? 1 : SHARED;
     const unsigned blocks = (unsigned)((Nq * share + SEARCH_THREADS - 1) / SEARCH_THREADS);
 #define S3D_KNN_SEARCH(KL, SHARE)                                                                                   \
     if (root) tree_search_kernel<KL, SHARE, true><<<blocks, SEARCH_THREADS, 0, st>>>(K, qo, B, Nq, t, idx, dist);   \
     else tree_search_kernel<KL, SHARE, false><<<blocks, SEARCH_THREADS, 0, st>>>(K, qo, B, Nq, t, idx, dist)
     if (K <= 3) { S3D_KNN_SEARCH(3, 1); }
-    else if (K <= 8 && share == 2) { S3D_KNN_SEARCH(8, 2); }
-    else if (K <= 8) { S3D_KNN_SEARCH(8, 4); }
-    else if (share == 2) { S3D_KNN_SEARCH(16, 2); }
-    else { S3D_KNN_SEARCH(16, 4); }
+    else if (K <= 8) { S3D_KNN_SEARCH(8, SHARED); }
+    else { S3D_KNN_SEARCH(16, SHARED); }
 #undef S3D_KNN_SEARCH
     if (cudaGetLastError() != cudaSuccess) return S3D_ERR_LAUNCH;
     // tied queries: a block each while they are few, otherwise the thread-per-query scan; both kernels read
