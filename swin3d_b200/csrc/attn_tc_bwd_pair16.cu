@@ -159,20 +159,21 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
                 ++ti;
                 tj = 0;
             } else {
-                ++w;
-                have = w < w_end;
-                if (have) {
-                    n = n_nx;
-                    base = base_nx;
-                    if (w + 1 < w_end) {
-                        n_nx = __ldg(P.w_sizes + w + 1);
-                        base_nx = __ldg(P.w2n + w + 1);
+                ti = tj = 0;
+                do {                              // an empty window has no items; the next one may have some
+                    ++w;
+                    have = w < w_end;
+                    if (have) {
+                        n = n_nx;
+                        base = base_nx;
+                        if (w + 1 < w_end) {
+                            n_nx = __ldg(P.w_sizes + w + 1);
+                            base_nx = __ldg(P.w2n + w + 1);
+                        }
                     }
-                    nt = (n + QT - 1) / QT;
-                    ts = nt > 0 ? (n + nt - 1) / nt : 0;      // equal tiles of at most QT voxels
-                    ti = tj = 0;
-                    have = n > 0;
-                }
+                } while (have && n < 1);
+                nt = (n + QT - 1) / QT;
+                ts = nt > 0 ? (n + nt - 1) / nt : 0;      // equal tiles of at most QT voxels
             }
             nq = have ? min(ts, n - ti * ts) : 0;
             nk = have ? min(ts, n - tj * ts) : 0;

@@ -355,6 +355,26 @@ def test_backward_kernels_at_the_edges_of_their_tiles(dtype, H, hd, ws, crse):
             assert table_row_errors(a, b, H * hd, tol, 2e-2) == [], name
 
 
+@pytest.mark.parametrize("dtype,H,hd", [("float32", 3, 8), ("float32", 1, 16), ("float16", 2, 8), ("float16", 1, 16), ("float16", 2, 16)])
+def test_windows_without_voxels_are_passed_over(dtype, H, hd):
+    """Entries of 0 at the start, in the middle and at the end of w_sizes, several windows per block so that a block's
+    range begins with some: the rows are those of the call without these entries, bit for bit."""
+    from tests.gpu_helpers import cuda_fwd_bwd
+    p = make_problem(seed=95, ws=5, H=H, hd=hd, crse="XYZ_RGB", scene=_scene_of_window_sizes(5, [40, 3, 33, 20] * 150),
+                     round_fp16=dtype == "float16")
+    full = cuda_fwd_bwd(p, getattr(torch, dtype))
+    at = np.repeat(np.arange(len(p.w_sizes) + 1), 3)              # 3 empty entries before every window and after the last
+    p.w_sizes, p.w2n = np.insert(p.w_sizes, at, 0), np.insert(p.w2n, at, np.append(p.w2n, p.N).astype(p.w2n.dtype)[at])
+    stale = [torch.full((p.N, H, hd), float("nan"), dtype=getattr(torch, dtype), device="cuda") for _ in range(12)]
+    del stale                                                     # what the allocator hands out next holds no old result
+    holes = cuda_fwd_bwd(p, getattr(torch, dtype))
+    assert np.array_equal(full[0], holes[0]) and np.array_equal(full[1], holes[1])
+    for name, a, b in zip("dq dk dv".split(), full[2], holes[2]):
+        assert np.array_equal(a, b), name
+    for name, a, b in zip("dtq dtk dtv".split(), full[2][3:], holes[2][3:]):   # fp32 atomics across blocks
+        assert rel_err(a, b) < 1e-4, name
+
+
 @pytest.mark.parametrize("H,hd,ws,crse", [(2, 8, 5, "XYZ_RGB_NORM"), (4, 8, 7, "XYZ_RGB"), (2, 8, 7, "XYZ"), (10, 8, 7, "XYZ_RGB_NORM"),
                                           (1, 16, 5, "XYZ_RGB_NORM"), (3, 16, 7, "XYZ_RGB"), (1, 16, 7, "XYZ")])
 def test_fp16_forward_at_the_edges_of_its_tiles(H, hd, ws, crse):
