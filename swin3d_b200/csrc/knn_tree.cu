@@ -20,6 +20,8 @@
 // Bound: instruction issue of the leaf evaluation for K = 3, the merges of the lists and their latency for
 // K = 16.  Measured, whole search: 8 scenes x (200 k queries, 50 k sources), K = 3: 0.42 ms, the scan of knn.cu
 // 16.9; 4 x (30 k, 120 k), K = 16: 0.37 ms (the scan: 62).
+#include <climits>
+
 #include "knn_common.cuh"
 #include "knn_kernels.cuh"
 #include "scan.cuh"
@@ -494,7 +496,7 @@ tree_search_kernel(int K, const int32_t *__restrict__ qo, int B, int64_t Nq, Tre
             }
         };
         auto visit = [&](int leaf) {
-            const float *p = points + leaf * (4 * LEAF) + sub * PER;
+            const float *p = points + (int64_t)leaf * (4 * LEAF) + sub * PER;
 #pragma unroll 2
             for (int j = 0; j < PER; j += 8) {
                 float d[8];
@@ -917,14 +919,22 @@ knn_warp_kernel(int K, const float *__restrict__ src, const float *__restrict__ 
 
 }  // namespace
 
+// Row numbers of points are int.  The kernels of this file count past the last row of a scene by less than one
+// round (the tie kernel), one batch of the warp scan or one node, so this is where they stop and the
+// thread-per-query scan takes over; offsets into the planes (128 floats per leaf) are formed in 64 bits.
+constexpr int64_t MAX_POINTS = ((int64_t)1 << 31) - (1 << 13);
+static_assert(MAX_POINTS + TIE_WARPS * 32 * TIE_PER < INT_MAX && MAX_POINTS + 2 * 32 * WARP_BATCH < INT_MAX &&
+              MAX_POINTS + LEAF * 32 < INT_MAX, "int row numbers");
+static_assert(MAX_POINTS / LEAF * 4 * LEAF > INT_MAX, "plane offsets need 64 bits");
+
 bool knn_tree_supported(int K, int B, int64_t Ns, int64_t Nq)
 {
-    return K <= 16 && Ns + Nq < ((int64_t)1 << 31) && B <= 65535;
+    return K <= 16 && Ns + Nq <= MAX_POINTS && B <= 65535;
 }
 
 bool knn_warp_wanted(int K, int B, int64_t Ns, int64_t Nq)
 {
-    return Nq * (Ns / B) <= 20000000;
+    return Ns <= MAX_POINTS && Nq * (Ns / B) <= 20000000;
 }
 
 int64_t knn_tree_bytes(int B, int64_t Ns, int64_t Nq) { return tree_bufs(nullptr, B, Ns, Nq).total; }

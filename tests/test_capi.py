@@ -74,6 +74,19 @@ def test_argument_validation_without_device():
     assert L.s3d_window_build_workspace_bytes(1000) > 1000 * 24
 
 
+def test_knn_index_stops_where_its_row_numbers_do():
+    """The search over the index counts rows in int and runs up to 3840 (the tie kernel's round) past the last
+    one of a scene: it takes no call whose rows plus that pass 2^31 - 1; below, offsets of 128 floats per
+    32 rows exceed 2^31 and are the kernel's 64-bit business."""
+    from swin3d_b200 import _lib
+    need = _lib.lib.s3d_knn_workspace_bytes
+    most = 2 ** 31 - 2 ** 13
+    assert most + 3840 < 2 ** 31 - 1
+    for K in (3, 16):
+        assert need(K, 1, most - 5, 5) > (most - 5) * 16
+        assert need(K, 1, most - 4, 5) == 0 and need(K, 1, 2 ** 31 - 10, 5) == 0
+
+
 def test_python_wrappers_reject_cpu_tensors():
     import torch
     from swin3d_b200.sparse_dl.attn.attn_coff import (SelfAttnAIOFunction, PosEmb, TableDims,
