@@ -24,6 +24,15 @@ namespace tc {
 
 constexpr int P16_STAGES = 2;
 
+// Windows of up to P16_SLOTS tiles (7^3 cells are 11) run over their tile pairs (i, j) once, j innermost: dQ of a query
+// tile is complete after its last key tile, dK and dV of every key tile with the last query tile.  Until then the thread
+// that stores a row piece keeps its sum in fp32, for dK and dV one per key tile (local memory: 0.7 KB a thread, L1 and L2
+// hold it; rows in fp16 that every pair adds to were as fast and cost half the precision: 6.0 against 3.8e-4 of the norm
+// for windows of 343 voxels).  Larger windows run over their pairs twice, for dQ (and dTq, dTv) with j innermost and
+// for dK, dV (and dTk) with i innermost, so that one sum suffices.
+constexpr int P16_SLOTS = 11;
+enum { ROLE_Q = 1, ROLE_K = 2, Q_FIRST = 4, Q_LAST = 8, K_FIRST = 16, K_LAST = 32 };
+
 template <int D>
 struct P16Split {
     static constexpr int NW = p16_warps(D);
@@ -111,7 +120,7 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
     float *s_lses = reinterpret_cast<float *>(smem + L.off_misc);       // [stage][32][2]
     float *s_dels = s_lses + P16_STAGES * 64;                           // [stage][32][2]
     int *s_rowi = reinterpret_cast<int *>(s_dels + P16_STAGES * 64);    // [stage][query tile, key tile][32]
-    int *s_n = s_rowi + P16_STAGES * 64;                                // [stage][8]: nq, nk, j > 0, i > 0, used tiles; nq = 0: no more items
+    int *s_n = s_rowi + P16_STAGES * 64;                                // [stage][8]: nq, nk, roles, slot, used tiles; nq = 0: no more items
     int *s_fail = s_n + P16_STAGES * 8;
     uint64_t *s_full = reinterpret_cast<uint64_t *>(smem + L.off_misc + 1792), *s_empty = s_full + P16_STAGES;
 
@@ -143,6 +152,7 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
         // by the row number) inside the iteration, under the tile-mask arithmetic.
         int64_t w = w_begin - 1;
         int n = 0, base = 0, nt = 0, ts = 0, ti = 0, tj = 0;
+        int unit = 0, unit_end = 0, role = 0;              // a window is one unit of both roles, or 2 nt of one
         int n_nx = 0, base_nx = 0;                         // sizes of window w + 1
         if (w_begin < w_end) {
             n_nx = __ldg(P.w_sizes + w_begin);
@@ -153,27 +163,31 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
         float cq[D], ck[D];
         // descriptor of the next item and the loads that depend on the sorted position only
         auto advance = [&]() {
-            if (have && tj + 1 < nt) {
+            if (have && (role & ROLE_Q) && tj + 1 < nt) {
                 ++tj;
-            } else if (have && ti + 1 < nt) {
+            } else if (have && (role & ROLE_K) && ti + 1 < nt) {
                 ++ti;
-                tj = 0;
+                if (role & ROLE_Q) tj = 0;
             } else {
-                ti = tj = 0;
-                do {                              // an empty window has no items; the next one may have some
+                ++unit;
+                while (unit >= unit_end) {                 // the next window with voxels
                     ++w;
                     have = w < w_end;
-                    if (have) {
-                        n = n_nx;
-                        base = base_nx;
-                        if (w + 1 < w_end) {
-                            n_nx = __ldg(P.w_sizes + w + 1);
-                            base_nx = __ldg(P.w2n + w + 1);
-                        }
+                    if (!have) break;
+                    n = n_nx;
+                    base = base_nx;
+                    if (w + 1 < w_end) {
+                        n_nx = __ldg(P.w_sizes + w + 1);
+                        base_nx = __ldg(P.w2n + w + 1);
                     }
-                } while (have && n < 1);
-                nt = (n + QT - 1) / QT;
-                ts = nt > 0 ? (n + nt - 1) / nt : 0;      // equal tiles of at most QT voxels
+                    nt = (n + QT - 1) / QT;
+                    ts = nt > 0 ? (n + nt - 1) / nt : 0;   // equal tiles of at most QT voxels
+                    unit = 0;
+                    unit_end = nt > P16_SLOTS ? 2 * nt : (nt > 0 ? 1 : 0);
+                }
+                role = unit_end == 1 ? ROLE_Q | ROLE_K : (unit < nt ? ROLE_Q : ROLE_K);
+                ti = role == ROLE_Q ? unit : 0;
+                tj = role == ROLE_K ? unit - nt : 0;
             }
             nq = have ? min(ts, n - ti * ts) : 0;
             nk = have ? min(ts, n - tj * ts) : 0;
@@ -241,8 +255,8 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
             if (lane == 0) {
                 s_n[s * 8] = nq;
                 s_n[s * 8 + 1] = nk;
-                s_n[s * 8 + 2] = tj > 0;
-                s_n[s * 8 + 3] = ti > 0;
+                s_n[s * 8 + 2] = role | (tj == 0 ? Q_FIRST : 0) | (tj + 1 == nt ? Q_LAST : 0) | (ti == 0 ? K_FIRST : 0) | (ti + 1 == nt ? K_LAST : 0);
+                s_n[s * 8 + 3] = role & ROLE_Q ? tj : 0;      // sums of dK and dV: slot
                 s_n[s * 8 + 4] = (int)used;
             }
             mbar_arrive(s_full + s);
@@ -277,6 +291,10 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
 #pragma unroll
             for (int j = 0; j < 4; ++j) dt_acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
 
+    // sums of the store phase: this thread's entries, dQ (slot 0) or dK and dV of a key tile
+    constexpr int EPT = (512 + NT - 1) / NT;
+    float4 run[P16_SLOTS][EPT][2];
+
     for (int it = 0;; ++it) {
         const int s = it % P16_STAGES;
         if (!mbar_wait(s_full + s, (it / P16_STAGES) & 1)) {
@@ -285,7 +303,8 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
         }
         consumer_sync<NT>();          // the previous item's stores are over; the flag is settled
         const int nq = s_n[s * 8], nk = s_n[s * 8 + 1];
-        const bool add_q = s_n[s * 8 + 2] != 0, add_k = s_n[s * 8 + 3] != 0;   // not the first share of dQ / of dK, dV
+        const int roles = s_n[s * 8 + 2], slot = s_n[s * 8 + 3];
+        const bool do_q = roles & ROLE_Q, do_k = roles & ROLE_K;
         const uint32_t used = (uint32_t)s_n[s * 8 + 4];
         if (nq == 0 || *s_fail) break;
         const __half *s_q = s_rows + s * (4 * ROWS), *s_do = s_q + ROWS, *s_k = s_do + ROWS, *s_v = s_k + ROWS;
@@ -374,27 +393,33 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
         for (int i = tid; i < L.R16 * QT / 4; i += NT)                       // 128 16-byte pieces per 16-row tile
             if ((used >> (i >> 7)) & 1u) {
                 const uint4 z = make_uint4(0, 0, 0, 0);
-                reinterpret_cast<uint4 *>(s_hq)[i] = z;
-                reinterpret_cast<uint4 *>(s_hv)[i] = z;
-                reinterpret_cast<uint4 *>(s_hk)[i] = z;
+                if (do_q) {
+                    reinterpret_cast<uint4 *>(s_hq)[i] = z;
+                    reinterpret_cast<uint4 *>(s_hv)[i] = z;
+                }
+                if (do_k) reinterpret_cast<uint4 *>(s_hk)[i] = z;
             }
         consumer_sync<NT>();
         // ---- histograms and pair products -----------------------------------------------------------------------
         if (wid < D) {
-            hist_query_side(s_hq + mypos, L.R16 * QT, s_P, s_DS, s_W0, s_W1, s_lut, pm.lut_stride, wid, nk, lane);
-        } else if (wid < D + NKW) {
+            if (do_q) hist_query_side(s_hq + mypos, L.R16 * QT, s_P, s_DS, s_W0, s_W1, s_lut, pm.lut_stride, wid, nk, lane);
+        } else if (wid < D + NKW && do_k) {
             for (int d = 2 * (wid - D); d < 2 * (wid - D) + 2 && d < D; ++d)
                 hist_key_side(s_hk + mypos, s_DS, s_W0, s_W1, s_lut, pm.lut_stride, d, nq, lane);
         }
         if (wid == GEMM_WARP) {
             float acc[2][2][2][4];
-            p16_zero(acc);
-            p16_pair_gemm<false>(acc, s_DS, s_k, nk, g, t);                     // dQ[q] = sum_k ds K[k]
-            p16_store(s_pg, acc, g, t);
-            p16_zero(acc);
-            p16_pair_gemm<true>(acc, s_DS, s_q, nq, g, t);                      // dK[k] = sum_q ds Q[q]
-            p16_store(s_pg + 2048, acc, g, t);
-        } else if (wid == DV_WARP) {
+            if (do_q) {
+                p16_zero(acc);
+                p16_pair_gemm<false>(acc, s_DS, s_k, nk, g, t);                 // dQ[q] = sum_k ds K[k]
+                p16_store(s_pg, acc, g, t);
+            }
+            if (do_k) {
+                p16_zero(acc);
+                p16_pair_gemm<true>(acc, s_DS, s_q, nq, g, t);                  // dK[k] = sum_q ds Q[q]
+                p16_store(s_pg + 2048, acc, g, t);
+            }
+        } else if (wid == DV_WARP && do_k) {
             float acc[2][2][2][4];
             p16_zero(acc);
             p16_pair_gemm<true>(acc, s_P, s_do, nq, g, t);                      // dV[k] = sum_q p dO[q]
@@ -402,7 +427,7 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
         }
         consumer_sync<NT>();
         // ---- dTq, dTv, dTk | dQ += histQ.Tq, dK += histK.Tk --------------------------------------------------------
-        if (dtg < 3) {
+        if (dtg < 3 && (dtg < 2 ? do_q : do_k)) {
             const __half *X = dtg == 0 ? s_q : (dtg == 1 ? s_do : s_k);
             const uint32_t *hist = dtg == 0 ? s_hq : (dtg == 1 ? s_hv : s_hk);
             uint32_t b[2][2][2][2];                            // [k-step][slot][parity][half]
@@ -449,7 +474,7 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
 #pragma unroll
                 for (int j = 0; j < 4; ++j) dt_acc[i][j] = c[j];
             }
-        } else if (side < 2) {
+        } else if (side < 2 && (side == 0 ? do_q : do_k)) {
             const __half *T = side == 0 ? P.tq : P.tk;
             const uint32_t *hist = side == 0 ? s_hq : s_hk;
             float acc[2][2][2][4];
@@ -469,22 +494,37 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
             p16_store(s_part + (side * SG + ws2) * 1024, acc, g, t);
         }
         consumer_sync<NT>();
-        // ---- reduce and store dQ (first half of the entries), dK and dV (second half), four channels each ----------
-        for (int e = tid; e < 512; e += NT) {
-            const int sd = e >> 8, xx = (e >> 3) & 31, ch = (e & 7) * 4;
-            if (xx < (sd == 0 ? nq : nk)) {
-                float4 a = *reinterpret_cast<const float4 *>(s_pg + (sd == 0 ? 0 : 2048) + xx * 32 + ch);
+        // ---- reduce dQ (first half of the entries), dK and dV (second half), four channels each; sum over the tile pairs
+        // of a row, store after the last ---------------------------------------------------------------------------
+#pragma unroll
+        for (int k = 0; k < EPT; ++k) {
+            const int e = tid + NT * k, sd = e >> 8, xx = (e >> 3) & 31, ch = (e & 7) * 4;
+            if (e < 512 && (sd == 0 ? do_q && xx < nq : do_k && xx < nk)) {
+                float4 a = *reinterpret_cast<const float4 *>(s_pg + (sd == 0 ? 0 : 2048) + xx * 32 + ch), v = make_float4(0.f, 0.f, 0.f, 0.f);
                 const float *pp = s_part + sd * SG * 1024 + xx * 32 + ch;
 #pragma unroll
                 for (int ww = 0; ww < SG; ++ww) {
                     const float4 pr = *reinterpret_cast<const float4 *>(pp + ww * 1024);
                     a.x += pr.x; a.y += pr.y; a.z += pr.z; a.w += pr.w;
                 }
-                const bool add = sd == 0 ? add_q : add_k;
-                const int64_t o = (int64_t)(sd == 0 ? s_rowq : s_rowk)[xx] * HC + co + ch;
-                // the same thread writes every share of a row
-                add_store_h4((sd == 0 ? P.dq : P.dk) + o, a, add);
-                if (sd == 1) add_store_h4(P.dv + o, *reinterpret_cast<const float4 *>(s_pg + 1024 + xx * 32 + ch), add);
+                if (sd == 1) v = *reinterpret_cast<const float4 *>(s_pg + 1024 + xx * 32 + ch);
+                const int at = sd == 0 ? 0 : slot;
+                if (!(roles & (sd == 0 ? Q_FIRST : K_FIRST))) {
+                    const float4 b = run[at][k][0];
+                    a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+                    if (sd == 1) {
+                        const float4 c = run[at][k][1];
+                        v.x += c.x; v.y += c.y; v.z += c.z; v.w += c.w;
+                    }
+                }
+                if (roles & (sd == 0 ? Q_LAST : K_LAST)) {
+                    const int64_t o = (int64_t)(sd == 0 ? s_rowq : s_rowk)[xx] * HC + co + ch;
+                    store_h4((sd == 0 ? P.dq : P.dk) + o, a);
+                    if (sd == 1) store_h4(P.dv + o, v);
+                } else {
+                    run[at][k][0] = a;
+                    if (sd == 1) run[at][k][1] = v;
+                }
             }
         }
         __syncwarp();

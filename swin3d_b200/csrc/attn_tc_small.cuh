@@ -279,16 +279,10 @@ __device__ __forceinline__ void hist_key_side(uint32_t *cell, const uint32_t *s_
     }
 }
 
-// Four fp16 channels of a result row: written, or added to what the same thread wrote before.
-__device__ __forceinline__ void add_store_h4(__half *p, float4 a, bool add)
+// Four fp16 channels of a result row.
+__device__ __forceinline__ void store_h4(__half *p, float4 a)
 {
-    uint2 *d = reinterpret_cast<uint2 *>(p);
-    if (add) {
-        const uint2 old = *d;
-        const float2 lo = __half22float2(u32_as_h2(old.x)), hi = __half22float2(u32_as_h2(old.y));
-        a.x += lo.x; a.y += lo.y; a.z += hi.x; a.w += hi.y;
-    }
-    *d = make_uint2(h2_as_u32(__floats2half2_rn(a.x, a.y)), h2_as_u32(__floats2half2_rn(a.z, a.w)));
+    *reinterpret_cast<uint2 *>(p) = make_uint2(h2_as_u32(__floats2half2_rn(a.x, a.y)), h2_as_u32(__floats2half2_rn(a.z, a.w)));
 }
 
 __device__ __forceinline__ void store_part(float *red, const float (&part)[2][2][4], int g, int t)

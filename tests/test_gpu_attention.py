@@ -375,6 +375,21 @@ def test_windows_without_voxels_are_passed_over(dtype, H, hd):
         assert rel_err(a, b) < 1e-4, name
 
 
+@pytest.mark.parametrize("crse", ["XYZ", "XYZ_RGB", "XYZ_RGB_NORM"])
+def test_fp16_gradients_of_large_windows_are_rounded_once(crse):
+    """dQ, dK, dV of windows of 11 tiles (343 voxels) and 22: the error does not grow with the tiles.  An element of a
+    gradient carries the rounding of the result, of its ds or p and of a histogram entry, each 2^-11 / sqrt(3) of
+    the norm at most: 2^-11 together.  (Rounded after every tile pair, eleven times: 6e-4.)"""
+    from tests.gpu_helpers import cuda_fwd_bwd
+    p = make_problem(seed=96, ws=7, H=2, hd=16, crse=crse, scene=_scene_of_window_sizes(7, [343] * 3), round_fp16=True)
+    p.w_sizes, p.w2n = np.array([686, 343], p.w_sizes.dtype), p.w2n[[0, 2]]
+    _, _, g_ref = oracle_fwd_bwd(p, np.float64)
+    _, _, grads = cuda_fwd_bwd(p, torch.float16)
+    for name, a, b in zip("dq dk dv".split(), grads, g_ref):
+        for rows in (p.n2n[:686], p.n2n[686:]):
+            assert np.linalg.norm(a[rows] - b[rows]) < 2.0 ** -11 * np.linalg.norm(b[rows]), name
+
+
 @pytest.mark.parametrize("H,hd,ws,crse", [(2, 8, 5, "XYZ_RGB_NORM"), (4, 8, 7, "XYZ_RGB"), (2, 8, 7, "XYZ"), (10, 8, 7, "XYZ_RGB_NORM"),
                                           (1, 16, 5, "XYZ_RGB_NORM"), (3, 16, 7, "XYZ_RGB"), (1, 16, 7, "XYZ")])
 def test_fp16_forward_at_the_edges_of_its_tiles(H, hd, ws, crse):
