@@ -325,29 +325,47 @@ struct UsedTiles {
     }
 };
 
-// The share of block blockIdx.x of gridDim.x: a contiguous range of equal cost, the cost of a window being its number of
-// 32 x 32 tile pairs.  Every block scans all window sizes (a few hundred KB from L2), so the assignment needs no global
-// counter and is the same on every run.  The range is [(w_begin, i_begin), (w_end, i_end)) in (window, query tile) units,
-// a query tile costing as many tile pairs as its window has tiles; with whole windows (BY_WINDOW) i_begin = i_end = 0.
-// Windows of fewer than n_min or more than n_max voxels cost nothing.
+// Work units of a window: `count` of them, of equal cost.
+struct Units {
+    int count;
+    int64_t each;
+};
+
+// A window of n voxels as one unit (whole windows), and as one unit per query tile; the cost is the number of 32 x 32
+// tile pairs.
+struct UnitsWhole {
+    __device__ __forceinline__ Units operator()(int n) const
+    {
+        const int64_t nt = (n + QT - 1) / QT;
+        return {nt > 0 ? 1 : 0, nt * nt};
+    }
+};
+struct UnitsPerQueryTile {
+    int n_min, n_max;                             // windows of other sizes have no units
+    __device__ __forceinline__ Units operator()(int n) const
+    {
+        const int nt = n >= n_min && n <= n_max ? (n + QT - 1) / QT : 0;
+        return {nt, nt};
+    }
+};
+
+// The share of block blockIdx.x of gridDim.x: a contiguous range [(w_begin, i_begin), (w_end, i_end)) of (window, unit)
+// of equal cost.  Every block scans all window sizes (a few hundred KB from L2), so the assignment needs no global
+// counter and is the same on every run.  With one unit per window i_begin = i_end = 0.
 // All NTA threads of the block call this; scratch: (NTA + 6) * 8 bytes of shared memory.
-template <int NTA, bool BY_WINDOW>
-__device__ __forceinline__ void balanced_units(const int32_t *__restrict__ w_sizes, int64_t W, void *scratch, int64_t &w_begin,
-                                               int64_t &w_end, int &i_begin, int &i_end, int n_min = 1, int n_max = 0x7fffffff)
+template <int NTA, typename F>
+__device__ __forceinline__ void balanced_units(const int32_t *__restrict__ w_sizes, int64_t W, void *scratch, const F units, int64_t &w_begin,
+                                               int64_t &w_end, int &i_begin, int &i_end)
 {
     int64_t *s_seg = static_cast<int64_t *>(scratch);                  // [NTA + 1] segment sums, then their exclusive scan
-    int64_t *s_range = s_seg + NTA + 2;                                // [4] window and tile of the first unit, of one past the last
+    int64_t *s_range = s_seg + NTA + 2;                                // [4] window and unit of the first, of one past the last
     const int tid = threadIdx.x, lane = tid & 31;
     const int64_t per = (W + NTA - 1) / NTA;
     const int64_t w0 = (int64_t)tid * per, w1 = w0 + per < W ? w0 + per : W;
-    auto tiles = [&](int64_t w) {
-        const int n = __ldg(w_sizes + w);
-        return (int64_t)(n >= n_min && n <= n_max ? (n + QT - 1) / QT : 0);
-    };
     int64_t sum = 0;
     for (int64_t w = w0; w < w1; ++w) {
-        const int64_t nt = tiles(w);
-        sum += nt * nt;
+        const Units u = units(__ldg(w_sizes + w));
+        sum += u.count * u.each;
     }
     s_seg[tid] = sum;
     __syncthreads();
@@ -368,7 +386,7 @@ __device__ __forceinline__ void balanced_units(const int32_t *__restrict__ w_siz
     }
     __syncthreads();
     const int64_t total = s_seg[NTA];
-    // the first unit (window) at which the cumulative cost reaches the target
+    // the first unit at which the cumulative cost reaches the target
     const int64_t lo_t = total * blockIdx.x / gridDim.x, hi_t = total * (blockIdx.x + 1) / gridDim.x;
     const int64_t mine = s_seg[tid], next = tid + 1 < NTA ? s_seg[tid + 1] : total + 1;
 #pragma unroll
@@ -379,13 +397,13 @@ __device__ __forceinline__ void balanced_units(const int32_t *__restrict__ w_siz
         } else if (mine <= target && target < next && w0 < w1) {
             int64_t acc = mine, w = w0, i = 0;
             for (; w < w1 && acc < target; ++w) {
-                const int64_t nt = tiles(w);
-                if (!BY_WINDOW && acc + nt * nt > target) {
-                    i = (target - acc + nt - 1) / nt;
-                    if (i < nt) break;
+                const Units u = units(__ldg(w_sizes + w));
+                if (acc + u.count * u.each > target) {
+                    i = (target - acc + u.each - 1) / u.each;
+                    if (i < u.count) break;
                     i = 0;
                 }
-                acc += nt * nt;
+                acc += u.count * u.each;
             }
             s_range[2 * k] = w;
             s_range[2 * k + 1] = i;
@@ -403,7 +421,7 @@ template <int NTA>
 __device__ __forceinline__ void balanced_range(const int32_t *__restrict__ w_sizes, int64_t W, void *scratch, int64_t &w_begin, int64_t &w_end)
 {
     int i_begin, i_end;
-    balanced_units<NTA, true>(w_sizes, W, scratch, w_begin, w_end, i_begin, i_end);
+    balanced_units<NTA>(w_sizes, W, scratch, UnitsWhole{}, w_begin, w_end, i_begin, i_end);
 }
 
 // Head modes of the tiled kernels.  A thread block always works on two "slots" packed as half2:

@@ -31,6 +31,58 @@ constexpr int P16_STAGES = 2;
 // for windows of 343 voxels).  Larger windows run over their pairs twice, for dQ (and dTq, dTv) with j innermost and
 // for dK, dV (and dTk) with i innermost, so that one sum suffices.
 constexpr int P16_SLOTS = 11;
+//
+// The same two halves serve calls of few windows: a block that takes whole windows runs over up to 121 pairs in a row
+// while others have none.  A window of several tiles is then 2 nt units, (query tile i, all j) for dQ and (key tile j, all
+// i) for dK and dV, dealt to the blocks one by one.  An item of one role costs about two thirds of one of both.
+struct P16UnitsWhole {
+    __device__ __forceinline__ Units operator()(int n) const
+    {
+        const int64_t nt = (n + QT - 1) / QT;
+        return {nt > 0 ? 1 : 0, (nt > P16_SLOTS ? 4 : 3) * nt * nt};
+    }
+};
+struct P16UnitsSplit {
+    __device__ __forceinline__ Units operator()(int n) const
+    {
+        const int nt = (n + QT - 1) / QT;
+        return nt > 1 ? Units{2 * nt, 2 * nt} : Units{nt, 3};
+    }
+};
+
+// Whether the windows of this call are split: the longest share of a block, estimated for both ways.  Whole windows: the
+// average share and half of the largest window, or that window alone; split: the average and the largest unit.  All
+// blocks come to the same answer.  Called by all NTA threads; scratch: 32 bytes of shared memory.
+template <int NTA>
+__device__ __forceinline__ bool split_windows(const int32_t *__restrict__ w_sizes, int64_t W, void *scratch)
+{
+    if (W >= 32 * (int64_t)gridDim.x) return false;               // enough windows for the shares to even out
+    unsigned long long *s_sum = static_cast<unsigned long long *>(scratch);   // tile pairs, windows of one tile
+    int *s_max = reinterpret_cast<int *>(s_sum + 2);
+    if (threadIdx.x == 0) {
+        s_sum[0] = s_sum[1] = 0;
+        *s_max = 0;
+    }
+    __syncthreads();
+    unsigned long long sum = 0, single = 0;
+    int mx = 0;
+    for (int64_t w = threadIdx.x; w < W; w += NTA) {
+        const int nt = (__ldg(w_sizes + w) + QT - 1) / QT;
+        if (nt > 0) sum += (unsigned long long)nt * nt;
+        single += nt == 1;
+        mx = max(mx, nt);
+    }
+    atomicAdd(s_sum, sum);
+    atomicAdd(s_sum + 1, single);
+    atomicMax(s_max, mx);
+    __syncthreads();
+    const float all = (float)s_sum[0], one = (float)s_sum[1], nt = (float)*s_max, share = 1.f / gridDim.x;
+    __syncthreads();
+    const float whole = 3.f * fmaxf(all * share + 0.5f * nt * nt, nt * nt);
+    const float split = (4.f * (all - one) + 3.f * one) * share + 2.f * nt;
+    return split < whole;
+}
+
 enum { ROLE_Q = 1, ROLE_K = 2, Q_FIRST = 4, Q_LAST = 8, K_FIRST = 16, K_LAST = 32 };
 
 template <int D>
@@ -140,9 +192,12 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
         const int row = perm_table_row(pm, r);
         s_map[r] = row < 0 ? (uint16_t)0xffff : (uint16_t)row;
     }
-    // this block's windows: a contiguous range of equal cost
+    // this block's share: a contiguous range of equal cost
+    const bool split = split_windows<(NW + 1) * 32>(P.w_sizes, P.W, smem + L.off_pq);
     int64_t w_begin, w_end;
-    balanced_range<(NW + 1) * 32>(P.w_sizes, P.W, smem + L.off_pq, w_begin, w_end);
+    int u_begin, u_end;                          // first unit of window w_begin, one past the last of window w_end
+    if (split) balanced_units<(NW + 1) * 32>(P.w_sizes, P.W, smem + L.off_pq, P16UnitsSplit{}, w_begin, w_end, u_begin, u_end);
+    else balanced_units<(NW + 1) * 32>(P.w_sizes, P.W, smem + L.off_pq, P16UnitsWhole{}, w_begin, w_end, u_begin, u_end);
 
     if (wid == NW) {
         // ================================ producer warp ================================================
@@ -152,9 +207,10 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
         // by the row number) inside the iteration, under the tile-mask arithmetic.
         int64_t w = w_begin - 1;
         int n = 0, base = 0, nt = 0, ts = 0, ti = 0, tj = 0;
-        int unit = 0, unit_end = 0, role = 0;              // a window is one unit of both roles, or 2 nt of one
+        int unit = 0, unit_end = 0, role = 0;              // a window is one unit of both roles, or (halves) 2 nt of one
+        bool halves = false;
         int n_nx = 0, base_nx = 0;                         // sizes of window w + 1
-        if (w_begin < w_end) {
+        if (w_begin < P.W) {
             n_nx = __ldg(P.w_sizes + w_begin);
             base_nx = __ldg(P.w2n + w_begin);
         }
@@ -172,20 +228,21 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
                 ++unit;
                 while (unit >= unit_end) {                 // the next window with voxels
                     ++w;
-                    have = w < w_end;
+                    have = w < w_end || (w == w_end && u_end > 0);
                     if (!have) break;
                     n = n_nx;
                     base = base_nx;
-                    if (w + 1 < w_end) {
+                    if (w + 1 < P.W) {
                         n_nx = __ldg(P.w_sizes + w + 1);
                         base_nx = __ldg(P.w2n + w + 1);
                     }
                     nt = (n + QT - 1) / QT;
                     ts = nt > 0 ? (n + nt - 1) / nt : 0;   // equal tiles of at most QT voxels
-                    unit = 0;
-                    unit_end = nt > P16_SLOTS ? 2 * nt : (nt > 0 ? 1 : 0);
+                    halves = nt > P16_SLOTS || (split && nt > 1);
+                    unit = w == w_begin ? u_begin : 0;
+                    unit_end = w == w_end ? u_end : (halves ? 2 * nt : (nt > 0 ? 1 : 0));
                 }
-                role = unit_end == 1 ? ROLE_Q | ROLE_K : (unit < nt ? ROLE_Q : ROLE_K);
+                role = !halves ? ROLE_Q | ROLE_K : (unit < nt ? ROLE_Q : ROLE_K);
                 ti = role == ROLE_Q ? unit : 0;
                 tj = role == ROLE_K ? unit - nt : 0;
             }
@@ -295,7 +352,8 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
     constexpr int EPT = (512 + NT - 1) / NT;
     float4 run[P16_SLOTS][EPT][2];
 
-    for (int it = 0;; ++it) {
+    int it = 0;
+    for (;; ++it) {
         const int s = it % P16_STAGES;
         if (!mbar_wait(s_full + s, (it / P16_STAGES) & 1)) {
             *s_fail = 1;
@@ -532,7 +590,7 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
     }
 
     // ---- the table gradients of this block -----------------------------------------------------------------------------
-    if (dtg < 3) {
+    if (dtg < 3 && it > 0) {
         float *dst = dtg == 0 ? P.dtq : (dtg == 1 ? P.dtv : P.dtk);
 #pragma unroll 1
         for (int i = 0; i < NU; ++i) {
@@ -559,7 +617,6 @@ static int launch_pair16(const P16Params &p, const CrseMeta &meta, const PermMet
     if (rc != S3D_OK) return rc;
     const int hp = p.H / 2;
     int gx = sms / hp;
-    if (gx > p.W) gx = (int)p.W;
     if (gx < 1) gx = 1;
     kern<<<dim3((unsigned)gx, (unsigned)hp), (p16_warps(D) + 1) * 32, L.total, st>>>(p, pm, make_pair_consts(meta));
     const cudaError_t le = cudaGetLastError();

@@ -20,6 +20,8 @@
 // Bound: latency between the barriers and shared-memory wavefronts.  Second stage of Swin3D-L, 144 k voxels, 10 heads:
 // 3.48 -> 3.18 ms against a tiled kernel with an online softmax (all row tiles, whole windows per block); deepest stage of
 // one room (4 windows of up to 150 voxels, 24 heads): 96 -> 54 us.
+#include <climits>
+
 #include "attn_kernels.cuh"
 #include "attn_tc.cuh"
 #include "attn_tc_pair16.cuh"
@@ -124,7 +126,7 @@ attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, c
     }
     int64_t w_begin, w_end;
     int i_begin, i_end;                          // first query tile of window w_begin, one past the last of window w_end
-    balanced_units<(NW + 1) * 32, false>(P.w_sizes, P.W, smem + L.off_pq, w_begin, w_end, i_begin, i_end);
+    balanced_units<(NW + 1) * 32>(P.w_sizes, P.W, smem + L.off_pq, UnitsPerQueryTile{1, INT_MAX}, w_begin, w_end, i_begin, i_end);
 
     if (wid == NW) {
         // ================================ producer warp ================================================

@@ -137,7 +137,7 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
     }
     int64_t w_begin, w_end;
     int i_begin, i_end;                          // first query tile of window w_begin, one past the last of window w_end
-    balanced_units<(NW + 1) * 32, false>(P.w_sizes, P.W, smem + L.off_pq, w_begin, w_end, i_begin, i_end, P.n_min, P.n_max);
+    balanced_units<(NW + 1) * 32>(P.w_sizes, P.W, smem + L.off_pq, UnitsPerQueryTile{P.n_min, P.n_max}, w_begin, w_end, i_begin, i_end);
 
     if (wid == NW) {
         // ================================ producer warp ================================================

@@ -390,6 +390,41 @@ def test_fp16_gradients_of_large_windows_are_rounded_once(crse):
             assert np.linalg.norm(a[rows] - b[rows]) < 2.0 ** -11 * np.linalg.norm(b[rows]), name
 
 
+@pytest.mark.parametrize("crse", ["XYZ", "XYZ_RGB", "XYZ_RGB_NORM"])
+def test_fp16_backward_gives_the_same_rows_whether_windows_are_split_or_not(crse):
+    """With one pair of heads there are more blocks than windows and a window is dealt out by query and by key tiles;
+    with 148 pairs a block takes whole windows.  A row's sum runs over the tiles in the same order."""
+    from tests.gpu_helpers import dev
+    from swin3d_b200.sparse_dl.attn import attn_coff as C
+    H = 296
+    p = make_problem(seed=97, ws=7, H=2, hd=16, crse=crse, scene=_scene_of_window_sizes(7, [343, 343, 343, 343, 40, 33, 5, 320, 64]))
+    order = np.argsort(-p.w_sizes, kind="stable")
+    n2n = np.concatenate([p.n2n[a:a + n] for a, n in zip(p.w2n[order], p.w_sizes[order])])
+    nc = np.concatenate([p.n_crse[a:a + n] for a, n in zip(p.w2n[order], p.w_sizes[order])])
+    sizes = [686] + sorted(p.w_sizes.tolist(), reverse=True)[2:]  # 22, 11, 11, 10, 2, 2, 2 and 1 tiles
+    w = np.array(sizes, np.int32)
+    geo = (dev(w), dev((np.cumsum(w) - w).astype(np.int32)), dev(n2n), dev(nc))
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    rnd = lambda *s: torch.randn(s, generator=gen, device="cuda").half()
+    rows = sum(p.sizes) // 32
+    q, k, v, g = (rnd(p.N, H, 16) for _ in range(4))
+    t = [rnd(rows, H, 16) * 0.02 for _ in range(3)]
+
+    def run(h):
+        x = [a[:, :h].contiguous() for a in (q, k, v, g)]
+        tab = [a[:, :h].reshape(-1).contiguous() for a in t]
+        size = [s // 32 * h * 16 for s in p.sizes]
+        out, lse = C.attn_forward_raw(*x[:3], *tab, size, *geo)
+        return C.attn_backward_raw(*x[:3], *tab, size, *geo, out, lse, x[3])
+
+    few, many = run(2), run(H)
+    for name, a, b in zip("dq dk dv".split(), few, many):
+        assert torch.equal(a, b[:, :2]), name
+    for name, a, b in zip("dtq dtk dtv".split(), few[3:], many[3:]):           # summed over the blocks in another order
+        a, b = a.view(rows, 2, 16), b.view(rows, H, 16)[:, :2]
+        assert rel_err(a.cpu().numpy(), b.cpu().numpy()) < 1e-4, name
+
+
 @pytest.mark.parametrize("H,hd,ws,crse", [(2, 8, 5, "XYZ_RGB_NORM"), (4, 8, 7, "XYZ_RGB"), (2, 8, 7, "XYZ"), (10, 8, 7, "XYZ_RGB_NORM"),
                                           (1, 16, 5, "XYZ_RGB_NORM"), (3, 16, 7, "XYZ_RGB"), (1, 16, 7, "XYZ")])
 def test_fp16_forward_at_the_edges_of_its_tiles(H, hd, ws, crse):
