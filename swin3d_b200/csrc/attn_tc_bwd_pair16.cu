@@ -88,8 +88,8 @@ enum { ROLE_Q = 1, ROLE_K = 2, Q_FIRST = 4, Q_LAST = 8, K_FIRST = 16, K_LAST = 3
 template <int D>
 struct P16Split {
     static constexpr int NW = p16_warps(D);
-    static constexpr int DTW = D == 9 ? 3 : (D == 6 ? 2 : 1);        // gradient warps per table
-    static constexpr int NU = D == 9 ? 8 : (D == 6 ? 10 : 12);       // row tiles per gradient warp, at most
+    static constexpr int DTW = D == 3 ? 2 : 3;                       // gradient warps per table
+    static constexpr int NU = D == 9 ? 8 : (D == 6 ? 7 : 6);        // row tiles per gradient warp, at most
     static constexpr int HT0 = 3 * DTW;                              // first warp of the hist.T products
     static constexpr int SG = (NW - HT0) / 2;                        // warps per side of them
 };

@@ -13,7 +13,7 @@ namespace s3d {
 namespace tc {
 
 constexpr int P16_RS = 40;                       // halves per staged voxel row: 32 + 8, so that 8 rows start in different banks
-__host__ __device__ constexpr int p16_warps(int D) { return D == 9 ? 15 : (D == 6 ? 11 : 7); }
+__host__ __device__ constexpr int p16_warps(int D) { return D == 3 ? 11 : 15; }
 
 __device__ __forceinline__ void mma_f32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
