@@ -546,7 +546,7 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
                 const P16TileB cur = tile;
                 const int nx = tiles.next();
                 if (nx >= 0) tile.fetch(T, HC, co, s_map, nx, g, t);
-                p16_hist_t(acc, hist, cur, ks, lane, g, t);
+                p16_hist_t(acc, hist, P16FragB(cur), ks, lane, g, t);
                 ks = nx;
             }
             p16_store(s_part + (side * SG + ws2) * 1024, acc, g, t);

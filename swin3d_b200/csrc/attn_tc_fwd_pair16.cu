@@ -13,7 +13,10 @@
 //   histogram  warp d: hist[row][q] += p for dimension d; warp D: P.V                                      [tensor cores]
 //   products   += hist.Tv, row tiles dealt to the warps                                                   [tensor cores]
 //   merge      reduce over the warps, merge, store after the last key tile
-// Rows are numbered and row tiles skipped as in the backward (PermMeta); table operands come from L1/L2 a tile ahead.
+// Rows are numbered and row tiles skipped as in the backward (PermMeta); the producer lists the used tiles.  The three
+// tables of the pair of heads stand in shared memory in the order in which the lanes of an mma take them (71 KB at 23 row
+// tiles; fetched from L1/L2 for every item through the row map, a tile ahead, the projections took 4.7 k cycles of an
+// item's 18 k and the products 6.8 k).
 //
 // The blocks take contiguous ranges of (window, query tile) units of equal cost, so that the deep stages -- a handful of
 // windows of some hundred voxels -- still spread over the GPU.
@@ -32,18 +35,18 @@ namespace s3d {
 namespace tc {
 
 constexpr int F16_STAGES = 2;
-__host__ __device__ constexpr int f16_warps(int D) { return D == 9 ? 15 : (D == 6 ? 11 : 8); }   // the merge takes 256 threads
+__host__ __device__ constexpr int f16_warps(int D) { return 15; }   // with the producer, four warps per scheduler
 
 // Warps of the hist.Tv products: their partial outputs (4 KB each) go where P_k was.
 template <int D>
 struct F16Split {
     static constexpr int NW = f16_warps(D);
-    static constexpr int NHT = D == 9 ? 12 : (D == 6 ? 8 : 6);
+    static constexpr int NHT = D == 9 ? 12 : (D == 6 ? 9 : 6);
 };
 
 struct F16Smem {
     int R16, Rp;
-    int off_pq, off_pk, off_e, off_rows, off_c, off_lut, off_map, off_misc, total;
+    int off_pq, off_pk, off_e, off_rows, off_c, off_ta, off_tb, off_lut, off_map, off_misc, total;
 };
 
 template <int D>
@@ -59,6 +62,8 @@ __host__ __device__ inline F16Smem make_f16_layout(int R, int lut_entries)
     L.off_e = off; off += 2 * 32 * ES * 8;                           // pair entries, two planes; S0 before
     L.off_rows = off; off += F16_STAGES * 3 * 32 * P16_RS * 2;       // Q (query tile), K, V (key tile), per stage
     L.off_c = off; off += F16_STAGES * 2 * 32 * 12 * 4;
+    L.off_ta = off; off += 2 * (L.R16 / 16) * 1024;                  // Tq and Tk as operands of the projections
+    L.off_tb = off; off += (L.R16 / 16) * 1024;                      // Tv as operand of the products
     L.off_lut = off; off += (lut_entries * 2 + 15) / 16 * 16;
     L.off_map = off; off += (L.R16 * 2 + 15) / 16 * 16;
     L.off_misc = off; off += 6144;
@@ -99,13 +104,16 @@ attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, c
     float *s_part = reinterpret_cast<float *>(smem + L.off_pk);      // [NHT][32][32]
     __half *s_rows = reinterpret_cast<__half *>(smem + L.off_rows);  // [stage][Q,K,V][32][RS]
     float *s_cs = reinterpret_cast<float *>(smem + L.off_c);         // [stage][query tile, key tile][32][12]
+    uint4 *s_ta = reinterpret_cast<uint4 *>(smem + L.off_ta);        // [Tq, Tk][row tile][2][lane]
+    uint4 *s_tb = reinterpret_cast<uint4 *>(smem + L.off_tb);        // [row tile][2][lane]
     uint16_t *s_lut = reinterpret_cast<uint16_t *>(smem + L.off_lut);
     uint16_t *s_map = reinterpret_cast<uint16_t *>(smem + L.off_map);
     float *s_max = reinterpret_cast<float *>(smem + L.off_misc);     // [32][2]
     float *s_lsum = s_max + 64;                                      // [NW][32][2]
     int *s_rowi = reinterpret_cast<int *>(s_lsum + 16 * 64);         // [stage][32] rows of the query tile
-    int *s_n = s_rowi + F16_STAGES * 32;                             // [stage][8]: nq, nk, first key tile, last key tile, used tiles; nq = 0: no more items
+    int *s_n = s_rowi + F16_STAGES * 32;                             // [stage][8]: nq, nk, first key tile, last key tile, used tiles, stop
     int *s_fail = s_n + F16_STAGES * 8;
+    uint8_t *s_tiles = reinterpret_cast<uint8_t *>(s_fail + 1);      // [stage][32] the used tiles in order
     uint64_t *s_full = reinterpret_cast<uint64_t *>(smem + L.off_misc + 6144 - 64), *s_empty = s_full + F16_STAGES;
 
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -123,6 +131,26 @@ attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, c
     for (int r = tid; r < L.R16; r += blockDim.x) {
         const int row = perm_table_row(pm, r);
         s_map[r] = row < 0 ? (uint16_t)0xffff : (uint16_t)row;
+    }
+    __syncthreads();
+    // the tables of this pair of heads, in the order the lanes of an mma take them
+    const int g = lane >> 2, t = lane & 3, n_mt = L.R16 / 16;
+    for (int u = wid; u < 3 * n_mt; u += NW + 1) {
+        const int tab = u / n_mt, mt = u - tab * n_mt;
+        if (tab < 2) {
+            P16TileA a;
+            a.fetch(tab == 0 ? P.tq : P.tk, HC, co, s_map, mt, g, t);
+            uint4 *o = s_ta + u * 64 + lane;
+            o[0] = make_uint4(a.f[0][0].x, a.f[0][0].y, a.f[0][1].x, a.f[0][1].y);
+            o[32] = make_uint4(a.f[1][0].x, a.f[1][0].y, a.f[1][1].x, a.f[1][1].y);
+        } else {
+            P16TileB raw;
+            raw.fetch(P.tv, HC, co, s_map, mt, g, t);
+            const P16FragB f(raw);
+            uint4 *o = s_tb + mt * 64 + lane;
+            o[0] = make_uint4(f.b[0][0][0], f.b[0][0][1], f.b[0][1][0], f.b[0][1][1]);
+            o[32] = make_uint4(f.b[1][0][0], f.b[1][0][1], f.b[1][1][0], f.b[1][1][1]);
+        }
     }
     int64_t w_begin, w_end;
     int i_begin, i_end;                          // first query tile of window w_begin, one past the last of window w_end
@@ -185,7 +213,7 @@ attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, c
         };
         advance();
         for (int it = 0;; ++it) {
-            const uint32_t used = item_tile_mask<D>(cq, ck, nq, nk, s_lut, pm, pc, lane);
+            const uint32_t used = item_tile_mask<D>(cq, ck, nq, nk, s_lut, pm, pc, lane) & (n_mt < 32 ? (1u << n_mt) - 1u : 0xffffffffu);
             const int s = it % F16_STAGES;
             bool stop = !have;
             if (it >= F16_STAGES && !mbar_wait(s_empty + s, ((it / F16_STAGES) - 1) & 1)) {
@@ -201,6 +229,7 @@ attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, c
                 cs[384 + lane * 12 + d] = ck[d];
             }
             s_rowi[s * 32 + lane] = rowq;
+            if ((used >> lane) & 1u) s_tiles[s * 32 + __popc(used & ((1u << lane) - 1u))] = (uint8_t)lane;
             if (lane == 0) {
                 s_n[s * 8] = nq;
                 s_n[s * 8 + 1] = nk;
@@ -221,8 +250,7 @@ attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, c
     }
 
     // ==================================== consumer warps ===============================================
-    const int g = lane >> 2, t = lane & 3;
-    const int n_mt = L.R16 / 16, Rp = L.Rp;
+    const int Rp = L.Rp;
     const int mypos = qpos(lane);
     const bool od = g & 1;
     constexpr float LOG2E = 1.4426950408889634f;
@@ -242,30 +270,29 @@ attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, c
         const int nq = s_n[s * 8], nk = s_n[s * 8 + 1];
         const bool first = s_n[s * 8 + 2] != 0, last = s_n[s * 8 + 3] != 0;
         const uint32_t used = (uint32_t)s_n[s * 8 + 4];
+        const int n_used = __popc(used);
+        const uint8_t *tiles = s_tiles + s * 32;
         if (s_n[s * 8 + 5] || *s_fail) break;
         const __half *s_q = s_rows + s * (3 * ROWS), *s_k = s_q + ROWS, *s_v = s_k + ROWS;
         const float *s_c = s_cs + s * 768, *s_ck = s_c + 384;
         if (tid < 64) s_max[tid] = -INFINITY;
         // ---- projections, S0 ------------------------------------------------------------------------------------
         if (pside < 2) {
-            const __half *T = pside == 0 ? P.tq : P.tk;
-            UsedTiles tiles(used, n_mt, wsub, HALF);
-            int mt = tiles.next();
-            P16TileA tile;
-            if (mt >= 0) tile.fetch(T, HC, co, s_map, mt, g, t);
             const int nv = pside == 0 ? nq : nk;
             uint2 bf[8];
             p16_feat_frag(bf, pside == 0 ? s_q : s_k, nv, g, t);
 #pragma unroll 1
-            while (mt >= 0) {
-                const P16TileA cur = tile;
-                const int nx = tiles.next();
-                if (nx >= 0) tile.fetch(T, HC, co, s_map, nx, g, t);
+            for (int i = wsub; i < n_used; i += HALF) {
+                const int mt = tiles[i];
+                const uint4 *f = s_ta + (pside * n_mt + mt) * 64 + lane;
+                const uint4 x = f[0], y = f[32];
+                P16TileA cur;
+                cur.f[0][0] = make_uint2(x.x, x.y); cur.f[0][1] = make_uint2(x.z, x.w);
+                cur.f[1][0] = make_uint2(y.x, y.y); cur.f[1][1] = make_uint2(y.z, y.w);
                 uint32_t d0[8], d1[8];
                 p16_project(d0, d1, cur, bf, nv, od);
                 if (pside == 0) store_lane_major(s_pq, d0, d1, mt, g, t);
                 else store_key_major(s_pk, d0, d1, mt, Rp, nv, g, t);
-                mt = nx;
             }
         }
         for (int u = NW - 1 - wid; u < 16; u += NW) {
@@ -380,17 +407,11 @@ attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, c
         consumer_sync<NT>();
         // ---- O += hist . Tv ---------------------------------------------------------------------------------------
         if (wid < NHT) {
-            UsedTiles tiles(used, n_mt, wid, NHT);
-            int ks = tiles.next();
-            P16TileB tile;
-            if (ks >= 0) tile.fetch(P.tv, HC, co, s_map, ks, g, t);
 #pragma unroll 1
-            while (ks >= 0) {
-                const P16TileB cur = tile;
-                const int nx = tiles.next();
-                if (nx >= 0) tile.fetch(P.tv, HC, co, s_map, nx, g, t);
-                p16_hist_t(acc, s_hist, cur, ks, lane, g, t);
-                ks = nx;
+            for (int i = wid; i < n_used; i += NHT) {
+                const int ks = tiles[i];
+                const uint4 *f = s_tb + ks * 64 + lane;
+                p16_hist_t(acc, s_hist, P16FragB(f[0], f[32]), ks, lane, g, t);
             }
             p16_store(s_part + wid * 1024, acc, g, t);       // P_k is dead since the scores
         }

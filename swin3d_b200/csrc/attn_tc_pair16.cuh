@@ -52,6 +52,22 @@ struct P16TileB {
     }
 };
 
+// The operands of the products themselves: b[slot][even / odd channels][half].
+struct P16FragB {
+    uint32_t b[2][2][2];
+    __device__ __forceinline__ explicit P16FragB(const P16TileB &tile)
+    {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                b[h][0][half] = pack_lo(tile.raw[h][half][0], tile.raw[h][half][1]);
+                b[h][1][half] = pack_hi(tile.raw[h][half][0], tile.raw[h][half][1]);
+            }
+    }
+    __device__ __forceinline__ P16FragB(const uint4 &x, const uint4 &y) : b{{{x.x, x.y}, {x.z, x.w}}, {{y.x, y.y}, {y.z, y.w}}} {}
+};
+
 // acc[slot][even / odd channels][m-tile] += A . rows with A from a [32][ES] plane of half2 pair entries: TRANSPOSED = false:
 // m = query, k = key (entry [k][m]); true: m = key, k = query (entry [m][k]).
 // WORDS: 4-byte words per entry (the half2 comes first).
@@ -151,7 +167,7 @@ __device__ __forceinline__ void p16_dot_block(float (&c)[4], const __half *Y, in
 }
 
 // acc += hist(16 rows of k-step ks) . T(the same rows) for the 32 voxels (m).
-__device__ __forceinline__ void p16_hist_t(float (&acc)[2][2][2][4], const uint32_t *hist, const P16TileB &tb, int ks, int lane, int g, int t)
+__device__ __forceinline__ void p16_hist_t(float (&acc)[2][2][2][4], const uint32_t *hist, const P16FragB &tb, int ks, int lane, int g, int t)
 {
     uint4 y[4];
     load_hist_rows(y, hist, ks, lane, g, t);       // y[i] = row t + 4i, queries {g, g+8, g+16, g+24}
@@ -162,12 +178,9 @@ __device__ __forceinline__ void p16_hist_t(float (&acc)[2][2][2][4], const uint3
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            const uint32_t b0 = p == 0 ? pack_lo(tb.raw[h][0][0], tb.raw[h][0][1]) : pack_hi(tb.raw[h][0][0], tb.raw[h][0][1]);
-            const uint32_t b1 = p == 0 ? pack_lo(tb.raw[h][1][0], tb.raw[h][1][1]) : pack_hi(tb.raw[h][1][0], tb.raw[h][1][1]);
+        for (int p = 0; p < 2; ++p)
 #pragma unroll
-            for (int i = 0; i < 2; ++i) mma_f32(acc[h][p][i], a[h][i], b0, b1);
-        }
+            for (int i = 0; i < 2; ++i) mma_f32(acc[h][p][i], a[h][i], tb.b[h][p][0], tb.b[h][p][1]);
 }
 
 }  // namespace tc
