@@ -10,9 +10,10 @@
 // L2 holds; a warp touches the tiles an item uses, 16 bytes per lane and access.  The gradients run on
 // 3 warps per table, the hist.T products on the others at the same time.
 //
-// Bound: shared-memory wavefronts of the look-ups and histograms, then latency between the barriers.
-// Against the two-sweep kernels of attn_tc_bwd.cu (scores twice, no tile skipping): second stage of
-// Swin3D-L, 144 k voxels, 10 heads: 11.84 -> 5.78 ms.
+// Bound: instruction issue and shared-memory wavefronts of the look-ups and histograms (half of the slots, three quarters of
+// the L1 pipe), then latency between the barriers.  Against the two-sweep kernels of attn_tc_bwd.cu (scores twice, no tile
+// skipping), forward and backward of 144 k voxels, 10 heads: 16.8 -> 9.4 ms; 8 k voxels, 20 heads, 4.5 key tiles per query
+// tile: 2.63 -> 2.15 ms.
 #include "attn_kernels.cuh"
 #include "attn_tc.cuh"
 #include "attn_tc_pair16.cuh"
@@ -104,7 +105,7 @@ __host__ __device__ inline P16Smem make_p16_layout(int R, int lut_entries)
 {
     P16Smem L;
     L.R16 = (R + 15) / 16 * 16;
-    L.Rp = (L.R16 + 31) / 32 * 32 + 8;
+    L.Rp = (L.R16 + 15) / 16 * 16 + 4;                             // see p16_store_key_major
     const int lane_arr = L.R16 * QT * 4, pk = 32 * L.Rp * 4;
     int off = 0;
     L.off_pq = off; off += lane_arr;                               // P_q, later histQ
@@ -376,29 +377,30 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
             P16TileA tile;
             if (mt >= 0) tile.fetch(Tproj, HC, co, s_map, mt, g, t);
             const int nv = tg == 2 ? nk : nq;
-            uint2 bf[8];
+            uint2 bf[4][2];
             p16_feat_frag(bf, tg == 0 ? s_q : (tg == 1 ? s_do : s_k), nv, g, t);
 #pragma unroll 1
             while (mt >= 0) {
                 const P16TileA cur = tile;
                 const int nx = tiles.next();
                 if (nx >= 0) tile.fetch(Tproj, HC, co, s_map, nx, g, t);
-                uint32_t d0[8], d1[8];
-                p16_project(d0, d1, cur, bf, nv, od);
-                if (tg < 2) store_lane_major(tg == 0 ? s_pq : s_db, d0, d1, mt, g, t);
-                else store_key_major(s_pk, d0, d1, mt, Rp, nv, g, t);
+                uint32_t d[2][2][4];
+                p16_project(d, cur, bf, nv);
+                if (tg < 2) p16_store_lane_major(tg == 0 ? s_pq : s_db, d, mt, g, t);
+                else p16_store_key_major(s_pk, d, mt, Rp, nv, g, t);
                 mt = nx;
             }
         }
-        for (int u = wid; u < 32; u += NW) {
-            const int a = u >> 4, mt = (u >> 3) & 1, j = u & 7;     // key rows 16mt.., query columns 4j..
-            if (16 * mt < nk && 4 * j < nq) {
-                float c[4];
-                p16_dot_block(c, a == 0 ? s_k : s_v, 16 * mt, a == 0 ? s_q : s_do, 4 * j, g, t);
-                float *e0 = reinterpret_cast<float *>(s_s0 + (16 * mt + g) * ES + 4 * j + t) + 2 * a;
-                float *e1 = reinterpret_cast<float *>(s_s0 + (16 * mt + g + 8) * ES + 4 * j + t) + 2 * a;
-                *reinterpret_cast<float2 *>(e0) = make_float2(c[0], c[1]);
-                *reinterpret_cast<float2 *>(e1) = make_float2(c[2], c[3]);
+        for (int u = NW - 1 - wid; u < 16; u += NW) {
+            const int a = u >> 3, mt = (u >> 2) & 1, j = u & 3;     // key rows 16mt.., query columns 8j..
+            if (16 * mt < nk && 8 * j < nq) {
+                float c[2][2][2];
+                p16_dot_block(c, a == 0 ? s_k : s_v, 16 * mt, a == 0 ? s_q : s_do, 8 * j, g, t);
+#pragma unroll
+                for (int rr = 0; rr < 2; ++rr)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        *reinterpret_cast<float2 *>(reinterpret_cast<float *>(s_s0 + (16 * mt + g + 8 * rr) * ES + 8 * j + 2 * t + e) + 2 * a) = make_float2(c[rr][e][0], c[rr][e][1]);
             }
         }
         consumer_sync<NT>();

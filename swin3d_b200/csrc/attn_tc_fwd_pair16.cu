@@ -20,9 +20,10 @@
 //
 // The blocks take contiguous ranges of (window, query tile) units of equal cost, so that the deep stages -- a handful of
 // windows of some hundred voxels -- still spread over the GPU.
-// Bound: latency between the barriers and shared-memory wavefronts.  Second stage of Swin3D-L, 144 k voxels, 10 heads:
-// 3.48 -> 3.18 ms against a tiled kernel with an online softmax (all row tiles, whole windows per block); deepest stage of
-// one room (4 windows of up to 150 voxels, 24 heads): 96 -> 54 us.
+// Bound: instruction issue (half of the slots, four warps a scheduler) and the barriers.  A forward call, tiled kernel with an
+// online softmax that did the work of a query tile once / this one with tables from L1/L2 / now: 144 k voxels, 10 heads,
+// 2.8 key tiles per query tile 3.85 / 3.79 / 3.08 ms; 8 k voxels, 20 heads, 4.5 key tiles 611 / 732 / 588 us, three signal
+// dimensions 383 / 516 / 381 us; 4 windows of up to 150 voxels, 24 heads 108 / 62 / 60 us.
 #include <climits>
 
 #include "attn_kernels.cuh"
@@ -54,7 +55,7 @@ __host__ __device__ inline F16Smem make_f16_layout(int R, int lut_entries)
 {
     F16Smem L;
     L.R16 = (R + 15) / 16 * 16;
-    L.Rp = (L.R16 + 31) / 32 * 32 + 8;
+    L.Rp = (L.R16 + 15) / 16 * 16 + 4;                               // see p16_store_key_major
     int off = 0;
     L.off_pq = off; off += L.R16 * QT * 4 > 8192 ? L.R16 * QT * 4 : 8192;          // P_q, later the histogram
     const int pk = 32 * L.Rp * 4, part = F16Split<D>::NHT * 4096;
@@ -252,7 +253,6 @@ attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, c
     // ==================================== consumer warps ===============================================
     const int Rp = L.Rp;
     const int mypos = qpos(lane);
-    const bool od = g & 1;
     constexpr float LOG2E = 1.4426950408889634f;
     const int pside = wid / HALF, wsub = wid - pside * HALF;         // projections: 0 = Tq with Q, 1 = Tk with K
     // the store phase: this thread's query and four channels, merged over the key tiles
@@ -279,7 +279,7 @@ attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, c
         // ---- projections, S0 ------------------------------------------------------------------------------------
         if (pside < 2) {
             const int nv = pside == 0 ? nq : nk;
-            uint2 bf[8];
+            uint2 bf[4][2];
             p16_feat_frag(bf, pside == 0 ? s_q : s_k, nv, g, t);
 #pragma unroll 1
             for (int i = wsub; i < n_used; i += HALF) {
@@ -289,19 +289,22 @@ attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, c
                 P16TileA cur;
                 cur.f[0][0] = make_uint2(x.x, x.y); cur.f[0][1] = make_uint2(x.z, x.w);
                 cur.f[1][0] = make_uint2(y.x, y.y); cur.f[1][1] = make_uint2(y.z, y.w);
-                uint32_t d0[8], d1[8];
-                p16_project(d0, d1, cur, bf, nv, od);
-                if (pside == 0) store_lane_major(s_pq, d0, d1, mt, g, t);
-                else store_key_major(s_pk, d0, d1, mt, Rp, nv, g, t);
+                uint32_t d[2][2][4];
+                p16_project(d, cur, bf, nv);
+                if (pside == 0) p16_store_lane_major(s_pq, d, mt, g, t);
+                else p16_store_key_major(s_pk, d, mt, Rp, nv, g, t);
             }
         }
-        for (int u = NW - 1 - wid; u < 16; u += NW) {
-            const int mt = u >> 3, j = u & 7;       // key rows 16mt.., query columns 4j..
-            if (16 * mt < nk && 4 * j < nq) {
-                float c[4];
-                p16_dot_block(c, s_k, 16 * mt, s_q, 4 * j, g, t);
-                *reinterpret_cast<float2 *>(s_elo + (16 * mt + g) * ES + 4 * j + t) = make_float2(c[0], c[1]);
-                *reinterpret_cast<float2 *>(s_elo + (16 * mt + g + 8) * ES + 4 * j + t) = make_float2(c[2], c[3]);
+        for (int u = NW - 1 - wid; u < 8; u += NW) {
+            const int mt = u >> 2, j = u & 3;       // key rows 16mt.., query columns 8j..
+            if (16 * mt < nk && 8 * j < nq) {
+                float c[2][2][2];
+                p16_dot_block(c, s_k, 16 * mt, s_q, 8 * j, g, t);
+#pragma unroll
+                for (int rr = 0; rr < 2; ++rr)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        *reinterpret_cast<float2 *>(s_elo + (16 * mt + g + 8 * rr) * ES + 8 * j + 2 * t + e) = make_float2(c[rr][e][0], c[rr][e][1]);
             }
         }
         consumer_sync<NT>();
@@ -385,22 +388,27 @@ attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, c
             const uint16_t *lut = s_lut + d * pm.lut_stride;
             uint32_t *cell = s_hist + mypos;
             auto row_of = [&](uint2 e) { return (uint32_t)lut[((lo ? e.y : e.x) >> sh) & ((1u << IDX_BITS) - 1u)] * QT; };
-            uint2 e0 = ecol[0], e1 = ecol[ES];              // keys beyond the tile hold zero entries
-            int kk = 0;
-            for (; kk + 1 < nk; kk += 2) {
-                const uint32_t p0 = lo ? e0.x : e0.y, p1 = lo ? e1.x : e1.y;
-                uint32_t *a0 = cell + row_of(e0), *a1 = cell + row_of(e1);
+            // the rows of this step are known; its cells, the rows of the next step and the entries after that are
+            // fetched together (keys beyond the tile hold zero entries)
+            uint2 e0 = ecol[0], e1 = ecol[ES];
+            uint32_t r0 = row_of(e0), r1 = row_of(e1);
+            uint32_t p0 = lo ? e0.x : e0.y, p1 = lo ? e1.x : e1.y;
+            e0 = ecol[2 * ES];
+            e1 = ecol[3 * ES];
+            for (int kk = 0; kk < nk; kk += 2) {
+                uint32_t *a0 = cell + r0, *a1 = cell + r1;
                 const uint32_t c0 = *a0, c1 = *a1;
-                e0 = ecol[min(kk + 2, QT - 1) * ES];
-                e1 = ecol[min(kk + 3, QT - 1) * ES];
-                const __half2 s0 = __hadd2(u32_as_h2(c0), u32_as_h2(p0));
-                const __half2 s1 = __hadd2(a1 == a0 ? s0 : u32_as_h2(c1), u32_as_h2(p1));
+                const bool same = r1 == r0, second = kk + 1 < nk;
+                const __half2 h0 = u32_as_h2(p0), h1 = u32_as_h2(p1);
+                r0 = row_of(e0);
+                r1 = row_of(e1);
+                p0 = lo ? e0.x : e0.y;
+                p1 = lo ? e1.x : e1.y;
+                e0 = ecol[min(kk + 4, QT - 1) * ES];
+                e1 = ecol[min(kk + 5, QT - 1) * ES];
+                const __half2 s0 = __hadd2(u32_as_h2(c0), h0), s1 = __hadd2(same ? s0 : u32_as_h2(c1), h1);
                 *a0 = h2_as_u32(s0);
-                *a1 = h2_as_u32(s1);
-            }
-            if (kk < nk) {
-                uint32_t *a0 = cell + row_of(e0);
-                *a0 = h2_as_u32(__hadd2(u32_as_h2(*a0), u32_as_h2(lo ? e0.x : e0.y)));
+                if (second) *a1 = h2_as_u32(s1);
             }
         }
         if (wid == PV_WARP) p16_pair_gemm<false, 2>(acc, reinterpret_cast<const uint32_t *>(s_elo), s_v, nk, g, t);   // O[q] = sum_k p V[k]

@@ -1,8 +1,7 @@
 // Pieces of the kernels that serve two heads of 16 channels per block (half2 entries = two heads).
 //
-// A product that contracts over channels runs as two k-steps: an mma lane t holds channels 4t, 4t+1 in the first and
-// 4t+2, 4t+3 in the second (any split serves as long as both operands use it), so that its part of a row is one 8-byte
-// load.  A product whose columns are channels runs once for the even and once for the odd channels: lane g loads
+// A product that contracts over channels is one k-step: an mma lane t holds channels 4t, 4t+1 in its first and 4t+2, 4t+3
+// in its second half (any split serves as long as both operands use it), so that its part of a row is one 8-byte load.  A product whose columns are channels runs once for the even and once for the odd channels: lane g loads
 // channels 2g, 2g+1 of the two rows of a k pair with 4-byte loads and swaps halves, and an accumulator lane ends with
 // channels 4t..4t+3.
 #pragma once
@@ -133,37 +132,78 @@ __device__ __forceinline__ void p16_zero(float (&acc)[2][2][2][4])
             for (int i = 0; i < 2; ++i) acc[h][p][i][0] = acc[h][p][i][1] = acc[h][p][i][2] = acc[h][p][i][3] = 0.f;
 }
 
-// Feature fragments of a staged array (voxel 4j + g/2, slot g&1, channels 4t..4t+3), and one projection unit: the 16 rows
-// of a tile against them; d0 / d1 = rows g / g + 8, voxels 4j + t.
-__device__ __forceinline__ void p16_project(uint32_t (&d0)[8], uint32_t (&d1)[8], const P16TileA &a, const uint2 (&bf)[8], int nv, bool od)
+// Feature fragments of a staged array for the projections: [voxels 8j + g][slot], channels 4t..4t+3.
+__device__ __forceinline__ void p16_feat_frag(uint2 (&bf)[4][2], const __half *rows, int nv, int g, int t)
+{
+    const __half *feat = rows + g * P16_RS + 4 * t;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) bf[j][h] = 8 * j < nv ? *reinterpret_cast<const uint2 *>(feat + 8 * j * P16_RS + h * 16) : make_uint2(0, 0);
+}
+
+// One projection unit: the 16 rows of a table tile against 32 voxels, one product per slot and 8 voxels; d[row g / g + 8]
+// [2t + e][j] = voxel 8j + 2t + e, both slots.  (Block-diagonal operands, as at head_dim 8, would take two products
+// for four voxels: twice the tensor work, and a second rounding of the sum to fp16.)
+__device__ __forceinline__ void p16_project(uint32_t (&d)[2][2][4], const P16TileA &a, const uint2 (&bf)[4][2], int nv)
 {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        d0[j] = d1[j] = 0u;
-        if (4 * j < nv) {
-            mma_k16_h(d0[j], d1[j], a.f[0][0].x, a.f[0][1].x, a.f[1][0].x, a.f[1][1].x, od ? 0u : bf[j].x, od ? bf[j].x : 0u);
-            mma_k16_ha(d0[j], d1[j], a.f[0][0].y, a.f[0][1].y, a.f[1][0].y, a.f[1][1].y, od ? 0u : bf[j].y, od ? bf[j].y : 0u);
+    for (int j = 0; j < 4; ++j) {
+        d[0][0][j] = d[0][1][j] = d[1][0][j] = d[1][1][j] = 0u;
+        if (8 * j < nv) {
+            uint32_t x0, x1, y0, y1;
+            mma_k16_h(x0, x1, a.f[0][0].x, a.f[0][1].x, a.f[0][0].y, a.f[0][1].y, bf[j][0].x, bf[j][0].y);
+            mma_k16_h(y0, y1, a.f[1][0].x, a.f[1][1].x, a.f[1][0].y, a.f[1][1].y, bf[j][1].x, bf[j][1].y);
+            d[0][0][j] = pack_lo(x0, y0);
+            d[0][1][j] = pack_hi(x0, y0);
+            d[1][0][j] = pack_lo(x1, y1);
+            d[1][1][j] = pack_hi(x1, y1);
         }
     }
 }
 
-__device__ __forceinline__ void p16_feat_frag(uint2 (&bf)[8], const __half *rows, int nv, int g, int t)
-{
-    const __half *feat = rows + (g >> 1) * P16_RS + (g & 1) * 16 + 4 * t;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) bf[j] = 4 * j < nv ? *reinterpret_cast<const uint2 *>(feat + 4 * j * P16_RS) : make_uint2(0, 0);
-}
-
-// A 16 x (4 voxels x 2 slots) block of Y . X^T (both slots): c = rows y0 + g / + 8, columns (voxel x0 + t, slots 0, 1).
-__device__ __forceinline__ void p16_dot_block(float (&c)[4], const __half *Y, int y0, const __half *X, int x0, int g, int t)
+// Its stores.  Lane-major [row][qpos(voxel)]: voxels 8j + 2t + e, j = 0..3, are the four columns from 4 (2t + e) on; odd rows
+// write e = 1 first, so that the eight lanes of a quarter warp (rows g, g + 1; t = 0..3) cover all 32 banks.
+__device__ __forceinline__ void p16_store_lane_major(uint32_t *dst, const uint32_t (&d)[2][2][4], int mt, int g, int t)
 {
     const bool od = g & 1;
-    const __half *y = Y + (y0 + g) * P16_RS + 4 * t;
-    const uint2 x = *reinterpret_cast<const uint2 *>(X + (x0 + (g >> 1)) * P16_RS + (g & 1) * 16 + 4 * t);
-    const uint2 a0 = *reinterpret_cast<const uint2 *>(y), a1 = *reinterpret_cast<const uint2 *>(y + 8 * P16_RS);
-    const uint2 a2 = *reinterpret_cast<const uint2 *>(y + 16), a3 = *reinterpret_cast<const uint2 *>(y + 8 * P16_RS + 16);
-    mma_k16_z(c, a0.x, a1.x, a2.x, a3.x, od ? 0u : x.x, od ? x.x : 0u);
-    mma_k16(c, a0.y, a1.y, a2.y, a3.y, od ? 0u : x.y, od ? x.y : 0u);
+    uint32_t *r = dst + (mt * 16 + g) * QT + 8 * t;
+    const int o0 = od ? 4 : 0, o1 = 4 - o0;
+#pragma unroll
+    for (int rr = 0; rr < 2; ++rr) {
+        const uint4 a = make_uint4(d[rr][0][0], d[rr][0][1], d[rr][0][2], d[rr][0][3]), b = make_uint4(d[rr][1][0], d[rr][1][1], d[rr][1][2], d[rr][1][3]);
+        *reinterpret_cast<uint4 *>(r + rr * 8 * QT + o0) = od ? b : a;
+        *reinterpret_cast<uint4 *>(r + rr * 8 * QT + o1) = od ? a : b;
+    }
+}
+
+// Key-major [voxel][Rp], the first nv voxels rounded up to a multiple of eight; Rp = 4 (mod 16): voxels 2t lie 8 banks apart.
+__device__ __forceinline__ void p16_store_key_major(uint32_t *dst, const uint32_t (&d)[2][2][4], int mt, int Rp, int nv, int g, int t)
+{
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (8 * j < nv) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                uint32_t *p = dst + (8 * j + 2 * t + e) * Rp + mt * 16 + g;
+                p[0] = d[0][e][j];
+                p[8] = d[1][e][j];
+            }
+        }
+}
+
+// A 16 x 8 block of Y . X^T (both slots): c[row y0 + g / + 8][voxel x0 + 2t / + 1][slot].
+__device__ __forceinline__ void p16_dot_block(float (&c)[2][2][2], const __half *Y, int y0, const __half *X, int x0, int g, int t)
+{
+    const __half *y = Y + (y0 + g) * P16_RS + 4 * t, *x = X + (x0 + g) * P16_RS + 4 * t;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint2 b = *reinterpret_cast<const uint2 *>(x + h * 16);
+        const uint2 a0 = *reinterpret_cast<const uint2 *>(y + h * 16), a1 = *reinterpret_cast<const uint2 *>(y + 8 * P16_RS + h * 16);
+        float d[4];
+        mma_k16_z(d, a0.x, a1.x, a0.y, a1.y, b.x, b.y);
+        c[0][0][h] = d[0]; c[0][1][h] = d[1]; c[1][0][h] = d[2]; c[1][1][h] = d[3];
+    }
 }
 
 // acc += hist(16 rows of k-step ks) . T(the same rows) for the 32 voxels (m).

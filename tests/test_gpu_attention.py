@@ -425,6 +425,24 @@ def test_fp16_backward_gives_the_same_rows_whether_windows_are_split_or_not(crse
         assert rel_err(a.cpu().numpy(), b.cpu().numpy()) < 1e-4, name
 
 
+@pytest.mark.parametrize("H,ws,crse", [(2, 7, "XYZ_RGB_NORM"), (4, 5, "XYZ_RGB"), (2, 7, "XYZ")])
+def test_fp16_pairs_of_16_channel_heads_at_the_edges_of_their_products(H, ws, crse):
+    """Products go by 8 voxels, pair products by 16, tiles by 32: each side of these.  Element by element the result
+    carries an fp16 rounding (2^-11 of it) and those of its terms, which average out over a window; together
+    below 2^-8 of the largest element of the array, and 2^-10 of the norm."""
+    from tests.gpu_helpers import cuda_fwd_bwd
+    sizes = [1, 2, 7, 8, 9, 15, 16, 17, 23, 24, 25, 31, 32, 33, 39, 40, 41, 47, 48, 49, 63, 64, 65, 79, 81]
+    p = make_problem(seed=98, ws=ws, H=H, hd=16, crse=crse, scene=_scene_of_window_sizes(ws, sizes), round_fp16=True)
+    o_ref, lse_ref, g_ref = oracle_fwd_bwd(p, np.float64)
+    out, lse, grads = cuda_fwd_bwd(p, torch.float16)
+    assert np.abs(lse - lse_ref).max() < 2.0 ** -8
+    for name, a, b in zip("out dq dk dv".split(), (out,) + grads[:3], (o_ref,) + g_ref[:3]):
+        assert rel_err(a, b) < 2.0 ** -8, name
+        assert np.linalg.norm(a - b) < 2.0 ** -10 * np.linalg.norm(b), name
+    for name, a, b in zip("dtq dtk dtv".split(), grads[3:], g_ref[3:]):
+        assert rel_err(a, b) < FP16_TOL, name
+
+
 @pytest.mark.parametrize("H,hd,ws,crse", [(2, 8, 5, "XYZ_RGB_NORM"), (4, 8, 7, "XYZ_RGB"), (2, 8, 7, "XYZ"), (10, 8, 7, "XYZ_RGB_NORM"),
                                           (1, 16, 5, "XYZ_RGB_NORM"), (3, 16, 7, "XYZ_RGB"), (1, 16, 7, "XYZ")])
 def test_fp16_forward_at_the_edges_of_its_tiles(H, hd, ws, crse):
