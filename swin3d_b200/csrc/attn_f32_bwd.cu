@@ -3,8 +3,9 @@
 // per block.
 //
 // A window of n voxels is cut into nt = ceil(n / 32) tiles and the work item is a tile pair (query tile i,
-// key tile j); items of a window run one after the other in the same block, later shares of dQ, dK, dV
-// are added to the rows already written.  Per item, phases separated by a barrier of the consumer warps:
+// key tile j); items of a row run one after the other in the same block, later shares of dQ, dK, dV are
+// added to the rows already written.  In calls of few windows a window's query and key tiles go to different
+// blocks (split_windows).  Per item, phases separated by a barrier of the consumer warps:
 //   project    P_q = Tq.Q^T, dB = Tv.dO^T as [row][query], P_k = Tk.K^T as [key][row]; lane = voxel with
 //              its row in registers, table rows broadcast from a staged 16-row tile
 //   scores     lane = query, keys dealt to the warps: q.k and dO.v, D indices, 3*D look-ups, p = exp(s - lse),
@@ -37,7 +38,9 @@ using tc::IDX_BITS;
 
 constexpr int STAGES = 2;
 constexpr int ES = 33;                                       // row stride of the pair planes
-__host__ __device__ constexpr int warps_for(int D) { return D == 9 ? 15 : (D == 6 ? 11 : 7); }
+enum { ROLE_Q = 1, ROLE_K = 2 };                             // what an item contributes to: dQ, dTq, dTv; dK, dV, dTk
+// head_dim 16 with six signal dimensions: 15 warps leave 128 registers and spill (8 k voxels, 6 heads 1.90 -> 2.15 ms)
+__host__ __device__ constexpr int warps_for(int D, int HD) { return D == 3 || (D == 6 && HD == 16) ? 11 : 15; }
 
 // How the warps share the last two kinds of products.  A step of the table gradients reads a voxel row per
 // lane, and every 32-row unit a warp holds reuses it: head_dim 8 gives the gradients to 3 * DTW warps
@@ -47,10 +50,10 @@ __host__ __device__ constexpr int warps_for(int D) { return D == 9 ? 15 : (D == 
 // registers: every warp takes its share of both, up to three units.
 template <int D, int HD>
 struct Split {
-    static constexpr int NW = warps_for(D);
+    static constexpr int NW = warps_for(D, HD);
     static constexpr bool APART = HD == 8;
-    static constexpr int DTW = APART ? (D == 9 ? 3 : (D == 6 ? 2 : 1)) : NW / 3;   // gradient warps per table
-    static constexpr int NDT = APART ? (D == 9 ? 4 : (D == 6 ? 5 : 6)) : 3;        // 32-row units per warp
+    static constexpr int DTW = APART ? (D == 3 ? 2 : 3) : NW / 3;                  // gradient warps per table
+    static constexpr int NDT = APART ? (D == 3 ? 3 : 4) : 3;                       // 32-row units per warp
     static constexpr int HT0 = APART ? 3 * DTW : 0;                                // first warp of the hist.T products
     static constexpr int SG = (NW - HT0) / 2;                                      // warps per side of them
 };
@@ -64,7 +67,7 @@ struct Smem {
 template <int D, int HD>
 __host__ __device__ inline Smem make_smem(int R, int lut_entries)
 {
-    constexpr int nw = warps_for(D), hd = HD, rs = row_stride(HD);
+    constexpr int nw = warps_for(D, HD), hd = HD, rs = row_stride(HD);
     Smem L;
     L.R16 = (R + 15) / 16 * 16;
     L.Rp = L.R16 + 1;                                        // odd: lanes = keys write P_k without conflicts
@@ -188,10 +191,10 @@ struct TableTile {
 };
 
 template <int D, int HD>
-__global__ void __launch_bounds__((warps_for(D) + 1) * 32, 1)
+__global__ void __launch_bounds__((warps_for(D, HD) + 1) * 32, 1)
 attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
 {
-    constexpr int NW = warps_for(D), NT = NW * 32;
+    constexpr int NW = warps_for(D, HD), NT = NW * 32;
     constexpr int TG = NW / 3;                   // warps per table (projections and table gradients)
     constexpr int NKW = (D + 1) / 2;             // warps of the key-side histogram, two dimensions each
     constexpr int GEMM_WARP = D + NKW;           // dQ and dK pair products
@@ -218,7 +221,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
     float *s_lses = reinterpret_cast<float *>(smem + L.off_misc);       // [stage][32]
     float *s_dels = s_lses + STAGES * 32;                               // [stage][32]
     int *s_rowi = reinterpret_cast<int *>(s_dels + STAGES * 32);        // [stage][query tile, key tile][32]
-    int *s_n = s_rowi + STAGES * 64;                                    // [stage][8]: nq, nk, j > 0, i > 0, used tiles; nq = 0: no more items
+    int *s_n = s_rowi + STAGES * 64;                                    // [stage][8]: nq, nk, j > 0, i > 0, used tiles, roles; nq = 0: no more items
     int *s_fail = s_n + STAGES * 8;
     uint64_t *s_full = reinterpret_cast<uint64_t *>(smem + L.off_misc + 1792), *s_empty = s_full + STAGES;
 
@@ -238,9 +241,12 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
         const int row = tc::perm_table_row(pm, r);
         s_map[r] = row < 0 ? (uint16_t)0xffff : (uint16_t)row;
     }
-    // this block's windows: a contiguous range of equal cost
+    // this block's share: a contiguous range of equal cost
+    const bool split = tc::split_windows<(NW + 1) * 32, 7, 8>(P.w_sizes, P.W, smem + L.off_pq);
     int64_t w_begin, w_end;
-    tc::balanced_range<(NW + 1) * 32>(P.w_sizes, P.W, smem + L.off_pq, w_begin, w_end);
+    int u_begin, u_end;                          // first unit of window w_begin, one past the last of window w_end
+    if (split) tc::balanced_units<(NW + 1) * 32>(P.w_sizes, P.W, smem + L.off_pq, tc::UnitsSplit<7, 8>{}, w_begin, w_end, u_begin, u_end);
+    else tc::balanced_units<(NW + 1) * 32>(P.w_sizes, P.W, smem + L.off_pq, tc::UnitsWhole{}, w_begin, w_end, u_begin, u_end);
 
     if (wid == NW) {
         // ================================ producer warp ================================================
@@ -249,8 +255,10 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
         // are loaded inside it.
         int64_t w = w_begin - 1;
         int n = 0, base = 0, nt = 0, ts = 0, ti = 0, tj = 0;
+        int unit = 0, unit_end = 0, role = 0;              // a window is one unit of both roles, or (halves) 2 nt of one
+        bool halves = false;
         int n_nx = 0, base_nx = 0;
-        if (w_begin < w_end) {
+        if (w_begin < P.W) {
             n_nx = __ldg(P.w_sizes + w_begin);
             base_nx = __ldg(P.w2n + w_begin);
         }
@@ -258,27 +266,32 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
         int nq = 0, nk = 0, rowq = 0, rowk = 0;
         float cq[D], ck[D];
         auto advance = [&]() {
-            if (have && tj + 1 < nt) {
+            if (have && (role & ROLE_Q) && tj + 1 < nt) {
                 ++tj;
-            } else if (have && ti + 1 < nt) {
+            } else if (have && (role & ROLE_K) && ti + 1 < nt) {
                 ++ti;
-                tj = 0;
+                if (role & ROLE_Q) tj = 0;
             } else {
-                ti = tj = 0;
-                do {                              // an empty window has no items; the next one may have some
+                ++unit;
+                while (unit >= unit_end) {                 // the next window with voxels
                     ++w;
-                    have = w < w_end;
-                    if (have) {
-                        n = n_nx;
-                        base = base_nx;
-                        if (w + 1 < w_end) {
-                            n_nx = __ldg(P.w_sizes + w + 1);
-                            base_nx = __ldg(P.w2n + w + 1);
-                        }
+                    have = w < w_end || (w == w_end && u_end > 0);
+                    if (!have) break;
+                    n = n_nx;
+                    base = base_nx;
+                    if (w + 1 < P.W) {
+                        n_nx = __ldg(P.w_sizes + w + 1);
+                        base_nx = __ldg(P.w2n + w + 1);
                     }
-                } while (have && n < 1);
-                nt = (n + QT - 1) / QT;
-                ts = nt > 0 ? (n + nt - 1) / nt : 0;
+                    nt = (n + QT - 1) / QT;
+                    ts = nt > 0 ? (n + nt - 1) / nt : 0;
+                    halves = split && nt > 1;
+                    unit = w == w_begin ? u_begin : 0;
+                    unit_end = w == w_end ? u_end : (halves ? 2 * nt : (nt > 0 ? 1 : 0));
+                }
+                role = !halves ? ROLE_Q | ROLE_K : (unit < nt ? ROLE_Q : ROLE_K);
+                ti = role == ROLE_Q ? unit : 0;
+                tj = role == ROLE_K ? unit - nt : 0;
             }
             nq = have ? min(ts, n - ti * ts) : 0;
             nk = have ? min(ts, n - tj * ts) : 0;
@@ -336,6 +349,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
                 s_n[s * 8 + 1] = nk;
                 s_n[s * 8 + 2] = tj > 0;
                 s_n[s * 8 + 3] = ti > 0;
+                s_n[s * 8 + 5] = role;
                 s_n[s * 8 + 4] = (int)used;
             }
             mbar_arrive(s_full + s);
@@ -365,7 +379,8 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
 #pragma unroll
         for (int i = 0; i < HP; ++i) dt_acc[u][i] = 0ull;
 
-    for (int it = 0;; ++it) {
+    int it = 0;
+    for (;; ++it) {
         const int s = it % STAGES;
         if (!mbar_wait(s_full + s, (it / STAGES) & 1)) {
             *s_fail = 1;
@@ -374,6 +389,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
         consumer_sync<NT>();          // the previous item's stores are over; the flag is settled
         const int nq = s_n[s * 8], nk = s_n[s * 8 + 1];
         const bool add_q = s_n[s * 8 + 2] != 0, add_k = s_n[s * 8 + 3] != 0;
+        const bool do_q = s_n[s * 8 + 5] & ROLE_Q, do_k = s_n[s * 8 + 5] & ROLE_K;
         const uint32_t used = (uint32_t)s_n[s * 8 + 4];
         if (nq == 0 || *s_fail) break;
         const float *s_q = s_rows + s * (4 * 32 * RS), *s_do = s_q + 32 * RS, *s_k = s_do + 32 * RS, *s_v = s_k + 32 * RS;
@@ -453,13 +469,15 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
         for (int i = tid; i < L.R16 * QT / 4; i += NT)                 // 128 16-byte pieces per 16-row tile
             if ((used >> (i >> 7)) & 1u) {
                 const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-                reinterpret_cast<float4 *>(s_hq)[i] = z;
-                reinterpret_cast<float4 *>(s_hv)[i] = z;
-                reinterpret_cast<float4 *>(s_hk)[i] = z;
+                if (do_q) {
+                    reinterpret_cast<float4 *>(s_hq)[i] = z;
+                    reinterpret_cast<float4 *>(s_hv)[i] = z;
+                }
+                if (do_k) reinterpret_cast<float4 *>(s_hk)[i] = z;
             }
         consumer_sync<NT>();
         // ---- histograms and pair products ----------------------------------------------------------------------
-        if (wid < D) {
+        if (wid < D && do_q) {
             // lanes = queries, two keys per step, the next step's entries fetched before this step's stores
             const int d = wid;
             const bool lo = d < 5;
@@ -491,7 +509,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
                 a0[0] = sq0; a0[hv] = sv0;
                 if (second) { a1[0] = sq1; a1[hv] = sv1; }
             }
-        } else if (wid < D + NKW) {
+        } else if (wid >= D && wid < D + NKW && do_k) {
             // histK += ds ; lanes = keys, the planes are read column-wise
             for (int d = 2 * (wid - D); d < 2 * (wid - D) + 2 && d < D; ++d) {
                 const bool lo = d < 5;
@@ -522,17 +540,21 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
         }
         if (wid == GEMM_WARP) {
             uint64_t acc[HP];
+            if (do_q) {
 #pragma unroll
-            for (int i = 0; i < HP; ++i) acc[i] = 0ull;
+                for (int i = 0; i < HP; ++i) acc[i] = 0ull;
 #pragma unroll 4
-            for (int kk = 0; kk < nk; ++kk) axpy_row<HD>(acc, s_DS[kk * ES + lane], s_k + kk * RS);      // dQ[q] = sum_k ds K[k]
-            store_row<HD>(s_pg + lane * HD, acc);
+                for (int kk = 0; kk < nk; ++kk) axpy_row<HD>(acc, s_DS[kk * ES + lane], s_k + kk * RS);  // dQ[q] = sum_k ds K[k]
+                store_row<HD>(s_pg + lane * HD, acc);
+            }
+            if (do_k) {
 #pragma unroll
-            for (int i = 0; i < HP; ++i) acc[i] = 0ull;
+                for (int i = 0; i < HP; ++i) acc[i] = 0ull;
 #pragma unroll 4
-            for (int qq = 0; qq < nq; ++qq) axpy_row<HD>(acc, s_DS[lane * ES + qq], s_q + qq * RS);      // dK[k] = sum_q ds Q[q]
-            store_row<HD>(s_pg + (64 + lane) * HD, acc);
-        } else if (wid == DV_WARP) {
+                for (int qq = 0; qq < nq; ++qq) axpy_row<HD>(acc, s_DS[lane * ES + qq], s_q + qq * RS);  // dK[k] = sum_q ds Q[q]
+                store_row<HD>(s_pg + (64 + lane) * HD, acc);
+            }
+        } else if (wid == DV_WARP && do_k) {
             uint64_t acc[HP];
 #pragma unroll
             for (int i = 0; i < HP; ++i) acc[i] = 0ull;
@@ -542,25 +564,26 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
         }
         consumer_sync<NT>();
         // ---- table gradients: lane = row of a 32-row unit ---------------------------------------------------------
-        if (dtg < 3) {
+        if (dtg < 3 && (dtg < 2 ? do_q : do_k)) {
             const float *hist = dtg == 0 ? s_hq : (dtg == 1 ? s_hv : s_hk);
             const float *X = dtg == 0 ? s_q : (dtg == 1 ? s_do : s_k);
-            bool on[NDT];
+            bool on[NDT], any[NDT];
             const float *hrow[NDT];
 #pragma unroll
             for (int u = 0; u < NDT; ++u) {
                 const int tile = 2 * (dsub + DTW * u) + (lane >> 4);
                 on[u] = tile < n_mt && ((used >> tile) & 1u);
+                any[u] = __any_sync(0xffffffffu, on[u]);
                 hrow[u] = hist + (on[u] ? (dsub + DTW * u) * 32 + lane : 0) * QT;
             }
-            constexpr int STEP = 2;
+            constexpr int STEP = D == 9 && HD == 16 ? 1 : 2;       // two rows of 16 channels ahead spill beside three units
             for (int i = 0; i < QT; i += STEP) {
                 uint64_t x[STEP][HP];
 #pragma unroll
                 for (int j = 0; j < STEP; ++j) load_row<HD>(x[j], X + ((i + j + lane) & 31) * RS);
 #pragma unroll
                 for (int u = 0; u < NDT; ++u)
-                    if (__any_sync(0xffffffffu, on[u])) {
+                    if (any[u]) {
 #pragma unroll
                         for (int j = 0; j < STEP; ++j) {
                             const float h = on[u] ? hrow[u][(i + j + lane) & 31] : 0.f;
@@ -572,7 +595,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
             }
         }
         // ---- dQ += histQ.Tq, dK += histK.Tk: lane = voxel -----------------------------------------------------------
-        if (side < 2) {
+        if (side < 2 && (side == 0 ? do_q : do_k)) {
             const float *T = side == 0 ? P.tq : P.tk, *hist = side == 0 ? s_hq : s_hk;
             uint64_t acc[HP];
 #pragma unroll
@@ -598,7 +621,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
         // ---- reduce and store ---------------------------------------------------------------------------------------
         for (int e = tid; e < 2 * 32 * HP; e += NT) {
             const int sd = e / (32 * HP), xx = e / HP & 31, ch = e % HP * 2;
-            if (xx < (sd == 0 ? nq : nk)) {
+            if (sd == 0 ? do_q && xx < nq : do_k && xx < nk) {
                 const float2 pg = *reinterpret_cast<const float2 *>(s_pg + ((sd == 0 ? 0 : 64) + xx) * HD + ch);
                 float a = pg.x, b = pg.y;
                 const float *pp = s_part + (sd * SG * 32 + xx) * HD + ch;
@@ -634,7 +657,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
     }
 
     // ---- the table gradients of this block ---------------------------------------------------------------------------
-    if (dtg < 3) {
+    if (dtg < 3 && it > 0) {
         float *dst = dtg == 0 ? P.dtq : (dtg == 1 ? P.dtv : P.dtk);
 #pragma unroll
         for (int u = 0; u < NDT; ++u) {
@@ -654,14 +677,13 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
 template <int D, int HD>
 static int launch(const Params &p, const CrseMeta &meta, const PermMeta &pm, cudaStream_t st)
 {
-    constexpr int NW = warps_for(D);
+    constexpr int NW = warps_for(D, HD);
     const Smem L = make_smem<D, HD>(pm.R, pm.D * pm.lut_stride);
     auto kern = attn_bwd_f32_kernel<D, HD>;
     int sms = 0;
     const int rc = tc::kernel_setup(reinterpret_cast<const void *>(kern), sms);
     if (rc != S3D_OK) return rc;
     int gx = sms / p.H;
-    if (gx > p.W) gx = (int)p.W;
     if (gx < 1) gx = 1;
     kern<<<dim3((unsigned)gx, (unsigned)p.H), (NW + 1) * 32, L.total, st>>>(p, pm, tc::make_pair_consts(meta));
     const cudaError_t le = cudaGetLastError();

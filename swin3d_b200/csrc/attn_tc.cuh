@@ -424,6 +424,51 @@ __device__ __forceinline__ void balanced_range(const int32_t *__restrict__ w_siz
     balanced_units<NTA>(w_sizes, W, scratch, UnitsWhole{}, w_begin, w_end, i_begin, i_end);
 }
 
+// Backwards in calls of few windows: a block that takes whole windows runs over up to 121 tile pairs in a row while others
+// have none.  A window of nt > 1 tiles is then 2 nt units, (query tile i, all j) for dQ, dTq and dTv, and (key tile j, all i)
+// for dK, dV and dTk, dealt to the blocks one by one.  An item of one role costs ONE / BOTH of an item of both.
+template <int ONE, int BOTH>
+struct UnitsSplit {
+    __device__ __forceinline__ Units operator()(int n) const
+    {
+        const int nt = (n + QT - 1) / QT;
+        return nt > 1 ? Units{2 * nt, ONE * nt} : Units{nt, BOTH};
+    }
+};
+
+// Whether the windows of this call are split: the longest share of a block, estimated for both ways.  Whole windows: the
+// average share and half of the largest window, or that window alone; split: the average and the largest unit.  All
+// blocks come to the same answer.  Called by all NTA threads; scratch: 32 bytes of shared memory.
+template <int NTA, int ONE, int BOTH>
+__device__ __forceinline__ bool split_windows(const int32_t *__restrict__ w_sizes, int64_t W, void *scratch)
+{
+    if (W >= 32 * (int64_t)gridDim.x) return false;               // enough windows for the shares to even out
+    unsigned long long *s_sum = static_cast<unsigned long long *>(scratch);   // tile pairs, windows of one tile
+    int *s_max = reinterpret_cast<int *>(s_sum + 2);
+    if (threadIdx.x == 0) {
+        s_sum[0] = s_sum[1] = 0;
+        *s_max = 0;
+    }
+    __syncthreads();
+    unsigned long long sum = 0, single = 0;
+    int mx = 0;
+    for (int64_t w = threadIdx.x; w < W; w += NTA) {
+        const int nt = (__ldg(w_sizes + w) + QT - 1) / QT;
+        if (nt > 0) sum += (unsigned long long)nt * nt;
+        single += nt == 1;
+        mx = max(mx, nt);
+    }
+    atomicAdd(s_sum, sum);
+    atomicAdd(s_sum + 1, single);
+    atomicMax(s_max, mx);
+    __syncthreads();
+    const float all = (float)s_sum[0], one = (float)s_sum[1], nt = (float)*s_max, share = 1.f / gridDim.x;
+    __syncthreads();
+    const float whole = BOTH * fmaxf(all * share + 0.5f * nt * nt, nt * nt);
+    const float split = (2.f * ONE * (all - one) + BOTH * one) * share + ONE * nt;
+    return split < whole;
+}
+
 // Head modes of the tiled kernels.  A thread block always works on two "slots" packed as half2:
 //   HDM_PAIR8   head_dim 8 : slots = heads 2hp, 2hp+1, 8 channels each, one plane
 //   HDM_SINGLE16 head_dim 16: slots = the two 8-channel halves of head hp (partial scores are summed)

@@ -33,9 +33,7 @@ constexpr int P16_STAGES = 2;
 // for dK, dV (and dTk) with i innermost, so that one sum suffices.
 constexpr int P16_SLOTS = 11;
 //
-// The same two halves serve calls of few windows: a block that takes whole windows runs over up to 121 pairs in a row
-// while others have none.  A window of several tiles is then 2 nt units, (query tile i, all j) for dQ and (key tile j, all
-// i) for dK and dV, dealt to the blocks one by one.  An item of one role costs about two thirds of one of both.
+// The same two halves serve calls of few windows (split_windows).
 struct P16UnitsWhole {
     __device__ __forceinline__ Units operator()(int n) const
     {
@@ -43,47 +41,6 @@ struct P16UnitsWhole {
         return {nt > 0 ? 1 : 0, (nt > P16_SLOTS ? 4 : 3) * nt * nt};
     }
 };
-struct P16UnitsSplit {
-    __device__ __forceinline__ Units operator()(int n) const
-    {
-        const int nt = (n + QT - 1) / QT;
-        return nt > 1 ? Units{2 * nt, 2 * nt} : Units{nt, 3};
-    }
-};
-
-// Whether the windows of this call are split: the longest share of a block, estimated for both ways.  Whole windows: the
-// average share and half of the largest window, or that window alone; split: the average and the largest unit.  All
-// blocks come to the same answer.  Called by all NTA threads; scratch: 32 bytes of shared memory.
-template <int NTA>
-__device__ __forceinline__ bool split_windows(const int32_t *__restrict__ w_sizes, int64_t W, void *scratch)
-{
-    if (W >= 32 * (int64_t)gridDim.x) return false;               // enough windows for the shares to even out
-    unsigned long long *s_sum = static_cast<unsigned long long *>(scratch);   // tile pairs, windows of one tile
-    int *s_max = reinterpret_cast<int *>(s_sum + 2);
-    if (threadIdx.x == 0) {
-        s_sum[0] = s_sum[1] = 0;
-        *s_max = 0;
-    }
-    __syncthreads();
-    unsigned long long sum = 0, single = 0;
-    int mx = 0;
-    for (int64_t w = threadIdx.x; w < W; w += NTA) {
-        const int nt = (__ldg(w_sizes + w) + QT - 1) / QT;
-        if (nt > 0) sum += (unsigned long long)nt * nt;
-        single += nt == 1;
-        mx = max(mx, nt);
-    }
-    atomicAdd(s_sum, sum);
-    atomicAdd(s_sum + 1, single);
-    atomicMax(s_max, mx);
-    __syncthreads();
-    const float all = (float)s_sum[0], one = (float)s_sum[1], nt = (float)*s_max, share = 1.f / gridDim.x;
-    __syncthreads();
-    const float whole = 3.f * fmaxf(all * share + 0.5f * nt * nt, nt * nt);
-    const float split = (4.f * (all - one) + 3.f * one) * share + 2.f * nt;
-    return split < whole;
-}
-
 enum { ROLE_Q = 1, ROLE_K = 2, Q_FIRST = 4, Q_LAST = 8, K_FIRST = 16, K_LAST = 32 };
 
 template <int D>
@@ -194,10 +151,10 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
         s_map[r] = row < 0 ? (uint16_t)0xffff : (uint16_t)row;
     }
     // this block's share: a contiguous range of equal cost
-    const bool split = split_windows<(NW + 1) * 32>(P.w_sizes, P.W, smem + L.off_pq);
+    const bool split = split_windows<(NW + 1) * 32, 2, 3>(P.w_sizes, P.W, smem + L.off_pq);
     int64_t w_begin, w_end;
     int u_begin, u_end;                          // first unit of window w_begin, one past the last of window w_end
-    if (split) balanced_units<(NW + 1) * 32>(P.w_sizes, P.W, smem + L.off_pq, P16UnitsSplit{}, w_begin, w_end, u_begin, u_end);
+    if (split) balanced_units<(NW + 1) * 32>(P.w_sizes, P.W, smem + L.off_pq, UnitsSplit<2, 3>{}, w_begin, w_end, u_begin, u_end);
     else balanced_units<(NW + 1) * 32>(P.w_sizes, P.W, smem + L.off_pq, P16UnitsWhole{}, w_begin, w_end, u_begin, u_end);
 
     if (wid == NW) {
