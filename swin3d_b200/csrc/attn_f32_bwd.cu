@@ -127,6 +127,14 @@ __device__ __forceinline__ float sum2(uint64_t a)
     return x + y;
 }
 
+// __expf rounds x * log2(e) before the exponential; the rounding error is put back to first order.
+__device__ __forceinline__ float exp_rounded_once(float x)
+{
+    constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
+    const float t = x * LOG2E, e = tc::ex2_approx(t);
+    return fabsf(t) < 126.f ? fmaf(e, fmaf(x, LOG2E, -t) * LN2, e) : e;
+}
+
 // A row of HD floats as HD/2 packed pairs (16-byte loads).
 template <int HD>
 __device__ __forceinline__ void load_row(uint64_t (&r)[HD / 2], const float *p)
@@ -441,7 +449,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
                         float ck[D];
                         tc::load_coords12<D>(s_ck + kk * 12, ck);
                         const float *pk_row = s_pk + kk * Rp;
-                        float b0 = dot_row<HD>(q2, s_k + kk * RS), b1 = 0.f, b2 = dot_row<HD>(g2, s_v + kk * RS);
+                        float b0 = 0.f, b1 = 0.f, b2 = 0.f;      // table terms, small beside the products: summed first
 #pragma unroll
                         for (int d = 0; d < D; ++d) {
                             const uint32_t idx = tc::crse_index_pc(cx[d], ck[d], pc.half[d], pc.clamp[d]);
@@ -453,8 +461,8 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
                             else w1 |= idx << (IDX_BITS * (d - 5));
                         }
                         if (lane < nq) {
-                            p = __expf(b0 + b1 - lse);
-                            ds = p * (b2 - del);
+                            p = exp_rounded_once(dot_row<HD>(q2, s_k + kk * RS) - lse + (b0 + b1));
+                            ds = p * (dot_row<HD>(g2, s_v + kk * RS) - del + b2);
                         }
                     }
                     s_P[kk * ES + lane] = p;
