@@ -458,9 +458,17 @@ __device__ __forceinline__ bool split_windows(const int32_t *__restrict__ w_size
         single += nt == 1;
         mx = max(mx, nt);
     }
-    atomicAdd(s_sum, sum);
-    atomicAdd(s_sum + 1, single);
-    atomicMax(s_max, mx);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        single += __shfl_xor_sync(0xffffffffu, single, o);
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(s_sum, sum);
+        atomicAdd(s_sum + 1, single);
+        atomicMax(s_max, mx);
+    }
     __syncthreads();
     const float all = (float)s_sum[0], one = (float)s_sum[1], nt = (float)*s_max, share = 1.f / gridDim.x;
     __syncthreads();
