@@ -18,6 +18,9 @@
 //              from 32 different banks
 //   products   dQ += histQ.Tq, dK += histK.Tk: lane = voxel, row tiles dealt to the warps
 //   store      reduce over the warps, write or add the rows
+// The last two run over whole row tiles, with zeros where no pair touches a row.  Where the other operand is not finite
+// (flags found beside the projections, and once per block for the tables) the zeros are passed over
+// there, so that a result becomes infinite or NaN only through a pair that reaches it.
 // All products are fp32 FMAs, two per instruction (fma.f32x2): no operand is rounded to fewer bits.
 // Row numbering and tile skipping as in PermMeta (attn_tc.cuh).
 //
@@ -127,6 +130,11 @@ __device__ __forceinline__ float sum2(uint64_t a)
     return x + y;
 }
 
+__device__ __forceinline__ bool finite4(const float4 &v)
+{
+    return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))) < INFINITY && v.x == v.x && v.y == v.y && v.z == v.z && v.w == v.w;
+}
+
 // __expf rounds x * log2(e) before the exponential; the rounding error is put back to first order.
 __device__ __forceinline__ float exp_rounded_once(float x)
 {
@@ -231,6 +239,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
     int *s_rowi = reinterpret_cast<int *>(s_dels + STAGES * 32);        // [stage][query tile, key tile][32]
     int *s_n = s_rowi + STAGES * 64;                                    // [stage][8]: nq, nk, j > 0, i > 0, used tiles, roles; nq = 0: no more items
     int *s_fail = s_n + STAGES * 8;
+    int *s_odd = s_fail + 1;                                            // not finite: Q, dO, K of the item, Tq, Tk
     uint64_t *s_full = reinterpret_cast<uint64_t *>(smem + L.off_misc + 1792), *s_empty = s_full + STAGES;
 
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -242,12 +251,22 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
             mbar_init(s_empty + s, NW);
         }
         *s_fail = 0;
+        s_odd[3] = s_odd[4] = 0;
         mbar_init_fence();
     }
     tc::fill_perm_lut(s_lut, pm, tid, blockDim.x);
     for (int r = tid; r < L.R16; r += blockDim.x) {
         const int row = tc::perm_table_row(pm, r);
         s_map[r] = row < 0 ? (uint16_t)0xffff : (uint16_t)row;
+    }
+    __syncthreads();
+    for (int e = tid; e < L.R16 * (HD / 4); e += blockDim.x) {
+        const int row = s_map[e / (HD / 4)];
+        if (row != 0xffff) {
+            const int64_t o = (int64_t)row * HC + co + e % (HD / 4) * 4;
+            if (!finite4(__ldg(reinterpret_cast<const float4 *>(P.tq + o)))) s_odd[3] = 1;
+            if (!finite4(__ldg(reinterpret_cast<const float4 *>(P.tk + o)))) s_odd[4] = 1;
+        }
     }
     // this block's share: a contiguous range of equal cost
     const bool split = tc::split_windows<(NW + 1) * 32, 7, 8>(P.w_sizes, P.W, smem + L.off_pq);
@@ -407,6 +426,13 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
         if (tg < 3) {
             uint64_t x[HP];
             load_row<HD>(x, (tg == 0 ? s_q : (tg == 1 ? s_do : s_k)) + lane * RS);
+            if (wsub == 0) {                                          // 0 * x is zero for every finite x
+                uint64_t z = mul2(x[0], 0ull);
+#pragma unroll
+                for (int i = 1; i < HP; ++i) z = fma2(x[i], 0ull, z);
+                const bool odd = __any_sync(0xffffffffu, sum2(z) != 0.f);
+                if (lane == 0) s_odd[tg] = odd;
+            }
             TableTile<HD> tile;
             tc::UsedTiles tiles(used, n_mt, wsub, TG);
             int mt = tiles.next();
@@ -571,6 +597,26 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
             store_row<HD>(s_pg + (32 + lane) * HD, acc);
         }
         consumer_sync<NT>();
+        // ---- rows of the item that are not finite: NaN to the histogram entries of their pairs, zeros in their place (passing
+        // over zero entries in the loop below made every item 3 % slower) -------------------------------------------
+        if (__builtin_expect(s_odd[0] | s_odd[1] | s_odd[2], 0)) {
+            float *rows = s_rows + s * (4 * 32 * RS);
+            float *const X[3] = {rows, rows + 32 * RS, rows + 64 * RS}, *const hist[3] = {s_hq, s_hv, s_hk};
+#pragma unroll 1
+            for (int e = tid; e < 3 * 32 * HD; e += NT) {
+                const int tab = e / (32 * HD), v = e / HD & 31;
+                if (fabsf(X[tab][v * RS + e % HD]) < INFINITY || !(tab < 2 ? do_q : do_k)) continue;
+#pragma unroll 1
+                for (int r = 0; r < L.R16; ++r)
+                    if (((used >> (r >> 4)) & 1u) && hist[tab][r * QT + v] != 0.f) hist[tab][r * QT + v] = NAN;
+            }
+            consumer_sync<NT>();
+            for (int e = tid; e < 3 * 32 * HD; e += NT) {
+                float *x = X[e / (32 * HD)] + (e / HD & 31) * RS + e % HD;
+                if (!(fabsf(*x) < INFINITY)) *x = 0.f;
+            }
+            consumer_sync<NT>();
+        }
         // ---- table gradients: lane = row of a 32-row unit ---------------------------------------------------------
         if (dtg < 3 && (dtg < 2 ? do_q : do_k)) {
             const float *hist = dtg == 0 ? s_hq : (dtg == 1 ? s_hv : s_hk);
@@ -605,6 +651,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
         // ---- dQ += histQ.Tq, dK += histK.Tk: lane = voxel -----------------------------------------------------------
         if (side < 2 && (side == 0 ? do_q : do_k)) {
             const float *T = side == 0 ? P.tq : P.tk, *hist = side == 0 ? s_hq : s_hk;
+            const bool odd_table = s_odd[3 + side];
             uint64_t acc[HP];
 #pragma unroll
             for (int i = 0; i < HP; ++i) acc[i] = 0ull;
@@ -619,8 +666,14 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
                 const int nx = tiles.next();
                 if (nx >= 0) tile.fetch(T, HC, co, s_map, nx, lane);
                 const float *h = hist + mt * 16 * QT + lane;
+                if (__builtin_expect(odd_table, 0)) {
+#pragma unroll 1
+                    for (int r = 0; r < 16; ++r)
+                        if (h[r * QT] != 0.f) axpy_row<HD>(acc, h[r * QT], st + r * HD);
+                } else {
 #pragma unroll 4
-                for (int r = 0; r < 16; ++r) axpy_row<HD>(acc, h[r * QT], st + r * HD);
+                    for (int r = 0; r < 16; ++r) axpy_row<HD>(acc, h[r * QT], st + r * HD);
+                }
                 mt = nx;
             }
             store_row<HD>(s_part + ((side * SG + ws2) * 32 + lane) * HD, acc);

@@ -443,6 +443,50 @@ def test_fp16_pairs_of_16_channel_heads_at_the_edges_of_their_products(H, ws, cr
         assert rel_err(a, b) < FP16_TOL, name
 
 
+def _rows_of_pairs(p, queries, keys):
+    """Table rows that the pairs (query, key) of sorted positions touch, index L of a dimension being the next one's row 0."""
+    L = [s // (p.H * p.hd) for s in p.sizes]
+    rows = set()
+    for d, n in enumerate(L):
+        rel = p.n_crse[queries][:, None, d] - p.n_crse[keys][None, :, d] + np.float32(n // 2)
+        idx = np.clip(rel, 0, n - 1 if d == p.D - 1 else n).astype(np.int64)
+        rows |= set((sum(L[:d]) + idx).ravel().tolist())
+    return rows
+
+
+@pytest.mark.parametrize("crse,hd,what", [(c, h, w) for c, h in [("XYZ_RGB_NORM", 8), ("XYZ_RGB", 16)] for w in ("q", "g", "k", "tq", "tk")] +
+                         [("XYZ", 8, "q"), ("XYZ", 8, "g")])          # without colours a window touches every row
+def test_fp32_a_value_that_is_not_finite_reaches_its_own_pairs_only(crse, hd, what):
+    """An infinite q or gradient row spoils the pairs of that query, a key row or table entry those of its window; rows and
+    table rows that no spoiled pair touches are those of the finite problem."""
+    from tests.gpu_helpers import cuda_fwd_bwd
+    p = make_problem(seed=99, ws=5, H=2, hd=hd, crse=crse, scene=_scene_of_window_sizes(5, [40, 70, 33, 5, 20]))
+    a, n = int(p.w2n[1]), int(p.w_sizes[1])
+    window = np.arange(a, a + n)
+    spoiled = _rows_of_pairs(p, window[3:4] if what in "qg" else window, window)
+    clean = cuda_fwd_bwd(p)
+    if what in ("tq", "tk"):
+        others = [np.arange(b, b + m) for b, m in zip(p.w2n, p.w_sizes) if b != a]
+        row = sorted(spoiled - set().union(*[_rows_of_pairs(p, w, w) for w in others]))[0]
+        getattr(p, what).reshape(-1, 2, hd)[row, 1, 3] = np.inf
+    else:
+        getattr(p, what)[p.n2n[a + 3], 1, 2] = np.inf
+    bad = cuda_fwd_bwd(p)
+    rows = np.setdiff1d(np.arange(p.N), p.n2n[window])            # voxels of the other windows
+    keep = np.setdiff1d(np.arange(sum(p.sizes) // (2 * hd)), sorted(spoiled))
+    assert len(rows) and len(keep)
+    for name, x, y in zip("out dq dk dv".split(), (bad[0],) + bad[2][:3], (clean[0],) + clean[2][:3]):
+        assert np.array_equal(x[rows], y[rows]), name
+        assert np.array_equal(x[:, 0][rows], y[:, 0][rows])
+    for name, x, y in zip("dtq dtk dtv".split(), bad[2][3:], clean[2][3:]):
+        x, y = x.reshape(-1, 2, hd), y.reshape(-1, 2, hd)
+        assert np.abs(x[keep] - y[keep]).max() < 1e-5 * np.abs(y).max(), name    # atomics in another order
+    if what == "q":
+        own = np.setdiff1d(p.n2n[window], p.n2n[a + 3])           # the other queries of the window
+        assert np.array_equal(bad[2][0][own], clean[2][0][own])
+        assert not np.isfinite(bad[2][0][p.n2n[a + 3], 1]).any()
+
+
 @pytest.mark.parametrize("H,hd,ws,crse", [(2, 8, 5, "XYZ_RGB_NORM"), (4, 8, 7, "XYZ_RGB"), (2, 8, 7, "XYZ"), (10, 8, 7, "XYZ_RGB_NORM"),
                                           (1, 16, 5, "XYZ_RGB_NORM"), (3, 16, 7, "XYZ_RGB"), (1, 16, 7, "XYZ")])
 def test_fp16_forward_at_the_edges_of_its_tiles(H, hd, ws, crse):
