@@ -75,16 +75,15 @@ def test_argument_validation_without_device():
 
 
 def test_knn_index_stops_where_its_row_numbers_do():
-    """The search over the index counts rows in int and runs up to 3840 (the tie kernel's round) past the last
-    one of a scene: it takes no call whose rows plus that pass 2^31 - 1; below, offsets of 128 floats per
-    32 rows exceed 2^31 and are the kernel's 64-bit business."""
+    """The search over the index numbers rows, and floats in its planes of 128 per 32 rows, in int, and runs up to 3840
+    (the tie kernel's round) past the last row of a scene: it takes no call for which these pass 2^31 - 1."""
     from swin3d_b200 import _lib
     need = _lib.lib.s3d_knn_workspace_bytes
-    most = 2 ** 31 - 2 ** 13
-    assert most + 3840 < 2 ** 31 - 1
+    most = 2 ** 29 - 2 ** 13
+    assert (most + 31) // 32 * 128 < 2 ** 31 and most + 3840 < 2 ** 31
     for K in (3, 16):
         assert need(K, 1, most - 5, 5) > (most - 5) * 16
-        assert need(K, 1, most - 4, 5) == 0 and need(K, 1, 2 ** 31 - 10, 5) == 0
+        assert need(K, 1, most - 4, 5) == 0 and need(K, 1, 2 ** 29, 5) == 0 and need(K, 1, 2 ** 31 - 10, 5) == 0
 
 
 def test_python_wrappers_reject_cpu_tensors():
