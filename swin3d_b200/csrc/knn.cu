@@ -84,14 +84,12 @@ __device__ __forceinline__ float knn_threshold(float top, float sq, float pmax2)
 // The heaps are thread-private arrays (local memory beyond a few entries; heaps in shared memory as
 // [entry][thread] were measured at the same speed for K = 16: the cost there is the number of heap
 // updates, K (1 + ln(N / K)) per query, each entered by a whole warp).
-// LIST: the queries are those of a list in device memory (tied queries of the search over the spatial
-// index), walked by a fixed grid; nothing happens unless it holds more than list_min.
-template <int KMAX, int NQ, int NT, int QCAP, bool LIST>
+// GATED: nothing happens unless *count is larger than most (the search over the spatial index left that many tied queries).
+template <int KMAX, int NQ, int NT, int QCAP, bool GATED>
 __global__ void __launch_bounds__(NT)
 knn_kernel(int K, const float *__restrict__ src, const float *__restrict__ query,
            const int32_t *__restrict__ src_offset, const int32_t *__restrict__ query_offset,
-           int B, int64_t Nq, const int32_t *__restrict__ list, const int *__restrict__ list_count, int list_min,
-           bool root, int32_t *__restrict__ ret_idx, float *__restrict__ ret_dist)
+           int B, int64_t Nq, const int *__restrict__ count, int64_t most, bool root, int32_t *__restrict__ ret_idx, float *__restrict__ ret_dist)
 {
     // planes x, y, z, |p|^2 of a tile; a step may read past the last point
     __shared__ __align__(16) float s_p[4][KNN_TILE + KNN_STEP];
@@ -99,10 +97,8 @@ knn_kernel(int K, const float *__restrict__ src, const float *__restrict__ query
     __shared__ int s_lo, s_hi;
     __shared__ unsigned s_pmax;                    // bits of the largest |p|^2 loaded so far
 
-    const int64_t total = LIST ? (int64_t)__ldg(list_count) : Nq;
-    if (LIST && total <= list_min) return;
-    for (int64_t blk = blockIdx.x; blk * (NT * NQ) < total; blk += gridDim.x) {
-    const int64_t g0 = blk * (NT * NQ) + threadIdx.x;
+    if (GATED && __ldg(count) <= most) return;
+    const int64_t g0 = (int64_t)blockIdx.x * (NT * NQ) + threadIdx.x;
 
     float heap[NQ][KMAX];
     int hidx[NQ][KMAX];
@@ -110,7 +106,6 @@ knn_kernel(int K, const float *__restrict__ src, const float *__restrict__ query
     uint64_t a2[NQ], b2[NQ], c2[NQ];
     int s0[NQ], s1[NQ], qn[NQ];
     bool active[NQ];
-    int64_t gq[NQ];
 #pragma unroll
     for (int r = 0; r < NQ; ++r) {
 #pragma unroll
@@ -118,10 +113,8 @@ knn_kernel(int K, const float *__restrict__ src, const float *__restrict__ query
             heap[r][i] = 2147483648.0f;  // (float)0x7fffffff
             hidx[r][i] = 0;
         }
-        const int64_t at = g0 + (int64_t)r * NT;
-        active[r] = at < total;
-        const int64_t g = LIST && active[r] ? (int64_t)__ldg(list + at) : at;
-        gq[r] = g;
+        const int64_t g = g0 + (int64_t)r * NT;
+        active[r] = g < Nq;
         qx[r] = qy[r] = qz[r] = 0.f;
         s0[r] = s1[r] = 0;
         qn[r] = 0;
@@ -138,7 +131,6 @@ knn_kernel(int K, const float *__restrict__ src, const float *__restrict__ query
         c2[r] = pack2(-2.f * qz[r], -2.f * qz[r]);
         sq[r] = __fmaf_rn(qz[r], qz[r], __fmaf_rn(qy[r], qy[r], __fmul_rn(qx[r], qx[r])));
     }
-    if (LIST) __syncthreads();                     // the previous round of the block is over
     if (threadIdx.x == 0) { s_lo = 0x7fffffff; s_hi = 0; s_pmax = 0u; }
     __syncthreads();
 #pragma unroll
@@ -275,41 +267,29 @@ knn_kernel(int K, const float *__restrict__ src, const float *__restrict__ query
 #pragma unroll
     for (int r = 0; r < NQ; ++r) {
         if (!active[r]) continue;
+        const int64_t g = g0 + (int64_t)r * NT;
         knn_heap_sort(heap[r], hidx[r], K);
         for (int i = 0; i < K; ++i) {
-            ret_dist[gq[r] * K + i] = root ? __fsqrt_rn(heap[r][i]) : heap[r][i];
-            ret_idx[gq[r] * K + i] = hidx[r][i];
+            ret_dist[g * K + i] = root ? __fsqrt_rn(heap[r][i]) : heap[r][i];
+            ret_idx[g * K + i] = hidx[r][i];
         }
-    }
     }
 }
 
 template <int KMAX, int NQ, int NT, int QCAP>
 static int knn_launch_as(int K, const float *src, const float *query, const int32_t *src_offset,
-                         const int32_t *query_offset, int B, int64_t Nq, bool root, int32_t *ret_idx, float *ret_dist,
-                         cudaStream_t st)
+                         const int32_t *query_offset, int B, int64_t Nq, const int *count, int64_t most, bool root,
+                         int32_t *ret_idx, float *ret_dist, cudaStream_t st)
 {
     const unsigned blocks = (unsigned)((Nq + NT * NQ - 1) / (NT * NQ));
-    knn_kernel<KMAX, NQ, NT, QCAP, false><<<blocks, NT, 0, st>>>(K, src, query, src_offset, query_offset, B, Nq, nullptr, nullptr, 0, root, ret_idx, ret_dist);
-    return cudaGetLastError() == cudaSuccess ? S3D_OK : S3D_ERR_LAUNCH;
-}
-
-int knn_launch_list(int K, const float *src, const float *query, const int32_t *src_offset,
-                    const int32_t *query_offset, int B, int64_t Nq, const int32_t *list, const int *list_count,
-                    int list_min, bool root, int32_t *ret_idx, float *ret_dist, cudaStream_t st)
-{
-    if (K > 16) return S3D_ERR_UNSUPPORTED;
-    const unsigned blocks = (unsigned)((Nq + 127) / 128 < 148 * 8 ? (Nq + 127) / 128 : 148 * 8);
-    if (K <= 4)
-        knn_kernel<4, 1, 128, KNN_STEP + 4, true><<<blocks, 128, 0, st>>>(K, src, query, src_offset, query_offset, B, Nq, list, list_count, list_min, root, ret_idx, ret_dist);
-    else
-        knn_kernel<16, 1, 128, KNN_STEP + 4, true><<<blocks, 128, 0, st>>>(K, src, query, src_offset, query_offset, B, Nq, list, list_count, list_min, root, ret_idx, ret_dist);
+    if (count) knn_kernel<KMAX, NQ, NT, QCAP, true><<<blocks, NT, 0, st>>>(K, src, query, src_offset, query_offset, B, Nq, count, most, root, ret_idx, ret_dist);
+    else knn_kernel<KMAX, NQ, NT, QCAP, false><<<blocks, NT, 0, st>>>(K, src, query, src_offset, query_offset, B, Nq, nullptr, 0, root, ret_idx, ret_dist);
     return cudaGetLastError() == cudaSuccess ? S3D_OK : S3D_ERR_LAUNCH;
 }
 
 int knn_launch(int K, const float *src, const float *query, const int32_t *src_offset,
                const int32_t *query_offset, int B, int64_t Nq, bool root, int32_t *ret_idx, float *ret_dist,
-               cudaStream_t st)
+               cudaStream_t st, const int *count, int64_t most)
 {
     if (Nq == 0) return S3D_OK;
     // few neighbours: the scan dominates, two queries per thread halve its shared-memory loads;
@@ -318,14 +298,14 @@ int knn_launch(int K, const float *src, const float *query, const int32_t *src_o
     // queries: smaller blocks of one query per thread keep more warps resident (measured on 200 k to
     // 1.6 M queries: the smaller blocks win below about 300 k queries for K <= 4, 600 k for K <= 16)
     if (K <= 4) {
-        if (Nq < 300000) return knn_launch_as<4, 1, 128, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, root, ret_idx, ret_dist, st);
-        return knn_launch_as<4, 2, 128, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, root, ret_idx, ret_dist, st);
+        if (Nq < 300000) return knn_launch_as<4, 1, 128, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, count, most, root, ret_idx, ret_dist, st);
+        return knn_launch_as<4, 2, 128, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, count, most, root, ret_idx, ret_dist, st);
     }
     if (K <= 16) {
-        if (Nq < 600000) return knn_launch_as<16, 1, 128, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, root, ret_idx, ret_dist, st);
-        return knn_launch_as<16, 1, 256, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, root, ret_idx, ret_dist, st);
+        if (Nq < 600000) return knn_launch_as<16, 1, 128, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, count, most, root, ret_idx, ret_dist, st);
+        return knn_launch_as<16, 1, 256, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, count, most, root, ret_idx, ret_dist, st);
     }
-    return knn_launch_as<64, 1, 256, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, root, ret_idx, ret_dist, st);
+    return knn_launch_as<64, 1, 256, KNN_STEP + 4>(K, src, query, src_offset, query_offset, B, Nq, count, most, root, ret_idx, ret_dist, st);
 }
 
 }  // namespace s3d

@@ -5,14 +5,11 @@
 
 namespace s3d {
 
-// thread-per-query scan; root: write distances instead of squared distances
+// thread-per-query scan; root: write distances instead of squared distances; with count (device memory) nothing happens
+// unless *count is larger than most
 int knn_launch(int K, const float *src, const float *query, const int32_t *src_offset,
                const int32_t *query_offset, int B, int64_t Nq, bool root, int32_t *ret_idx, float *ret_dist,
-               cudaStream_t st);
-// the same for the queries of a list in device memory; nothing happens unless it holds more than list_min
-int knn_launch_list(int K, const float *src, const float *query, const int32_t *src_offset,
-                    const int32_t *query_offset, int B, int64_t Nq, const int32_t *list, const int *list_count,
-                    int list_min, bool root, int32_t *ret_idx, float *ret_dist, cudaStream_t st);
+               cudaStream_t st, const int *count = nullptr, int64_t most = 0);
 
 // warp-per-query scan
 bool knn_warp_wanted(int K, int B, int64_t Ns, int64_t Nq);

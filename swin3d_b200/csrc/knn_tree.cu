@@ -682,14 +682,14 @@ __device__ __forceinline__ void finish_heap(float *heap, int *hidx, int K, int64
 // The heap is a serial chain over the candidates that enter it, several thousand when the sources are in
 // spatial order.  Warp 0 runs it; the other warps scan the sources ahead of it, 8 per lane and round, and
 // hand over, in index order, those below the heap root of two rounds ago -- all that can still enter.
-// A list of more than list_max queries is left to the thread-per-query scan.
+// A list of more than list_max queries is left to the thread-per-query scan (few_ties).
 constexpr int TIE_THREADS = 512, TIE_WARPS = TIE_THREADS / 32 - 1, TIE_PER = 8;
 
 template <bool ROOT>
 __global__ void __launch_bounds__(TIE_THREADS)
 knn_tie_kernel(int K, const float *__restrict__ src, const float *__restrict__ query, const int32_t *__restrict__ so,
                const int32_t *__restrict__ qo, int B, const int32_t *__restrict__ list, const int *__restrict__ list_count,
-               int list_max, int32_t *__restrict__ ret_idx, float *__restrict__ ret_dist)
+               int64_t list_max, int32_t *__restrict__ ret_idx, float *__restrict__ ret_dist)
 {
     __shared__ float s_d[2][TIE_WARPS][32 * TIE_PER];
     __shared__ uint16_t s_o[2][TIE_WARPS][32 * TIE_PER];     // offset from the first source of the warp's share
@@ -938,6 +938,18 @@ bool knn_warp_wanted(int K, int B, int64_t Ns, int64_t Nq)
     return Ns <= MAX_POINTS && Nq * (Ns / B) <= 20000000;
 }
 
+// Up to this many tied queries get a block each (knn_tie_kernel); with more of them the thread-per-query scan does all
+// queries again.  Both kernels read the count, and one of them returns at once.  4 x 120 k sources: a tied query costs 0.40 /
+// 0.47 / 0.57 us (K = 3 / 8 / 16), the scan of 4 x 30 k queries 7.0 / 13.4 / 21 ms, which is an eighth, a fifth and three
+// tenths of them; fewer than 10,000 queries do not fill the GPU in the scan (2,100 of 120 k sources: 3.1 / 3.5 / 3.8 ms
+// against 0.6 / 0.7 / 0.8).  Many ties cost the index on top of the scan: all queries tied, K = 3, 1 to 5 % more than
+// the scan alone.
+static int64_t few_ties(int K, int64_t Nq)
+{
+    const int64_t part = K <= 4 ? Nq / 8 : (K <= 8 ? Nq / 5 : Nq * 3 / 10);
+    return part > 10000 ? part : 10000;
+}
+
 int64_t knn_tree_bytes(int B, int64_t Ns, int64_t Nq) { return tree_bufs(nullptr, B, Ns, Nq).total; }
 
 int knn_launch_warp(int K, const float *src, const float *query, const int32_t *so, const int32_t *qo, int B, int64_t Nq,
@@ -962,6 +974,7 @@ int knn_launch_tree(int K, const float *src, const float *query, const int32_t *
     scan_in_place(t.hist, t.tile, t.n_tiles, st);
     tree_sort_kernel<false><<<nb, KT_THREADS, 0, st>>>(src, query, so, qo, B, Ns, Nq, t);
     tree_boxes_kernel<<<(unsigned)(Ns / (LEAF * 32) + B), 1024, 0, st>>>(B, t);
+    const int64_t few = few_ties(K, Nq);
     const int share = K <= 3 ? 1 : SHARED;
     const unsigned blocks = (unsigned)((Nq * share + SEARCH_THREADS - 1) / SEARCH_THREADS);
 #define S3D_KNN_SEARCH(KL, SHARE)                                                                                   \
@@ -972,14 +985,11 @@ int knn_launch_tree(int K, const float *src, const float *query, const int32_t *
     else { S3D_KNN_SEARCH(16, SHARED); }
 #undef S3D_KNN_SEARCH
     if (cudaGetLastError() != cudaSuccess) return S3D_ERR_LAUNCH;
-    // tied queries: a block each while they are few, otherwise the thread-per-query scan; both kernels read
-    // the count and one of them returns at once
-    constexpr int FEW = 2048;
     const unsigned tie_blocks = (unsigned)(Nq < 148 * 4 ? Nq : 148 * 4);
-    if (root) knn_tie_kernel<true><<<tie_blocks, TIE_THREADS, 0, st>>>(K, src, query, so, qo, B, t.ties, t.tie_count, FEW, idx, dist);
-    else knn_tie_kernel<false><<<tie_blocks, TIE_THREADS, 0, st>>>(K, src, query, so, qo, B, t.ties, t.tie_count, FEW, idx, dist);
+    if (root) knn_tie_kernel<true><<<tie_blocks, TIE_THREADS, 0, st>>>(K, src, query, so, qo, B, t.ties, t.tie_count, few, idx, dist);
+    else knn_tie_kernel<false><<<tie_blocks, TIE_THREADS, 0, st>>>(K, src, query, so, qo, B, t.ties, t.tie_count, few, idx, dist);
     if (cudaGetLastError() != cudaSuccess) return S3D_ERR_LAUNCH;
-    return Nq > FEW ? knn_launch_list(K, src, query, so, qo, B, Nq, t.ties, t.tie_count, FEW, root, idx, dist, st) : S3D_OK;
+    return Nq > few ? knn_launch(K, src, query, so, qo, B, Nq, root, idx, dist, st, t.tie_count, few) : S3D_OK;
 }
 
 }  // namespace s3d

@@ -246,6 +246,29 @@ def test_knn_index_hands_many_ties_to_the_scan():
         _lib.lib.s3d_debug_knn_path(was)
 
 
+@pytest.mark.parametrize("K", [3, 4, 5, 16])
+@pytest.mark.parametrize("n_tied", [9_999, 10_001, 12_001, 18_001, 60_000])
+def test_knn_tied_queries_either_side_of_the_handover(K, n_tied):
+    """60,000 queries on a lattice of sources, n_tied of them on lattice points (every neighbour distance tied), the rest
+    off them: a block per tied query up to 10,000 (K = 5: 12,000, K = 16: 18,000), all queries by the scan beyond."""
+    from swin3d_b200 import _lib
+    from swin3d_b200.sparse_dl.knn.knn import knn_raw
+    rng = np.random.default_rng(K)
+    src = np.stack(np.meshgrid(np.arange(40), np.arange(25), [0, 9], indexing="ij"), -1).reshape(-1, 3).astype(np.float32)
+    qry = src[rng.integers(0, len(src), 60_000)] + rng.uniform(0.01, 0.4, (60_000, 3)).astype(np.float32)
+    at = rng.permutation(60_000)[:n_tied]
+    qry[at] = np.floor(qry[at])
+    a = [_dev(src), _dev(qry), _dev(np.array([1200, 2000], np.int32)), _dev(np.array([30_000, 60_000], np.int32))]
+    was = _lib.lib.s3d_debug_knn_path(3)
+    try:
+        idx, d2 = knn_raw(K, *a)
+        _lib.lib.s3d_debug_knn_path(1)
+        want_idx, want_d2 = knn_raw(K, *a)
+    finally:
+        _lib.lib.s3d_debug_knn_path(was)
+    assert torch.equal(idx, want_idx) and torch.equal(d2, want_d2)
+
+
 @pytest.mark.parametrize("n_query", [3_001, 65_536])
 @pytest.mark.parametrize("K", [4, 5, 8, 9, 16])
 def test_knn_index_lanes_of_a_query_agree_with_the_heap(K, n_query):
