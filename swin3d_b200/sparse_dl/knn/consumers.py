@@ -9,7 +9,7 @@ Swin3D/modules/swin3d_layers.py): ``knn_linear_interpolation`` (:53-73), ``query
 import torch
 from torch.autograd.function import Function
 
-from ... import _lib
+from ... import _lib, _stream
 from .knn import KNN
 
 
@@ -62,10 +62,8 @@ class KNNInterpolate(Function):
         Nq, K = idx.shape
         C = src_feat.shape[1]
         out = torch.empty((Nq, C), dtype=src_feat.dtype, device=src_feat.device)
-        with torch.cuda.device(src_feat.device):
-            st = torch.cuda.current_stream().cuda_stream
-            rc = _lib.lib.s3d_knn_interpolate_fwd(idx.data_ptr(), dist.data_ptr(), src_feat.data_ptr(),
-                                                  out.data_ptr(), Nq, K, C, _dtype_code(src_feat), st)
+        rc = _stream.call(src_feat.device, _lib.lib.s3d_knn_interpolate_fwd, idx.data_ptr(), dist.data_ptr(),
+                          src_feat.data_ptr(), out.data_ptr(), Nq, K, C, _dtype_code(src_feat))
         _lib.check(rc, "s3d_knn_interpolate_fwd")
         ctx.save_for_backward(idx, dist)
         ctx.n_src = src_feat.shape[0]
@@ -80,19 +78,14 @@ class KNNInterpolate(Function):
         work, nbytes = _gather_workspace(ctx.n_src, Nq, K, grad_out.device)
         if work is not None and grad_out.data_ptr() % 16 == 0:
             dsrc = torch.empty((ctx.n_src, C), dtype=grad_out.dtype, device=grad_out.device)
-            with torch.cuda.device(grad_out.device):
-                st = torch.cuda.current_stream().cuda_stream
-                rc = _lib.lib.s3d_knn_interpolate_gather_bwd(idx.data_ptr(), dist.data_ptr(), grad_out.data_ptr(),
-                                                             dsrc.data_ptr(), Nq, ctx.n_src, K, C, _dtype_code(grad_out),
-                                                             work.data_ptr(), nbytes, st)
+            rc = _stream.call(grad_out.device, _lib.lib.s3d_knn_interpolate_gather_bwd, idx.data_ptr(), dist.data_ptr(),
+                              grad_out.data_ptr(), dsrc.data_ptr(), Nq, ctx.n_src, K, C, _dtype_code(grad_out),
+                              work.data_ptr(), nbytes)
             _lib.check(rc, "s3d_knn_interpolate_gather_bwd")
             return dsrc, None, None
         dsrc = torch.empty((ctx.n_src, C), dtype=torch.float32, device=grad_out.device)
-        with torch.cuda.device(grad_out.device):
-            st = torch.cuda.current_stream().cuda_stream
-            rc = _lib.lib.s3d_knn_interpolate_bwd(idx.data_ptr(), dist.data_ptr(), grad_out.data_ptr(),
-                                                  dsrc.data_ptr(), Nq, ctx.n_src, K, C,
-                                                  _dtype_code(grad_out), st)
+        rc = _stream.call(grad_out.device, _lib.lib.s3d_knn_interpolate_bwd, idx.data_ptr(), dist.data_ptr(), grad_out.data_ptr(),
+                          dsrc.data_ptr(), Nq, ctx.n_src, K, C, _dtype_code(grad_out))
         _lib.check(rc, "s3d_knn_interpolate_bwd")
         return dsrc.to(grad_out.dtype), None, None
 
@@ -116,10 +109,8 @@ class KNNMaxPool(Function):
         C = g.shape[1]
         out = torch.empty((Nq, C), dtype=g.dtype, device=g.device)
         arg = torch.empty((Nq, C), dtype=torch.int32, device=g.device)
-        with torch.cuda.device(g.device):
-            st = torch.cuda.current_stream().cuda_stream
-            rc = _lib.lib.s3d_knn_maxpool_fwd(idx.data_ptr(), g.data_ptr(), out.data_ptr(),
-                                              arg.data_ptr(), Nq, K, C, _dtype_code(g), st)
+        rc = _stream.call(g.device, _lib.lib.s3d_knn_maxpool_fwd, idx.data_ptr(), g.data_ptr(), out.data_ptr(),
+                          arg.data_ptr(), Nq, K, C, _dtype_code(g))
         _lib.check(rc, "s3d_knn_maxpool_fwd")
         ctx.save_for_backward(arg)
         ctx.n_src = g.shape[0]
@@ -132,10 +123,8 @@ class KNNMaxPool(Function):
         grad_out = grad_out.contiguous()
         Nq, C = grad_out.shape
         dg = torch.empty((ctx.n_src, C), dtype=torch.float32, device=grad_out.device)
-        with torch.cuda.device(grad_out.device):
-            st = torch.cuda.current_stream().cuda_stream
-            rc = _lib.lib.s3d_knn_maxpool_bwd(arg.data_ptr(), grad_out.data_ptr(), dg.data_ptr(),
-                                              Nq, ctx.n_src, C, _dtype_code(grad_out), st)
+        rc = _stream.call(grad_out.device, _lib.lib.s3d_knn_maxpool_bwd, arg.data_ptr(), grad_out.data_ptr(), dg.data_ptr(),
+                          Nq, ctx.n_src, C, _dtype_code(grad_out))
         _lib.check(rc, "s3d_knn_maxpool_bwd")
         return dg.to(grad_out.dtype), None
 
@@ -152,10 +141,8 @@ class _KNNMaxPoolSlots(Function):
         C = g.shape[1]
         out = torch.empty((Nq, C), dtype=g.dtype, device=g.device)
         slot = torch.empty((Nq, C), dtype=torch.uint8, device=g.device)
-        with torch.cuda.device(g.device):
-            st = torch.cuda.current_stream().cuda_stream
-            rc = _lib.lib.s3d_knn_maxpool_slots_fwd(idx.data_ptr(), g.data_ptr(), out.data_ptr(), slot.data_ptr(),
-                                                    Nq, K, C, _dtype_code(g), st)
+        rc = _stream.call(g.device, _lib.lib.s3d_knn_maxpool_slots_fwd, idx.data_ptr(), g.data_ptr(), out.data_ptr(), slot.data_ptr(),
+                          Nq, K, C, _dtype_code(g))
         _lib.check(rc, "s3d_knn_maxpool_slots_fwd")
         ctx.save_for_backward(idx, slot)
         ctx.n_src = g.shape[0]
@@ -172,10 +159,8 @@ class _KNNMaxPoolSlots(Function):
         dg = torch.empty((ctx.n_src, C), dtype=grad_out.dtype, device=grad_out.device)
         nbytes = _lib.lib.s3d_knn_gather_workspace_bytes(ctx.n_src, Nq, K)
         work = torch.empty(nbytes, dtype=torch.uint8, device=grad_out.device)
-        with torch.cuda.device(grad_out.device):
-            st = torch.cuda.current_stream().cuda_stream
-            rc = _lib.lib.s3d_knn_maxpool_slots_bwd(idx.data_ptr(), slot.data_ptr(), grad_out.data_ptr(), dg.data_ptr(),
-                                                    Nq, ctx.n_src, K, C, _dtype_code(grad_out), work.data_ptr(), nbytes, st)
+        rc = _stream.call(grad_out.device, _lib.lib.s3d_knn_maxpool_slots_bwd, idx.data_ptr(), slot.data_ptr(),
+                          grad_out.data_ptr(), dg.data_ptr(), Nq, ctx.n_src, K, C, _dtype_code(grad_out), work.data_ptr(), nbytes)
         _lib.check(rc, "s3d_knn_maxpool_slots_bwd")
         return dg, None
 

@@ -172,3 +172,41 @@ def test_gather_backwards_match_the_scatter(dtype, K, C, n_src, Nq):
     size = torch.zeros((n_src, C), dtype=torch.float64, device="cuda").scatter_add_(0, arg.long(), dout.double().abs())
     if K <= n_src:                                    # a row listed twice by a query: the first position counts, as here
         assert ((got.double() - ref.double()).abs() <= size * n_max * 2.0 ** -23 + 2 * ref.double().abs() * eps + 2.0 ** -24).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("K,C,n_src,Nq,counts", [(3, 80, 500, 3_000, (64, 65, 66)), (3, 640, 40, 3_000, (1279, 1280, 1281, 2561)),
+                                                 (16, 8, 300, 5_000, (255, 256, 257, 511, 512, 513)), (3, 16, 20_000, 40_000, (20_000, 70, 65)),
+                                                 (1, 4, 3, 3_000, (700, 2_000)), (3, 2064, 9, 700, (100, 300))])
+def test_gather_backwards_of_long_rows(dtype, K, C, n_src, Nq, counts):
+    """Source rows with more entries than a thread sums (64) and than a block takes at a time (the larger of 256 and 2 C),
+    each side of both, among rows without any; more pieces in a row than threads in a block."""
+    if dtype == torch.float16 and C % 8:
+        pytest.skip("rows of fp16 are whole 16-byte pieces")
+    from swin3d_b200.sparse_dl.knn import KNNInterpolate, consumers
+    g = torch.Generator(device="cuda").manual_seed(C + Nq)
+    rest = torch.randint(len(counts) + 1, max(n_src, len(counts) + 2), (Nq * K - sum(counts),), generator=g, device="cuda") % n_src
+    idx = torch.cat([torch.full((c,), i, device="cuda") for i, c in enumerate(counts)] + [rest])
+    idx = idx[torch.randperm(Nq * K, generator=g, device="cuda")].view(Nq, K).int()
+    dist = torch.rand((Nq, K), generator=g, device="cuda")
+    feat = torch.randn((n_src, C), generator=g, device="cuda").to(dtype).requires_grad_()
+    dout = torch.randn((Nq, C), generator=g, device="cuda").to(dtype)
+    w = 1.0 / (dist + 1e-8)
+    w = (w / w.sum(1, keepdim=True)).double()
+    size, want = (torch.zeros((n_src, C), dtype=torch.float64, device="cuda") for _ in range(2))
+    for i in range(K):
+        want.index_add_(0, idx[:, i].long(), w[:, i, None] * dout.double())
+        size.index_add_(0, idx[:, i].long(), w[:, i, None] * dout.double().abs())
+    eps = 2.0 ** -24 if dtype == torch.float32 else 2.0 ** -11
+    n_max = int(torch.bincount(idx.flatten().long(), minlength=n_src).max()) + 8
+    was, consumers.GATHER_MOST_PER_SOURCE = consumers.GATHER_MOST_PER_SOURCE, 1 << 30
+    try:
+        (got,) = torch.autograd.grad(KNNInterpolate.apply(feat, idx, dist), [feat], dout)
+        out = consumers._KNNMaxPoolSlots.apply(feat, idx)
+        (pooled,) = torch.autograd.grad(out, [feat], dout)
+    finally:
+        consumers.GATHER_MOST_PER_SOURCE = was
+    assert ((got.double() - want).abs() <= size * n_max * 2.0 ** -24 + want.abs() * eps + 2.0 ** -24).all()
+    arg = torch.gather(idx.long()[:, :, None].expand(-1, -1, C), 1, feat.detach()[idx.long()].argmax(1, keepdim=True))[:, 0]
+    ref, size = (torch.zeros((n_src, C), dtype=torch.float64, device="cuda").scatter_add_(0, arg, d) for d in (dout.double(), dout.double().abs()))
+    assert ((pooled.double() - ref).abs() <= size * n_max * 2.0 ** -24 + ref.abs() * eps + 2.0 ** -24).all()
