@@ -237,9 +237,9 @@ int s3d_window_build_static(const int32_t *coords, const float *feats, int64_t N
  * reasonably well (no sort: a dense grid of windows with a bit per cell).
  *  xyz, rest: the first three and the other F - 3 signals of a voxel, rows xyz_stride / rest_stride floats
  *  apart.  w2m int64[N]: exclusive sum of the squared window sizes.  counts_host[4] (host memory):
- *  windows, attention pairs, largest window, flags: 1 = a coordinate outside the supported range,
- *  2 = the box holds too many windows, 4 = repeated voxels; with a flag set the outputs are incomplete
- *  and (2, 4) s3d_window_build does the job.
+ *  windows, attention pairs, largest window, flags: 1 = a coordinate outside the supported range (the
+ *  outputs are incomplete), 2 = the box holds too many windows, 4 = repeated voxels: sorted, as by
+ *  s3d_window_build, and w2m is not written.
  *  workspace: s3d_window_groups_workspace_bytes, 16-byte aligned device memory.
  */
 int64_t s3d_window_groups_workspace_bytes(int64_t N, int ws);

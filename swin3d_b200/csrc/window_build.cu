@@ -30,7 +30,7 @@ constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
-constexpr int NPASS = 8;
+constexpr int NPASS = WB_MAX_PASSES;
 
 // ---- keys ------------------------------------------------------------------------------------
 // range[0..3] = min of (batch, wx, wy, wz), range[4..7] = max; also flags coordinates outside the
@@ -255,57 +255,64 @@ radix_scatter_kernel(SortBufs b, int pass, int64_t N, int nblk, const uint32_t *
                      const int *__restrict__ skip)
 {
     if (skip[pass]) return;
-    __shared__ uint32_t s_run[256];
+    // a warp takes 256 consecutive keys: their ranks among the warp's keys of the same digit, then the warps' counts of a
+    // digit one after the other, so that earlier keys get lower positions (stability). 
+    __shared__ uint32_t s_cnt[WB_THREADS / 32][256];
     const int src = b.cur[pass];
     const uint64_t *kin = b.keys[src];
     const uint32_t *vin = b.vals[src];
     uint64_t *kout = b.keys[src ^ 1];
     uint32_t *vout = b.vals[src ^ 1];
-    s_run[threadIdx.x] = excl[(int64_t)threadIdx.x * nblk + blockIdx.x];
-    __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t base = (int64_t)blockIdx.x * WB_TILE;
+#pragma unroll
+    for (int w = 0; w < WB_THREADS / 32; ++w) s_cnt[w][threadIdx.x] = 0;
+    __syncthreads();
+    const int64_t base = (int64_t)blockIdx.x * WB_TILE + warp * (32 * WB_ITEMS) + lane;
+    uint64_t key[WB_ITEMS];
+    uint32_t val[WB_ITEMS], rank[WB_ITEMS];
+#pragma unroll
     for (int j = 0; j < WB_ITEMS; ++j) {
-        const int64_t i = base + j * WB_THREADS + threadIdx.x;
-        const bool valid = i < N;
-        uint64_t key = 0;
-        uint32_t val = 0;
-        int digit = 256 + lane;  // unique per lane: invalid lanes match nobody
-        if (valid) {
-            key = kin[i];
-            val = vin[i];
-            digit = (int)((key >> (8 * pass)) & 255);
-        }
-        const uint32_t peers = __match_any_sync(0xffffffffu, digit);
-        const int rank = __popc(peers & ((1u << lane) - 1u));
-        const int leader = __ffs(peers) - 1;
-        // warps take turns so that earlier keys get lower positions (stability)
-        for (int wv = 0; wv < WB_THREADS / 32; ++wv) {
-            uint32_t start = 0;
-            if (warp == wv) {
-                if (valid && lane == leader) {
-                    start = s_run[digit];
-                    s_run[digit] = start + __popc(peers);
-                }
-                start = __shfl_sync(0xffffffffu, start, leader);
-                if (valid) {
-                    kout[start + rank] = key;
-                    vout[start + rank] = val;
-                }
-            }
-            __syncthreads();
-        }
+        const int64_t i = base + 32 * j;
+        key[j] = i < N ? kin[i] : 0;
+        val[j] = i < N ? vin[i] : 0;
     }
+#pragma unroll
+    for (int j = 0; j < WB_ITEMS; ++j) {
+        const bool valid = base + 32 * j < N;
+        const int digit = valid ? (int)((key[j] >> (8 * pass)) & 255) : 256 + lane;      // invalid lanes match nobody
+        const uint32_t peers = __match_any_sync(0xffffffffu, digit);
+        const uint32_t before = valid ? s_cnt[warp][digit] : 0;
+        rank[j] = before + __popc(peers & ((1u << lane) - 1u));
+        __syncwarp();
+        if (valid && lane == __ffs(peers) - 1) s_cnt[warp][digit] = before + __popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    uint32_t run = excl[(int64_t)threadIdx.x * nblk + blockIdx.x];
+#pragma unroll
+    for (int w = 0; w < WB_THREADS / 32; ++w) {
+        const uint32_t c = s_cnt[w][threadIdx.x];
+        s_cnt[w][threadIdx.x] = run;
+        run += c;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < WB_ITEMS; ++j)
+        if (base + 32 * j < N) {
+            const uint32_t at = s_cnt[warp][(key[j] >> (8 * pass)) & 255] + rank[j];
+            kout[at] = key[j];
+            vout[at] = val[j];
+        }
 }
 
 // ---- windows from sorted keys ------------------------------------------------------------------------
-__global__ void wb_flags_kernel(SortBufs b, int64_t N, int ws, int F,
-                                const float *__restrict__ feats, uint32_t *__restrict__ flags,
+__global__ void wb_flags_kernel(SortBufs b, int passes, int64_t N, int ws, int F, const float *__restrict__ xyz, int xyz_stride,
+                                const float *__restrict__ rest, int rest_stride, uint32_t *__restrict__ flags,
                                 int32_t *__restrict__ n2n, float *__restrict__ n_coords)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
-    const int fin = b.cur[NPASS];
+    const int fin = b.cur[passes];
     const uint64_t key = b.keys[fin][i];
     const uint32_t vid = b.vals[fin][i];
     const uint64_t win = key >> CELL_BITS;
@@ -313,12 +320,12 @@ __global__ void wb_flags_kernel(SortBufs b, int64_t N, int ws, int F,
     n2n[i] = (int32_t)vid;
     const int cell = (int)(key & ((1 << CELL_BITS) - 1));
     const int cz = cell % ws, cy = (cell / ws) % ws, cx = cell / (ws * ws);
-    const float *f = feats + (int64_t)vid * F;
+    const float *f = xyz + (int64_t)vid * xyz_stride, *r = rest + (int64_t)vid * rest_stride;
     float *o = n_coords + i * F;
     o[0] = (float)cx + __ldg(f);
     o[1] = (float)cy + __ldg(f + 1);
     o[2] = (float)cz + __ldg(f + 2);
-    for (int j = 3; j < F; ++j) o[j] = __ldg(f + j);
+    for (int j = 3; j < F; ++j) o[j] = __ldg(r + j - 3);
 }
 
 __global__ void wb_heads_kernel(const uint32_t *__restrict__ flags, const uint32_t *__restrict__ excl,
@@ -396,10 +403,18 @@ static constexpr WbLayout wb_layout(int64_t N)
 
 int64_t window_build_workspace_bytes(int64_t N) { return wb_layout(N).total; }
 
-int window_build_launch(const int32_t *coords, const float *feats, int64_t N, int F, int stride,
-                        int ws, int shift, int32_t *n2n, float *n_coords, int32_t *w_sizes,
+int window_build_passes(const int *span)
+{
+    int bits = CELL_BITS;
+    for (int k = 0; k < 4; ++k)
+        for (int v = span[k]; v > 0; v >>= 1) ++bits;
+    return bits < 64 ? (bits + 7) / 8 : NPASS;
+}
+
+int window_build_launch(const int32_t *coords, const float *xyz, int xyz_stride, const float *rest, int rest_stride, int64_t N,
+                        int F, int stride, int ws, int shift, int32_t *n2n, float *n_coords, int32_t *w_sizes,
                         int32_t *w2n, int64_t *counts, void *workspace, int64_t workspace_bytes,
-                        cudaStream_t st)
+                        cudaStream_t st, int passes)
 {
     const WbLayout L = wb_layout(N);
     if (workspace_bytes < L.total) return S3D_ERR_WORKSPACE;
@@ -423,13 +438,13 @@ int window_build_launch(const int32_t *coords, const float *feats, int64_t N, in
     const unsigned nb = (unsigned)((N + 255) / 256);
     wb_range_kernel<<<nb < 148u * 8u ? nb : 148u * 8u, 256, 0, st>>>(coords, N, stride, ws, shift, range, counts);
     wb_keys_kernel<<<nb, 256, 0, st>>>(coords, N, stride, ws, shift, range, b.keys[0], b.vals[0], live);
-    for (int pass = 0; pass < NPASS; ++pass) {
+    for (int pass = 0; pass < passes; ++pass) {
         radix_hist_kernel<<<L.nblk, WB_THREADS, 0, st>>>(b, pass, N, L.nblk, hist, live);
         scan_excl_u32(hist, excl, (int64_t)256 * L.nblk, sums, st, live + pass);
         radix_decide_kernel<<<1, 256, 0, st>>>(b, pass, N, L.nblk, excl, skip, live);
         radix_scatter_kernel<<<L.nblk, WB_THREADS, 0, st>>>(b, pass, N, L.nblk, excl, skip);
     }
-    wb_flags_kernel<<<nb, 256, 0, st>>>(b, N, ws, F, feats, flags, n2n, n_coords);
+    wb_flags_kernel<<<nb, 256, 0, st>>>(b, passes, N, ws, F, xyz, xyz_stride, rest, rest_stride, flags, n2n, n_coords);
     scan_excl_u32(flags, excl, N, sums, st);
     wb_heads_kernel<<<nb, 256, 0, st>>>(flags, excl, N, w2n, counts);
     wb_sizes_kernel<<<148 * 4, 256, 0, st>>>(w2n, N, w_sizes, counts);
@@ -495,6 +510,6 @@ extern "C" int s3d_window_build_static(const int32_t *coords, const float *feats
     // Nothing in the scratch has to start at zero: every field the kernels read is written earlier
     // in the same call (keys, values, digit histograms, scans, flags, pass bookkeeping), so the
     // contents left behind by the previous call are simply overwritten.
-    return s3d::window_build_launch(coords, feats, N, F, stride, ws, shift, n2n, n_coords, w_sizes, w2n,
+    return s3d::window_build_launch(coords, feats, F, feats ? feats + 3 : nullptr, F, N, F, stride, ws, shift, n2n, n_coords, w_sizes, w2n,
                                     counts_out, scratch, WB_STATIC_BYTES, static_cast<cudaStream_t>(stream));
 }

@@ -135,7 +135,8 @@ wd_mark_kernel(const int32_t *__restrict__ coords, int64_t N, WindowGrid w, WdBu
     const VoxelWindow v = voxel_window(coords, i, w);
     const uint32_t bit = 1u << (v.cell & 31);
     const uint32_t old = atomicOr(b.mask + (int64_t)wd_index(x, v) * b.words + (v.cell >> 5), bit);
-    if (old & bit) atomicOr(reinterpret_cast<unsigned long long *>(b.counts + 3), (unsigned long long)WD_REPEATED);
+    if ((old & bit) && !(*(volatile int64_t *)(b.counts + 3) & WD_REPEATED))      // half of a million voxels repeated: 300 us of atomics
+        atomicOr(reinterpret_cast<unsigned long long *>(b.counts + 3), (unsigned long long)WD_REPEATED);
 }
 
 __device__ __forceinline__ uint32_t wd_count(const WdBufs &b, uint32_t win, uint32_t total)
@@ -149,6 +150,7 @@ __device__ __forceinline__ uint32_t wd_count(const WdBufs &b, uint32_t win, uint
 __global__ void __launch_bounds__(WD_THREADS)
 wd_tile_kernel(WdBufs b)
 {
+    if (b.counts[3]) return;                                   // the sort takes over
     const uint32_t total = wd_box(b).total;
     if (blockIdx.x * (uint32_t)WD_TILE >= total) return;
     unsigned long long sq = 0;
@@ -191,6 +193,7 @@ wd_tile_kernel(WdBufs b)
 __global__ void __launch_bounds__(WD_THREADS)
 wd_scan_kernel(WdBufs b, int32_t *__restrict__ w_sizes, int32_t *__restrict__ w2n, int64_t *__restrict__ w2m)
 {
+    if (b.counts[3]) return;
     const uint32_t total = wd_box(b).total;
     const uint32_t base = blockIdx.x * (uint32_t)WD_TILE;
     if (base >= total) return;
@@ -257,7 +260,7 @@ wd_scatter_kernel(const int32_t *__restrict__ coords, const float *__restrict__ 
                   int rest_stride, int64_t N, int F, WindowGrid w, WdBufs b,
                   int32_t *__restrict__ n2n, float *__restrict__ n_coords)
 {
-    if (b.counts[3]) return;                                   // the host takes the other path
+    if (b.counts[3]) return;
     const WdBox x = wd_box(b);
     const int64_t i = (int64_t)blockIdx.x * WD_THREADS + threadIdx.x;
     if (i >= N) return;
@@ -281,11 +284,11 @@ int64_t window_dense_workspace_bytes(int64_t N, int ws) { return wd_layout(nullp
 
 int window_dense_launch(const int32_t *coords, const float *xyz, int xyz_stride, const float *rest, int rest_stride,
                         int64_t N, int F, int stride, int ws, int shift, int32_t *n2n, float *n_coords, int32_t *w_sizes,
-                        int32_t *w2n, int64_t *w2m, int64_t **counts, void *workspace, int64_t workspace_bytes, cudaStream_t st)
+                        int32_t *w2n, int64_t *w2m, uint32_t **state, void *workspace, int64_t workspace_bytes, cudaStream_t st)
 {
     const WdBufs b = wd_layout(static_cast<char *>(workspace), N, ws);
     if (workspace_bytes < b.total) return S3D_ERR_WORKSPACE;
-    *counts = b.counts;
+    *state = b.range;
     if (cudaMemsetAsync(b.range, 0, (size_t)b.cleared, st) != cudaSuccess) return S3D_ERR_LAUNCH;
     if (N == 0) return S3D_OK;
     const WindowGrid w{stride, ws, shift};

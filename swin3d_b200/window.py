@@ -8,7 +8,7 @@ order.  Windows are emitted in lexicographic (batch, wx, wy, wz) order; the refe
 whatever MinkowskiEngine's pooling returns and attention does not depend on it.
 """
 import ctypes
-from dataclasses import dataclass
+from dataclasses import dataclass, field
 from typing import Optional
 
 import torch
@@ -24,15 +24,23 @@ class WindowIndex:
     w2n: torch.Tensor        # int32 [W]  first sorted position of each window
     num_pairs: int           # M = sum w^2
     max_window: int
-    w2m: Optional[torch.Tensor] = None   # int64 [W]  exclusive sum of w^2
+    w2m: Optional[torch.Tensor] = field(default_factory=lambda: None)   # int64 [W]  exclusive sum of w^2; made when asked for
+
+    def __post_init__(self):
+        if self.w2m is None:
+            del self.w2m
+
+    def __getattr__(self, name):
+        if name != "w2m":
+            raise AttributeError(name)
+        w2 = self.w_sizes.to(torch.int64) ** 2
+        self.w2m = torch.cumsum(w2, 0) - w2
+        return self.w2m
 
     def reference_indices(self, n_crse: torch.Tensor):
         """The six-tensor list ``SelfAttnAIOFunction.apply`` takes for IndexMode.INDIRECT.
         ``m2w`` (one entry per attention pair in the reference) is never read by the fused
         kernels, so an empty tensor stands in for it; ``w2m`` is the exclusive sum of w^2."""
-        if self.w2m is None:
-            w2 = self.w_sizes.to(torch.int64) ** 2
-            self.w2m = torch.cumsum(w2, 0) - w2
         m2w = torch.empty(0, dtype=torch.int64, device=self.n2n.device)
         return [m2w, self.w_sizes, self.w2m, self.w2n, self.n2n, n_crse]
 
@@ -52,8 +60,8 @@ def _build(coords, xyz, rest, feats, window_size: int, shift: int, stride: int) 
     w2n = torch.empty(max(N, 1), dtype=torch.int32, device=dev)
     w2m = torch.empty(max(N, 1), dtype=torch.int64, device=dev)
     lib = _lib.lib
-    # distinct voxels that fill their box of windows reasonably well: no sort, and the library reads the
-    # window count back itself (the one host sync of the builder)
+    # distinct voxels that fill their box of windows reasonably well are not sorted (others are, after a second
+    # look); the library reads the window count back itself
     wbytes = lib.s3d_window_groups_workspace_bytes(N, window_size)
     if wbytes:
         work = torch.empty(wbytes, dtype=torch.uint8, device=dev)
@@ -66,8 +74,7 @@ def _build(coords, xyz, rest, feats, window_size: int, shift: int, stride: int) 
         W, M, mx, flags = host
         if flags & 1:
             raise ValueError(_RANGE_ERROR)
-        if not flags:
-            return WindowIndex(n2n, n_coords, w_sizes[:W], w2n[:W], M, mx, w2m[:W])
+        return WindowIndex(n2n, n_coords, w_sizes[:W], w2n[:W], M, mx, None if flags else w2m[:W])
     counts = torch.empty(4, dtype=torch.int64, device=dev)
     wbytes = lib.s3d_window_build_workspace_bytes(N)
     work = torch.empty(wbytes, dtype=torch.uint8, device=dev)
@@ -78,8 +85,7 @@ def _build(coords, xyz, rest, feats, window_size: int, shift: int, stride: int) 
     W, M, mx, err = (int(x) for x in counts.tolist())
     if err:
         raise ValueError(_RANGE_ERROR)
-    w2 = w_sizes[:W].to(torch.int64) ** 2
-    return WindowIndex(n2n, n_coords, w_sizes[:W], w2n[:W], M, mx, torch.cumsum(w2, 0) - w2)
+    return WindowIndex(n2n, n_coords, w_sizes[:W], w2n[:W], M, mx)
 
 
 def build_windows(coords: torch.Tensor, feats: torch.Tensor, window_size: int, shift: int = 0,
