@@ -165,6 +165,12 @@ int s3d_debug_crse_indices_variant(const float *n_coords, const int32_t *table_s
 int s3d_debug_crse_index_values(const float *cq, const float *ck, int64_t n, int L, int last_dim,
                                 int variant, int32_t *idx_out, void *stream);
 
+/* The attention kernels wait for their own copies with a limit.  Should a limit ever run out, the kernel ends
+ * with rows unwritten and notes it on its device.  This call waits for the current device, reads the notes and
+ * clears them: *kernels (host) = 0, or bits 1, 2 = a forward (head_dim 8 or odd head counts, head_dim 16), 4, 8 = the
+ * fp16 backwards of the same, 16 = the fp32 backward.                                                       */
+int s3d_async_error(int *kernels);
+
 /* The three fp32 tables of a layer (n elements each) rounded to fp16 in one launch: dst[t*n + i] =
  * half(src_t[i]), the cast that the fp16 modes make before every call
  * (Swin3D/sparse_dl/attn/attn_coff.py:172-178).  dst: 3 n halves.                                */

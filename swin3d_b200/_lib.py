@@ -42,6 +42,7 @@ SIGNATURES = {
     "s3d_debug_crse_indices_variant": (_i32, [_c_void_p, _c_void_p, _i32, _i32, _i32, _i32, _i32, _i32,
                                               _c_void_p, _c_void_p]),
     "s3d_debug_crse_index_values": (_i32, [_c_void_p, _c_void_p, _i64, _i32, _i32, _i32, _c_void_p, _c_void_p]),
+    "s3d_async_error": (_i32, [_c_void_p]),
     "s3d_cast_tables": (_i32, [_c_void_p] * 3 + [_i64, _c_void_p, _c_void_p]),
     "s3d_gather_rows": (_i32, [_c_void_p, _i32, _c_void_p, _i64, _i64, _c_void_p, _i64, _c_void_p]),
     "s3d_scatter_rows": (_i32, [_c_void_p, _i32, _c_void_p, _i64, _i64, _i64, _i64, _i64, _c_void_p, _c_void_p]),

@@ -1,16 +1,32 @@
-// Asynchronous staging primitives (sm_90+/sm_100a): mbarrier objects in shared memory and the bulk
-// asynchronous copy engine (cp.async.bulk, global -> this block's shared memory, completion counted
-// in bytes on an mbarrier).  Every copy here reads the launching GPU's own global memory and lands in
-// the issuing block's shared memory; none addresses another block or another GPU.
+// Asynchronous staging primitives (sm_80+/sm_90+): mbarrier objects in shared memory and 16-byte asynchronous copies
+// global -> this block's shared memory (cp.async) whose completion arrives on an mbarrier.  Every copy here reads the
+// launching GPU's own global memory and lands in the issuing block's shared memory.
 //
 // Every wait is bounded: mbar_wait gives up after MBAR_WAIT_TRIES polls and returns false, and the
-// kernels then leave their loops through a block-uniform flag and record the event in an error word.
+// kernels then leave their loops through a block-uniform flag and set g_async_error (s3d_async_error()).
 #pragma once
+#include <cuda_runtime.h>
 #include <stdint.h>
 
 namespace s3d {
 
 constexpr int MBAR_WAIT_TRIES = 1 << 22;
+
+// Set when a bounded wait of this file's kernels ran out (it never should); one word per including source file.
+static __device__ int g_async_error;
+
+// Whether it is set on the current device, and clears it.  Waits for the device.
+static inline cudaError_t take_async_error(bool &set)
+{
+    int v = 0;
+    cudaError_t e = cudaMemcpyFromSymbol(&v, g_async_error, sizeof(v));
+    set = e == cudaSuccess && v != 0;
+    if (set) {
+        v = 0;
+        e = cudaMemcpyToSymbol(g_async_error, &v, sizeof(v));
+    }
+    return e;
+}
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p)
 {
@@ -28,20 +44,9 @@ __device__ __forceinline__ void mbar_init_fence()
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
-// Orders this thread's earlier generic-proxy accesses to shared memory before later asynchronous copies.
-__device__ __forceinline__ void async_proxy_fence()
-{
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
 }
 
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, unsigned parity)

@@ -102,9 +102,6 @@ struct Params {
     int H;
 };
 
-// Set when a bounded wait of this kernel ran out (it never should).
-__device__ int g_f32_async_error;
-
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
 {
     uint64_t r;
@@ -357,7 +354,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
             }
             const int s = it % STAGES;
             if (it >= STAGES && !mbar_wait(s_empty + s, ((it / STAGES) - 1) & 1)) {
-                g_f32_async_error = 1;
+                g_async_error = 1;
                 nq = nk = 0;                                  // tell the consumers to stop
             }
             float *rq = s_rows + s * (4 * 32 * RS);
@@ -411,7 +408,7 @@ attn_bwd_f32_kernel(const Params P, const PermMeta pm, const PairConsts pc)
         const int s = it % STAGES;
         if (!mbar_wait(s_full + s, (it / STAGES) & 1)) {
             *s_fail = 1;
-            g_f32_async_error = 2;
+            g_async_error = 2;
         }
         consumer_sync<NT>();          // the previous item's stores are over; the flag is settled
         const int nq = s_n[s * 8], nk = s_n[s * 8 + 1];
@@ -798,5 +795,7 @@ int attn_f32_backward(const AttnArgs &a, cudaStream_t st)
     }
 #undef S3D_F32_BWD
 }
+
+cudaError_t attn_f32_bwd_async_error(bool &set) { return take_async_error(set); }
 
 }  // namespace s3d

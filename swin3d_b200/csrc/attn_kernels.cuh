@@ -61,6 +61,13 @@ int attn_tc_forward_pair16(const AttnArgs &a, cudaStream_t st);
 bool attn_tc_bwd_pair16_supported(const AttnArgs &a);         // attn_tc_bwd_pair16.cu: head_dim 16, even head count
 int attn_tc_backward_pair16(const AttnArgs &a, cudaStream_t st);
 
+// Whether a bounded wait of a file's kernels has run out on the current device since the last call (async_stage.cuh).
+cudaError_t attn_tc_fwd_small_async_error(bool &set);
+cudaError_t attn_tc_fwd_pair16_async_error(bool &set);
+cudaError_t attn_tc_bwd_small_async_error(bool &set);
+cudaError_t attn_tc_bwd_pair16_async_error(bool &set);
+cudaError_t attn_f32_bwd_async_error(bool &set);
+
 // fp32 backward, factorised (attn_f32_bwd.cu): head_dim 8 and 16, tables of at most 63 rows per dimension
 bool attn_f32_bwd_supported(const AttnArgs &a);
 int attn_f32_backward(const AttnArgs &a, cudaStream_t st);

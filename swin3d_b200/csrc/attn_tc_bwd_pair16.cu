@@ -95,9 +95,6 @@ struct P16Params {
     int H;
 };
 
-// Set when a bounded wait of this kernel ran out (it never should).
-__device__ int g_bwd_p16_async_error;
-
 template <int D>
 __global__ void __launch_bounds__((p16_warps(D) + 1) * 32, 1)
 attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc)
@@ -251,7 +248,7 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
             }
             const int s = it % P16_STAGES;
             if (it >= P16_STAGES && !mbar_wait(s_empty + s, ((it / P16_STAGES) - 1) & 1)) {
-                g_bwd_p16_async_error = 1;
+                g_async_error = 1;
                 nq = nk = 0;                              // tell the consumers to stop
             }
             __half *rq = s_rows + s * (4 * ROWS);
@@ -315,7 +312,7 @@ attn_bwd_pair16_kernel(const P16Params P, const PermMeta pm, const PairConsts pc
         const int s = it % P16_STAGES;
         if (!mbar_wait(s_full + s, (it / P16_STAGES) & 1)) {
             *s_fail = 1;
-            g_bwd_p16_async_error = 2;
+            g_async_error = 2;
         }
         consumer_sync<NT>();          // the previous item's stores are over; the flag is settled
         const int nq = s_n[s * 8], nk = s_n[s * 8 + 1];
@@ -621,5 +618,7 @@ int attn_tc_backward_pair16(const AttnArgs &a, cudaStream_t st)
         default: return S3D_ERR_UNSUPPORTED;
     }
 }
+
+cudaError_t attn_tc_bwd_pair16_async_error(bool &set) { return take_async_error(set); }
 
 }  // namespace s3d

@@ -112,9 +112,6 @@ struct BwdMirrors {
     Mirrors dq, dk, dv;
 };
 
-// Set when a bounded wait of a kernel in this file ran out (it never should).
-__device__ int g_bwd_small_async_error;
-
 template <int D, int NPU /*projection + dT units per warp*/, int NHU /*hist.T units per warp*/, bool HD16,
           bool MIRROR /*also store the rows to other GPUs' arrays*/>
 __global__ void __launch_bounds__((bwd_small_warps(D) + 1) * 32, 1)
@@ -260,7 +257,7 @@ attn_bwd_small_kernel(const SmallParams P, const PermMeta pm, const PairConsts p
             }
             const int s = it % BS_STAGES;
             if (it >= BS_STAGES && !mbar_wait(s_empty + s, ((it / BS_STAGES) - 1) & 1)) {
-                g_bwd_small_async_error = 1;
+                g_async_error = 1;
                 nq = nk = 0;                              // tell the consumers to stop
             }
             __half *rq = s_rows + s * 2048;
@@ -354,7 +351,7 @@ attn_bwd_small_kernel(const SmallParams P, const PermMeta pm, const PairConsts p
         const int s = it % BS_STAGES;
         if (!mbar_wait(s_full + s, (it / BS_STAGES) & 1)) {
             *s_fail = 1;
-            g_bwd_small_async_error = 2;
+            g_async_error = 2;
         }
         consumer_sync<NT>();          // the previous window's stores are over; the flag is settled
         S3D_PHASE_MARK(0)
@@ -685,5 +682,7 @@ int attn_tc_backward_small(const AttnArgs &a0, cudaStream_t st)
 #undef S3D_SMALL
 #undef S3D_SMALL_H
 }
+
+cudaError_t attn_tc_bwd_small_async_error(bool &set) { return take_async_error(set); }
 
 }  // namespace s3d

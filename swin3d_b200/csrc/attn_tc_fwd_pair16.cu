@@ -83,8 +83,6 @@ struct F16Params {
     Mirrors m_out;
 };
 
-__device__ int g_fwd_p16_async_error;
-
 template <int D>
 __global__ void __launch_bounds__((f16_warps(D) + 1) * 32, 1)
 attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, const PairConsts pc)
@@ -218,7 +216,7 @@ attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, c
             const int s = it % F16_STAGES;
             bool stop = !have;
             if (it >= F16_STAGES && !mbar_wait(s_empty + s, ((it / F16_STAGES) - 1) & 1)) {
-                g_fwd_p16_async_error = 1;
+                g_async_error = 1;
                 stop = true;                      // tell the consumers to stop
             }
             if (stop) nq = nk = 0;
@@ -264,7 +262,7 @@ attn_fwd_pair16_kernel(const __grid_constant__ F16Params P, const PermMeta pm, c
         const int s = it % F16_STAGES;
         if (!mbar_wait(s_full + s, (it / F16_STAGES) & 1)) {
             *s_fail = 1;
-            g_fwd_p16_async_error = 2;
+            g_async_error = 2;
         }
         consumer_sync<NT>();          // the previous item's merge is over; the flag is settled
         const int nq = s_n[s * 8], nk = s_n[s * 8 + 1];
@@ -514,5 +512,7 @@ int attn_tc_forward_pair16(const AttnArgs &a, cudaStream_t st)
         default: return S3D_ERR_UNSUPPORTED;
     }
 }
+
+cudaError_t attn_tc_fwd_pair16_async_error(bool &set) { return take_async_error(set); }
 
 }  // namespace s3d

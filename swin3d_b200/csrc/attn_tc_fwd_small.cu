@@ -89,10 +89,6 @@ struct FwdSmallParams {
     Mirrors m_out;
 };
 
-// Set when a bounded wait of a kernel in this file ran out (it never should); read and cleared by
-// s3d_debug_async_error().
-__device__ int g_fwd_small_async_error;
-
 // Block = NW consumer warps + one producer warp.  The producer walks the block's tile pairs ahead of the
 // consumers: it reads row numbers and coordinates and copies the 32-byte Q, K, V pieces of the voxels
 // into the next stage of shared memory (cp.async, completion on the stage's "full" mbarrier); the
@@ -202,7 +198,7 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
         for (int it = 0;; ++it) {
             const int s = it % FS_STAGES;
             if (it >= FS_STAGES && !mbar_wait(s_empty + s, ((it / FS_STAGES) - 1) & 1)) {
-                g_fwd_small_async_error = 1;
+                g_async_error = 1;
                 have = false;                             // tell the consumers to stop
             }
             if (!have) nq = nk = 0;
@@ -281,7 +277,7 @@ attn_fwd_small_kernel(const __grid_constant__ FwdSmallParams P, const CrseMeta m
         const int s = it % FS_STAGES;
         if (!mbar_wait(s_full + s, (it / FS_STAGES) & 1)) {
             *s_fail = 1;
-            g_fwd_small_async_error = 2;
+            g_async_error = 2;
         }
         consumer_sync<NT>();          // the previous item's epilogue is over; the flag is settled
         S3D_PHASE_MARK(0)
@@ -573,5 +569,7 @@ int attn_tc_forward_small(const AttnArgs &a0, cudaStream_t st)
 #undef S3D_FS_D
 #undef S3D_FS
 }
+
+cudaError_t attn_tc_fwd_small_async_error(bool &set) { return take_async_error(set); }
 
 }  // namespace s3d

@@ -310,6 +310,25 @@ int s3d_window_build(const int32_t *coords, const float *feats, int64_t N, int F
                                counts_out, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
 }
 
+int s3d_async_error(int *kernels)
+{
+    if (!kernels) return S3D_ERR_BAD_ARG;
+    cudaError_t (*const files[])(bool &) = {attn_tc_fwd_small_async_error, attn_tc_fwd_pair16_async_error, attn_tc_bwd_small_async_error,
+                                            attn_tc_bwd_pair16_async_error, attn_f32_bwd_async_error};
+    *kernels = 0;
+    if (cudaDeviceSynchronize() != cudaSuccess) return S3D_ERR_LAUNCH;
+    for (int i = 0; i < (int)(sizeof(files) / sizeof(files[0])); ++i) {
+        bool set = false;
+        const cudaError_t e = files[i](set);
+        if (e != cudaSuccess) {
+            note_cuda_error(e);
+            return S3D_ERR_LAUNCH;
+        }
+        if (set) *kernels |= 1 << i;
+    }
+    return S3D_OK;
+}
+
 // Set through s3d_debug_knn_path(): 0 = by size, 1 = thread-per-query scan, 2 = warp-per-query scan,
 // 3 = spatial index where it exists (K <= 16).  The tests run every kernel at every size with it.
 static int g_knn_path = 0;

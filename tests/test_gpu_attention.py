@@ -770,3 +770,16 @@ def test_views_that_are_not_16_byte_aligned_are_copied_by_the_wrapper_and_refuse
                                2, 8, _lib.S3D_F16, out1.data_ptr(),
                                lse1.data_ptr(), None)
     assert rc == 1
+
+
+def test_no_bounded_wait_of_the_attention_kernels_has_run_out():
+    """After the calls of this file, whose kernels all wait with a limit; and after one of each here."""
+    import ctypes
+    from swin3d_b200 import _lib
+    from tests.gpu_helpers import cuda_fwd_bwd
+    for dtype, H, hd in (("float16", 2, 8), ("float16", 2, 16), ("float16", 1, 16), ("float32", 1, 8)):
+        p = make_problem(seed=5, n_voxels=300, grid=12, H=H, hd=hd, round_fp16=dtype == "float16")
+        cuda_fwd_bwd(p, getattr(torch, dtype))
+    kernels = ctypes.c_int(-1)
+    assert _lib.lib.s3d_async_error(ctypes.addressof(kernels)) == 0 and kernels.value == 0
+    assert _lib.lib.s3d_async_error(None) == 1
