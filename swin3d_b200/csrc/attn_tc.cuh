@@ -585,17 +585,16 @@ constexpr int WL_NSEG = WL_CHUNK / 32;
 constexpr int WL_BYTES = WL_NSEG * WL_SEG * 2 + 64;
 
 // s_list: uint16 [WL_NSEG][WL_SEG], s_cnt: int [WL_NSEG + 1] (the last entry: overflow flag, cleared by
-// the caller before).  All threads of the block call this between two __syncthreads().  Windows of at
-// most `skip_upto` voxels are left out.
+// the caller before).  All threads of the block call this between two __syncthreads().
 __device__ __forceinline__ void build_work_list(const int32_t *__restrict__ w_sizes, int64_t W, int64_t c0,
-                                                int skip_upto, uint16_t *s_list, int *s_cnt)
+                                                uint16_t *s_list, int *s_cnt)
 {
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     if (tid >= WL_CHUNK) return;
     const int nb = gridDim.x, b = blockIdx.x;
     const int64_t w = c0 + tid;
     const int n = w < W ? __ldg(w_sizes + w) : 0;
-    const int tiles = n > skip_upto ? (n + QT - 1) / QT : 0;
+    const int tiles = n > 0 ? (n + QT - 1) / QT : 0;
     int t = (int)(((int64_t)b - w) % nb);
     if (t < 0) t += nb;
     int pos = 0;
@@ -619,7 +618,7 @@ __device__ __forceinline__ void build_work_list(const int32_t *__restrict__ w_si
 // pos = segment * WL_SEG + index, or, when the list overflowed, the window and tile of a direct walk).
 // -> true and (window, first voxel of the tile), false at the end of the chunk.
 __device__ __forceinline__ bool next_work_item(const uint16_t *list, const int *cnt, const int32_t *__restrict__ w_sizes,
-                                               int64_t W, int64_t c0, int skip_upto, int &pos, int &dw, int &dt,
+                                               int64_t W, int64_t c0, int &pos, int &dw, int &dt,
                                                int64_t &win, int &x0)
 {
     if (cnt[WL_NSEG] == 0) {
@@ -635,7 +634,7 @@ __device__ __forceinline__ bool next_work_item(const uint16_t *list, const int *
     for (;;) {
         if (dw >= 0 && dw < WL_CHUNK && c0 + dw < W && dt >= 0) {
             const int n = __ldg(w_sizes + c0 + dw);
-            const int tiles = n > skip_upto ? (n + QT - 1) / QT : 0;
+            const int tiles = n > 0 ? (n + QT - 1) / QT : 0;
             if (dt < tiles) {
                 win = c0 + dw;
                 x0 = dt * QT;

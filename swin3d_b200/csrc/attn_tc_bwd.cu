@@ -67,7 +67,6 @@ struct BwdParams {
     const float *n_coords;
     int64_t W;
     int H;
-    int skip_upto;   // windows with at most this many voxels are left to the single-sweep kernel
 };
 
 // Projection GEMM  P^T[row][(voxel, slot)] = T . F^T  for 8 n-tiles of 4 voxels, written either in the
@@ -262,12 +261,12 @@ attn_bwd_tc_kernel(const BwdParams P, const CrseMeta meta)
         __syncthreads();            // every warp has left the item loop of the previous chunk
         if (tid == 0) s_wcnt[WL_NSEG] = 0;
         __syncthreads();
-        build_work_list(P.w_sizes, P.W, c0, P.skip_upto, s_wlist, s_wcnt);
+        build_work_list(P.w_sizes, P.W, c0, s_wlist, s_wcnt);
         __syncthreads();
         int it_pos = 0, it_dw = -1, it_dt = -1;
         int64_t w;
         int x0;
-        while (next_work_item(s_wlist, s_wcnt, P.w_sizes, P.W, c0, P.skip_upto, it_pos, it_dw, it_dt, w, x0)) {
+        while (next_work_item(s_wlist, s_wcnt, P.w_sizes, P.W, c0, it_pos, it_dw, it_dt, w, x0)) {
             const int n = __ldg(P.w_sizes + w), base = __ldg(P.w2n + w);
             const int nx = min(QT, n - x0);
             // ---- item set-up: x rows, x coordinates, projections of the x side, empty histograms --------
@@ -677,10 +676,9 @@ static int launch_side(const BwdParams &p, const CrseMeta &meta, cudaStream_t st
 }
 
 template <int D, int MTW, int HDM>
-static int launch_both(const AttnArgs &a, int skip_upto, cudaStream_t st)
+static int launch_both(const AttnArgs &a, cudaStream_t st)
 {
     BwdParams pq{};
-    pq.skip_upto = skip_upto;
     pq.x0 = (const __half *)a.q;   pq.x1 = (const __half *)a.dout;
     pq.y0 = (const __half *)a.k;   pq.y1 = (const __half *)a.v;
     pq.o = (const __half *)a.out;  pq.lse = a.lse;
@@ -703,12 +701,12 @@ static int launch_both(const AttnArgs &a, int skip_upto, cudaStream_t st)
 }
 
 template <int D, int MTW>
-static int launch_mode(const AttnArgs &a, int hdm, int skip_upto, cudaStream_t st)
+static int launch_mode(const AttnArgs &a, int hdm, cudaStream_t st)
 {
     switch (hdm) {
-        case HDM_PAIR8: return launch_both<D, MTW, HDM_PAIR8>(a, skip_upto, st);
-        case HDM_SINGLE16: return launch_both<D, MTW, HDM_SINGLE16>(a, skip_upto, st);
-        default: return launch_both<D, MTW, HDM_PAIR16>(a, skip_upto, st);
+        case HDM_PAIR8: return launch_both<D, MTW, HDM_PAIR8>(a, st);
+        case HDM_SINGLE16: return launch_both<D, MTW, HDM_SINGLE16>(a, st);
+        default: return launch_both<D, MTW, HDM_PAIR16>(a, st);
     }
 }
 
@@ -735,18 +733,17 @@ int attn_tc_backward(const AttnArgs &a0, cudaStream_t st)
     AttnArgs a = a0;
     a.meta = tc::internal_meta(a0.meta);   // kernels work in the internal row numbering
     const int hdm = attn_tc_head_mode(a0);
-    int skip_upto = 0;
-    // the single-sweep kernel serves head pairs of 8 channels and single heads of 16, windows of any size
-    if (hdm != tc::HDM_PAIR16 && attn_tc_bwd_small_supported(a0))
-        return attn_tc_backward_small(a0, st);      // tile pairs: windows of any size
+    // the single-sweep kernels serve what fits their shared memory; the two-sweep ones larger tables: head pairs of 16
+    // channels with six signal dimensions and 337 to 368 rows, the others from about 300 rows on
+    if (hdm != tc::HDM_PAIR16 && attn_tc_bwd_small_supported(a0)) return attn_tc_backward_small(a0, st);
     if (hdm == tc::HDM_PAIR16 && attn_tc_bwd_pair16_supported(a0)) return attn_tc_backward_pair16(a0, st);
     if (a0.m_dq.n) return S3D_ERR_UNSUPPORTED;      // the two-sweep kernels have no mirrored stores
     const int n_mt = (a.meta.R + 15) / 16;
     const int mtw = (n_mt + tc::BW_NWARP - 1) / tc::BW_NWARP;
 #define S3D_TC_BWD(DD)                                            \
     switch (mtw) {                                                \
-        case 1: return tc::launch_mode<DD, 1>(a, hdm, skip_upto, st); \
-        case 2: return tc::launch_mode<DD, 2>(a, hdm, skip_upto, st); \
+        case 1: return tc::launch_mode<DD, 1>(a, hdm, st);           \
+        case 2: return tc::launch_mode<DD, 2>(a, hdm, st);           \
         default: return S3D_ERR_UNSUPPORTED;                      \
     }
     switch (a.meta.D) {

@@ -778,8 +778,21 @@ def test_no_bounded_wait_of_the_attention_kernels_has_run_out():
     from swin3d_b200 import _lib
     from tests.gpu_helpers import cuda_fwd_bwd
     for dtype, H, hd in (("float16", 2, 8), ("float16", 2, 16), ("float16", 1, 16), ("float32", 1, 8)):
-        p = make_problem(seed=5, n_voxels=300, grid=12, H=H, hd=hd, round_fp16=dtype == "float16")
+        p = make_problem(seed=5, n_voxels=300, H=H, hd=hd, round_fp16=dtype == "float16")
         cuda_fwd_bwd(p, getattr(torch, dtype))
     kernels = ctypes.c_int(-1)
     assert _lib.lib.s3d_async_error(ctypes.addressof(kernels)) == 0 and kernels.value == 0
     assert _lib.lib.s3d_async_error(None) == 1
+
+
+def test_fp16_backward_of_the_largest_tables_by_two_sweeps():
+    """Six signal dimensions of 60 rows, two heads of 16 channels: 365 rows, more than the single-sweep backward has
+    warps for.  Against the oracle."""
+    from tests.gpu_helpers import cuda_fwd_bwd
+    p = make_problem(seed=33, ws=5, H=2, hd=16, crse="XYZ_RGB", scene=_scene_of_window_sizes(5, [1, 20, 33, 70, 125]), round_fp16=True)
+    p.sizes = [60 * 32] * 6
+    p.tq, p.tk, p.tv = (t.astype(np.float16).astype(np.float32) for t in S.make_tables(34, p.sizes))
+    o_ref, _, g_ref = oracle_fwd_bwd(p, np.float64)
+    out, _, grads = cuda_fwd_bwd(p, torch.float16)
+    for name, a, b in zip("out dq dk dv dtq dtk dtv".split(), (out,) + grads, (o_ref,) + g_ref):
+        assert rel_err(a, b) < FP16_TOL, name
