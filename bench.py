@@ -494,7 +494,7 @@ def run_attention(args):
             finally:
                 C.HALF_FORWARD_FAST_BACKWARD = saved
         half_forward["note"] = ("through SelfAttnAIOFunction under autocast with fp32 arrays (casts included), one window set; default: "
-                                "fp32 backward on the generic kernels as in the reference; switch "
+                                "fp32 backward as in the reference; switch "
                                 "attn_coff.HALF_FORWARD_FAST_BACKWARD: fp16 tensor-core backward")
         del x32, g32
 

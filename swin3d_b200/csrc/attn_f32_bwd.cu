@@ -24,9 +24,10 @@
 // All products are fp32 FMAs, two per instruction (fma.f32x2): no operand is rounded to fewer bits.
 // Row numbering and tile skipping as in PermMeta (attn_tc.cuh).
 //
-// Bound: instruction issue (about half the slots used with 16 warps per SM; shared memory of 160 to
-// 220 KB allows one block).  The generic kernel this replaces recomputes every pair's table products
-// channel by channel, twice, and adds a histogram row by row for every (voxel, head).
+// Bound: instruction issue (51 % of the slots with 16 warps per SM; shared memory of 160 to 220 KB allows one
+// block) and shared-memory wavefronts (64 % of the pipe).  The generic kernel this replaces recomputes every pair's
+// table products channel by channel, twice, and adds a histogram row by row for every (voxel, head): 117 k voxels, 6
+// heads of 8 channels, mixed precision 8.40 -> 3.58 ms a training pass.
 #include "attn_kernels.cuh"
 #include "attn_tc.cuh"
 #include "async_stage.cuh"

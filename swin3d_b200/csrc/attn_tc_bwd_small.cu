@@ -10,10 +10,10 @@
 // Windows of at most 32 voxels -- most of them -- are a single item.
 //
 // Block = 15 / 11 / 7 consumer warps (9 / 6 / 3 signal dimensions) + one producer warp, one block per SM, serving one head pair
-// (head_dim 8) or one head (head_dim 16) for the windows x, x + gridDim.x, ...  The producer walks
+// (head_dim 8) or one head (head_dim 16) for a contiguous range of windows of equal cost.  The producer walks
 // the block's items ahead of the consumers: row numbers, coordinates, lse and delta = dO.O by plain
-// loads, the 32-byte Q, dO pieces of the query tile and K, V pieces of the key tile by the copy
-// engine (cp.async.bulk) into the next stage of shared memory; stages are handed over through
+// loads, the 32-byte Q, dO pieces of the query tile and K, V pieces of the key tile by 16-byte
+// cp.async into the next stage of shared memory; stages are handed over through
 // "full" / "empty" mbarriers.
 // Per window (consumers, phases separated by a barrier among the consumer warps):
 //   GEMM    P_q = Tq.Q^T, dB = Tv.dO^T (lane-major), P_k = Tk.K^T (key-major); a warp owns consecutive

@@ -24,7 +24,8 @@
 // The blocks take contiguous ranges of (window, query tile) units of equal cost (tile pairs).
 // grid = (x, H/2) (head_dim 8) or (x, H) (head_dim 16).
 //
-// Bound: shared-memory wavefronts (65 % of the pipe's peak) and instruction issue (58 %), see profiles/.
+// Bound: shared-memory wavefronts (66 % of the pipe's peak), instruction issue (55 %), barriers and staged rows (1.8 and 1.6
+// stall cycles per instruction); 241 k voxels, 10 heads.
 // Measured against the version for windows of at most 32 voxels (blocks took every gridDim.x-th window) plus a kernel of
 // one block per SM with an online softmax for the larger ones: 964 k voxels, 10 heads 8.38 -> 7.69 ms; 115 k
 // voxels, 6 heads 680 -> 559 us.

@@ -69,11 +69,11 @@ def _as_int32(t: Tensor) -> Tensor:
 CACHE_TABLE_OFFSETS = True
 
 # PrecisionMode.HALF_FORWARD (fp16_mode=1): the reference runs the backward on fp32 casts of q, k, v,
-# the tables and the gradient (attn_coff.py:207-217).  That is the default here too (generic fp32
-# kernels, 1e-4 agreement with the reference's fp32 backward).  With this switch on, the backward of
+# the tables and the gradient (attn_coff.py:207-217).  That is the default here too (fp32 kernels,
+# 1e-4 agreement with the reference's fp32 backward).  With this switch on, the backward of
 # that mode instead runs the tensor-core kernels on the fp16 values the forward used (fp16 storage,
-# fp32 accumulation, the 2e-2 tolerance of the fp16 modes) and returns fp32 gradients: about four
-# times faster, for callers who accept fp16-mode accuracy in the backward of fp16_mode=1.
+# fp32 accumulation, the 2e-2 tolerance of the fp16 modes) and returns fp32 gradients: about
+# twice as fast, for callers who accept fp16-mode accuracy in the backward of fp16_mode=1.
 HALF_FORWARD_FAST_BACKWARD = False
 _table_sizes_cache = {}
 

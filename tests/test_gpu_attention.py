@@ -691,7 +691,9 @@ def test_c_abi_calls_can_be_captured_in_a_cuda_graph():
 def test_tiled_kernels_work_list_overflow_falls_back_to_a_direct_walk():
     """150 heads leave one block per head pair, which then owns every tile of every window; nine
     dense 343-voxel windows give its first warp 99 work items, more than a list segment holds, so the
-    kernels walk the chunk's windows directly.  Checked against the generic kernels of the library."""
+    kernels walk the chunk's windows directly.  Checked against the generic kernels of the library.
+    (At these tables the tile-pair kernels answer, whose block takes all tile pairs of the nine windows; the
+    two-sweep backward, which has the list, is the next test's.)"""
     import os
     from tests.gpu_helpers import cuda_fwd_bwd
     g = np.stack(np.meshgrid(np.arange(21), np.arange(21), np.arange(7), indexing="ij"), -1).reshape(-1, 3)
@@ -708,6 +710,25 @@ def test_tiled_kernels_work_list_overflow_falls_back_to_a_direct_walk():
         slow = cuda_fwd_bwd(p, torch.float16)
     finally:
         __import__("swin3d_b200._lib", fromlist=["lib"]).lib.s3d_debug_force_generic(0)
+    assert rel_err(fast[0], slow[0]) < 5e-3
+    for a, b in zip(fast[2], slow[2]):
+        assert rel_err(a, b) < 1.5e-2
+
+
+def test_work_list_overflow_of_the_two_sweep_backward():
+    """150 pairs of 16-channel heads, tables of 365 rows, nine windows of 11 tiles: one block per pair, 99 work items for
+    a list segment of 64.  Against the generic kernels."""
+    from swin3d_b200 import _lib
+    from tests.gpu_helpers import cuda_fwd_bwd
+    p = make_problem(seed=35, ws=7, H=300, hd=16, crse="XYZ_RGB", scene=_scene_of_window_sizes(7, [343] * 9), round_fp16=True)
+    p.sizes = [60 * 300 * 16] * 6
+    p.tq, p.tk, p.tv = (t.astype(np.float16).astype(np.float32) for t in S.make_tables(36, p.sizes))
+    fast = cuda_fwd_bwd(p, torch.float16)
+    _lib.lib.s3d_debug_force_generic(1)
+    try:
+        slow = cuda_fwd_bwd(p, torch.float16)
+    finally:
+        _lib.lib.s3d_debug_force_generic(0)
     assert rel_err(fast[0], slow[0]) < 5e-3
     for a, b in zip(fast[2], slow[2]):
         assert rel_err(a, b) < 1.5e-2
