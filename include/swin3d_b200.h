@@ -314,8 +314,8 @@ int s3d_knn_maxpool_bwd(const int32_t *arg, const void *dout, float *dg,
  *  s3d_knn_maxpool_slots_fwd keeps slot uint8[Nq,C], the position (0..K-1) of the maximum in the query's
  *  list, instead of the source row.  The two _bwd calls turn idx around in `workspace`
  *  (s3d_knn_gather_workspace_bytes, 16-byte aligned device memory; 0: too large for this form) and
- *  write dsrc / dg [Ns,C] in `dtype`, every row once, summed in fp32.  The sum runs over the queries that
- *  refer to a row one after the other, so lists of many thousands are better scattered.
+ *  write dsrc / dg [Ns,C] in `dtype`, every row once, summed in fp32 (rows with more than 64 entries by blocks
+ *  that share their entries).
  */
 int64_t s3d_knn_gather_workspace_bytes(int64_t Ns, int64_t Nq, int K);
 int s3d_knn_interpolate_gather_bwd(const int32_t *idx, const float *dist, const void *dout, void *dsrc,

@@ -37,8 +37,8 @@ def get_offset(batch: torch.Tensor) -> torch.Tensor:
     return torch.cumsum(torch.bincount(batch.long()), 0).to(torch.int32)
 
 
-# The gather form of the backwards walks the queries of a source row one after the other: with more than
-# this many on average (few sources, many queries) the scatter form keeps more of the GPU busy.
+# With more entries per source row than this on average (few sources, many queries) the scatter form of the backwards
+# is taken: every row would be a long one of the gather form.
 GATHER_MOST_PER_SOURCE = 256
 
 

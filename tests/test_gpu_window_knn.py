@@ -232,7 +232,7 @@ def test_knn_kernels_agree_with_the_heap_at_every_size(path, case):
 
 
 def test_knn_index_hands_many_ties_to_the_scan():
-    """More tied queries than the block-per-query pass takes (2048): a lattice, where every query ties."""
+    """More tied queries than the block-per-query pass takes (10,000): a lattice, where each of the 27,000 ties."""
     from swin3d_b200 import _lib
     g = np.stack(np.meshgrid(*[np.arange(30)] * 3, indexing="ij"), -1).reshape(-1, 3).astype(np.float32)
     src, qry = g[::13], g + np.float32(0.5)
