@@ -450,7 +450,7 @@ void launch_gather_as(const uint8_t *slot, const void *dout, void *dsrc, int64_t
     inverse_gather_kernel<T, SLOT><<<blocks_of(Ns * (C / Vec<T>::N), KC_THREADS), KC_THREADS, 0, st>>>((const T *)dout, slot, (T *)dsrc, Ns, C, v);
     if (n > LONG_ROW) {
         const int64_t most = n / LONG_ROW + 1;
-        inverse_long_rows_kernel<T, SLOT><<<(unsigned)(most < 148 * 8 ? most : 148 * 8), KC_THREADS, 0, st>>>((const T *)dout, slot, (T *)dsrc, C, v);
+        inverse_long_rows_kernel<T, SLOT><<<(unsigned)(most < 148 * 4 ? most : 148 * 4), KC_THREADS, 0, st>>>((const T *)dout, slot, (T *)dsrc, C, v);
     }
 }
 

@@ -210,3 +210,25 @@ def test_gather_backwards_of_long_rows(dtype, K, C, n_src, Nq, counts):
     arg = torch.gather(idx.long()[:, :, None].expand(-1, -1, C), 1, feat.detach()[idx.long()].argmax(1, keepdim=True))[:, 0]
     ref, size = (torch.zeros((n_src, C), dtype=torch.float64, device="cuda").scatter_add_(0, arg, d) for d in (dout.double(), dout.double().abs()))
     assert ((pooled.double() - ref).abs() <= size * n_max * 2.0 ** -24 + ref.abs() * eps + 2.0 ** -24).all()
+
+
+@pytest.mark.parametrize("dtype,per_source,gathered", [(torch.float16, 190, True), (torch.float16, 200, False), (torch.float32, 22, True),
+                                                       (torch.float32, 26, False)])
+def test_pooling_either_side_of_the_gather(dtype, per_source, gathered):
+    """knn_max_pool takes the gathered backward up to its limit of entries per source, and both give the same gradient."""
+    from swin3d_b200.sparse_dl.knn import KNN, KNNMaxPool, knn_max_pool
+    K, n_src = 16, 800
+    rng = np.random.default_rng(per_source)
+    src, qry = (rng.random((n, 3), dtype=np.float32) for n in (n_src, per_source * n_src // K))
+    a = [_dev(src), _dev(qry)]
+    so, qo = _dev(np.array([len(src)], np.int32)), _dev(np.array([len(qry)], np.int32))
+    g = torch.randn((n_src, 16), device="cuda").to(dtype).requires_grad_()
+    dout = torch.randn((len(qry), 16), device="cuda").to(dtype)
+    out = knn_max_pool(K, *a, g, so, qo)
+    assert type(out.grad_fn).__name__ == ("_KNNMaxPoolSlotsBackward" if gathered else "KNNMaxPoolBackward")
+    ref = KNNMaxPool.apply(g, KNN.apply(K, *a, so, qo)[0])[0]
+    assert torch.equal(out, ref)
+    (x,), (y,) = torch.autograd.grad(out, [g], dout), torch.autograd.grad(ref, [g], dout)
+    # both sum in fp32, in another order, and round once
+    eps = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -16
+    assert ((x.double() - y.double()).abs() <= 2 * eps * y.double().abs() + 2.0 ** -14).all()
