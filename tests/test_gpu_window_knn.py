@@ -379,3 +379,28 @@ def test_get_index01_drop_in_returns_the_tuple_window_attention_unpacks(shift):
     assert rel_err(out.detach().cpu().numpy(), o_ref) < 1e-4
     for t, b in zip((q, k, v, tq, tk, tv), g_ref):
         assert rel_err(t.grad.cpu().numpy(), b) < 1e-4
+
+
+@pytest.mark.parametrize("signals", [0, 3, 6])
+@pytest.mark.parametrize("kind", ["repeated", "scattered", "one voxel twice"])
+def test_grouping_that_needs_the_sort_takes_its_signals_from_two_arrays(kind, signals):
+    """get_index01 on voxels that the dense grid cannot place: positions and other signals in arrays (and views) of their
+    own, no others at all, window offsets made on demand."""
+    from types import SimpleNamespace
+    from swin3d_b200.window import get_index01
+    rng = np.random.default_rng(signals)
+    n = 3_000
+    c = np.zeros((n, 4), np.int32)
+    c[:, 0] = np.sort(rng.integers(0, 3, n))
+    c[:, 1:] = rng.integers(0, 9, (n, 3)) if kind == "repeated" else rng.integers(-40_000, 40_000, (n, 3))
+    if kind == "one voxel twice":
+        c[:, 1:] = np.stack(np.meshgrid(*[np.arange(15)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+        c[:, 0] = 0
+        c[-1] = c[17]
+    feats = rng.random((n, 3 + signals), dtype=np.float32)
+    wide = _dev(np.concatenate([feats, feats], 1))                # rows wider than what is taken of them
+    got = get_index01(SimpleNamespace(C=_dev(c), tensor_stride=1), wide[:, :3], wide[:, 3:3 + signals], 5, 2)
+    n2n, n_coords, w_sizes, w2n = O.window_grouping(c, feats, 5, 2)
+    w2 = w_sizes.astype(np.int64) ** 2
+    for x, want in zip(got[3:], (w_sizes, w2n, n2n, np.cumsum(w2) - w2, n_coords)):
+        assert np.array_equal(x.cpu().numpy(), want)
